@@ -44,10 +44,16 @@ struct RuleBufs {
   DBuf<uint32_t> key_l, key_r, off_l, off_r, sorted_l, sorted_r;
   DBuf<dev::StrMeta> sorted_meta_r;
   DBuf<unsigned long long> item_off;
-  DBuf<uint32_t> part_u32;
-  DBuf<unsigned long long> part_u64;
-  uint32_t nb = 0;    // scan CTAs over the join key domain
-  uint32_t nb_l = 0;  // scan CTAs over the left key domain (word classes x keys)
+};
+
+// The tasks of a rule array's join kernels (kernels.cuh), and the histogram
+// words that they use, all at the front of hbx_session::counts.
+struct JoinLists {
+  std::vector<uint32_t> count, scatter, block_task;
+  std::vector<dev::ScanTask> scan;
+  DBuf<uint32_t> d_count, d_scatter, d_block_task;
+  DBuf<dev::ScanTask> d_scan;
+  uint64_t n_counts = 0;
 };
 
 template <class T>
@@ -76,8 +82,8 @@ struct hbx_session {
   hbx::DBuf<unsigned long long> seen;  // reported-pair set (plans with several rules)
   // key histograms and scatter cursors of every rule, one block: one memset
   hbx::DBuf<uint32_t> counts;
-  hbx::DBuf<unsigned long long> scan_sync;  // fused join: chunk totals and tickets (k_join_scan)
-  bool fused_join = false;  // every key domain small: join kernels covering all rules
+  hbx::DBuf<unsigned long long> scan_sync;  // chunk totals and tickets (k_join_scan)
+  hbx::JoinLists join_rules, join_groups;   // the joins of h_rules and of h_groups
   hbx::DBuf<uint32_t> bound_idx;              // per rule, n_partitions + 1 key indices
   hbx::DBuf<unsigned long long> bound_val;    // item_off at those keys
   hbx::dev::Side side_l{}, side_r{};
@@ -234,12 +240,35 @@ void launch_dependent(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, c
   HBX_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...));
 }
 
-// Chunks of kScanChunk keys in the largest left key domain of the session's
-// rules (the fused join's scan grid).
-uint32_t fused_chunks(const hbx_session* S) {
-  uint32_t max_d = 1;
-  for (const dev::Rule& d : S->h_rules) max_d = std::max(max_d, d.domain_l);
-  return (max_d + dev::kScanChunk - 1) / dev::kScanChunk;
+// The join tasks of a rule array, uploaded on st.
+void list_join(const std::vector<dev::Rule>& rules, JoinLists* J, cudaStream_t st) {
+  for (uint32_t r = 0; r < (uint32_t)rules.size(); r++) {
+    const dev::Rule& d = rules[r];
+    if (!d.n_members) {
+      if (!d.cmp_weight) continue;  // another rule's join counts its comparisons
+      J->count.push_back(dev::join_task(r, 1));
+      J->scatter.push_back(dev::join_task(r, 0));
+      continue;
+    }
+    for (int side : {0, 1}) {
+      J->count.push_back(dev::join_task(r, side));
+      J->scatter.push_back(dev::join_task(r, side));
+    }
+    for (uint32_t what = 0; what < 3; what++) {
+      const uint32_t D = what == 1 ? d.domain : d.domain_l;
+      dev::ScanTask t;
+      t.rule = r;
+      t.what = what;
+      t.first_block = (uint32_t)J->block_task.size();
+      t.n_chunks = (D + dev::kScanChunk - 1) / dev::kScanChunk;
+      J->block_task.insert(J->block_task.end(), t.n_chunks, (uint32_t)J->scan.size());
+      J->scan.push_back(t);
+    }
+  }
+  J->d_count.upload(J->count, st);
+  J->d_scatter.upload(J->scatter, st);
+  J->d_block_task.upload(J->block_task, st);
+  J->d_scan.upload(J->scan, st);
 }
 
 // Device state of a session whose side buffers hold the encoded tables.
@@ -280,13 +309,10 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
       d.thr[s] = re.thr[s];
     }
     d.domain = (uint32_t)re.domain;
-    // group left rows by the word class of the first similarity predicate's
-    // string, unless that would make the left key domain too large
-    const bool split = !re.sim_slot_l.empty() &&
-                       re.domain * dev::kWordClasses <= (uint64_t)kMaxKeyDomain * 4;
-    d.n_wclass = split ? dev::kWordClasses : 1u;
-    d.wclass_slot = split ? (uint32_t)re.sim_slot_l[0] : 0u;
-    d.domain_l = d.n_wclass * d.domain;
+    // one kernel per mask width runs every left string: no word classes
+    d.n_wclass = 1u;
+    d.wclass_slot = 0u;
+    d.domain_l = d.domain;
     dev::make_singleton(&d);
     RuleBufs& b = S->rb[r];
     b.key_l.alloc(nL);
@@ -297,10 +323,6 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
     b.sorted_r.alloc((size_t)nR + 4);
     if (d.n_sim) b.sorted_meta_r.alloc(nR);
     b.item_off.alloc((size_t)d.domain_l + 1);
-    b.nb = (uint32_t)((re.domain + dev::kScanChunk - 1) / dev::kScanChunk);
-    b.nb_l = (uint32_t)((d.domain_l + dev::kScanChunk - 1) / dev::kScanChunk);
-    b.part_u32.alloc(std::max(b.nb, b.nb_l));
-    b.part_u64.alloc(b.nb_l);
     d.key_l = b.key_l.p;
     d.key_r = b.key_r.p;
     d.off_l = b.off_l.p;
@@ -310,27 +332,51 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
     d.sorted_r = b.sorted_r.p;
     d.sorted_meta_r = d.n_sim ? b.sorted_meta_r.p : nullptr;
   }
-  // histograms and cursors: [cnt_l | cur_l | cnt_r | cur_r] per rule
-  {
-    size_t total = 0;
-    for (const dev::Rule& d : S->h_rules) total += 2ull * d.domain_l + 2ull * d.domain;
-    S->counts.alloc(std::max<size_t>(total, 1));
-    size_t pos = 0;
-    S->fused_join = true;
-    for (dev::Rule& d : S->h_rules) {
-      d.cnt_l = S->counts.p + pos;
-      d.cur_l = d.cnt_l + d.domain_l;
-      d.cnt_r = d.cur_l + d.domain_l;
-      d.cur_r = d.cnt_r + d.domain;
-      pos += 2ull * d.domain_l + 2ull * d.domain;
-      if (d.domain_l > dev::kFusedJoinMaxDomain) S->fused_join = false;
-    }
-    if (S->fused_join) S->scan_sync.alloc(E.rules.size() * 3 * (fused_chunks(S) + 1));
-  }
   S->h_groups = group_rules(S->h_rules);
   S->groups = false;
   for (const dev::Rule& g : S->h_groups)
     if (g.n_members > 1) S->groups = true;
+  // histograms and cursors of every rule, one block: first what the groups'
+  // join uses (a member that counts its comparisons: cnt_r), then the rest
+  {
+    size_t total = 0;
+    for (const dev::Rule& d : S->h_rules) total += 2ull * d.domain_l + 2ull * d.domain;
+    S->counts.alloc(std::max<size_t>(total, 1));
+    uint32_t* next = S->counts.p;
+    auto take = [&](size_t words) {
+      uint32_t* p = next;
+      next += words;
+      return p;
+    };
+    for (size_t r = 0; r < S->h_rules.size(); r++) {
+      dev::Rule& d = S->h_rules[r];
+      const dev::Rule& g = S->h_groups[r];
+      if (g.n_members || g.cmp_weight) d.cnt_r = take(d.domain);
+      if (!g.n_members) continue;
+      d.cnt_l = take(d.domain_l);
+      d.cur_l = take(d.domain_l);
+      d.cur_r = take(d.domain);
+    }
+    S->join_groups.n_counts = (uint64_t)(next - S->counts.p);
+    for (dev::Rule& d : S->h_rules) {
+      if (!d.cnt_r) d.cnt_r = take(d.domain);
+      if (!d.cnt_l) d.cnt_l = take(d.domain_l);
+      if (!d.cur_l) d.cur_l = take(d.domain_l);
+      if (!d.cur_r) d.cur_r = take(d.domain);
+    }
+    S->join_rules.n_counts = (uint64_t)(next - S->counts.p);
+    for (size_t r = 0; r < S->h_rules.size(); r++) {
+      const dev::Rule& d = S->h_rules[r];
+      dev::Rule& g = S->h_groups[r];
+      g.cnt_l = d.cnt_l;
+      g.cnt_r = d.cnt_r;
+      g.cur_l = d.cur_l;
+      g.cur_r = d.cur_r;
+    }
+  }
+  list_join(S->h_rules, &S->join_rules, st);
+  list_join(S->h_groups, &S->join_groups, st);
+  S->scan_sync.alloc(S->join_rules.block_task.size() + S->join_rules.scan.size());
   S->d_rules.alloc(E.rules.size());
   S->d_groups.alloc(E.rules.size());
   S->d_rule_base.alloc(E.rules.size() + 1);
@@ -516,6 +562,25 @@ std::vector<dev::Rule> group_rules(const std::vector<dev::Rule>& singles) {
   }
   for (dev::Rule& G : g)
     if (G.n_members) dev::fill_extras_table(&G);
+  // rules with the same equalities have the same pair-comparisons: one of
+  // them counts for all, a rule with work items where there is one
+  for (size_t r = 0; r < n; r++) {
+    if (!g[r].cmp_weight) continue;
+    size_t keep = r;
+    std::vector<size_t> same;
+    for (size_t q = r; q < n; q++)
+      if (g[q].cmp_weight && eqset(q) == eqset(r)) {
+        same.push_back(q);
+        if (g[q].n_members && !g[keep].n_members) keep = q;
+      }
+    uint32_t rest = 0;
+    for (size_t q : same)
+      if (q != keep && !g[q].n_members) {
+        rest++;
+        g[q].cmp_weight = 0;
+      }
+    g[keep].cmp_weight = 1 + rest;
+  }
   return g;
 }
 
@@ -526,65 +591,34 @@ __global__ void k_gather_bounds(const dev::Rule* rules, uint32_t n_rules, uint32
   out[i] = rules[i / per_rule].item_off[idx[i]];
 }
 
-// Enqueues counter reset + the joins of every rule, with the rule array
-// `rules` (d_rules or d_groups: the same join state; in d_groups a group's
-// first column may lead another predicate, and members have no items).
-// Returns launches.
-uint32_t enqueue_join(hbx_session* S, cudaStream_t st, const dev::Rule* rules) {
-  uint32_t launches = 1;  // k_reset
-  const uint64_t n_sync = S->fused_join ? S->scan_sync.n : 0;
+// Enqueues counter reset + the joins of a rule array: h_rules (groups =
+// false) or h_groups (the same join state; there a group's first column may
+// lead another predicate, and members have no items).  Returns launches.
+uint32_t enqueue_join(hbx_session* S, cudaStream_t st, bool groups) {
+  const JoinLists& J = groups ? S->join_groups : S->join_rules;
+  const dev::Rule* rules = groups ? S->d_groups.p : S->d_rules.p;
+  const uint32_t n_blocks = (uint32_t)J.block_task.size();
   {  // counters, histograms, the duplicate set and the join scan's tickets, one launch
     const uint64_t n_seen = S->seen.p ? S->seen.n : 0;
-    const uint64_t n = std::max<uint64_t>(std::max<uint64_t>(S->counts.n, n_seen), std::max<uint64_t>(n_sync, 32));
-    dev::k_reset<<<row_grid(n, S->ctx->n_sm), 256, 0, st>>>(S->d_ctr.p, S->counts.p, S->counts.n,
+    const uint64_t n_sync = n_blocks + J.scan.size();
+    const uint64_t n = std::max<uint64_t>(std::max<uint64_t>(J.n_counts, n_seen), std::max<uint64_t>(n_sync, 32));
+    dev::k_reset<<<row_grid(n, S->ctx->n_sm), 256, 0, st>>>(S->d_ctr.p, S->counts.p, J.n_counts,
                                                             S->seen.p, n_seen, S->scan_sync.p,
                                                             n_sync);
   }
-  const uint32_t nL = S->side_l.n_rows, nR = S->side_r.n_rows;
-  const int n_sm = S->ctx->n_sm;
-  const uint32_t n_rules = (uint32_t)S->rb.size();
-  if (S->fused_join) {
-    uint32_t max_d = 1;
-    for (const dev::Rule& d : S->h_rules) max_d = std::max(max_d, d.domain_l);
-    const size_t smem = std::min<uint32_t>(max_d, dev::kSharedHistKeys) * sizeof(uint32_t);
-    // rows per block row: each (rule, table) pair gets its own blocks
-    const dim3 grid(row_grid(std::max(nL, nR), n_sm), n_rules, 2);
-    const uint32_t nb = fused_chunks(S);
-    unsigned long long* comparisons = &S->d_ctr.p->comparisons;
-    launch_dependent(dev::k_join_count, grid, dim3(256), smem, st, S->side_l, S->side_r, rules);
-    launch_dependent(dev::k_join_scan, dim3(nb, 3, n_rules), dim3(1024), 0, st, rules,
-                     S->tile_right, nb, S->scan_sync.p, comparisons, S->d_ctr.p);
-    launch_dependent(dev::k_join_scatter, grid, dim3(256), 0, st, S->side_l, S->side_r, rules,
-                     n_rules, S->d_rule_base.p, &S->d_ctr.p->items_total);
-    launch_check("join kernels");
-    return launches + 3;
-  }
-  for (size_t r = 0; r < S->rb.size(); r++) {
-    RuleBufs& b = S->rb[r];
-    const uint32_t D = S->h_rules[r].domain;
-    const uint32_t DL = S->h_rules[r].domain_l;
-    if (nL) dev::k_keys_hist<<<row_grid(nL, n_sm), 256, 0, st>>>(S->side_l, rules, (uint32_t)r, 0);
-    if (nR) dev::k_keys_hist<<<row_grid(nR, n_sm), 256, 0, st>>>(S->side_r, rules, (uint32_t)r, 1);
-    dev::k_scan_partial_u32<<<b.nb_l, 1024, 0, st>>>(S->h_rules[r].cnt_l, DL, b.part_u32.p);
-    dev::k_scan_top_u32<<<1, 1024, 0, st>>>(b.part_u32.p, b.nb_l);
-    dev::k_scan_final_u32<<<b.nb_l, 1024, 0, st>>>(S->h_rules[r].cnt_l, DL, b.part_u32.p, b.off_l.p);
-    dev::k_scan_partial_u32<<<b.nb, 1024, 0, st>>>(S->h_rules[r].cnt_r, D, b.part_u32.p);
-    dev::k_scan_top_u32<<<1, 1024, 0, st>>>(b.part_u32.p, b.nb);
-    dev::k_scan_final_u32<<<b.nb, 1024, 0, st>>>(S->h_rules[r].cnt_r, D, b.part_u32.p, b.off_r.p);
-    dev::k_items_partial<<<b.nb_l, 1024, 0, st>>>(rules, (uint32_t)r, S->tile_right,
-                                                  b.part_u64.p, &S->d_ctr.p->comparisons);
-    dev::k_scan_top_u64<<<1, 1024, 0, st>>>(b.part_u64.p, b.nb_l);
-    dev::k_items_final<<<b.nb_l, 1024, 0, st>>>(rules, (uint32_t)r, S->tile_right,
-                                                b.part_u64.p);
-    if (nL) dev::k_scatter<<<row_grid(nL, n_sm), 256, 0, st>>>(S->side_l, rules, (uint32_t)r, 0);
-    if (nR) dev::k_scatter<<<row_grid(nR, n_sm), 256, 0, st>>>(S->side_r, rules, (uint32_t)r, 1);
-    launches += 9 + (nL ? 2 : 0) + (nR ? 2 : 0);
-  }
-  dev::k_rule_base<<<1, 32, 0, st>>>(rules, n_rules, S->d_rule_base.p,
-                                     &S->d_ctr.p->items_total);
-  launches++;
+  uint32_t max_d = 1;
+  for (const dev::Rule& d : S->h_rules) max_d = std::max(max_d, d.domain_l);
+  const size_t smem = std::min<uint32_t>(max_d, dev::kSharedHistKeys) * sizeof(uint32_t);
+  const int row_blocks = row_grid(std::max(S->side_l.n_rows, S->side_r.n_rows), S->ctx->n_sm);
+  launch_dependent(dev::k_join_count, dim3(row_blocks, (uint32_t)J.count.size()), dim3(256), smem,
+                   st, S->side_l, S->side_r, rules, J.d_count.p);
+  launch_dependent(dev::k_join_scan, dim3(n_blocks), dim3(1024), 0, st, rules, S->tile_right,
+                   J.d_scan.p, J.d_block_task.p, S->scan_sync.p, S->d_ctr.p);
+  launch_dependent(dev::k_join_scatter, dim3(row_blocks, (uint32_t)J.scatter.size()), dim3(256), 0,
+                   st, S->side_l, S->side_r, rules, (uint32_t)S->rb.size(), J.d_scatter.p,
+                   S->d_rule_base.p, S->d_ctr.p);
   launch_check("join kernels");
-  return launches;
+  return 4;
 }
 
 // Output slots of the next run: the caller's buffer or the session's own.
@@ -641,7 +675,7 @@ uint32_t enqueue_batched(hbx_session* S, cudaStream_t st) {
       cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
   HBX_CUDA(cudaEventRecordWithFlags(S->ev0, st, rec_flags));
   // the batched form evaluates rule groups: one join's items for several rules
-  uint32_t launches = enqueue_join(S, st, S->d_groups.p);
+  uint32_t launches = enqueue_join(S, st, true);
   dev::EvalParams P = eval_params(S, S->d_groups.p);
   P.n_seg = 0;  // every work item of every group
   const int grid = S->ctx->n_sm * S->blocks_per_sm;
@@ -729,7 +763,7 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
   }
   // PLAIN: join, then one launch per (partition, rule)
   HBX_CUDA(cudaEventRecord(S->ev0, st));
-  uint32_t n = enqueue_join(S, st, S->d_rules.p);
+  uint32_t n = enqueue_join(S, st, false);
   const uint32_t n_rules = (uint32_t)S->rb.size();
   const uint32_t per_class = (uint32_t)S->E.n_partitions + 1;
   const uint32_t per_rule = per_class * dev::kWordClasses;
@@ -796,7 +830,7 @@ std::string autotune_path() {
 
 std::string workload_signature(const hbx_session* S) {
   std::string sig = S->ctx->device_name;
-  sig += "|k4";  // evaluation kernel generation: entries of earlier kernels do not apply
+  sig += "|k5";  // evaluation kernel generation: entries of earlier kernels do not apply
   auto bucket = [](uint64_t n) {  // power-of-two bucket
     uint32_t b = 0;
     while ((1ull << b) < n) b++;

@@ -202,27 +202,38 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // pdl_wait); called once every block of this grid has started.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 
-// ---- fused join for small key domains (every rule's left key domain at most
-// kFusedJoinMaxDomain): one launch for keys + histograms, one for offsets +
-// work items, one for the scatter, each covering every rule and both
-// tables.  The row kernels run one block row per (rule, table)
-// (blockIdx.y = rule, blockIdx.z = table), so the rules' and tables'
-// dependent load -> atomic -> store chains run side by side.
+// ---- the join of every rule of a session: one launch for keys + histograms,
+// one for offsets + work items, one for the scatter, each covering every
+// rule and both tables.  The row kernels run one block row per task
+// (blockIdx.y: one table of one rule), so the rules' and tables' dependent
+// load -> atomic -> store chains run side by side.
+//
+// A rule evaluated in another rule's group needs no offsets, only its number
+// of pair-comparisons, sum over left rows of the right rows with their key:
+// its right rows are counted with the others' and its left rows add up their
+// counts in the scatter launch, so no pass runs over its key domain (8 rules,
+// 30,012 x 29,990 rows: the key + venue rules have 64 partitions x 250 keys x
+// 500 venues = 8M keys).  Bound by launches and memory latency: reset, count,
+// scan and scatter take 46 us there and 158 us at 150k x 150k rows, against
+// 1.57 and 1.83 ms with a scan of every rule's domain, times 5 length
+// classes, in launches per rule; 38 us against 44 us for 2 rules, 2,601 x
+// 64,264 rows.
 
-// Keys and key histograms of every rule for both tables; histograms of
+// Keys and key histograms of every task's rule and table; histograms of
 // domains up to kSharedHistKeys are kept per block in shared memory.
-__global__ void k_join_count(Side L, Side R, const Rule* rules) {
+__global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* tasks) {
   extern __shared__ uint32_t s_cnt[];
   pdl_trigger();
   pdl_wait();  // the histograms are cleared (k_reset)
-  const int side = blockIdx.z;
+  const uint32_t task = tasks[blockIdx.y];
+  const int side = task & kTaskRight ? 1 : 0;
   const Side& S = side ? R : L;
   if ((unsigned long long)blockIdx.x * blockDim.x >= S.n_rows) return;  // whole block
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const Rule& Q = rules[blockIdx.y];
+  const Rule& Q = rules[task & ~kTaskRight];
   const uint32_t D = side ? Q.domain : Q.domain_l;
-  uint32_t* keys = side ? Q.key_r : Q.key_l;
+  uint32_t* keys = !Q.n_members ? nullptr : side ? Q.key_r : Q.key_l;
   uint32_t* cnt = side ? Q.cnt_r : Q.cnt_l;
   const bool split = !side && Q.n_wclass > 1;
   const bool sh = D <= kSharedHistKeys;
@@ -233,7 +244,7 @@ __global__ void k_join_count(Side L, Side R, const Rule* rules) {
   for (uint32_t row = t0; row < S.n_rows; row += stride) {
     uint32_t k = row_key(S, Q, row);
     if (split) k += Q.domain * word_class(S.str_meta[(size_t)Q.wclass_slot * S.n_rows + row].loc.y);
-    keys[row] = k;
+    if (keys) keys[row] = k;
     atomicAdd(sh ? s_cnt + k : cnt + k, 1u);
   }
   if (sh) {
@@ -243,95 +254,90 @@ __global__ void k_join_count(Side L, Side R, const Rule* rules) {
   }
 }
 
-// The three independent scans of every rule -- row offsets per left key
-// (y = 0), row offsets per right key (y = 1), work items per left key with
-// the rule's pair-comparison count (y = 2) -- in chunks of kScanChunk keys,
-// one block of 1024 threads per (chunk, y, rule), in one launch.  A block
-// takes its chunk from a ticket counter of its (y, rule) when it starts,
-// publishes the chunk's total (flag bit kScanFlag set) before it reads
-// anything of the other chunks, then adds the totals of the chunks before
-// its own: those blocks took their tickets earlier, so they are running or
-// done, and every wait ends (bounded all the same: a wait that gives up
-// counts a watchdog trip, which fails the run).
-__device__ __forceinline__ uint32_t join_scan_domain(const Rule& Q, uint32_t y) {
-  return y == 1 ? Q.domain : Q.domain_l;
-}
-
-// The value of key k (< D): its row count, or its work items (y = 2, with
+// The value of key k (< D): its row count, or its work items (what = 2, with
 // the key's pair comparisons added to *pairs).
-__device__ __forceinline__ unsigned long long join_scan_value(const Rule& Q, uint32_t y,
+__device__ __forceinline__ unsigned long long join_scan_value(const Rule& Q, uint32_t what,
                                                               uint32_t tile_right, uint32_t k,
                                                               unsigned long long* pairs) {
-  if (y == 2) {
+  if (what == 2) {
     unsigned long long p = 0;
     const unsigned long long v = key_items(Q, k, tile_right, &p);
     *pairs += p;
     return v;
   }
-  return (y == 1 ? Q.cnt_r : Q.cnt_l)[k];
+  return (what == 1 ? Q.cnt_r : Q.cnt_l)[k];
 }
 
 constexpr unsigned long long kScanFlag = 1ull << 63;
 constexpr uint32_t kScanWaitPolls = 1u << 20;
 
-__global__ void k_join_scan(const Rule* rules, uint32_t tile_right, uint32_t nb,
-                            unsigned long long* sync, unsigned long long* comparisons,
-                            Counters* ctr) {
+// The scans of every rule with work items (ScanTask), one block of 1024
+// threads per chunk of kScanChunk keys, in one launch.  A block takes its
+// chunk from its task's ticket counter when it starts, publishes the chunk's
+// total (flag bit kScanFlag set) before it reads anything of the other
+// chunks, then adds the totals of the chunks before its own, a thread per
+// chunk: those blocks took their tickets earlier, so they are running or
+// done, and every wait ends (bounded all the same: a wait that gives up
+// counts a watchdog trip, which fails the run).
+__global__ void k_join_scan(const Rule* rules, uint32_t tile_right, const ScanTask* tasks,
+                            const uint32_t* block_task, unsigned long long* sync, Counters* ctr) {
   __shared__ unsigned long long s_w64[32];
   __shared__ unsigned long long s_t64, s_base;
   __shared__ uint32_t s_chunk;
   pdl_trigger();
   pdl_wait();  // the histograms are complete (k_join_count)
-  const uint32_t y = blockIdx.y, r = blockIdx.z;
-  // sync: per (rule, y) nb chunk totals, then one ticket counter each
-  unsigned long long* totals = sync + ((size_t)r * 3 + y) * nb;
-  unsigned long long* ticket = sync + (size_t)gridDim.z * 3 * nb + (size_t)r * 3 + y;
-  if (threadIdx.x == 0) s_chunk = (uint32_t)atomicAdd(ticket, 1ull);
+  const uint32_t ti = block_task[blockIdx.x];
+  const ScanTask T = tasks[ti];
+  unsigned long long* totals = sync + T.first_block;
+  if (threadIdx.x == 0) s_chunk = (uint32_t)atomicAdd(sync + gridDim.x + ti, 1ull);
   __syncthreads();
   const uint32_t c = s_chunk;
-  const Rule& Q = rules[r];
-  const uint32_t D = join_scan_domain(Q, y);
-  if ((unsigned long long)c * kScanChunk >= D) return;
+  const Rule& Q = rules[T.rule];
+  const uint32_t D = T.what == 1 ? Q.domain : Q.domain_l;
   const uint32_t b = c * kScanChunk + threadIdx.x * 4u;
   unsigned long long v[4], pairs = 0;
 #pragma unroll
-  for (int k = 0; k < 4; k++) v[k] = b + k < D ? join_scan_value(Q, y, tile_right, b + k, &pairs) : 0ull;
+  for (int k = 0; k < 4; k++)
+    v[k] = b + k < D ? join_scan_value(Q, T.what, tile_right, b + k, &pairs) : 0ull;
   unsigned long long ex = block_excl_scan<unsigned long long>(v[0] + v[1] + v[2] + v[3], s_w64, &s_t64);
   const unsigned long long chunk_total = s_t64;
   if (threadIdx.x == 0) {
+    s_base = 0;
     __threadfence();
     atomicExch(totals + c, chunk_total | kScanFlag);
   }
-  if (threadIdx.x < 32) {  // the chunks before this one: at most 15
-    unsigned long long t = 0;
-    for (uint32_t j = threadIdx.x; j < c; j += 32) {
-      unsigned long long f = 0;
-      uint32_t polls = 0;
-      while (!((f = atomicAdd(totals + j, 0ull)) & kScanFlag) && ++polls < kScanWaitPolls)
-        __nanosleep(64);
-      if (!(f & kScanFlag)) atomicAdd(&ctr->watchdog_trips, 1ull);
-      t += f & ~kScanFlag;
-    }
+  if (c) {  // the chunks before this one
+    __syncthreads();  // s_base is 0
+    if ((threadIdx.x & ~31u) < c) {  // whole warps
+      unsigned long long t = 0;
+      for (uint32_t j = threadIdx.x; j < c; j += blockDim.x) {
+        unsigned long long f = 0;
+        uint32_t polls = 0;
+        while (!((f = atomicAdd(totals + j, 0ull)) & kScanFlag) && ++polls < kScanWaitPolls)
+          __nanosleep(64);
+        if (!(f & kScanFlag)) atomicAdd(&ctr->watchdog_trips, 1ull);
+        t += f & ~kScanFlag;
+      }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
-    if (threadIdx.x == 0) s_base = t;
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+      if ((threadIdx.x & 31) == 0) atomicAdd(&s_base, t);
+    }
   }
   __syncthreads();
   const unsigned long long base = s_base;
   ex += base;
-  if (y == 2) {
+  if (T.what == 2) {
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       if (b + k < D) Q.item_off[b + k] = ex;
       ex += v[k];
     }
-    if ((unsigned long long)(c + 1) * kScanChunk >= D && threadIdx.x == 0)
-      Q.item_off[D] = base + chunk_total;
+    if (c + 1 == T.n_chunks && threadIdx.x == 0) Q.item_off[D] = base + chunk_total;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(kFull, pairs, o);
-    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(comparisons, pairs);
+    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&ctr->comparisons, pairs * Q.cmp_weight);
   } else {
-    uint32_t* off = y == 1 ? Q.off_r : Q.off_l;
+    uint32_t* off = T.what == 1 ? Q.off_r : Q.off_l;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       if (b + k < D) off[b + k] = (uint32_t)ex;
@@ -340,13 +346,15 @@ __global__ void k_join_scan(const Rule* rules, uint32_t tile_right, uint32_t nb,
   }
 }
 
-// Rows of every rule grouped by key (counting-sort scatter, right rows with
-// their first similarity column's metadata), and the rules' item bases.
+// Rows of every rule with work items grouped by key (counting-sort scatter,
+// right rows with their first similarity column's metadata), the
+// pair-comparisons of the others, and the rules' item bases.
 __global__ void k_join_scatter(Side L, Side R, const Rule* rules, uint32_t n_rules,
-                               unsigned long long* rule_base, unsigned long long* items_total) {
+                               const uint32_t* tasks, unsigned long long* rule_base,
+                               Counters* ctr) {
   pdl_trigger();
   pdl_wait();  // offsets and work items are complete (k_join_scan)
-  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
     unsigned long long acc = 0;
     for (uint32_t r = 0; r < n_rules; r++) {
       rule_base[r] = acc;
@@ -354,18 +362,13 @@ __global__ void k_join_scatter(Side L, Side R, const Rule* rules, uint32_t n_rul
       if (rules[r].n_members) acc += rules[r].item_off[rules[r].domain_l];
     }
     rule_base[n_rules] = acc;
-    if (items_total) *items_total = acc;
+    ctr->items_total = acc;
   }
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const Rule& Q = rules[blockIdx.y];
-  if (!Q.n_members) return;  // evaluated in another rule's group: counted, never enumerated
-  if (blockIdx.z == 0) {
-    for (uint32_t row = t0; row < L.n_rows; row += stride) {
-      const uint32_t k = Q.key_l[row];
-      Q.sorted_l[Q.off_l[k] + atomicAdd(Q.cur_l + k, 1u)] = row;
-    }
-  } else {
+  const uint32_t task = tasks[blockIdx.y];
+  const Rule& Q = rules[task & ~kTaskRight];
+  if (task & kTaskRight) {
     const StrMeta* meta_in = R.str_meta + (size_t)Q.sim_r[0] * R.n_rows;
     for (uint32_t row = t0; row < R.n_rows; row += stride) {
       const uint32_t k = Q.key_r[row];
@@ -373,6 +376,17 @@ __global__ void k_join_scatter(Side L, Side R, const Rule* rules, uint32_t n_rul
       Q.sorted_r[pos] = row;
       if (Q.sorted_meta_r) Q.sorted_meta_r[pos] = sorted_meta(R, Q, meta_in, row);
     }
+  } else if (Q.n_members) {
+    for (uint32_t row = t0; row < L.n_rows; row += stride) {
+      const uint32_t k = Q.key_l[row];
+      Q.sorted_l[Q.off_l[k] + atomicAdd(Q.cur_l + k, 1u)] = row;
+    }
+  } else {
+    unsigned long long pairs = 0;
+    for (uint32_t row = t0; row < L.n_rows; row += stride) pairs += Q.cnt_r[row_key(L, Q, row)];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(kFull, pairs, o);
+    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&ctr->comparisons, pairs * Q.cmp_weight);
   }
 }
 

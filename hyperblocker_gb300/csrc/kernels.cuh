@@ -1,13 +1,13 @@
 // kernels.cuh -- sm_103a device code of the blocking engine.
 //
 // Pipeline per run (all on one stream; the batched form is a CUDA graph):
-//   1. k_keys_hist    join key of every row per rule (partition bucket and
+//   1. k_join_count   join key of every row per rule (partition bucket and
 //                     equality dictionary codes in mixed radix, or a dense
 //                     composite id) + histogram of keys per side.
-//   2. scan kernels   exclusive scans: row offsets per key, and work items
+//   2. k_join_scan    exclusive scans: row offsets per key, and work items
 //                     per key (a work item = one left row x up to TR right rows
 //                     of one candidate block).
-//   3. k_scatter      rows grouped by key (counting sort) -> candidate blocks
+//   3. k_join_scatter rows grouped by key (counting sort) -> candidate blocks
 //                     L_key x R_key.
 //   4. k_peq_build    Peq bitmask table of every left string (built with
 //                     __match_any), in device memory.
@@ -150,8 +150,12 @@ struct Rule {
   // match count; members that pass go on with their other predicates, and
   // the pair matches when one member passes them all (OR across rules).
   // n_members == 0: the rule is a member of another rule's group and has no
-  // work items of its own (its join still counts its pair-comparisons).
+  // work items of its own; its pair-comparisons are still counted.
   uint32_t n_members;
+  // Rules whose pair-comparisons this rule's join counts: itself and, in a
+  // grouped rule array, the rules with the same equality slots that have no
+  // join of their own (their cmp_weight is 0).
+  uint32_t cmp_weight;
   uint32_t n_xslots;
   uint32_t xslot[kMaxEq];
   float thr_min;  // smallest member threshold on the first column
@@ -185,6 +189,7 @@ inline void fill_extras_table(Rule* g) {
 // and any rule no group takes in).
 inline void make_singleton(Rule* d) {
   d->n_members = 1;
+  d->cmp_weight = 1;
   d->n_xslots = 0;
   Member& m = d->mem[0];
   m = Member{};
@@ -356,20 +361,32 @@ __global__ void k_rule_base(const Rule* rules, uint32_t n_rules, unsigned long l
 __global__ void k_reset(Counters* ctr, uint32_t* counts, uint64_t n_counts,
                         unsigned long long* seen, uint64_t n_seen, unsigned long long* zero64,
                         uint64_t n_zero64);
-// fused join (every rule's left key domain <= kFusedJoinMaxDomain); k_join_count
-// and k_join_scatter run on grid (blocks, rules, 2 tables); k_join_count
-// takes min(max domain, kSharedHistKeys) * 4 bytes of dynamic shared memory;
-// k_join_scan runs 1024 threads per (chunk of kScanChunk keys, scan, rule):
-// grid (nb = max domain / kScanChunk rounded up, 3, rules); sync holds
-// rules * 3 * (nb + 1) words, zero before the launch (k_reset)
-constexpr uint32_t kFusedJoinMaxDomain = 1u << 16;
+// The join of a rule array in three launches, whatever the key domains.
+// k_join_count and k_join_scatter run on grid (blocks, tasks): a task is one
+// table of one rule (join_task).  Count: both tables of the rules with work
+// items, the right one of the members that only count their comparisons;
+// kSharedHistKeys * 4 bytes of dynamic shared memory, or 4 bytes per key of
+// the largest domain when that is less.  Scatter: both tables of the rules
+// with work items, the left one of the members.  k_join_scan runs 1024
+// threads per chunk of kScanChunk keys of each ScanTask; sync holds one total
+// per block of its grid, then one ticket per task, zero before the launch
+// (k_reset).
 constexpr uint32_t kSharedHistKeys = 8192;
-__global__ void k_join_count(Side L, Side R, const Rule* rules);
-__global__ void k_join_scan(const Rule* rules, uint32_t tile_right, uint32_t nb,
-                            unsigned long long* sync, unsigned long long* comparisons,
-                            Counters* ctr);
+constexpr uint32_t kTaskRight = 1u << 31;
+__host__ __device__ inline uint32_t join_task(uint32_t rule, int side) {
+  return rule | (side ? kTaskRight : 0u);
+}
+// One scan of a rule's join: 0 = row offsets per left key, 1 = row offsets
+// per right key, 2 = work items per left key with the rule's comparisons.
+struct ScanTask {
+  uint32_t rule, what, first_block, n_chunks;
+};
+__global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* tasks);
+__global__ void k_join_scan(const Rule* rules, uint32_t tile_right, const ScanTask* tasks,
+                            const uint32_t* block_task, unsigned long long* sync, Counters* ctr);
 __global__ void k_join_scatter(Side L, Side R, const Rule* rules, uint32_t n_rules,
-                               unsigned long long* rule_base, unsigned long long* items_total);
+                               const uint32_t* tasks, unsigned long long* rule_base,
+                               Counters* ctr);
 // ------------------------------------------------------------------ evaluation
 // Peq tables of every left string of n_slots string slots (PeqShape).
 __global__ void k_peq_build(Side L, uint32_t n_slots, PeqShape shape, uint32_t* peq);
