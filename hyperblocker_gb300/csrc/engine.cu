@@ -94,6 +94,7 @@ struct hbx_session {
   hbx::DBuf<uint32_t> peq;  // Peq tables of the left strings [slot][row]
   int variant = 0;  // evaluation kernel: 0 = k_eval, 1 = k_eval_wide
   bool groups = false;  // some rule evaluates others in the batched form (h_groups)
+  bool long_left = false;  // some left string has no Peq table (k_eval_long)
   bool tuned = false;
   bool one_shot = false;  // runs once (hbx_block): no graph is captured
   // output slots to start with; a run needing more than cap_limit (the
@@ -271,6 +272,9 @@ void list_join(const std::vector<dev::Rule>& rules, JoinLists* J, cudaStream_t s
   J->d_scan.upload(J->scan, st);
 }
 
+// Classes of left rows of the session's rules (dev::Rule).
+uint32_t n_classes(const hbx_session* S) { return S->long_left ? 2u : 1u; }
+
 // Device state of a session whose side buffers hold the encoded tables.
 void setup_session(hbx_session* S, uint64_t h2d_tables) {
   hbx_ctx* C = S->ctx;
@@ -288,6 +292,10 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
   bind(S->L, S->side_l, nL);
   bind(S->R, S->side_r, nR);
 
+  S->long_left = false;
+  for (const RuleEnc& re : E.rules)
+    for (int sl : re.sim_slot_l)
+      if (E.L.str_maxlen[(size_t)sl] > dev::kMaxTableLen) S->long_left = true;
   // join state of every rule (independent of the tile shape)
   S->rb.clear();
   S->rb.resize(E.rules.size());
@@ -309,10 +317,7 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
       d.thr[s] = re.thr[s];
     }
     d.domain = (uint32_t)re.domain;
-    // one kernel per mask width runs every left string: no word classes
-    d.n_wclass = 1u;
-    d.wclass_slot = 0u;
-    d.domain_l = d.domain;
+    dev::set_classes(&d, S->long_left);
     dev::make_singleton(&d);
     RuleBufs& b = S->rb[r];
     b.key_l.alloc(nL);
@@ -379,7 +384,7 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
   S->scan_sync.alloc(S->join_rules.block_task.size() + S->join_rules.scan.size());
   S->d_rules.alloc(E.rules.size());
   S->d_groups.alloc(E.rules.size());
-  S->d_rule_base.alloc(E.rules.size() + 1);
+  S->d_rule_base.alloc(dev::item_base_words(E.rules.size()));
   S->d_ctr.alloc(1);
   // one page-locked counter block per context: its sessions run one at a time
   if (!C->h_ctr) HBX_CUDA(cudaHostAlloc(&C->h_ctr, sizeof(dev::Counters), cudaHostAllocPortable));
@@ -408,13 +413,13 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
     }
   }
 
-  // partition boundaries of every rule's left key space, per word class
-  // (plain form): entry (rule, class, p) = first left key of partition p
+  // partition boundaries of every rule's left key space, per class (plain
+  // form): entry (rule, class, p) = first left key of partition p
   std::vector<uint32_t> idx;
   for (size_t r = 0; r < E.rules.size(); r++)
-    for (uint32_t c = 0; c < dev::kWordClasses; c++)
+    for (uint32_t c = 0; c < n_classes(S); c++)
       for (uint64_t p = 0; p <= E.n_partitions; p++) {
-        const uint32_t cc = std::min<uint32_t>(c, S->h_rules[r].n_wclass - 1);
+        const uint32_t cc = std::min<uint32_t>(c, S->h_rules[r].n_classes - 1);
         idx.push_back(cc * S->h_rules[r].domain + (uint32_t)E.rules[r].part_key_begin[p]);
       }
   S->bound_idx.upload(idx, st);
@@ -555,7 +560,7 @@ std::vector<dev::Rule> group_rules(const std::vector<dev::Rule>& singles) {
       G.sim_l[0] = sl;
       G.sim_r[0] = sr;
       G.thr[0] = t;
-      if (G.n_wclass > 1) G.wclass_slot = sl;
+      G.class_slot = sl;
     }
     dev::make_singleton(&G);
     roots.push_back(r);
@@ -664,6 +669,13 @@ dev::EvalParams eval_params(hbx_session* S, const dev::Rule* rules) {
 
 void queue_counters(hbx_session* S, cudaStream_t st);
 
+// The work items of long left strings (or the range of them in P's segment).
+void launch_long(hbx_session* S, dev::EvalParams P, cudaStream_t st) {
+  P.rule_item_base += P.n_rules + 1;
+  dev::k_eval_long<<<dev::long_grid(S->ctx->n_sm), kThreads, 0, st>>>(P);
+  launch_check("k_eval_long");
+}
+
 uint32_t enqueue_batched(hbx_session* S, cudaStream_t st) {
   // Inside stream capture a plain record would only be a capture dependency
   // marker; the external flag makes it an event-record node that can be
@@ -682,6 +694,10 @@ uint32_t enqueue_batched(hbx_session* S, cudaStream_t st) {
   HBX_CUDA(cudaEventRecordWithFlags(S->ev_eval0, st, rec_flags));
   dev::eval_kernel(S->variant, S->groups, S->peq_shape.w)<<<grid, kThreads, S->smem_bytes, st>>>(P);
   launch_check("k_eval");
+  if (S->long_left) {
+    launch_long(S, P, st);
+    launches++;
+  }
   HBX_CUDA(cudaEventRecordWithFlags(S->ev_eval1, st, rec_flags));
   // the counters travel back inside the run (graph nodes when captured)
   queue_counters(S, st);
@@ -766,16 +782,16 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
   uint32_t n = enqueue_join(S, st, false);
   const uint32_t n_rules = (uint32_t)S->rb.size();
   const uint32_t per_class = (uint32_t)S->E.n_partitions + 1;
-  const uint32_t per_rule = per_class * dev::kWordClasses;
+  const uint32_t per_rule = per_class * n_classes(S);
   const uint32_t total = n_rules * per_rule;
   k_gather_bounds<<<(total + 255) / 256, 256, 0, st>>>(S->d_rules.p, n_rules, per_rule,
                                                        S->bound_idx.p, S->bound_val.p);
   n++;
   launch_check("k_gather_bounds");
-  std::vector<unsigned long long> bounds(total), base(n_rules + 1);
+  std::vector<unsigned long long> bounds(total), base(dev::item_base_words(n_rules));
   HBX_CUDA(cudaMemcpyAsync(bounds.data(), S->bound_val.p, total * sizeof(unsigned long long),
                            cudaMemcpyDeviceToHost, st));
-  HBX_CUDA(cudaMemcpyAsync(base.data(), S->d_rule_base.p, (n_rules + 1) * sizeof(unsigned long long),
+  HBX_CUDA(cudaMemcpyAsync(base.data(), S->d_rule_base.p, base.size() * sizeof(unsigned long long),
                            cudaMemcpyDeviceToHost, st));
   HBX_CUDA(cudaStreamSynchronize(st));
   dev::EvalParams P = eval_params(S, S->d_rules.p);
@@ -783,25 +799,29 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
   HBX_CUDA(cudaEventRecord(S->ev_eval0, st));
   for (uint64_t p = 0; p < S->E.n_partitions; p++) {
     for (uint32_t r = 0; r < n_rules; r++) {
-      // the partition's items: one range per word class
-      P.n_seg = 0;
-      unsigned long long n_items = 0;
-      for (uint32_t c = 0; c < S->h_rules[r].n_wclass; c++) {
-        const size_t k = (size_t)r * per_rule + (size_t)c * per_class + p;
-        const unsigned long long b0 = base[r] + bounds[k], b1 = base[r] + bounds[k + 1];
-        if (b1 <= b0) continue;
-        P.seg_begin[P.n_seg] = b0;
-        P.seg_end[P.n_seg] = b1;
-        P.n_seg++;
-        n_items += b1 - b0;
+      // the partition's items, those of long left strings in a launch of
+      // their own
+      for (uint32_t c = 0; c < S->h_rules[r].n_classes; c++) {
+        const size_t k = (size_t)r * per_rule + (size_t)c * per_class;
+        // the class's first item of the rule, in its item space and in item_off
+        const unsigned long long base_c = base[c * (n_rules + 1) + r], off_c = bounds[k];
+        P.n_seg = 1;
+        P.seg_begin[0] = base_c + bounds[k + p] - off_c;
+        P.seg_end[0] = base_c + bounds[k + p + 1] - off_c;
+        if (P.seg_end[0] <= P.seg_begin[0]) continue;
+        unsigned long long* next = c ? &S->d_ctr.p->work_next_long : &S->d_ctr.p->work_next;
+        HBX_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned long long), st));
+        n++;
+        if (c) {
+          launch_long(S, P, st);
+          continue;
+        }
+        const unsigned long long ctas =
+            (P.seg_end[0] - P.seg_begin[0] + dev::kWarpsPerCta - 1) / dev::kWarpsPerCta;
+        const int grid = (int)std::min<unsigned long long>(ctas, (unsigned long long)max_grid);
+        dev::eval_kernel(S->variant, false, S->peq_shape.w)<<<grid, kThreads, S->smem_bytes, st>>>(P);
+        launch_check("k_eval (plain)");
       }
-      if (!n_items) continue;
-      HBX_CUDA(cudaMemsetAsync(&S->d_ctr.p->work_next, 0, sizeof(unsigned long long), st));
-      const unsigned long long ctas = (n_items + dev::kWarpsPerCta - 1) / dev::kWarpsPerCta;
-      const int grid = (int)std::min<unsigned long long>(ctas, (unsigned long long)max_grid);
-      dev::eval_kernel(S->variant, false, S->peq_shape.w)<<<grid, kThreads, S->smem_bytes, st>>>(P);
-      n++;
-      launch_check("k_eval (plain)");
     }
   }
   HBX_CUDA(cudaEventRecord(S->ev_eval1, st));

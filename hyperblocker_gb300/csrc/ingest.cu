@@ -306,12 +306,10 @@ __global__ void k_pack(ColDev c, uint32_t n, const uint32_t* off16, const uint8_
     }
     __syncwarp();
     uint32_t sw = 0;  // signature word `lane` (lanes 0-7)
-    if (lane < 8) {
-      if (len > dev::kSigMaxLen) {
-        sw = 0xffffffffu;
-      } else {
-        for (int k = 0; k < 4; k++) sw |= cnt[4 * lane + k] << (8 * k);
-      }
+    if (__any_sync(0xffffffffu, cnt[lane] > 255u)) {
+      sw = 0xffffffffu;
+    } else if (lane < 8) {
+      for (int k = 0; k < 4; k++) sw |= cnt[4 * lane + k] << (8 * k);
     }
     const uint32_t s = (lane < 16 && lane < len) ? sym[c.bytes[a + lane]] : 0u;
     uint32_t v = s << (8 * (lane & 3));

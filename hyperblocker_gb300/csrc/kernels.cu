@@ -23,11 +23,11 @@ __global__ void k_keys_hist(Side S, const Rule* rules, uint32_t rule, int side) 
   const Rule& R = rules[rule];
   uint32_t* keys = side ? R.key_r : R.key_l;
   uint32_t* cnt = side ? R.cnt_r : R.cnt_l;
-  const bool split = !side && R.n_wclass > 1;
+  const bool split = !side && R.n_classes > 1;
   for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < S.n_rows;
        row += gridDim.x * blockDim.x) {
     uint32_t k = row_key(S, R, row);
-    if (split) k += R.domain * word_class(S.str_meta[(size_t)R.wclass_slot * S.n_rows + row].loc.y);
+    if (split) k += R.domain * left_class(S.str_meta[(size_t)R.class_slot * S.n_rows + row].loc.y);
     keys[row] = k;
     atomicAdd(cnt + k, 1u);
   }
@@ -142,7 +142,7 @@ __global__ void k_scan_final_u32(const uint32_t* in, uint32_t n, const uint32_t*
   }
 }
 
-// Work items of left key j (word class j / D, join key j % D).
+// Work items of left key j (class j / D, join key j % D).
 __device__ __forceinline__ unsigned long long key_items(const Rule& R, uint32_t j,
                                                         uint32_t tile_right,
                                                         unsigned long long* pairs) {
@@ -235,7 +235,7 @@ __global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* 
   const uint32_t D = side ? Q.domain : Q.domain_l;
   uint32_t* keys = !Q.n_members ? nullptr : side ? Q.key_r : Q.key_l;
   uint32_t* cnt = side ? Q.cnt_r : Q.cnt_l;
-  const bool split = !side && Q.n_wclass > 1;
+  const bool split = !side && Q.n_classes > 1;
   const bool sh = D <= kSharedHistKeys;
   if (sh) {
     for (uint32_t k = threadIdx.x; k < D; k += blockDim.x) s_cnt[k] = 0;
@@ -243,7 +243,7 @@ __global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* 
   }
   for (uint32_t row = t0; row < S.n_rows; row += stride) {
     uint32_t k = row_key(S, Q, row);
-    if (split) k += Q.domain * word_class(S.str_meta[(size_t)Q.wclass_slot * S.n_rows + row].loc.y);
+    if (split) k += Q.domain * left_class(S.str_meta[(size_t)Q.class_slot * S.n_rows + row].loc.y);
     if (keys) keys[row] = k;
     atomicAdd(sh ? s_cnt + k : cnt + k, 1u);
   }
@@ -346,6 +346,25 @@ __global__ void k_join_scan(const Rule* rules, uint32_t tile_right, const ScanTa
   }
 }
 
+// Writes the item bases (item_base_words); returns the number of all items.
+// A rule evaluated in another rule's group has no items of its own.
+__device__ __forceinline__ unsigned long long item_bases(const Rule* rules, uint32_t n_rules,
+                                                         unsigned long long* base) {
+  unsigned long long acc = 0, acc1 = 0;
+  for (uint32_t r = 0; r < n_rules; r++) {
+    base[r] = acc;
+    base[n_rules + 1 + r] = acc1;
+    if (!rules[r].n_members) continue;
+    const unsigned long long n0 = rules[r].item_off[rules[r].domain];
+    acc += n0;
+    acc1 += rules[r].item_off[rules[r].domain_l] - n0;
+  }
+  base[n_rules] = acc;
+  base[2 * n_rules + 1] = acc1;
+  base[2 * n_rules + 2] = acc + acc1;
+  return acc + acc1;
+}
+
 // Rows of every rule with work items grouped by key (counting-sort scatter,
 // right rows with their first similarity column's metadata), the
 // pair-comparisons of the others, and the rules' item bases.
@@ -355,14 +374,7 @@ __global__ void k_join_scatter(Side L, Side R, const Rule* rules, uint32_t n_rul
   pdl_trigger();
   pdl_wait();  // offsets and work items are complete (k_join_scan)
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
-    unsigned long long acc = 0;
-    for (uint32_t r = 0; r < n_rules; r++) {
-      rule_base[r] = acc;
-      // a rule evaluated in another rule's group has no items of its own
-      if (rules[r].n_members) acc += rules[r].item_off[rules[r].domain_l];
-    }
-    rule_base[n_rules] = acc;
-    ctr->items_total = acc;
+    ctr->items_total = item_bases(rules, n_rules, rule_base);
   }
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -390,17 +402,8 @@ __global__ void k_join_scatter(Side L, Side R, const Rule* rules, uint32_t n_rul
   }
 }
 
-__global__ void k_rule_base(const Rule* rules, uint32_t n_rules, unsigned long long* base,
-                            unsigned long long* items_total) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    unsigned long long acc = 0;
-    for (uint32_t r = 0; r < n_rules; r++) {
-      base[r] = acc;
-      if (rules[r].n_members) acc += rules[r].item_off[rules[r].domain_l];
-    }
-    base[n_rules] = acc;
-    if (items_total) *items_total = acc;
-  }
+__global__ void k_rule_base(const Rule* rules, uint32_t n_rules, unsigned long long* base) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) item_bases(rules, n_rules, base);
 }
 
 __global__ void k_reset(Counters* ctr, uint32_t* counts, uint64_t n_counts,
@@ -454,8 +457,8 @@ __device__ __forceinline__ void load_row(const uint32_t* row, uint32_t (&pe)[S])
 
 // The reference's Jaro loops (device_func.cuh:71-111) on symbol strings, with
 // position 256 usable like any other (the reference's uint16_t idx[256] is
-// indexed at 256 there).  Used for pairs whose left string is longer than the
-// fast path handles and for the cross-rule duplicate check.
+// indexed at 256 there).  Used for the predicates after the first of a pair
+// whose left string there is longer than a Peq table covers.
 __device__ __noinline__ uint32_t jaro_m_ref(const uint8_t* s1, uint32_t l1, const uint8_t* s2,
                                             uint32_t l2) {
   const uint8_t* s = s1;
@@ -494,6 +497,74 @@ __device__ __noinline__ uint32_t jaro_m_ref(const uint8_t* s1, uint32_t l1, cons
         m++;
         break;
       }
+    }
+  }
+  return m;
+}
+
+// jaro_m_ref for one pair by a whole warp (every lane calls it with the same
+// arguments): lane k holds positions 8k .. 8k + 7 of the shorter string as
+// bytes of a 64-bit word, with a byte mask of those in the window and not yet
+// matched; a symbol of the longer string takes the lowest candidate position,
+// found by one ballot.  Position 256 (used by the reference's second loop
+// only) is kept beside it.
+// A step is about 30 instructions and one vote; one lane alone searches up to
+// 256 bytes per symbol (jaro_m_ref).
+__device__ __noinline__ uint32_t jaro_m_warp(const uint8_t* s1, uint32_t l1, const uint8_t* s2,
+                                             uint32_t l2) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint8_t* s = s1;
+  const uint8_t* t = s2;
+  uint32_t ls = l1, lt = l2;
+  if (l1 > l2) {
+    s = s2;
+    t = s1;
+    ls = l2;
+    lt = l1;
+  }
+  const uint32_t h = (ls + 1u) / 2u;
+  constexpr unsigned long long kHigh = 0x8080808080808080ull;
+  // strings are padded to 16 bytes with zeros, which equal no symbol
+  const uint2 own = lane * 8u < ls ? *reinterpret_cast<const uint2*>(s + lane * 8u) : make_uint2(0, 0);
+  const uint32_t s256 = ls > 256u ? s[256] : 0u;
+  unsigned long long avail = kHigh;
+  // byte mask of the lane's positions below n
+  auto below = [&](uint32_t n) {
+    const uint32_t b = lane * 8u;
+    if (n >= b + 8u) return kHigh;
+    return n <= b ? 0ull : kHigh & ((1ull << (8u * (n - b))) - 1ull);
+  };
+  auto zero_bytes = [](uint32_t x) {  // 0x80 in every byte of x that is 0
+    return ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x | 0x7f7f7f7fu);
+  };
+  auto candidates = [&](uint32_t c) {
+    const uint32_t cc = c * 0x01010101u;
+    return (unsigned long long)zero_bytes(own.y ^ cc) << 32 | zero_bytes(own.x ^ cc);
+  };
+  const uint32_t to = min(ls + h, lt);
+  uint32_t m = 0;
+  bool free256 = true;
+  unsigned long long win = below(h + 1u);
+  uint32_t w = 0;
+  for (uint32_t i = 0; i < to; i++) {
+    if ((i & 3u) == 0) w = *reinterpret_cast<const uint32_t*>(t + i);
+    const uint32_t c = w & 0xffu;
+    w >>= 8;
+    if (i == h) win = kHigh;  // second loop: from position i - h on
+    const unsigned long long cand = candidates(c) & avail & win;
+    const unsigned v = __ballot_sync(kFull, cand != 0ull);
+    if (v) {
+      m++;
+      if (lane == (uint32_t)__ffs(v) - 1u) avail &= ~(cand & (0ull - cand));
+    } else if (i >= h && i - h <= 256u && free256 && s256 == c) {
+      m++;
+      free256 = false;
+    }
+    // the position that enters (first loop) or leaves (second) for the next symbol
+    const uint32_t j = i < h ? i + h + 1u : i - h;
+    if ((j >> 3) == lane) {
+      const unsigned long long bit = 0x80ull << (8u * (j & 7u));
+      win = i < h ? win | bit : win & ~bit;
     }
   }
   return m;
@@ -562,8 +633,11 @@ __device__ __forceinline__ bool jw_decide(uint32_t m, uint32_t ls, uint32_t ll, 
 // 0.1 * (1/ls) / 3 >= 1.3e-4 per match (c <= 0.9, shorter length ls <= 256 on
 // the path that uses this), so staying 0.05 matches below the real-valued
 // bound keeps a 6.5e-6 gap, far above the float rounding of j (6e-8) and of
-// this computation (< 3e-4 matches).  p >= 10 reaches 1.0: no bound.  A NaN
-// threshold never fails a pair in the reference, so it gives no bound either.
+// this computation (< 3e-4 matches).  For shorter lengths up to kReachMaxLen
+// = 1024 (can_reach) the gap is 0.05 / 3 / 1024 = 1.6e-5 of j, against the same
+// 6e-8, and the computation errs by less than 3e-3 matches.  p >= 10 reaches
+// 1.0: no bound.  A NaN threshold never fails a pair in the reference, so it
+// gives no bound either.
 __device__ __forceinline__ int m_need_lo(uint32_t ls, uint32_t ll, uint32_t p, float thr) {
   if (p >= 10u) return 0;
   const float c = 0.1f * (float)p;
@@ -578,33 +652,6 @@ __device__ __forceinline__ int m_need_lo(uint32_t ls, uint32_t ll, uint32_t p, f
   const float v = ceilf(mr - 0.05f);
   if (!(v > 0.0f)) return 0;
   return v > 1.0e6f ? 1000000 : (int)v;
-}
-
-// Slow exact similarity check of one pair (any lengths).  Out of line and
-// with plain pointer/scalar arguments only: passing the kernel parameters by
-// reference would copy them into local memory for the whole kernel.
-__device__ __noinline__ bool sim_pass_slow(const uint8_t* a, uint32_t la, const uint8_t* b,
-                                           uint32_t lb, float thr, Counters* ctr) {
-  if (la == 0 || lb == 0) return jw_exact(0, la, lb, 0, thr, &ctr->ambiguous);
-  const uint32_t mn = min(la, lb);
-  if (mn > 256) atomicAdd(&ctr->long_pairs, 1ull);
-  const uint32_t m = jaro_m_ref(a, la, b, lb);
-  const uint32_t p = prefix_len(a, b, mn);
-  return jw_exact(m, mn, max(la, lb), p, thr, &ctr->ambiguous);
-}
-
-// The match count and common prefix of one pair by the reference's own
-// loops (any lengths; 0 and 0 when a string is empty), for decisions against
-// several thresholds.  Out of line like sim_pass_slow.
-__device__ __noinline__ void sim_m_slow(const uint8_t* a, uint32_t la, const uint8_t* b,
-                                        uint32_t lb, Counters* ctr, uint32_t* m, uint32_t* p) {
-  *m = 0;
-  *p = 0;
-  if (la == 0 || lb == 0) return;
-  const uint32_t mn = min(la, lb);
-  if (mn > 256) atomicAdd(&ctr->long_pairs, 1ull);
-  *m = jaro_m_ref(a, la, b, lb);
-  *p = prefix_len(a, b, mn);
 }
 
 // Threshold decision on one similarity column of a pair from its match
@@ -763,6 +810,40 @@ __device__ __forceinline__ uint32_t prefix16(const uint4& a, const uint4& b) {
   for (int k = 0; k < 4; k++)
     if (d[k]) return 4u * k + ((uint32_t)(__ffs(d[k]) - 1) >> 3);
   return 16u;
+}
+
+// Can a pair of non-empty strings whose left one has no Peq table reach thr?
+// The filters of the scanned pairs, in front of the reference's own loops:
+// the loops match each position of either string at most once, so lengths
+// and count signatures bound their count too.  false = JW < thr for certain.
+// Longer strings than kReachMaxLen and prefixes of 16 and more are not
+// decided here.
+constexpr uint32_t kReachMaxLen = 1024;
+__device__ __forceinline__ bool can_reach(const StrMeta* am, const StrMeta* bm, uint32_t la,
+                                          uint32_t lb, float thr) {
+  const uint32_t ls = min(la, lb), ll = max(la, lb);
+  if (ls > kReachMaxLen) return true;
+  const uint32_t p16 = prefix16(am->head, bm->head);
+  if (p16 == 16u && ls > 16u) return true;
+  const int need = m_need_lo(ls, ll, min(p16, ls), thr);
+  if (need > (int)ls) return false;
+  return need <= 0 ||
+         (int)sig_bound(am->sig[0], am->sig[1], bm->sig[0], bm->sig[1]) >= need;
+}
+
+// Slow exact similarity check of one pair (any lengths).  Out of line and
+// with plain pointer/scalar arguments only: passing the kernel parameters by
+// reference would copy them into local memory for the whole kernel.
+__device__ __noinline__ bool sim_pass_slow(const StrMeta* am, const StrMeta* bm, const uint8_t* a,
+                                           const uint8_t* b, float thr, Counters* ctr) {
+  const uint32_t la = am->loc.y, lb = bm->loc.y;
+  if (la == 0 || lb == 0) return jw_exact(0, la, lb, 0, thr, &ctr->ambiguous);
+  const uint32_t mn = min(la, lb);
+  if (mn > 256) atomicAdd(&ctr->long_pairs, 1ull);
+  if (!can_reach(am, bm, la, lb, thr)) return false;
+  const uint32_t m = jaro_m_ref(a, la, b, lb);
+  const uint32_t p = prefix_len(a, b, mn);
+  return jw_exact(m, mn, max(la, lb), p, thr, &ctr->ambiguous);
 }
 
 // Per-lane work counts of the evaluation loop, summed into Counters at exit:
@@ -924,7 +1005,7 @@ __device__ __forceinline__ int advance_rule(const EvalParams& P, uint32_t rule, 
     const uint8_t* b = P.R.arena + 16ull * bl.x;
     if (!has_table(P, la)) {  // the reference's own loops
       if (la && lb) ops->ops += jw_eval_ops(min(la, lb), max(la, lb));
-      if (!sim_pass_slow(a, la, b, lb, thr, P.ctr)) return 0;
+      if (!sim_pass_slow(am, bm, a, b, thr, P.ctr)) return 0;
       continue;
     }
     if (lb == 0) {
@@ -1014,7 +1095,7 @@ __device__ __forceinline__ int advance_group(const EvalParams& P, uint32_t rule,
       const uint8_t* b = P.R.arena + 16ull * bl.x;
       if (!has_table(P, la)) {  // the reference's own loops
         if (la && lb) ops->ops += jw_eval_ops(min(la, lb), max(la, lb));
-        if (!sim_pass_slow(a, la, b, lb, thr, P.ctr)) break;
+        if (!sim_pass_slow(am, bm, a, b, thr, P.ctr)) break;
         continue;
       }
       if (lb == 0) {
@@ -1080,6 +1161,10 @@ struct ItemDesc {
   int32_t lcode[2];  // the left row's codes of the group's first two extra slots
 };
 constexpr uint32_t kOutBuf = 64;  // matches a warp holds before writing them out
+struct OutBuf {  // matches not yet written out (emit): fewer than 32 between calls
+  uint2 pair[kOutBuf];
+  uint32_t n;
+};
 struct WarpCtl {
   ItemDesc desc[kMaxClaimChunk];  // claimed items not yet staged
   uint32_t c_rule[kMaxStageBufs], c_lrow[kMaxStageBufs];  // claim per staging buffer
@@ -1089,12 +1174,10 @@ struct WarpCtl {
   int32_t c_lcode[kMaxStageBufs][2];
   // the item being filtered; i_lcode: its left row's codes of the group's
   // extra equality slots
-  uint32_t i_rule, i_lrow, i_kind, i_fast, i_all;
+  uint32_t i_rule, i_lrow, i_kind, i_all;
   float i_thr;
   int32_t i_lcode[kMaxEq];
-  // matches not yet written out (emit): fewer than 32 between calls
-  uint2 out_buf[kOutBuf];
-  uint32_t out_n;
+  OutBuf out;
 };
 static_assert(sizeof(WarpCtl) <= kWarpCtlWords * 4, "warp control block outgrows its words");
 
@@ -1102,36 +1185,36 @@ static_assert(sizeof(WarpCtl) <= kWarpCtlWords * 4, "warp control block outgrows
 // together (flush_pairs), so the duplicate-set probes and the output
 // reservation pay their round trips once per 32 matches instead of once per
 // step with a match.
-__device__ __forceinline__ void emit(const EvalParams& P, WarpCtl* C, bool pass, uint32_t lrow,
+__device__ __forceinline__ void emit(const EvalParams& P, OutBuf* O, bool pass, uint32_t lrow,
                                      uint32_t rrow, int lane) {
   const unsigned pm = __ballot_sync(kFull, pass);
   if (!pm) return;
-  const uint32_t n0 = C->out_n;
-  if (pass) C->out_buf[n0 + __popc(pm & ((1u << lane) - 1u))] = make_uint2(lrow, rrow);
+  const uint32_t n0 = O->n;
+  if (pass) O->pair[n0 + __popc(pm & ((1u << lane) - 1u))] = make_uint2(lrow, rrow);
   const uint32_t n = n0 + __popc(pm);
   __syncwarp();
   if (n < 32) {
-    if (lane == 0) C->out_n = n;
+    if (lane == 0) O->n = n;
     __syncwarp();
     return;
   }
-  const uint2 e = C->out_buf[lane];
+  const uint2 e = O->pair[lane];
   const bool more = (uint32_t)lane + 32u < n;
-  const uint2 t = more ? C->out_buf[32 + lane] : make_uint2(0u, 0u);
+  const uint2 t = more ? O->pair[32 + lane] : make_uint2(0u, 0u);
   __syncwarp();
-  if (more) C->out_buf[lane] = t;
-  if (lane == 0) C->out_n = n - 32u;
+  if (more) O->pair[lane] = t;
+  if (lane == 0) O->n = n - 32u;
   __syncwarp();
   flush_pairs(P, true, e.x, e.y, lane);
 }
 
 // Writes out the matches emit still holds (at the end of the warp's loop).
-__device__ __forceinline__ void emit_drain(const EvalParams& P, WarpCtl* C, int lane) {
-  const uint32_t n = C->out_n;
+__device__ __forceinline__ void emit_drain(const EvalParams& P, OutBuf* O, int lane) {
+  const uint32_t n = O->n;
   const bool have = (uint32_t)lane < n;
-  const uint2 e = have ? C->out_buf[lane] : make_uint2(0u, 0u);
+  const uint2 e = have ? O->pair[lane] : make_uint2(0u, 0u);
   __syncwarp();
-  if (lane == 0) C->out_n = 0;
+  if (lane == 0) O->n = 0;
   __syncwarp();
   flush_pairs(P, have, e.x, e.y, lane);
 }
@@ -1192,21 +1275,11 @@ __device__ __forceinline__ uint32_t filter_batch(const EvalParams& P, WarpCtl* C
   int need = 0;
   if (live) {
     const uint32_t lb = loc.y;
-    if (!C->i_fast) {  // the reference's own loops
-      if (la && lb) ops->ops += jw_eval_ops(min(la, lb), max(la, lb));
-      if constexpr (G) {
-        uint32_t m = 0, pp = 0;
-        sim_m_slow(P.L.arena + 16ull * a_off, la, P.R.arena + 16ull * loc.x, lb, P.ctr, &m, &pp);
-        pass1 = first_pass(R, live, m, la, lb, pp, &P.ctr->ambiguous);
-      } else {
-        pass1 = sim_pass_slow(P.L.arena + 16ull * a_off, la, P.R.arena + 16ull * loc.x, lb, thr,
-                              P.ctr) ? 1u : 0u;
-      }
-    } else if (lb == 0) {
+    if (la == 0 || lb == 0) {
       if constexpr (G)
-        pass1 = first_pass(R, live, 0, la, 0, 0, &P.ctr->ambiguous);
+        pass1 = first_pass(R, live, 0, la, lb, 0, &P.ctr->ambiguous);
       else
-        pass1 = jw_exact(0, la, 0, 0, thr, &P.ctr->ambiguous) ? 1u : 0u;
+        pass1 = jw_exact(0, la, lb, 0, thr, &P.ctr->ambiguous) ? 1u : 0u;
     } else {
       const uint32_t ls = min(la, lb), ll = max(la, lb);
       ops->ops += jw_eval_ops(ls, ll);
@@ -1246,7 +1319,7 @@ __device__ __forceinline__ uint32_t filter_batch(const EvalParams& P, WarpCtl* C
                               __float_as_uint(thr))
                  : make_uint4(lrow, la, a_off, C->i_rule);
   }
-  emit(P, C, done, lrow, rrow, lane);
+  emit(P, &C->out, done, lrow, rrow, lane);
   return __popc(qm);
 }
 
@@ -1324,6 +1397,22 @@ __device__ __forceinline__ uint32_t find_key_in(const unsigned long long* item_o
   return lo;
 }
 
+// The left row and the rows [rb0, rb1) of sorted_r of item `local` of a rule's
+// item space, under left key jl.
+__device__ __forceinline__ void item_rows(const EvalParams& P, const Rule& R, uint32_t jl,
+                                          unsigned long long local, uint32_t* lrow, uint32_t* rb0,
+                                          uint32_t* rb1) {
+  const uint32_t key = jl < R.domain ? jl : jl - R.domain;  // join key
+  const unsigned long long in_key = local - R.item_off[jl];
+  const uint32_t nl = R.cnt_l[jl];
+  const uint32_t ri = (uint32_t)(in_key / nl);
+  const uint32_t li = (uint32_t)(in_key - (unsigned long long)ri * nl);
+  *lrow = R.sorted_l[R.off_l[jl] + li];
+  const uint32_t offr = R.off_r[key];
+  *rb0 = offr + ri * P.tile_right;
+  *rb1 = min(*rb0 + P.tile_right, offr + R.cnt_r[key]);
+}
+
 // Claims up to `chunk` consecutive work positions with one atomic and
 // computes their item descriptors into C->desc, one lane per item, so the
 // dependent loads of every item (rule fields included) overlap.  Within one rule, the first and
@@ -1345,24 +1434,17 @@ __device__ __forceinline__ uint32_t claim_chunk(const EvalParams& P, WarpCtl* C,
   const Rule& R = P.rules[r];
   const unsigned long long local = it - P.rule_item_base[r];
   const uint32_t r_first = __shfl_sync(kFull, r, 0), r_last = __shfl_sync(kFull, r, n - 1);
-  uint32_t jl;  // left key (word class, join key)
+  uint32_t jl;  // left key (items of class 0 only: the join key)
   if (r_first == r_last) {
     uint32_t kb = 0;
-    if (k == 0 || k == n - 1) kb = find_key(R.item_off, R.domain_l, local);
+    if (k == 0 || k == n - 1) kb = find_key(R.item_off, R.domain, local);
     const uint32_t k0 = __shfl_sync(kFull, kb, 0), k1 = __shfl_sync(kFull, kb, n - 1);
     jl = find_key_in(R.item_off, k0, k1 + 1, local);
   } else {
-    jl = find_key(R.item_off, R.domain_l, local);
+    jl = find_key(R.item_off, R.domain, local);
   }
-  const uint32_t key = jl % R.domain;  // join key
-  const unsigned long long in_key = local - R.item_off[jl];
-  const uint32_t nl = R.cnt_l[jl];
-  const uint32_t ri = (uint32_t)(in_key / nl);
-  const uint32_t li = (uint32_t)(in_key - (unsigned long long)ri * nl);
-  const uint32_t lrow = R.sorted_l[R.off_l[jl] + li];
-  const uint32_t offr = R.off_r[key];
-  const uint32_t rb0 = offr + ri * P.tile_right;
-  const uint32_t rb1 = min(rb0 + P.tile_right, offr + R.cnt_r[key]);
+  uint32_t lrow, rb0, rb1;
+  item_rows(P, R, jl, local, &lrow, &rb0, &rb1);
   const uint32_t a0 = rb0 & ~3u;
   ItemDesc d;
   const bool sim = R.n_sim != 0;
@@ -1417,7 +1499,7 @@ __device__ __forceinline__ void claim_item(const EvalParams& P, WarpCtl* C, uint
       for (uint32_t e = 0; e < d.n; e += 32) {
         const uint32_t k = e + (uint32_t)lane;
         const uint32_t rrow = k < d.n ? d.rows_src[d.shift + k] : 0u;
-        emit(P, C, k < d.n, d.lrow, rrow, lane);
+        emit(P, &C->out, k < d.n, d.lrow, rrow, lane);
       }
       (*done)++;
       continue;
@@ -1466,7 +1548,7 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
   WarpCtl* C = reinterpret_cast<WarpCtl*>(region + P.ctl_off);
   uint64_t* bar0 = reinterpret_cast<uint64_t*>(region + P.mbar_off);
   const long long t_start = clock64();
-  if (lane == 0) C->out_n = 0;
+  if (lane == 0) C->out.n = 0;
   __syncwarp();
   // work positions per claim: every warp gets about eight claims, at most
   // kMaxClaimChunk items each
@@ -1530,23 +1612,20 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
         mbar_wait(bar0 + cb, ((phs >> cb) & 1u) ^ 1u);
         for (uint32_t b = 0; b < P.n_bufs; b++)
           if (b != cb && C->c_n[b]) mbar_wait(bar0 + b, (phs >> b) & 1u);
-        emit_drain(P, C, lane);
+        emit_drain(P, &C->out, lane);
         return;
       }
       active = true;
       in_pos = 0;
       (*done)++;
-      const StrMeta* lm = reinterpret_cast<const StrMeta*>(buf + P.buf_lmeta_off);
       const uint32_t ir = C->c_rule[cb], il = C->c_lrow[cb], kind = C->c_kind[cb];
       const float thr = C->c_thr[cb];
-      const uint32_t la = lm->loc.y;
       __syncwarp();  // the previous item's fields are read
       C->i_rule = ir;
       C->i_lrow = il;
       C->i_thr = thr;
       C->i_kind = kind;
       C->i_all = (1u << item_members(kind)) - 1u;
-      C->i_fast = has_table(P, la) ? 1u : 0u;
       if (G && (kind & kItemExtras)) {  // the left row's codes of the extra equality slots
         const uint32_t nx = (kind >> 12) & 15u;
         if (lane < 2) {
@@ -1656,10 +1735,10 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
         }
       }
     }
-    emit(P, C, fin && pass, lrow, rrow, lane);
+    emit(P, &C->out, fin && pass, lrow, rrow, lane);
     if (!__any_sync(kFull, busy) && head == tail && !active && cur_n == 0) break;
   }
-  emit_drain(P, C, lane);
+  emit_drain(P, &C->out, lane);
 }
 
 // The evaluation kernel body for masks of W words, instantiated below with
@@ -1703,6 +1782,144 @@ __device__ __forceinline__ void eval_body(const EvalParams& P) {
     if (rest) atomicAdd(&P.ctr->rest_scans, rest);
     if (tally.wsteps) atomicAdd(&P.ctr->scan_warp_steps, (unsigned long long)tally.wsteps);
   }
+}
+
+// One pair, by the whole warp (arguments the same in every lane): does a
+// member of `pass`, the members whose threshold on the group's first column
+// the pair reaches, pass all its other predicates?
+__device__ __noinline__ bool long_pair_rest(const EvalParams& P, const Rule* R, uint32_t pass,
+                                            uint32_t lrow, uint32_t rrow) {
+  const int lane = threadIdx.x & 31;
+  uint32_t memo = 0xffffffffu, m = 0, p = 0;  // the last column counted (advance_group)
+  for (uint32_t x = pass; x; x &= x - 1) {
+    const Member* M = R->mem + (__ffs(x) - 1);
+    uint32_t k = 0;
+    for (; k < M->n_rest; k++) {
+      const uint32_t sl = M->rest_l[k], sr = M->rest_r[k];
+      const float thr = M->rest_thr[k];
+      const StrMeta* am = P.L.str_meta + (size_t)sl * P.L.n_rows + lrow;
+      const StrMeta* bm = P.R.str_meta + (size_t)sr * P.R.n_rows + rrow;
+      const uint4 al = am->loc, bl = bm->loc;
+      const uint32_t la = al.y, lb = bl.y, mn = min(la, lb), mx = max(la, lb);
+      if (mn && memo != (sl << 16 | sr)) {
+        if (lane == 0) {
+          atomicAdd(&P.ctr->jw_word_ops, jw_eval_ops(mn, mx));
+          if (mn > kMaxTableLen) atomicAdd(&P.ctr->long_pairs, 1ull);
+        }
+        if (!can_reach(am, bm, la, lb, thr)) break;
+        const uint8_t* a = P.L.arena + 16ull * al.x;
+        const uint8_t* b = P.R.arena + 16ull * bl.x;
+        m = jaro_m_warp(a, la, b, lb);
+        p = prefix_len(a, b, mn);
+        memo = sl << 16 | sr;
+      }
+      bool ok = false;
+      if (lane == 0) ok = mn ? jw_exact(m, mn, mx, p, thr, &P.ctr->ambiguous)
+                             : jw_exact(0, la, lb, 0, thr, &P.ctr->ambiguous);
+      if (!__shfl_sync(kFull, ok ? 1 : 0, 0)) break;
+    }
+    if (k == M->n_rest) return true;
+  }
+  return false;
+}
+
+// Work items whose left string has no Peq table (longer than kMaxTableLen).
+// A warp takes one item at a time from the class-1 item space and goes over
+// its right rows 32 at a time: a lane per row tests the extra equalities and
+// the filters of the scanned pairs (can_reach), and the few pairs left are
+// counted one after the other by the whole warp (jaro_m_warp).  As items
+// of the evaluation kernels -- a lane per pair, every pair through the
+// reference's loops -- they were most of the time: 40,014 x 60,000 rows of
+// 64-256 characters, 2 % of the authors over 256 symbols, evaluation 37.5 ms
+// against 2.51 ms; and the evaluation kernels without that path need fewer
+// registers (8 rules, 150k x 150k rows: 14.06 against 13.91 ms).
+__global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_eval_long(
+    const __grid_constant__ EvalParams P) {
+  __shared__ OutBuf s_out[kWarpsPerCta];
+  const int lane = threadIdx.x & 31;
+  OutBuf* O = s_out + (threadIdx.x >> 5);
+  if (lane == 0) O->n = 0;
+  __syncwarp();
+  const unsigned long long n_work =
+      P.n_seg ? P.seg_end[0] - P.seg_begin[0] : P.rule_item_base[P.n_rules];
+  const long long t_start = clock64();
+  unsigned long long done = 0, word_ops = 0;
+  for (;;) {
+    unsigned long long v = 0;
+    if (lane == 0) v = atomicAdd(&P.ctr->work_next_long, 1ull);
+    v = __shfl_sync(kFull, v, 0);
+    if (v >= n_work) break;
+    if (P.watchdog_cycles && (unsigned long long)(clock64() - t_start) > P.watchdog_cycles) {
+      if (lane == 0) atomicAdd(&P.ctr->watchdog_trips, 1ull);
+      break;
+    }
+    const unsigned long long it = P.n_seg ? P.seg_begin[0] + v : v;
+    uint32_t r = 0;
+    while (r + 1 < P.n_rules && P.rule_item_base[r + 1] <= it) r++;
+    const Rule* R = P.rules + r;
+    const unsigned long long local = it - P.rule_item_base[r] + R->item_off[R->domain];
+    const uint32_t jl =
+        R->domain + find_key(R->item_off + R->domain, R->domain_l - R->domain, local);
+    uint32_t lrow, rb0, rb1;
+    item_rows(P, *R, jl, local, &lrow, &rb0, &rb1);
+    const StrMeta* lm = P.L.str_meta + (size_t)R->sim_l[0] * P.L.n_rows + lrow;
+    const uint32_t la = lm->loc.y;
+    const uint8_t* a = P.L.arena + 16ull * lm->loc.x;
+    const uint32_t all = (1u << R->n_members) - 1u, nx = R->n_xslots;
+    for (uint32_t e0 = rb0; e0 < rb1; e0 += 32) {
+      const uint32_t e = e0 + (uint32_t)lane;
+      const bool act = e < rb1;
+      const uint32_t rrow = act ? R->sorted_r[e] : 0u;
+      const StrMeta* rm = R->sorted_meta_r + (act ? e : e0);
+      const uint4 loc = rm->loc;
+      const uint32_t lb = loc.y;
+      uint32_t live = act ? all : 0u, pass1 = 0;
+      if (act && nx) {  // members whose extra equalities hold
+        uint32_t eqm = 0;
+        for (uint32_t j = 0; j < nx; j++) {
+          const size_t xs = R->xslot[j];
+          if (P.R.eq_codes[xs * P.R.n_rows + rrow] == P.L.eq_codes[xs * P.L.n_rows + lrow])
+            eqm |= 1u << j;
+        }
+        for (uint32_t x = all; x; x &= x - 1) {
+          const uint32_t k = (uint32_t)__ffs(x) - 1u;
+          if (R->mem[k].xmask & ~eqm) live &= ~(1u << k);
+        }
+      }
+      bool count = false;
+      if (live) {
+        if (lb == 0) {
+          pass1 = first_pass(R, live, 0, la, 0, 0, &P.ctr->ambiguous);
+        } else {
+          word_ops += jw_eval_ops(min(la, lb), max(la, lb));
+          if (lb > kMaxTableLen) atomicAdd(&P.ctr->long_pairs, 1ull);
+          count = can_reach(lm, rm, la, lb, live_thr(R, live));
+        }
+      }
+      for (unsigned x = __ballot_sync(kFull, count); x; x &= x - 1) {
+        const int src = __ffs(x) - 1;
+        const uint8_t* b = P.R.arena + 16ull * __shfl_sync(kFull, loc.x, src);
+        const uint32_t m = jaro_m_warp(a, la, b, __shfl_sync(kFull, lb, src));
+        if (lane == src)
+          pass1 = first_pass(R, live, m, la, lb, prefix_len(a, b, min(la, lb)), &P.ctr->ambiguous);
+        __syncwarp();
+      }
+      bool match = pass1 && member_done(R, pass1);
+      for (unsigned x = __ballot_sync(kFull, pass1 && !match); x; x &= x - 1) {
+        const int src = __ffs(x) - 1;
+        const bool ok = long_pair_rest(P, R, __shfl_sync(kFull, pass1, src), lrow,
+                                       __shfl_sync(kFull, rrow, src));
+        if (lane == src) match = ok;
+      }
+      emit(P, O, match, lrow, rrow, lane);
+    }
+    done++;
+  }
+  emit_drain(P, O, lane);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) word_ops += __shfl_xor_sync(kFull, word_ops, o);
+  if (lane == 0 && done) atomicAdd(&P.ctr->items_done, done);
+  if (lane == 0 && word_ops) atomicAdd(&P.ctr->jw_word_ops, word_ops);
 }
 
 // Peq tables (PeqShape): one warp per (slot, row); the table is cleared,

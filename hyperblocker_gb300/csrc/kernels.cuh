@@ -55,11 +55,11 @@ constexpr float kDecisionMargin = 1e-4f;  // |approx JW - thr| below this -> exa
 // (any matching between equal symbols) is at most
 //     sum_k min(sig_a[k], sig_b[k]),
 // and pooling symbols into one bucket only raises that sum, so the bound is
-// exact.  A string longer than kSigMaxLen bytes, whose counts might not fit a
-// byte, gets 0xff in every bucket: min() then takes the other side's count,
-// which still bounds the matches from above.
+// exact.  A string with a count that does not fit a byte gets 0xff in every
+// bucket: min() then takes the other side's count, which still bounds the
+// matches from above (two such strings: 32 * 255, above every bound that is
+// asked for).
 constexpr uint32_t kSigBuckets = 32;
-constexpr uint32_t kSigMaxLen = 255;
 __host__ __device__ inline uint32_t sig_bucket(uint32_t sym) {  // sym >= 1
   return sym >= kSigBuckets ? kSigBuckets - 1 : sym - 1;
 }
@@ -77,14 +77,12 @@ struct __align__(16) StrMeta {
 // Host form of the signature of a string of symbols.
 inline void make_sig(const uint8_t* s, uint32_t len, uint4 out[2]) {
   uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (len > kSigMaxLen) {
-    for (int k = 0; k < 8; k++) w[k] = 0xffffffffu;
-  } else {
-    uint32_t c[kSigBuckets] = {0};
-    for (uint32_t i = 0; i < len; i++)
-      if (s[i]) c[sig_bucket(s[i])]++;
-    for (uint32_t k = 0; k < kSigBuckets; k++) w[k / 4] |= c[k] << (8 * (k % 4));
-  }
+  uint32_t c[kSigBuckets] = {0};
+  for (uint32_t i = 0; i < len; i++)
+    if (s[i]) c[sig_bucket(s[i])]++;
+  bool fits = true;
+  for (uint32_t k = 0; k < kSigBuckets; k++) fits = fits && c[k] <= 255u;
+  for (uint32_t k = 0; k < kSigBuckets; k++) w[k / 4] |= (fits ? c[k] : 255u) << (8 * (k % 4));
   out[0] = make_uint4(w[0], w[1], w[2], w[3]);
   out[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
@@ -118,13 +116,13 @@ struct Rule {
   uint32_t sim_l[kMaxSim], sim_r[kMaxSim];
   float thr[kMaxSim];
   uint32_t domain;    // D: join keys
-  // Left rows are grouped by (word class, key): the word class is the number
-  // of 32-symbol words of the left string of the first similarity predicate
-  // (1, 2, 3, 4, more).  Work items are ordered class by class, so warps that
-  // run at the same time mostly run the same scan variant.
-  uint32_t n_wclass;  // 1 (no split) or kWordClasses
-  uint32_t wclass_slot;  // left string slot that decides the class
-  uint32_t domain_l;  // n_wclass * D: left keys
+  // Where some left string has no Peq table (more than kMaxTableLen symbols),
+  // left rows are grouped by (class, key): class 1 holds the rows whose
+  // string of the first similarity predicate is that long.  Their work items
+  // follow all items of class 0 and are evaluated by k_eval_long.
+  uint32_t n_classes;   // 1, or 2 with long left strings
+  uint32_t class_slot;  // left string slot that decides the class
+  uint32_t domain_l;    // n_classes * D: left keys
   uint32_t* key_l;
   uint32_t* key_r;
   uint32_t* cnt_l;  // [domain_l]
@@ -205,8 +203,17 @@ inline void make_singleton(Rule* d) {
   fill_extras_table(d);
 }
 
-constexpr uint32_t kWordClasses = 5;
-constexpr uint32_t kMaxSegments = 8;
+constexpr uint32_t kMaxTableLen = 256;
+__host__ __device__ inline uint32_t left_class(uint32_t len) { return len > kMaxTableLen ? 1u : 0u; }
+
+// Host: a rule's left keys, in two classes when some left string is longer
+// than kMaxTableLen.  After domain, n_sim and sim_l are set.
+inline void set_classes(Rule* d, bool long_left) {
+  d->n_classes = long_left && d->n_sim ? 2u : 1u;
+  d->class_slot = d->n_sim ? d->sim_l[0] : 0u;
+  d->domain_l = d->n_classes * d->domain;
+}
+constexpr uint32_t kMaxSegments = 1;
 constexpr uint32_t kRingEntries = 64;
 constexpr uint32_t kRingWords = 12;  // words per ring entry (three 16-byte records)
 
@@ -275,11 +282,6 @@ inline WarpLayout warp_layout_fit(uint32_t tile_right, size_t smem_cap) {
   return warp_layout(tile_right, 1);
 }
 
-__host__ __device__ inline uint32_t word_class(uint32_t len) {
-  const uint32_t w = (len + 31u) >> 5;
-  return w == 0 ? 0u : (w > kWordClasses ? kWordClasses - 1 : w - 1);
-}
-
 struct Counters {
   unsigned long long out_count;
   unsigned long long comparisons;
@@ -296,6 +298,7 @@ struct Counters {
   unsigned long long items_total; // work items of the run (written by the join)
   unsigned long long scan_warp_steps;  // warp-level scan steps (any lane scanning)
   unsigned long long rest_scans;       // scans of predicates after a rule's or group's first
+  unsigned long long work_next_long;   // k_eval_long's work_next
 };
 
 struct EvalParams {
@@ -303,10 +306,12 @@ struct EvalParams {
   const Rule* rules;
   uint32_t n_rules;
   uint32_t n_symbols;
-  const unsigned long long* rule_item_base;  // [n_rules + 1], global item space
+  // [n_rules + 1], global item space of the class this launch evaluates (the
+  // two halves of ItemBases)
+  const unsigned long long* rule_item_base;
   // Work list of the launch: every item (n_seg == 0, the batched form), or the
   // concatenation of item ranges [seg_begin[k], seg_end[k]) (the plain form:
-  // one partition of one rule, one range per word class).
+  // one partition of one rule).
   uint32_t n_seg;
   unsigned long long seg_begin[kMaxSegments];
   unsigned long long seg_end[kMaxSegments];
@@ -354,8 +359,11 @@ __global__ void k_items_partial(const Rule* rules, uint32_t rule, uint32_t tile_
 __global__ void k_scan_top_u64(unsigned long long* partial, uint32_t nb);
 __global__ void k_items_final(const Rule* rules, uint32_t rule, uint32_t tile_right,
                               const unsigned long long* partial);
-__global__ void k_rule_base(const Rule* rules, uint32_t n_rules, unsigned long long* base,
-                            unsigned long long* items_total);
+// Item bases of a rule array: n_rules + 1 words for the items of class 0 (the
+// first item of each rule, then their number), the same for class 1, then
+// the number of all items.
+inline size_t item_base_words(size_t n_rules) { return 2 * (n_rules + 1) + 1; }
+__global__ void k_rule_base(const Rule* rules, uint32_t n_rules, unsigned long long* base);
 // One launch for a run's resets: the counters and histograms to 0, the
 // duplicate set (n_seen slots, may be 0) to empty.
 __global__ void k_reset(Counters* ctr, uint32_t* counts, uint64_t n_counts,
@@ -395,6 +403,11 @@ __global__ void k_peq_build(Side L, uint32_t n_slots, PeqShape shape, uint32_t* 
 // registers), or the same two over rule groups (k_eval_groups<W>,
 // k_eval_groups_wide<W>: launches where some rule evaluates others).
 using EvalKernel = void (*)(EvalParams);
+// The work items of left strings without a Peq table (class 1; rule_item_base
+// points at their bases), for groups and rules alike: grid
+// long_grid(number of SMs), kWarpsPerCta * 32 threads.
+__global__ void k_eval_long(const __grid_constant__ EvalParams P);
+inline int long_grid(int n_sm) { return n_sm * 4; }
 EvalKernel eval_kernel(int wide, bool groups, uint32_t peq_w);
 constexpr uint32_t kPeqWidths[] = {1, 2, 3, 4, 8};  // every PeqShape::w
 

@@ -89,7 +89,7 @@ __global__ void k_lookup(ing::ColDev lc, uint32_t n, const unsigned long long* k
 }
 
 // Left join key of the request rows [row0, row0 + n) for rule instance inst
-// (word class x equality codes in mixed radix), counted per key; rows with an
+// (class x equality codes in mixed radix), counted per key; rows with an
 // equality that has no resident partner get no key.
 __global__ void k_keys(const dev::Rule* rules, uint32_t inst, dev::Side L, uint32_t row0,
                        uint32_t n, uint32_t* key_l) {
@@ -107,8 +107,8 @@ __global__ void k_keys(const dev::Rule* rules, uint32_t inst, dev::Side L, uint3
       key_l[i] = 0xffffffffu;
       continue;
     }
-    if (R.n_wclass > 1)
-      key += R.domain * dev::word_class(L.str_meta[(size_t)R.wclass_slot * L.n_rows + row].loc.y);
+    if (R.n_classes > 1)
+      key += R.domain * dev::left_class(L.str_meta[(size_t)R.class_slot * L.n_rows + row].loc.y);
     key_l[i] = key;
     atomicAdd(R.cnt_l + key, 1u);
   }
@@ -247,6 +247,7 @@ struct Slot {
   uint64_t capacity = 0;
   uint64_t cmp_first = 0;  // comparisons counted by the first evaluation pass
   dev::PeqShape shape{};   // Peq tables of this batch's left strings
+  bool long_left = false;  // some left string may have no Peq table (k_eval_long)
   DBuf<uint32_t> peq;
   Pinned stage, h_out, h_ctr;  // h_ctr: Counters + total items + comparisons per instance
   ~Slot() {
@@ -553,9 +554,7 @@ void open_server(hbx_server* S, const hbx_plan* const* plans, int32_t n_plans, c
         d.thr[s] = pr.thr[s];
       }
       d.domain = (uint32_t)D;
-      d.n_wclass = (d.n_sim && D * dev::kWordClasses <= (1ull << 22)) ? dev::kWordClasses : 1u;
-      d.wclass_slot = d.n_sim ? d.sim_l[0] : 0u;
-      d.domain_l = d.n_wclass * d.domain;
+      dev::set_classes(&d, false);  // a batch with long left strings sets two
       dev::make_singleton(&d);
       // right half of the join: rows grouped by key, metadata in that order
       T->key_r.alloc(std::max<uint32_t>(nR, 1));
@@ -638,7 +637,9 @@ uint64_t estimate(const hbx_server* S, const Table& t, int32_t plan, uint32_t r0
   b += sizeof(dev::StrMeta) * n * S->lstr.size() + 4 * n * S->pairs.size();
   for (int r : S->plan_rules[(size_t)plan]) {
     const dev::Rule& d = S->rules[(size_t)r]->d;
-    b += 12ull * n + 20ull * d.domain_l + 64 + 8 * ((d.domain_l + dev::kScanChunk - 1) / dev::kScanChunk + 1);
+    // an upper bound on the classes of left keys
+    const uint64_t keys_l = (uint64_t)d.domain * (d.n_sim && d.domain * 5ull <= (1ull << 22) ? 5 : 1);
+    b += 12ull * n + 20ull * keys_l + 64 + 8 * ((keys_l + dev::kScanChunk - 1) / dev::kScanChunk + 1);
   }
   b += 16 * n + (S->any_multi_rule ? 64 * n : 0) + 4096;  // output share (grows if needed)
   return b;
@@ -749,11 +750,13 @@ void launch_batch(hbx_server* S, Slot& B) {
   check_launch("serving batch encode");
 
   // ---- rule instances: (request, rule of its plan)
+  B.long_left = max_len > (int64_t)dev::kMaxTableLen;
   B.inst.clear();
   B.h_rules.clear();
   for (size_t q = 0; q < nq; q++)
     for (int r : S->plan_rules[(size_t)B.ents[q].r->plan]) {
-      const dev::Rule& t = S->rules[(size_t)r]->d;
+      dev::Rule t = S->rules[(size_t)r]->d;
+      dev::set_classes(&t, B.long_left);
       B.inst.emplace_back();
       Inst& I = B.inst.back();
       I.req = (uint32_t)q;
@@ -782,7 +785,7 @@ void launch_batch(hbx_server* S, Slot& B) {
   B.d_rules.alloc(ni);
   HBX_CUDA(cudaMemcpyAsync(B.d_rules.p, B.h_rules.data(), ni * sizeof(dev::Rule),
                            cudaMemcpyHostToDevice, st));
-  B.d_base.alloc(ni + 1);
+  B.d_base.alloc(dev::item_base_words(ni));
   B.d_cmp.alloc(ni);
   B.d_ctr.alloc(1);
   HBX_CUDA(cudaMemsetAsync(B.d_cmp.p, 0, ni * 8ull, st));
@@ -801,7 +804,7 @@ void launch_batch(hbx_server* S, Slot& B) {
     dev::k_items_final<<<I.nb_l, 1024, 0, st>>>(B.d_rules.p, i, S->tile_right, I.part_u64.p);
     if (n) k_scatter_left<<<grid_for(n, C->n_sm), 256, 0, st>>>(B.d_rules.p, i, row0, n, I.key_l.p);
   }
-  dev::k_rule_base<<<1, 32, 0, st>>>(B.d_rules.p, ni, B.d_base.p, nullptr);
+  dev::k_rule_base<<<1, 32, 0, st>>>(B.d_rules.p, ni, B.d_base.p);
   check_launch("serving batch join");
 
   B.capacity = std::max<uint64_t>(1 << 16, 2ull * N);
@@ -840,10 +843,15 @@ void launch_eval(hbx_server* S, Slot& B) {
   P.seen_mask = B.seen.p ? B.seen.n - 1 : 0;
   const int grid = S->ctx->n_sm * S->blocks_per_sm;
   dev::eval_kernel(S->variant, false, B.shape.w)<<<grid, kThreads, S->smem_bytes, st>>>(P);
+  if (B.long_left) {
+    P.rule_item_base += ni + 1;
+    dev::k_eval_long<<<dev::long_grid(S->ctx->n_sm), kThreads, 0, st>>>(P);
+  }
   check_launch("serving k_eval");
   uint8_t* h = (uint8_t*)B.h_ctr.p;
   HBX_CUDA(cudaMemcpyAsync(h, B.d_ctr.p, sizeof(dev::Counters), cudaMemcpyDeviceToHost, st));
-  HBX_CUDA(cudaMemcpyAsync(h + sizeof(dev::Counters), B.d_base.p + ni, 8, cudaMemcpyDeviceToHost, st));
+  HBX_CUDA(cudaMemcpyAsync(h + sizeof(dev::Counters), B.d_base.p + dev::item_base_words(ni) - 1, 8,
+                           cudaMemcpyDeviceToHost, st));
   HBX_CUDA(cudaMemcpyAsync(h + sizeof(dev::Counters) + 8, B.d_cmp.p, 8ull * ni,
                            cudaMemcpyDeviceToHost, st));
   HBX_CUDA(cudaEventRecord(B.ev_eval, st));

@@ -148,6 +148,7 @@ struct Layout {
   hbx::dev::PeqShape shape{};
   uint32_t* peq = nullptr;
   uint32_t tile_right = 128;
+  bool long_left = false;  // some left string has no Peq table (k_eval_long)
 };
 
 // Places the join state, the Peq tables and the counters after the encoded
@@ -157,6 +158,10 @@ void place(Carve& c, const hbx::Encoded& E, size_t smem_cap, Layout* Y) {
   namespace dev = hbx::dev;
   const uint32_t nL = (uint32_t)E.L.n_rows, nR = (uint32_t)E.R.n_rows;
   uint32_t max_len = 1;
+  for (const hbx::RuleEnc& re : E.rules)
+    for (int sl : re.sim_slot_l) max_len = std::max(max_len, E.L.str_maxlen[(size_t)sl]);
+  const bool long_left = max_len > dev::kMaxTableLen;
+  Y->long_left = long_left;
   Y->rules.assign(E.rules.size(), dev::Rule{});
   Y->nb.assign(E.rules.size(), 0);
   Y->nb_l.assign(E.rules.size(), 0);
@@ -176,24 +181,25 @@ void place(Carve& c, const hbx::Encoded& E, size_t smem_cap, Layout* Y) {
       d.sim_l[s] = (uint32_t)re.sim_slot_l[s];
       d.sim_r[s] = (uint32_t)re.sim_slot_r[s];
       d.thr[s] = re.thr[s];
-      max_len = std::max(max_len, E.L.str_maxlen[(size_t)re.sim_slot_l[s]]);
     }
     d.domain = (uint32_t)re.domain;
-    const bool split = !re.sim_slot_l.empty() &&
-                       re.domain * dev::kWordClasses <= (uint64_t)hbx::kMaxKeyDomain * 4;
-    d.n_wclass = split ? dev::kWordClasses : 1u;
-    d.wclass_slot = split ? (uint32_t)re.sim_slot_l[0] : 0u;
-    d.domain_l = d.n_wclass * d.domain;
+    dev::set_classes(&d, long_left);
+    // room for five classes of left keys where they stay below four times
+    // kMaxKeyDomain, else for one (which long left strings may double): the
+    // sizes that are refused do not depend on the classes in use
+    const uint64_t room_l =
+        d.n_sim && re.domain * 5 <= (uint64_t)hbx::kMaxKeyDomain * 4
+            ? re.domain * 5 : std::max<uint64_t>(re.domain, d.domain_l);
     dev::make_singleton(&d);
     d.key_l = c.take<uint32_t>(nL);
     d.key_r = c.take<uint32_t>(nR);
-    d.cnt_l = c.take<uint32_t>(d.domain_l);
+    d.cnt_l = c.take<uint32_t>(room_l);
     d.cnt_r = c.take<uint32_t>(d.domain);
-    d.off_l = c.take<uint32_t>(d.domain_l);
+    d.off_l = c.take<uint32_t>(room_l);
     d.off_r = c.take<uint32_t>(d.domain);
-    d.cur_l = c.take<uint32_t>(d.domain_l);
+    d.cur_l = c.take<uint32_t>(room_l);
     d.cur_r = c.take<uint32_t>(d.domain);
-    d.item_off = c.take<unsigned long long>((size_t)d.domain_l + 1);
+    d.item_off = c.take<unsigned long long>((size_t)room_l + 1);
     d.sorted_l = c.take<uint32_t>(nL);
     d.sorted_r = c.take<uint32_t>((size_t)nR + 4);
     d.sorted_meta_r = d.n_sim ? c.take<dev::StrMeta>(nR) : nullptr;
@@ -209,7 +215,7 @@ void place(Carve& c, const hbx::Encoded& E, size_t smem_cap, Layout* Y) {
   Y->part_u32 = c.take<uint32_t>(max_nb);
   Y->part_u64 = c.take<unsigned long long>(max_nb);
   Y->d_rules = c.take<dev::Rule>(E.rules.size());
-  Y->rule_base = c.take<unsigned long long>(E.rules.size() + 1);
+  Y->rule_base = c.take<unsigned long long>(dev::item_base_words(E.rules.size()));
   Y->ctr = c.take<dev::Counters>(1);
 }
 
@@ -343,7 +349,7 @@ void run_static(int device, const hbx_plan* plan, const hbx_table* left, const h
     if (nL) dev::k_scatter<<<grid_for(nL), 256, 0, st>>>(Y.L, Y.d_rules, ru, 0);
     if (nR) dev::k_scatter<<<grid_for(nR), 256, 0, st>>>(Y.R, Y.d_rules, ru, 1);
   }
-  dev::k_rule_base<<<1, 32, 0, st>>>(Y.d_rules, (uint32_t)Y.rules.size(), Y.rule_base, nullptr);
+  dev::k_rule_base<<<1, 32, 0, st>>>(Y.d_rules, (uint32_t)Y.rules.size(), Y.rule_base);
   const uint32_t n_slots = (uint32_t)E.L.str_maxlen.size();
   if (n_slots && nL)
     dev::k_peq_build<<<grid_for((uint32_t)std::min<uint64_t>((uint64_t)n_slots * nL * 32, 1u << 30)), 256, 0,
@@ -379,12 +385,17 @@ void run_static(int device, const hbx_plan* plan, const hbx_table* left, const h
   int bps = 0;
   HBX_STATIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, dev::kWarpsPerCta * 32, smem));
   kern<<<n_sm * std::max(1, bps), dev::kWarpsPerCta * 32, smem, st>>>(P);
+  if (Y.long_left) {
+    P.rule_item_base += P.n_rules + 1;
+    dev::k_eval_long<<<dev::long_grid(n_sm), dev::kWarpsPerCta * 32, 0, st>>>(P);
+  }
   HBX_STATIC_CUDA(cudaGetLastError());
 
   dev::Counters c{};
   unsigned long long total_items = 0;
   HBX_STATIC_CUDA(cudaMemcpyAsync(&c, Y.ctr, sizeof c, cudaMemcpyDeviceToHost, st));
-  HBX_STATIC_CUDA(cudaMemcpyAsync(&total_items, Y.rule_base + Y.rules.size(), 8,
+  HBX_STATIC_CUDA(cudaMemcpyAsync(&total_items,
+                                  Y.rule_base + dev::item_base_words(Y.rules.size()) - 1, 8,
                                   cudaMemcpyDeviceToHost, st));
   HBX_STATIC_CUDA(cudaStreamSynchronize(st));
   drain.armed = false;  // the stream is idle
