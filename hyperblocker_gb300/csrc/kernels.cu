@@ -949,6 +949,12 @@ __device__ __forceinline__ bool scan_begin(Scan<W>& z, const uint32_t* tab, cons
 // (the scan is complete: *m = the match count) or 2 (the pair cannot reach
 // the scan's threshold).
 constexpr int kScanQuadUnroll = 1;
+// A loop turn scans until fewer than this many lanes are still scanning, then
+// decides the finished pairs and hands out the next ones: deciding and
+// picking up cost as much as two to three scan steps, whether one lane or all
+// take part.  8 rules, 150k x 150k rows, evaluation: 13.97 ms with one step
+// per turn, 12.18, 11.75, 11.74, 11.59, 11.34 ms with 24, 20, 16, 12, 8 lanes.
+constexpr uint32_t kTurnLanes = 8;
 template <int W>
 __device__ __forceinline__ int scan_step(Scan<W>& z, uint32_t* m_out, WorkTally* ops) {
   constexpr int S = row_words(W);
@@ -1681,12 +1687,20 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
       }
     }
     head += min(n_idle, avail);
-    // every lane votes (a warp vote must be reached by all lanes of its mask)
-    const bool any_busy = __any_sync(kFull, busy);
-    if (lane == 0 && any_busy) ops->wsteps++;
+    // scan steps until fewer than kTurnLanes lanes are left scanning (or, when
+    // fewer had a pair, one of them is decided): every lane votes
+    uint32_t m = 0;
+    int sc = 0;
+    {
+      uint32_t on = __popc(__ballot_sync(kFull, busy));
+      const uint32_t few = min(on, kTurnLanes);
+      while (on && on >= few) {
+        if (lane == 0) ops->wsteps++;
+        if (busy && !sc) sc = scan_step<W>(z, &m, ops);
+        on = __popc(__ballot_sync(kFull, busy && !sc));
+      }
+    }
     if (busy) {
-      uint32_t m = 0;
-      const int sc = scan_step<W>(z, &m, ops);
       if (sc) {
         busy = false;
         int st = 0;
