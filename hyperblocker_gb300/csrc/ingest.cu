@@ -306,11 +306,8 @@ __global__ void k_pack(ColDev c, uint32_t n, const uint32_t* off16, const uint8_
     }
     __syncwarp();
     uint32_t sw = 0;  // signature word `lane` (lanes 0-7)
-    if (__any_sync(0xffffffffu, cnt[lane] > 255u)) {
-      sw = 0xffffffffu;
-    } else if (lane < 8) {
-      for (int k = 0; k < 4; k++) sw |= cnt[4 * lane + k] << (8 * k);
-    }
+    if (lane < 8)
+      for (int k = 0; k < 4; k++) sw |= min(cnt[4 * lane + k], 255u) << (8 * k);
     const uint32_t s = (lane < 16 && lane < len) ? sym[c.bytes[a + lane]] : 0u;
     uint32_t v = s << (8 * (lane & 3));
     v |= __shfl_xor_sync(0xffffffffu, v, 1);

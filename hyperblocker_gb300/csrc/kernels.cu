@@ -33,17 +33,22 @@ __global__ void k_keys_hist(Side S, const Rule* rules, uint32_t rule, int side) 
   }
 }
 
-// A right row's metadata as the join stores it in sorted_meta_r: the string
-// metadata of the rule's first similarity column, with the row's dictionary
-// codes of the group's first two extra equality slots in loc.z and loc.w
-// (unused words of the string record), so that the filter compares them
-// from the staged copy.
-__device__ __forceinline__ StrMeta sorted_meta(const Side& S, const Rule& Q, const StrMeta* meta_in,
-                                               uint32_t row) {
+// Stores a right row's metadata at position pos of sorted_meta_r (its pieces
+// turned, meta_turn): the string metadata of the rule's first similarity
+// column, with the row's dictionary codes of the group's first two extra
+// equality slots in loc.z and loc.w (unused words of the string record), so
+// that the filter compares them from the staged copy.
+__device__ __forceinline__ void store_meta(const Side& S, const Rule& Q, const StrMeta* meta_in,
+                                           uint32_t row, uint32_t pos) {
   StrMeta m = meta_in[row];
   if (Q.n_xslots > 0) m.loc.z = (uint32_t)S.eq_codes[(size_t)Q.xslot[0] * S.n_rows + row];
   if (Q.n_xslots > 1) m.loc.w = (uint32_t)S.eq_codes[(size_t)Q.xslot[1] * S.n_rows + row];
-  return m;
+  uint4* out = reinterpret_cast<uint4*>(Q.sorted_meta_r + pos);
+  const uint32_t t = meta_turn(pos);
+  out[t] = m.loc;
+  out[1u ^ t] = m.head;
+  out[2u ^ t] = m.sig[0];
+  out[3u ^ t] = m.sig[1];
 }
 
 __global__ void k_scatter(Side S, const Rule* rules, uint32_t rule, int side) {
@@ -60,7 +65,7 @@ __global__ void k_scatter(Side S, const Rule* rules, uint32_t rule, int side) {
     const uint32_t k = keys[row];
     const uint32_t pos = off[k] + atomicAdd(cur + k, 1u);
     sorted[pos] = row;
-    if (meta_out) meta_out[pos] = sorted_meta(S, R, meta_in, row);
+    if (meta_out) store_meta(S, R, meta_in, row, pos);
   }
 }
 
@@ -386,7 +391,7 @@ __global__ void k_join_scatter(Side L, Side R, const Rule* rules, uint32_t n_rul
       const uint32_t k = Q.key_r[row];
       const uint32_t pos = Q.off_r[k] + atomicAdd(Q.cur_r + k, 1u);
       Q.sorted_r[pos] = row;
-      if (Q.sorted_meta_r) Q.sorted_meta_r[pos] = sorted_meta(R, Q, meta_in, row);
+      if (Q.sorted_meta_r) store_meta(R, Q, meta_in, row, pos);
     }
   } else if (Q.n_members) {
     for (uint32_t row = t0; row < L.n_rows; row += stride) {
@@ -721,6 +726,14 @@ __device__ __forceinline__ unsigned long long jw_eval_ops(uint32_t ls, uint32_t 
   return 6ull * to * ((ls + 63u) >> 6) + 2ull * ((ls + 3u) >> 2) + 16ull;
 }
 
+// The same below 2^32 (shorter lengths up to kMaxTableLen: at most 384 * 4 * 6
+// + 144).
+__device__ __forceinline__ uint32_t jw_eval_ops32(uint32_t ls, uint32_t ll) {
+  const uint32_t h = (ls + 1u) >> 1;
+  const uint32_t to = min(ls + h, ll);
+  return 6u * to * ((ls + 63u) >> 6) + 2u * ((ls + 3u) >> 2) + 16u;
+}
+
 // One character step of the bit-parallel match count: x = the unmatched
 // positions of the left string equal to `sym` inside the window; the lowest
 // one becomes matched; the window [i - h, i + h] moves one position right
@@ -786,30 +799,34 @@ __device__ __forceinline__ void flush_pairs(const EvalParams& P, bool pass, uint
   }
 }
 
-// Upper bound on the Jaro matches of two strings from their count signatures
-// (dev::StrMeta): sum over buckets of the smaller count.
-__device__ __forceinline__ uint32_t sig_bound(const uint4& a0, const uint4& a1, const uint4& b0,
-                                              const uint4& b1) {
-  constexpr unsigned kOnes = 0x01010101u;
-  uint32_t s = 0;
-  s = __dp4a(__vminu4(a0.x, b0.x), kOnes, s);
-  s = __dp4a(__vminu4(a0.y, b0.y), kOnes, s);
-  s = __dp4a(__vminu4(a0.z, b0.z), kOnes, s);
-  s = __dp4a(__vminu4(a0.w, b0.w), kOnes, s);
-  s = __dp4a(__vminu4(a1.x, b1.x), kOnes, s);
-  s = __dp4a(__vminu4(a1.y, b1.y), kOnes, s);
-  s = __dp4a(__vminu4(a1.z, b1.z), kOnes, s);
-  s = __dp4a(__vminu4(a1.w, b1.w), kOnes, s);
-  return s;
+// Twice an upper bound on the Jaro matches of two strings of lengths la and lb
+// from their count signatures (dev::StrMeta): the lengths less the sum of the
+// counts' differences, one vabsdiff4 per word (four minima per word, summed,
+// take five times as many instructions: 123 against 42 issue slots for a
+// bound and its operands in a loop).
+__device__ __forceinline__ int sig_bound2(uint32_t la, uint32_t lb, const uint4& a0,
+                                          const uint4& a1, const uint4& b0, const uint4& b1) {
+  uint32_t d = 0;
+  auto add = [&d](uint32_t a, uint32_t b) {
+    asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %0;" : "+r"(d) : "r"(a), "r"(b));
+  };
+  add(a0.x, b0.x);
+  add(a0.y, b0.y);
+  add(a0.z, b0.z);
+  add(a0.w, b0.w);
+  add(a1.x, b1.x);
+  add(a1.y, b1.y);
+  add(a1.z, b1.z);
+  add(a1.w, b1.w);
+  return (int)(la + lb - d);
 }
 
 // Common prefix of two 16-symbol little-endian heads; 16 when they agree.
 __device__ __forceinline__ uint32_t prefix16(const uint4& a, const uint4& b) {
-  const uint32_t d[4] = {a.x ^ b.x, a.y ^ b.y, a.z ^ b.z, a.w ^ b.w};
-#pragma unroll
-  for (int k = 0; k < 4; k++)
-    if (d[k]) return 4u * k + ((uint32_t)(__ffs(d[k]) - 1) >> 3);
-  return 16u;
+  const uint32_t d0 = a.x ^ b.x, d1 = a.y ^ b.y, d2 = a.z ^ b.z, d3 = a.w ^ b.w;
+  const uint32_t d = d0 ? d0 : d1 ? d1 : d2 ? d2 : d3;  // the first word that differs
+  const uint32_t k = d0 ? 0u : d1 ? 4u : d2 ? 8u : 12u;
+  return k + ((uint32_t)__clz((int)__brev(d)) >> 3);  // 12 + 32 / 8 when none does
 }
 
 // Can a pair of non-empty strings whose left one has no Peq table reach thr?
@@ -819,16 +836,15 @@ __device__ __forceinline__ uint32_t prefix16(const uint4& a, const uint4& b) {
 // Longer strings than kReachMaxLen and prefixes of 16 and more are not
 // decided here.
 constexpr uint32_t kReachMaxLen = 1024;
-__device__ __forceinline__ bool can_reach(const StrMeta* am, const StrMeta* bm, uint32_t la,
-                                          uint32_t lb, float thr) {
+__device__ __forceinline__ bool can_reach(const StrMeta* am, const uint4& b_head, const uint4& b_s0,
+                                          const uint4& b_s1, uint32_t la, uint32_t lb, float thr) {
   const uint32_t ls = min(la, lb), ll = max(la, lb);
   if (ls > kReachMaxLen) return true;
-  const uint32_t p16 = prefix16(am->head, bm->head);
+  const uint32_t p16 = prefix16(am->head, b_head);
   if (p16 == 16u && ls > 16u) return true;
   const int need = m_need_lo(ls, ll, min(p16, ls), thr);
   if (need > (int)ls) return false;
-  return need <= 0 ||
-         (int)sig_bound(am->sig[0], am->sig[1], bm->sig[0], bm->sig[1]) >= need;
+  return need <= 0 || sig_bound2(la, lb, am->sig[0], am->sig[1], b_s0, b_s1) >= 2 * need;
 }
 
 // Slow exact similarity check of one pair (any lengths).  Out of line and
@@ -840,7 +856,7 @@ __device__ __noinline__ bool sim_pass_slow(const StrMeta* am, const StrMeta* bm,
   if (la == 0 || lb == 0) return jw_exact(0, la, lb, 0, thr, &ctr->ambiguous);
   const uint32_t mn = min(la, lb);
   if (mn > 256) atomicAdd(&ctr->long_pairs, 1ull);
-  if (!can_reach(am, bm, la, lb, thr)) return false;
+  if (!can_reach(am, bm->head, bm->sig[0], bm->sig[1], la, lb, thr)) return false;
   const uint32_t m = jaro_m_ref(a, la, b, lb);
   const uint32_t p = prefix_len(a, b, mn);
   return jw_exact(m, mn, max(la, lb), p, thr, &ctr->ambiguous);
@@ -1030,7 +1046,7 @@ __device__ __forceinline__ int advance_rule(const EvalParams& P, uint32_t rule, 
       const uint32_t n_iter = min(lb, la + ((ls + 1u) >> 1));
       if (need > (int)min(n_iter, ls)) return 0;
       if (need > 0 &&
-          (int)sig_bound(am->sig[0], am->sig[1], bm->sig[0], bm->sig[1]) < need)
+          sig_bound2(la, lb, am->sig[0], am->sig[1], bm->sig[0], bm->sig[1]) < 2 * need)
         return 0;
     }
     ops->rest++;
@@ -1119,7 +1135,8 @@ __device__ __forceinline__ int advance_group(const EvalParams& P, uint32_t rule,
         need = m_need_lo(ls, ll, p, thr);
         const uint32_t n_iter = min(lb, la + ((ls + 1u) >> 1));
         if (need > (int)min(n_iter, ls)) break;
-        if (need > 0 && (int)sig_bound(am->sig[0], am->sig[1], bm->sig[0], bm->sig[1]) < need)
+        if (need > 0 &&
+            sig_bound2(la, lb, am->sig[0], am->sig[1], bm->sig[0], bm->sig[1]) < 2 * need)
           break;
       }
       // member *mi may pass: one scan for it and the later members testing
@@ -1155,14 +1172,14 @@ constexpr uint32_t kItemSim = 1u, kItemExtras = 2u, kItemMore = 4u;  // more: n_
 __device__ __forceinline__ uint32_t item_members(uint32_t kind) { return (kind >> 8) & 15u; }
 // A claimed work item: the sources of its bulk copies (right-row metadata
 // from the block's first row, right rows from the 16-byte boundary at or
-// before it, the left string's metadata), left row, rule, rows, the shift of
-// the first row past the boundary, its kind and the group's smallest
-// first-column threshold.
+// before it, the left string's metadata), left row, rule, rows, the first
+// row's position in sorted_r modulo 8 (modulo 4: past the boundary; meta_turn
+// needs the rest), its kind and the group's smallest first-column threshold.
 struct ItemDesc {
   const StrMeta* meta_src;
   const uint32_t* rows_src;
   const StrMeta* lm_src;
-  uint32_t lrow, rule, n, shift, kind;
+  uint32_t lrow, rule, n, pos, kind, slot;
   float thr0;
   int32_t lcode[2];  // the left row's codes of the group's first two extra slots
 };
@@ -1174,15 +1191,17 @@ struct OutBuf {  // matches not yet written out (emit): fewer than 32 between ca
 struct WarpCtl {
   ItemDesc desc[kMaxClaimChunk];  // claimed items not yet staged
   uint32_t c_rule[kMaxStageBufs], c_lrow[kMaxStageBufs];  // claim per staging buffer
-  uint32_t c_n[kMaxStageBufs], c_shift[kMaxStageBufs];    // (n = 0: none)
-  uint32_t c_kind[kMaxStageBufs];
+  uint32_t c_n[kMaxStageBufs], c_pos[kMaxStageBufs];      // (n = 0: none)
+  uint32_t c_kind[kMaxStageBufs], c_slot[kMaxStageBufs];
   float c_thr[kMaxStageBufs];
   int32_t c_lcode[kMaxStageBufs][2];
   // the item being filtered; i_lcode: its left row's codes of the group's
   // extra equality slots
-  uint32_t i_rule, i_lrow, i_kind, i_all;
+  uint32_t i_rule, i_lrow, i_kind, i_all, i_slot;  // i_slot: its first column's left slot
   float i_thr;
   int32_t i_lcode[kMaxEq];
+  uint32_t i_live[4];  // its group's Rule::x_live, x_thr (groups with extra slots)
+  float i_xthr[4];
   OutBuf out;
 };
 static_assert(sizeof(WarpCtl) <= kWarpCtlWords * 4, "warp control block outgrows its words");
@@ -1234,37 +1253,49 @@ __device__ __forceinline__ void emit_drain(const EvalParams& P, OutBuf* O, int l
 // decided here, the rest go to the ring with their first 16 symbols.  Pairs
 // decided without a scan that pass go to the ring for their members' further
 // predicates, or match at once when a passing member has none.  lm: the
-// item's left string metadata.  Returns the entries appended.
+// item's left string metadata; pos0: the item's first position in sorted_r
+// modulo 8.  Returns the entries appended.
 // G: the launch has rule groups; without, every rule is its own group of one
 // and its predicates take the plain path (one threshold per predicate).
+//
+// A chain of shared-memory loads and arithmetic, every candidate pair once:
+// issue slots and shared-memory wavefronts bound it.  With the bound from
+// differences (sig_bound2), the records turned (meta_turn) and the group's
+// table in shared memory a batch takes 1,620 cycles of its warp against
+// 2,150 (8 rules, 150k x 150k rows; evaluation 9.90 against 11.34 ms) and
+// 1,130 against 1,690 without groups (2,601 x 64,264 rows; 145 against
+// 179 us).
 template <bool G>
 __device__ __forceinline__ uint32_t filter_batch(const EvalParams& P, WarpCtl* C,
                                                  const StrMeta* lm, const uint32_t* rows,
-                                                 const StrMeta* meta, uint32_t n, uint32_t e0,
-                                                 uint4* q, uint32_t tail, WorkTally* ops) {
+                                                 const StrMeta* meta, uint32_t pos0, uint32_t n,
+                                                 uint32_t e0, uint4* q, uint32_t tail,
+                                                 WorkTally* ops) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const uint32_t e = e0 + (uint32_t)lane;
   const bool act = e < n;
   const uint32_t rrow = act ? rows[e] : 0u;
   const uint32_t la = lm->loc.y, a_off = lm->loc.x;
-  const Rule* R = P.rules + C->i_rule;
   const uint32_t all = C->i_all;
   uint32_t live = act ? all : 0u;
   float thr = C->i_thr;
+  const uint4* rec = reinterpret_cast<const uint4*>(meta + e);
+  const uint32_t turn = meta_turn(pos0 + e);
   uint4 loc = make_uint4(0, 0, 0, 0), head = make_uint4(0, 0, 0, 0);
-  if (act) loc = meta[e].loc;
+  if (act) loc = rec[turn];
   if (G && act && (C->i_kind & kItemExtras)) {
     // the right row's codes of the extra slots: the first two staged with
-    // its metadata (sorted_meta), the others from device memory
+    // its metadata (store_meta), the others from device memory
     uint32_t eqm = 0;
-    const uint32_t nx = R->n_xslots;
+    const uint32_t nx = (C->i_kind >> 12) & 15u;
     if ((int32_t)loc.z == C->i_lcode[0]) eqm |= 1u;
     if (nx > 1 && (int32_t)loc.w == C->i_lcode[1]) eqm |= 2u;
     if (nx <= 2u) {  // the group's table (Rule::x_live, x_thr)
-      live = R->x_live[eqm];
-      if (live != all) thr = R->x_thr[eqm];
+      live = C->i_live[eqm];
+      if (live != all) thr = C->i_xthr[eqm];
     } else {
+      const Rule* R = P.rules + C->i_rule;
       for (uint32_t j = 2; j < nx; j++)
         if (P.R.eq_codes[(size_t)R->xslot[j] * P.R.n_rows + rrow] == C->i_lcode[j]) eqm |= 1u << j;
       for (uint32_t x = all; x; x &= x - 1) {
@@ -1274,41 +1305,38 @@ __device__ __forceinline__ uint32_t filter_batch(const EvalParams& P, WarpCtl* C
       if (live != all) thr = live_thr(R, live);
     }
   }
-  if (live) head = meta[e].head;
   uint32_t pass1 = 0;  // members that passed the first column without a scan
   bool scan = false;
   uint32_t p = 0;
   int need = 0;
   if (live) {
+    head = rec[1u ^ turn];
     const uint32_t lb = loc.y;
     if (la == 0 || lb == 0) {
       if constexpr (G)
-        pass1 = first_pass(R, live, 0, la, lb, 0, &P.ctr->ambiguous);
+        pass1 = first_pass(P.rules + C->i_rule, live, 0, la, lb, 0, &P.ctr->ambiguous);
       else
         pass1 = jw_exact(0, la, lb, 0, thr, &P.ctr->ambiguous) ? 1u : 0u;
     } else {
       const uint32_t ls = min(la, lb), ll = max(la, lb);
-      ops->ops += jw_eval_ops(ls, ll);
+      ops->ops += jw_eval_ops32(ls, ll);
       const uint32_t p16 = prefix16(lm->head, head);
       if (p16 == 16u && ls > 16u) {
         scan = true;  // prefix longer than 16: measured exactly before the scan
         p = kPrefixUnknown;
       } else {
+        // out of reach when the need is above the shorter length, or above
+        // what the count signatures leave
         p = min(p16, ls);
         need = m_need_lo(ls, ll, p, thr);
-        const uint32_t n_iter = min(lb, la + ((ls + 1u) >> 1));
-        scan = need <= (int)min(n_iter, ls);  // else the threshold is out of reach
-        // the count signatures bound the matches from above: below the need,
-        // the pair cannot pass
-        if (scan && need > 0 &&
-            (int)sig_bound(lm->sig[0], lm->sig[1], meta[e].sig[0], meta[e].sig[1]) < need)
-          scan = false;
+        scan = need <= (int)ls &&
+               sig_bound2(la, lb, lm->sig[0], lm->sig[1], rec[2u ^ turn], rec[3u ^ turn]) >= 2 * need;
       }
     }
   }
   bool done;
   if constexpr (G)
-    done = pass1 && member_done(R, pass1);
+    done = pass1 && member_done(P.rules + C->i_rule, pass1);
   else
     done = pass1 && !(C->i_kind & kItemMore);
   const bool push = scan || (pass1 && !done);
@@ -1321,7 +1349,7 @@ __device__ __forceinline__ uint32_t filter_batch(const EvalParams& P, WarpCtl* C
                               : (ring_tag(0, 0, 0, pass1, (uint32_t)__ffs(pass1) - 1u) | kAdvance);
     en[0] = make_uint4(rrow, loc.x, loc.y, tag);
     en[1] = head;
-    en[2] = scan ? make_uint4(lrow, la | (min(R->sim_l[0], 127u) << 9) | (C->i_rule << 16), a_off,
+    en[2] = scan ? make_uint4(lrow, la | (min(C->i_slot, 127u) << 9) | (C->i_rule << 16), a_off,
                               __float_as_uint(thr))
                  : make_uint4(lrow, la, a_off, C->i_rule);
   }
@@ -1465,7 +1493,8 @@ __device__ __forceinline__ uint32_t claim_chunk(const EvalParams& P, WarpCtl* C,
   d.lrow = lrow;
   d.rule = r;
   d.n = rb1 - rb0;
-  d.shift = rb0 - a0;
+  d.pos = rb0 & 7u;
+  d.slot = sim ? R.sim_l[0] : 0u;
   d.thr0 = sim ? R.thr_min : 0.0f;
   __syncwarp();  // earlier reads of the descriptors are done
   if ((uint32_t)lane < n) C->desc[lane] = d;
@@ -1504,7 +1533,7 @@ __device__ __forceinline__ void claim_item(const EvalParams& P, WarpCtl* C, uint
     if (!(d.kind & kItemSim)) {  // equalities only: every candidate matches
       for (uint32_t e = 0; e < d.n; e += 32) {
         const uint32_t k = e + (uint32_t)lane;
-        const uint32_t rrow = k < d.n ? d.rows_src[d.shift + k] : 0u;
+        const uint32_t rrow = k < d.n ? d.rows_src[(d.pos & 3u) + k] : 0u;
         emit(P, &C->out, k < d.n, d.lrow, rrow, lane);
       }
       (*done)++;
@@ -1512,7 +1541,7 @@ __device__ __forceinline__ void claim_item(const EvalParams& P, WarpCtl* C, uint
     }
     if (lane == 0) {
       const uint32_t mbytes = d.n * (uint32_t)sizeof(StrMeta);
-      const uint32_t rbytes = ((d.n + d.shift) * 4u + 15u) & ~15u;
+      const uint32_t rbytes = ((d.n + (d.pos & 3u)) * 4u + 15u) & ~15u;
       // earlier reads of this buffer are done (__syncwarp before the claim);
       // order them before the asynchronous writes
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1524,8 +1553,9 @@ __device__ __forceinline__ void claim_item(const EvalParams& P, WarpCtl* C, uint
     C->c_rule[b] = d.rule;
     C->c_lrow[b] = d.lrow;
     C->c_n[b] = d.n;
-    C->c_shift[b] = d.shift;
+    C->c_pos[b] = d.pos;
     C->c_kind[b] = d.kind;
+    C->c_slot[b] = d.slot;
     C->c_thr[b] = d.thr0;
     C->c_lcode[b][0] = d.lcode[0];
     C->c_lcode[b][1] = d.lcode[1];
@@ -1595,8 +1625,9 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
       if (active) {
         if (in_pos < cur_n) {
           tail += filter_batch<G>(P, C, reinterpret_cast<const StrMeta*>(buf + P.buf_lmeta_off),
-                               buf + P.buf_rows_off + C->c_shift[cb],
-                               reinterpret_cast<const StrMeta*>(buf), cur_n, in_pos, q, tail, ops);
+                                  buf + P.buf_rows_off + (C->c_pos[cb] & 3u),
+                                  reinterpret_cast<const StrMeta*>(buf), C->c_pos[cb], cur_n,
+                                  in_pos, q, tail, ops);
           in_pos += 32;
           continue;
         }
@@ -1632,9 +1663,13 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
       C->i_thr = thr;
       C->i_kind = kind;
       C->i_all = (1u << item_members(kind)) - 1u;
+      C->i_slot = C->c_slot[cb];
       if (G && (kind & kItemExtras)) {  // the left row's codes of the extra equality slots
         const uint32_t nx = (kind >> 12) & 15u;
-        if (lane < 2) {
+        if (lane >= 28) {
+          C->i_live[lane - 28] = P.rules[ir].x_live[lane - 28];
+          C->i_xthr[lane - 28] = P.rules[ir].x_thr[lane - 28];
+        } else if (lane < 2) {
           C->i_lcode[lane] = C->c_lcode[cb][lane];  // loaded with the claim
         } else if ((uint32_t)lane < nx) {
           const Rule* R = P.rules + ir;
@@ -1820,7 +1855,7 @@ __device__ __noinline__ bool long_pair_rest(const EvalParams& P, const Rule* R, 
           atomicAdd(&P.ctr->jw_word_ops, jw_eval_ops(mn, mx));
           if (mn > kMaxTableLen) atomicAdd(&P.ctr->long_pairs, 1ull);
         }
-        if (!can_reach(am, bm, la, lb, thr)) break;
+        if (!can_reach(am, bm->head, bm->sig[0], bm->sig[1], la, lb, thr)) break;
         const uint8_t* a = P.L.arena + 16ull * al.x;
         const uint8_t* b = P.R.arena + 16ull * bl.x;
         m = jaro_m_warp(a, la, b, lb);
@@ -1884,8 +1919,9 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_eval_long(
       const uint32_t e = e0 + (uint32_t)lane;
       const bool act = e < rb1;
       const uint32_t rrow = act ? R->sorted_r[e] : 0u;
-      const StrMeta* rm = R->sorted_meta_r + (act ? e : e0);
-      const uint4 loc = rm->loc;
+      const uint32_t at = act ? e : e0, turn = meta_turn(at);
+      const uint4* rm = reinterpret_cast<const uint4*>(R->sorted_meta_r + at);
+      const uint4 loc = rm[turn];
       const uint32_t lb = loc.y;
       uint32_t live = act ? all : 0u, pass1 = 0;
       if (act && nx) {  // members whose extra equalities hold
@@ -1907,7 +1943,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_eval_long(
         } else {
           word_ops += jw_eval_ops(min(la, lb), max(la, lb));
           if (lb > kMaxTableLen) atomicAdd(&P.ctr->long_pairs, 1ull);
-          count = can_reach(lm, rm, la, lb, live_thr(R, live));
+          count = can_reach(lm, rm[1u ^ turn], rm[2u ^ turn], rm[3u ^ turn], la, lb,
+                            live_thr(R, live));
         }
       }
       for (unsigned x = __ballot_sync(kFull, count); x; x &= x - 1) {

@@ -50,15 +50,14 @@ __host__ __device__ constexpr int row_words(int w) { return w <= 1 ? 1 : w <= 2 
 constexpr float kDecisionMargin = 1e-4f;  // |approx JW - thr| below this -> exact path
 
 // Count signature of a string: byte k (of 32) counts the string's symbols in
-// bucket k, where the 31 most frequent symbols have a bucket each and the
-// rest share the last one.  For any two strings a, b the Jaro match count
-// (any matching between equal symbols) is at most
-//     sum_k min(sig_a[k], sig_b[k]),
-// and pooling symbols into one bucket only raises that sum, so the bound is
-// exact.  A string with a count that does not fit a byte gets 0xff in every
-// bucket: min() then takes the other side's count, which still bounds the
-// matches from above (two such strings: 32 * 255, above every bound that is
-// asked for).
+// bucket k (at most 255), where the 31 most frequent symbols have a bucket
+// each and the rest share the last one.  For any two strings a, b the Jaro
+// match count (any matching between equal symbols) is at most
+//     sum_k min(count_a[k], count_b[k])
+//         = (len_a + len_b - sum_k |count_a[k] - count_b[k]|) / 2,
+// and pooling symbols into one bucket only raises that sum.  Counts cut off
+// at 255 only lower the differences, so the signatures still give an upper
+// bound.
 constexpr uint32_t kSigBuckets = 32;
 __host__ __device__ inline uint32_t sig_bucket(uint32_t sym) {  // sym >= 1
   return sym >= kSigBuckets ? kSigBuckets - 1 : sym - 1;
@@ -80,12 +79,17 @@ inline void make_sig(const uint8_t* s, uint32_t len, uint4 out[2]) {
   uint32_t c[kSigBuckets] = {0};
   for (uint32_t i = 0; i < len; i++)
     if (s[i]) c[sig_bucket(s[i])]++;
-  bool fits = true;
-  for (uint32_t k = 0; k < kSigBuckets; k++) fits = fits && c[k] <= 255u;
-  for (uint32_t k = 0; k < kSigBuckets; k++) w[k / 4] |= (fits ? c[k] : 255u) << (8 * (k % 4));
+  for (uint32_t k = 0; k < kSigBuckets; k++) w[k / 4] |= (c[k] < 255u ? c[k] : 255u) << (8 * (k % 4));
   out[0] = make_uint4(w[0], w[1], w[2], w[3]);
   out[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
+
+// A record of Rule::sorted_meta_r holds its four 16-byte pieces (loc, head,
+// sig[0], sig[1]) in an order that depends on its position: piece p of record
+// pos is at index p ^ meta_turn(pos).  Lanes that read the same piece of
+// consecutive records from shared memory then spread over all banks (in
+// record order they would use two of eight 16-byte columns).
+__host__ __device__ inline uint32_t meta_turn(uint32_t pos) { return (pos >> 1) & 3u; }
 
 struct Side {
   const uint32_t* bucket;
@@ -135,8 +139,9 @@ struct Rule {
   uint32_t* sorted_l;
   uint32_t* sorted_r;  // [n_rows + 4]: the tail pads 16-byte bulk copies
   // right-row string metadata of the first similarity predicate in sorted_r
-  // order, so that a work item's metadata is one contiguous, 16-byte-aligned
-  // block for a bulk copy into shared memory (null without similarities)
+  // order (the pieces of a record turned, meta_turn), so that a work item's
+  // metadata is one contiguous, 16-byte-aligned block for a bulk copy into
+  // shared memory (null without similarities)
   StrMeta* sorted_meta_r;
   // Group evaluation.  The work items of this rule's join are evaluated for
   // n_members rules at once: member 0 is this rule, the others are rules whose
@@ -254,7 +259,7 @@ constexpr uint32_t kMaxStageBufs = 4;
 struct WarpLayout {
   uint32_t n_bufs, buf_off, buf_words, buf_rows_off, buf_lmeta_off, mbar_off, ctl_off, warp_words;
 };
-constexpr uint32_t kWarpCtlWords = 400;  // the warp's control block (kernels.cu: WarpCtl)
+constexpr uint32_t kWarpCtlWords = 448;  // the warp's control block (kernels.cu: WarpCtl)
 
 inline WarpLayout warp_layout(uint32_t tile_right, uint32_t n_bufs) {
   WarpLayout w;
@@ -262,11 +267,12 @@ inline WarpLayout warp_layout(uint32_t tile_right, uint32_t n_bufs) {
   const uint32_t meta_words = (uint32_t)(sizeof(StrMeta) / 4) * tile_right;
   w.buf_rows_off = meta_words;
   w.buf_lmeta_off = meta_words + (tile_right + 8 + 3) / 4 * 4;
-  w.buf_words = w.buf_lmeta_off + (uint32_t)(sizeof(StrMeta) / 4);
+  // (64-byte multiples: a record's turned pieces stay inside it)
+  w.buf_words = (w.buf_lmeta_off + (uint32_t)(sizeof(StrMeta) / 4) + 15) / 16 * 16;
   w.buf_off = kRingWords * kRingEntries;
   w.mbar_off = w.buf_off + w.n_bufs * w.buf_words;
   w.ctl_off = w.mbar_off + (2 * w.n_bufs + 3) / 4 * 4;
-  w.warp_words = w.ctl_off + kWarpCtlWords;
+  w.warp_words = (w.ctl_off + kWarpCtlWords + 15) / 16 * 16;
   return w;
 }
 
