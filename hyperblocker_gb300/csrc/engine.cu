@@ -618,7 +618,8 @@ uint32_t enqueue_join(hbx_session* S, cudaStream_t st, bool groups) {
   launch_dependent(dev::k_join_count, dim3(row_blocks, (uint32_t)J.count.size()), dim3(256), smem,
                    st, S->side_l, S->side_r, rules, J.d_count.p);
   launch_dependent(dev::k_join_scan, dim3(n_blocks), dim3(1024), 0, st, rules, S->tile_right,
-                   J.d_scan.p, J.d_block_task.p, S->scan_sync.p, S->d_ctr.p);
+                   J.d_scan.p, J.d_block_task.p, S->scan_sync.p, &S->d_ctr.p->comparisons, 0u,
+                   S->d_ctr.p);
   launch_dependent(dev::k_join_scatter, dim3(row_blocks, (uint32_t)J.scatter.size()), dim3(256), 0,
                    st, S->side_l, S->side_r, rules, (uint32_t)S->rb.size(), J.d_scatter.p,
                    S->d_rule_base.p, S->d_ctr.p);

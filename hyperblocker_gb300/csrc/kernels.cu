@@ -285,7 +285,8 @@ constexpr uint32_t kScanWaitPolls = 1u << 20;
 // done, and every wait ends (bounded all the same: a wait that gives up
 // counts a watchdog trip, which fails the run).
 __global__ void k_join_scan(const Rule* rules, uint32_t tile_right, const ScanTask* tasks,
-                            const uint32_t* block_task, unsigned long long* sync, Counters* ctr) {
+                            const uint32_t* block_task, unsigned long long* sync,
+                            unsigned long long* comparisons, uint32_t cmp_stride, Counters* ctr) {
   __shared__ unsigned long long s_w64[32];
   __shared__ unsigned long long s_t64, s_base;
   __shared__ uint32_t s_chunk;
@@ -340,7 +341,8 @@ __global__ void k_join_scan(const Rule* rules, uint32_t tile_right, const ScanTa
     if (c + 1 == T.n_chunks && threadIdx.x == 0) Q.item_off[D] = base + chunk_total;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(kFull, pairs, o);
-    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&ctr->comparisons, pairs * Q.cmp_weight);
+    if ((threadIdx.x & 31) == 0 && pairs)
+      atomicAdd(comparisons + (size_t)T.rule * cmp_stride, pairs * Q.cmp_weight);
   } else {
     uint32_t* off = T.what == 1 ? Q.off_r : Q.off_l;
 #pragma unroll
@@ -349,25 +351,6 @@ __global__ void k_join_scan(const Rule* rules, uint32_t tile_right, const ScanTa
       ex += v[k];
     }
   }
-}
-
-// Writes the item bases (item_base_words); returns the number of all items.
-// A rule evaluated in another rule's group has no items of its own.
-__device__ __forceinline__ unsigned long long item_bases(const Rule* rules, uint32_t n_rules,
-                                                         unsigned long long* base) {
-  unsigned long long acc = 0, acc1 = 0;
-  for (uint32_t r = 0; r < n_rules; r++) {
-    base[r] = acc;
-    base[n_rules + 1 + r] = acc1;
-    if (!rules[r].n_members) continue;
-    const unsigned long long n0 = rules[r].item_off[rules[r].domain];
-    acc += n0;
-    acc1 += rules[r].item_off[rules[r].domain_l] - n0;
-  }
-  base[n_rules] = acc;
-  base[2 * n_rules + 1] = acc1;
-  base[2 * n_rules + 2] = acc + acc1;
-  return acc + acc1;
 }
 
 // Rows of every rule with work items grouped by key (counting-sort scatter,

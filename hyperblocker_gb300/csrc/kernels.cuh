@@ -369,6 +369,26 @@ __global__ void k_items_final(const Rule* rules, uint32_t rule, uint32_t tile_ri
 // first item of each rule, then their number), the same for class 1, then
 // the number of all items.
 inline size_t item_base_words(size_t n_rules) { return 2 * (n_rules + 1) + 1; }
+#ifdef __CUDACC__
+// Writes them; returns the number of all items.  A rule evaluated in another
+// rule's group has no items of its own.
+__device__ __forceinline__ unsigned long long item_bases(const Rule* rules, uint32_t n_rules,
+                                                         unsigned long long* base) {
+  unsigned long long acc = 0, acc1 = 0;
+  for (uint32_t r = 0; r < n_rules; r++) {
+    base[r] = acc;
+    base[n_rules + 1 + r] = acc1;
+    if (!rules[r].n_members) continue;
+    const unsigned long long n0 = rules[r].item_off[rules[r].domain];
+    acc += n0;
+    acc1 += rules[r].item_off[rules[r].domain_l] - n0;
+  }
+  base[n_rules] = acc;
+  base[2 * n_rules + 1] = acc1;
+  base[2 * n_rules + 2] = acc + acc1;
+  return acc + acc1;
+}
+#endif
 __global__ void k_rule_base(const Rule* rules, uint32_t n_rules, unsigned long long* base);
 // One launch for a run's resets: the counters and histograms to 0, the
 // duplicate set (n_seen slots, may be 0) to empty.
@@ -396,8 +416,11 @@ struct ScanTask {
   uint32_t rule, what, first_block, n_chunks;
 };
 __global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* tasks);
+// comparisons: rule r's pair-comparisons are added to comparisons[r *
+// cmp_stride].
 __global__ void k_join_scan(const Rule* rules, uint32_t tile_right, const ScanTask* tasks,
-                            const uint32_t* block_task, unsigned long long* sync, Counters* ctr);
+                            const uint32_t* block_task, unsigned long long* sync,
+                            unsigned long long* comparisons, uint32_t cmp_stride, Counters* ctr);
 __global__ void k_join_scatter(Side L, Side R, const Rule* rules, uint32_t n_rules,
                                const uint32_t* tasks, unsigned long long* rule_base,
                                Counters* ctr);
