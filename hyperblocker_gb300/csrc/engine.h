@@ -16,7 +16,10 @@ void run_to_host(hbx_session* s, hbx_mode mode, std::vector<uint32_t>* l, std::v
 // does not overflow and repeat.
 void reserve_output(hbx_session* s, uint64_t pairs);
 struct Table;
-// sort.cu: sorts n device pairs by (left row, right row) in place.
+// sort.cu: sorts n device pairs by (left row, right row) in place; the first
+// form queues it on st.
+void queue_pair_sort(int n_sm, cudaStream_t st, uint32_t* l, uint32_t* r, uint64_t n,
+                     uint32_t n_left, uint32_t n_right);
 void sort_pairs_device(hbx_ctx* ctx, uint32_t* l, uint32_t* r, uint64_t n, uint32_t n_left,
                        uint32_t n_right);
 // writer.cu: appends the id lines of n device pairs to path.

@@ -95,14 +95,13 @@ __global__ void __launch_bounds__(kThreads) k_scatter(const unsigned long long* 
 
 }  // namespace srt
 
-// Sorts n pairs by (left row, right row) in place; rows below n_left /
-// n_right (the bytes of the keys beyond them are 0 and take no pass).
-void sort_pairs_device(hbx_ctx* C, uint32_t* l, uint32_t* r, uint64_t n, uint32_t n_left,
-                       uint32_t n_right) {
+// Queues the sort of n pairs by (left row, right row) in place on st; rows
+// below n_left / n_right (the bytes of the keys beyond them are 0 and take no
+// pass).  Its buffers come from the calling thread's pool on st.
+void queue_pair_sort(int n_sm, cudaStream_t st, uint32_t* l, uint32_t* r, uint64_t n,
+                     uint32_t n_left, uint32_t n_right) {
   if (n < 2) return;
   if (n >= (1ull << 32)) fail(HBX_ERR_UNSUPPORTED, "more than 2^32 pairs to sort");
-  cudaStream_t st = C->stream;
-  PoolScope scope(C->pool, st);
   auto bytes_of = [](uint32_t rows) {
     uint32_t b = 0;
     while (b < 4 && (uint64_t)rows > (1ull << (8 * b))) b++;
@@ -112,7 +111,7 @@ void sort_pairs_device(hbx_ctx* C, uint32_t* l, uint32_t* r, uint64_t n, uint32_
   DBuf<unsigned long long> a, b;
   a.alloc(n);
   b.alloc(n);
-  const int g = grid_for(n, C->n_sm);
+  const int g = grid_for(n, n_sm);
   srt::k_pack<<<g, 256, 0, st>>>(l, r, n, a.p);
   const uint32_t n_tiles = (uint32_t)((n + srt::kTile - 1) / srt::kTile);
   const uint64_t nh = 256ull * n_tiles;
@@ -134,7 +133,14 @@ void sort_pairs_device(hbx_ctx* C, uint32_t* l, uint32_t* r, uint64_t n, uint32_
   }
   srt::k_unpack<<<g, 256, 0, st>>>(src, n, l, r);
   check_launch("pair sort");
-  HBX_CUDA(cudaStreamSynchronize(st));
+}
+
+// The same on the context's stream; returns when the pairs are sorted.
+void sort_pairs_device(hbx_ctx* C, uint32_t* l, uint32_t* r, uint64_t n, uint32_t n_left,
+                       uint32_t n_right) {
+  PoolScope scope(C->pool, C->stream);
+  queue_pair_sort(C->n_sm, C->stream, l, r, n, n_left, n_right);
+  HBX_CUDA(cudaStreamSynchronize(C->stream));
 }
 
 }  // namespace hbx
