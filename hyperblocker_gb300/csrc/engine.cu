@@ -272,6 +272,13 @@ void list_join(const std::vector<dev::Rule>& rules, JoinLists* J, cudaStream_t s
   J->d_scan.upload(J->scan, st);
 }
 
+// Do rules of the array share all their candidates (dev::Rule::dup_always)?
+bool overlap(const std::vector<dev::Rule>& rules) {
+  for (const dev::Rule& d : rules)
+    if (d.n_members && d.dup_always) return true;
+  return false;
+}
+
 // Classes of left rows of the session's rules (dev::Rule).
 uint32_t n_classes(const hbx_session* S) { return S->long_left ? 2u : 1u; }
 
@@ -337,6 +344,7 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
     d.sorted_r = b.sorted_r.p;
     d.sorted_meta_r = d.n_sim ? b.sorted_meta_r.p : nullptr;
   }
+  dev::set_overlaps(S->h_rules.data(), S->h_rules.size());
   S->h_groups = group_rules(S->h_rules);
   S->groups = false;
   for (const dev::Rule& g : S->h_groups)
@@ -424,16 +432,19 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
       }
   S->bound_idx.upload(idx, st);
   S->bound_val.alloc(idx.size());
-  // output slots (and the duplicate set, twice as many) for the caller's
-  // capacity, but never more than the partitions can hold: a generous caller
-  // buffer does not size device buffers by itself
+  // output slots for the caller's capacity, but never more than the
+  // partitions can hold: a generous caller buffer does not size device buffers
+  // by itself.  The duplicate set: twice as many where rules may share every
+  // pair (load factor at most one half), else a quarter (dev::set_overlaps;
+  // a run that needs more repeats with a set of the size it asked for)
   const uint64_t cap0 =
       std::max<uint64_t>(1 << 16, std::min<uint64_t>(S->out_hint, E.pairs_covered + 1));
   S->out_l.alloc(cap0);
   S->out_r.alloc(cap0);
   if (E.rules.size() > 1) {
     uint64_t slots = 1 << 17;
-    while (slots < 2 * cap0) slots *= 2;  // load factor at most one half
+    const uint64_t want = overlap(S->h_groups) ? 2 * cap0 : cap0 / 4;
+    while (slots < want) slots *= 2;
     S->seen.alloc(slots);
   }
   HBX_CUDA(cudaEventCreate(&S->ev0));
@@ -586,6 +597,7 @@ std::vector<dev::Rule> group_rules(const std::vector<dev::Rule>& singles) {
       }
     g[keep].cmp_weight = 1 + rest;
   }
+  dev::set_overlaps(g.data(), n);
   return g;
 }
 
@@ -711,23 +723,26 @@ void grow_output(hbx_session* S, uint64_t need) {
   while (cap < need) cap *= 2;
   S->out_l.alloc(cap);
   S->out_r.alloc(cap);
-  if (S->seen.p) {
-    uint64_t slots = S->seen.n;
-    while (slots < 2 * cap) slots *= 2;  // load factor stays at or below one half
-    if (slots != S->seen.n) S->seen.alloc(slots);
-  }
   if (S->graph) {
     cudaGraphExecDestroy(S->graph);
     S->graph = nullptr;
   }
 }
 
-// Output pairs a repeated run must have room for: the distinct pairs of a
-// run whose output overflowed, or (duplicate set full) its pass count.
-uint64_t needed_capacity(const hbx_session* S, const dev::Counters& c) {
-  uint64_t need = c.out_count;
-  if (c.seen_overflow) need = std::max<uint64_t>(need, c.passes);
-  return std::max<uint64_t>(need, S->out_l.n + 1);
+// Distinct pairs of a run; with a full duplicate set an upper bound (its
+// reports, and all that it might have reported besides).
+uint64_t pair_count(const dev::Counters& c) {
+  return c.out_count + (c.seen_overflow ? c.passes : 0);
+}
+
+// A run's output or duplicate set was too small: room for its pairs.
+void grow_output(hbx_session* S, const dev::Counters& c) {
+  const uint64_t need = pair_count(c);
+  if (need > S->out_l.n) grow_output(S, need);
+  if (c.seen_overflow) {
+    S->seen_pairs = std::max<uint64_t>(S->seen_pairs, c.passes);
+    fit_seen(S, S->seen_pairs);
+  }
 }
 
 // Queues the copy of the counters (with the run's work-item total) into the
@@ -981,7 +996,7 @@ void autotune(hbx_session* S, cudaStream_t st) {
           S->seen_pairs = std::max<uint64_t>(2 * S->seen_pairs, c.passes);
           fit_seen(S, S->seen_pairs);
         } else {
-          grow_output(S, needed_capacity(S, c));
+          grow_output(S, c);
         }
         ms = timed_batched_run(S, st, &flush);
       }
@@ -1061,6 +1076,8 @@ void session_run(hbx_session* S, hbx_mode mode, cudaStream_t st) {
   if (!S->tuned && mode == HBX_MODE_BATCHED) autotune(S, st);
 
   uint32_t launches = 0;
+  if (mode == HBX_MODE_PLAIN && overlap(S->h_rules))
+    S->seen_pairs = std::max<uint64_t>(S->seen_pairs, std::min(out_cap(S), S->E.pairs_covered));
   fit_seen(S, S->seen_pairs);
   for (int attempt = 0; attempt < 8; attempt++) {
     dev::Counters c = run_once(S, mode, st, &launches);  // returns with the stream idle
@@ -1095,27 +1112,27 @@ void session_run(hbx_session* S, hbx_mode mode, cudaStream_t st) {
       fail(HBX_ERR_CUDA, "evaluation finished " + std::to_string(c.items_done) + " of " +
                              std::to_string(total_items) + " work items");
     if (c.seen_overflow == 0)
-      S->seen_pairs = std::max<uint64_t>(S->seen_pairs, c.out_count + c.out_count / 4);
+      S->seen_pairs = std::max<uint64_t>(S->seen_pairs, c.passes + c.passes / 4);
     if (c.out_count <= out_cap(S) && c.seen_overflow == 0) return;
+    if (c.seen_overflow)  // for the repeat, or the next run after a count
+      S->seen_pairs = std::max<uint64_t>(2 * S->seen_pairs, c.passes);
     if (S->ext_l) {
       // the caller's buffer: a result larger than it is only counted; a
       // full duplicate set is grown and the run repeated
-      if (c.out_count > S->ext_cap || (c.seen_overflow && c.passes > S->ext_cap)) {
-        S->stats.n_matches = c.seen_overflow ? std::max<uint64_t>(c.out_count, c.passes) : c.out_count;
+      if (c.out_count > S->ext_cap) {
+        S->stats.n_matches = pair_count(c);
         return;
       }
-      S->seen_pairs = std::max<uint64_t>(2 * S->seen_pairs, c.passes);
       fit_seen(S, S->seen_pairs);
       continue;
     }
-    const uint64_t need = needed_capacity(S, c);
-    if (S->cap_limit && need > S->cap_limit) {
+    if (S->cap_limit && c.out_count > S->cap_limit) {
       // the caller's buffer is too small anyway: report the count (an upper
       // bound when the duplicate set overflowed) instead of running again
-      S->stats.n_matches = c.seen_overflow ? std::max<uint64_t>(c.out_count, c.passes) : c.out_count;
+      S->stats.n_matches = pair_count(c);
       return;
     }
-    grow_output(S, need);
+    grow_output(S, c);
   }
   fail(HBX_ERR_CAPACITY, "output kept growing");
 }
@@ -1123,7 +1140,7 @@ void session_run(hbx_session* S, hbx_mode mode, cudaStream_t st) {
 void reserve_output(hbx_session* S, uint64_t pairs) {
   PoolScope scope(S->ctx->pool, S->ctx->stream);
   if (pairs > S->out_l.n) grow_output(S, pairs);
-  S->seen_pairs = std::max<uint64_t>(S->seen_pairs, pairs);
+  if (overlap(S->h_groups)) S->seen_pairs = std::max<uint64_t>(S->seen_pairs, pairs);
 }
 
 void run_to_host(hbx_session* S, hbx_mode mode, std::vector<uint32_t>* l, std::vector<uint32_t>* r) {
@@ -1404,6 +1421,7 @@ hbx_status hbx_internal_block_to_file(hbx_ctx* ctx, const hbx_plan* plan, const 
   auto S = std::make_unique<hbx_session>();
   S->ctx = ctx;
   S->one_shot = true;
+  S->out_hint = 1 << 22;  // 32 MiB: room for most results at the first run
   hbx_session* s = S.get();
   hbx_status st = guard(ctx, [&] {
     if (prefix_idx != INT_MAX && (prefix_idx < 0 || prefix_idx > INT_MAX))

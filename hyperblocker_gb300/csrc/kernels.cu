@@ -729,15 +729,27 @@ __device__ __forceinline__ void bp_step(const uint32_t* __restrict__ tab, uint32
   bp_update<W, S>(pe, win, mt, grow);
 }
 
-// First report of a pair?  With several rules a pair can match more than one
-// of them (the reference stops at the first rule that passes,
-// global_func.cuh:161-165); a device hash set of emitted (left, right) keys
-// keeps exactly one report.  Open addressing with linear probing over
+// May another rule of the launch report the pair too (Rule::dup_slot)?
+__device__ __forceinline__ bool shared_pair(const EvalParams& P, const Rule* R, uint32_t lrow,
+                                            uint32_t rrow) {
+  bool any = R->dup_always != 0;
+  for (uint32_t k = 0; k < R->n_dup && !any; k++) {
+    const size_t a = R->dup_slot[k][0], b = R->dup_slot[k][1];
+    any = P.L.eq_codes[a * P.L.n_rows + lrow] == P.R.eq_codes[a * P.R.n_rows + rrow] &&
+          (a == b || P.L.eq_codes[b * P.L.n_rows + lrow] == P.R.eq_codes[b * P.R.n_rows + rrow]);
+  }
+  return any;
+}
+
+// First report of a pair that several rules may report?  With several rules a
+// pair can match more than one of them (the reference stops at the first rule
+// that passes, global_func.cuh:161-165); a device hash set of emitted (left,
+// right) keys keeps exactly one report.  Open addressing with linear probing over
 // seen_mask + 1 slots (all ones = empty).  The set is sized for a load of at
 // most one half, where probe runs stay far below kMaxProbes; a run past it
 // means the set is too small for this run's distinct pairs: seen_overflow is
 // set, the host repeats the run with a set sized from the pass count
-// (Counters::passes, an upper bound on the distinct pairs).  Reports whose
+// (Counters::passes, an upper bound on the distinct pairs of the set).  Reports whose
 // probe run reaches kCheckProbe look at the overflow flag first and give up
 // once it is set, so an overflowing run costs a few probes per report; runs
 // of a set sized as intended rarely get that far and never read the flag.
@@ -758,15 +770,22 @@ __device__ __forceinline__ bool first_report(const EvalParams& P, uint32_t lrow,
   return false;
 }
 
-// Writes up to one match per lane to the output with one atomic per warp
-// (after the duplicate set, when the launch has one).
+// Writes up to one match per lane to the output with one atomic per warp,
+// the matches that another rule may report too after the duplicate set.  Most
+// matches of rules with different equalities are no other rule's candidates:
+// two loads each instead of a probe of a set larger than L2, which also had to
+// be cleared and, in a first run, grown (8 rules in two groups, 150k x 150k
+// rows, 7.9M matches: a run's reset and join 118 against 158 us; 30k x 30k
+// rows, the first run of a session 0.96 against 3.8 ms).
 __device__ __forceinline__ void flush_pairs(const EvalParams& P, bool pass, uint32_t lrow,
-                                            uint32_t rrow, int lane) {
+                                            uint32_t rrow, uint32_t rule, int lane) {
   if (P.seen) {
-    const unsigned cm = __ballot_sync(kFull, pass);
-    if (!cm) return;
-    if (lane == 0) atomicAdd(&P.ctr->passes, (unsigned long long)__popc(cm));
-    if (pass) pass = first_report(P, lrow, rrow);
+    const bool shared = pass && shared_pair(P, P.rules + rule, lrow, rrow);
+    const unsigned cm = __ballot_sync(kFull, shared);
+    if (cm) {
+      if (lane == 0) atomicAdd(&P.ctr->passes, (unsigned long long)__popc(cm));
+      if (shared) pass = first_report(P, lrow, rrow);
+    }
   }
   const unsigned pm = __ballot_sync(kFull, pass);
   if (!pm) return;
@@ -1169,6 +1188,7 @@ struct ItemDesc {
 constexpr uint32_t kOutBuf = 64;  // matches a warp holds before writing them out
 struct OutBuf {  // matches not yet written out (emit): fewer than 32 between calls
   uint2 pair[kOutBuf];
+  uint32_t rule[kOutBuf];
   uint32_t n;
 };
 struct WarpCtl {
@@ -1194,11 +1214,15 @@ static_assert(sizeof(WarpCtl) <= kWarpCtlWords * 4, "warp control block outgrows
 // reservation pay their round trips once per 32 matches instead of once per
 // step with a match.
 __device__ __forceinline__ void emit(const EvalParams& P, OutBuf* O, bool pass, uint32_t lrow,
-                                     uint32_t rrow, int lane) {
+                                     uint32_t rrow, uint32_t rule, int lane) {
   const unsigned pm = __ballot_sync(kFull, pass);
   if (!pm) return;
   const uint32_t n0 = O->n;
-  if (pass) O->pair[n0 + __popc(pm & ((1u << lane) - 1u))] = make_uint2(lrow, rrow);
+  if (pass) {
+    const uint32_t at = n0 + __popc(pm & ((1u << lane) - 1u));
+    O->pair[at] = make_uint2(lrow, rrow);
+    O->rule[at] = rule;
+  }
   const uint32_t n = n0 + __popc(pm);
   __syncwarp();
   if (n < 32) {
@@ -1207,13 +1231,18 @@ __device__ __forceinline__ void emit(const EvalParams& P, OutBuf* O, bool pass, 
     return;
   }
   const uint2 e = O->pair[lane];
+  const uint32_t er = O->rule[lane];
   const bool more = (uint32_t)lane + 32u < n;
   const uint2 t = more ? O->pair[32 + lane] : make_uint2(0u, 0u);
+  const uint32_t tr = more ? O->rule[32 + lane] : 0u;
   __syncwarp();
-  if (more) O->pair[lane] = t;
+  if (more) {
+    O->pair[lane] = t;
+    O->rule[lane] = tr;
+  }
   if (lane == 0) O->n = n - 32u;
   __syncwarp();
-  flush_pairs(P, true, e.x, e.y, lane);
+  flush_pairs(P, true, e.x, e.y, er, lane);
 }
 
 // Writes out the matches emit still holds (at the end of the warp's loop).
@@ -1221,10 +1250,11 @@ __device__ __forceinline__ void emit_drain(const EvalParams& P, OutBuf* O, int l
   const uint32_t n = O->n;
   const bool have = (uint32_t)lane < n;
   const uint2 e = have ? O->pair[lane] : make_uint2(0u, 0u);
+  const uint32_t er = have ? O->rule[lane] : 0u;
   __syncwarp();
   if (lane == 0) O->n = 0;
   __syncwarp();
-  flush_pairs(P, have, e.x, e.y, lane);
+  flush_pairs(P, have, e.x, e.y, er, lane);
 }
 
 // Filter one batch of 32 right rows of the item against its group's first
@@ -1336,7 +1366,7 @@ __device__ __forceinline__ uint32_t filter_batch(const EvalParams& P, WarpCtl* C
                               __float_as_uint(thr))
                  : make_uint4(lrow, la, a_off, C->i_rule);
   }
-  emit(P, &C->out, done, lrow, rrow, lane);
+  emit(P, &C->out, done, lrow, rrow, C->i_rule, lane);
   return __popc(qm);
 }
 
@@ -1517,7 +1547,7 @@ __device__ __forceinline__ void claim_item(const EvalParams& P, WarpCtl* C, uint
       for (uint32_t e = 0; e < d.n; e += 32) {
         const uint32_t k = e + (uint32_t)lane;
         const uint32_t rrow = k < d.n ? d.rows_src[(d.pos & 3u) + k] : 0u;
-        emit(P, &C->out, k < d.n, d.lrow, rrow, lane);
+        emit(P, &C->out, k < d.n, d.lrow, rrow, d.rule, lane);
       }
       (*done)++;
       continue;
@@ -1767,7 +1797,7 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
         }
       }
     }
-    emit(P, &C->out, fin && pass, lrow, rrow, lane);
+    emit(P, &C->out, fin && pass, lrow, rrow, rule, lane);
     if (!__any_sync(kFull, busy) && head == tail && !active && cur_n == 0) break;
   }
   emit_drain(P, &C->out, lane);
@@ -1945,7 +1975,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_eval_long(
                                        __shfl_sync(kFull, rrow, src));
         if (lane == src) match = ok;
       }
-      emit(P, O, match, lrow, rrow, lane);
+      emit(P, O, match, lrow, rrow, r, lane);
     }
     done++;
   }

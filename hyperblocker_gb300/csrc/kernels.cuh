@@ -105,6 +105,7 @@ struct Side {
 // the group root's (bits of Rule::xslot), and its other similarity
 // predicates in evaluation order.
 constexpr uint32_t kMaxMembers = 8;
+constexpr uint32_t kMaxDup = 4;
 struct Member {
   float thr_first;
   uint32_t xmask;
@@ -169,6 +170,12 @@ struct Rule {
   // looks them up instead of walking the members for every pair.
   uint32_t x_live[4];
   float x_thr[4];
+  // A pair can be reported by another rule of the launch too only where that
+  // rule's equalities also hold.  dup_always: it may at any pair (or there are
+  // more such rules than kMaxDup); else entry k: another rule and up to two of
+  // its equality slots that this rule's do not imply (set_overlaps).
+  uint32_t dup_always, n_dup;
+  uint32_t dup_slot[kMaxDup][2];
 };
 
 // Host: fills Rule::x_live / x_thr from the members, with the device's
@@ -193,6 +200,7 @@ inline void fill_extras_table(Rule* g) {
 inline void make_singleton(Rule* d) {
   d->n_members = 1;
   d->cmp_weight = 1;
+  d->dup_always = d->n_dup = 0;
   d->n_xslots = 0;
   Member& m = d->mem[0];
   m = Member{};
@@ -206,6 +214,34 @@ inline void make_singleton(Rule* d) {
   }
   d->thr_min = m.thr_first;
   fill_extras_table(d);
+}
+
+// Host: fills dup_always and dup_slot of the rules [0, n) that are evaluated
+// (those with members) over the same rows.
+inline void set_overlaps(Rule* rules, size_t n) {
+  auto has = [](const Rule& r, uint32_t slot) {
+    for (uint32_t e = 0; e < r.n_eq; e++)
+      if (r.eq_slot[e] == slot) return true;
+    return false;
+  };
+  for (size_t g = 0; g < n; g++) {
+    Rule& G = rules[g];
+    G.dup_always = G.n_dup = 0;
+    for (size_t h = 0; h < n && G.n_members; h++) {
+      const Rule& H = rules[h];
+      if (h == g || !H.n_members) continue;
+      uint32_t extra[2], k = 0;  // a slot may come twice: no harm
+      for (uint32_t e = 0; e < H.n_eq && k < 2; e++)
+        if (!has(G, H.eq_slot[e])) extra[k++] = H.eq_slot[e];
+      if (k == 0 || G.n_dup == kMaxDup) {
+        G.dup_always = 1;
+        break;
+      }
+      G.dup_slot[G.n_dup][0] = extra[0];
+      G.dup_slot[G.n_dup][1] = extra[k - 1];
+      G.n_dup++;
+    }
+  }
 }
 
 constexpr uint32_t kMaxTableLen = 256;
@@ -259,7 +295,7 @@ constexpr uint32_t kMaxStageBufs = 4;
 struct WarpLayout {
   uint32_t n_bufs, buf_off, buf_words, buf_rows_off, buf_lmeta_off, mbar_off, ctl_off, warp_words;
 };
-constexpr uint32_t kWarpCtlWords = 448;  // the warp's control block (kernels.cu: WarpCtl)
+constexpr uint32_t kWarpCtlWords = 512;  // the warp's control block (kernels.cu: WarpCtl)
 
 inline WarpLayout warp_layout(uint32_t tile_right, uint32_t n_bufs) {
   WarpLayout w;
@@ -298,7 +334,7 @@ struct Counters {
   unsigned long long items_done;
   unsigned long long jw_word_ops;  // algorithmic work of the JW evaluations
   unsigned long long seen_overflow;  // nonzero: the duplicate set had no room (run repeats)
-  unsigned long long passes;  // rule-level passes before de-duplication (plans with several rules)
+  unsigned long long passes;  // matches taken through the duplicate set (first_report)
   unsigned long long scans;       // pairs that reached a bit-parallel scan
   unsigned long long scan_steps;  // scan steps of 4 symbols
   unsigned long long items_total; // work items of the run (written by the join)
@@ -332,7 +368,8 @@ struct EvalParams {
   unsigned long long capacity;
   Counters* ctr;
   unsigned long long watchdog_cycles;  // 0 = no budget
-  // set of reported (left, right) keys when the plan has several rules, else null
+  // set of the reported (left, right) keys that another rule may report too
+  // (plans with several rules, else null)
   unsigned long long* seen;
   unsigned long long seen_mask;  // slots - 1 (a power of two minus one)
 };

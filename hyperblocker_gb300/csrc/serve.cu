@@ -604,6 +604,13 @@ void open_server(hbx_server* S, const hbx_plan* const* plans, int32_t n_plans, c
       S->rules.push_back(std::move(T));
     }
   }
+  // the rules of one plan run over the same request rows
+  for (const std::vector<int>& pr : S->plan_rules) {
+    std::vector<dev::Rule> v;
+    for (int r : pr) v.push_back(S->rules[(size_t)r]->d);
+    dev::set_overlaps(v.data(), v.size());
+    for (size_t k = 0; k < pr.size(); k++) S->rules[(size_t)pr[k]]->d = v[k];
+  }
   // a request batch's longest left string picks the mask width: the grid is
   // sized by the width with the fewest resident blocks
   S->blocks_per_sm = 1 << 20;
@@ -982,7 +989,7 @@ bool progress(hbx_server* S, Slot& B) {
       // grow and evaluate again (the join is unchanged)
       PoolScope scope(S->ctx->pool, B.st);
       uint64_t cap = B.capacity;
-      const uint64_t need = c.seen_overflow ? std::max<uint64_t>(c.out_count, c.passes) : c.out_count;
+      const uint64_t need = c.out_count + (c.seen_overflow ? c.passes : 0);
       while (cap < need || cap == B.capacity) cap *= 2;
       B.capacity = cap;
       B.out_l.alloc(cap);

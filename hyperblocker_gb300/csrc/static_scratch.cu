@@ -191,6 +191,7 @@ void place(Carve& c, const hbx::Encoded& E, size_t smem_cap, Layout* Y) {
         d.n_sim && re.domain * 5 <= (uint64_t)hbx::kMaxKeyDomain * 4
             ? re.domain * 5 : std::max<uint64_t>(re.domain, d.domain_l);
     dev::make_singleton(&d);
+    d.dup_always = E.rules.size() > 1 ? 1u : 0u;  // the set is sized for every report
     d.key_l = c.take<uint32_t>(nL);
     d.key_r = c.take<uint32_t>(nR);
     d.cnt_l = c.take<uint32_t>(room_l);

@@ -33,3 +33,50 @@ def test_domains_at_chunk_edges(ctx, n_keys, docs):
         got, st = hb.block(ctx, plan, left, right, 1, _util.INT_MAX, mode)
         assert np.array_equal(_util.sorted_pairs(got), want.pairs), mode
         assert st.pair_comparisons == want.pair_comparisons, mode
+
+
+def _rule8(eq_cols, sims):
+    return synth.rule_yaml(eq_cols, sims).replace("[0, 0, 1, 2, 3, 4]", "[0, 0, 1, 2, 3, 4, 5, 6, 7]") \
+        .replace("[1, 0, 1, 2, 3, 4]", "[1, 0, 1, 2, 3, 4, 5, 6, 7]")
+
+
+# rules that share pairs only where the other's equalities hold: one slot, two,
+# more than the two that are compared, the same ones, and more rules than are
+# listed (every pair then goes through the duplicate set)
+ROOTS = [
+    [([3], 1), ([4], 2)],
+    [([3], 1), ([4, 5], 1), ([5, 6, 7], 2)],
+    [([3], 1), ([3], 2), ([4], 1)],
+    [([], 1), ([4], 2)],
+    [([3], 1), ([4], 2), ([5], 1), ([6], 2), ([7], 1), ([3, 5], 2)],
+]
+
+
+@pytest.mark.parametrize("thr", [0.55, 0.0])
+@pytest.mark.parametrize("roots", range(len(ROOTS)))
+def test_pairs_of_several_rules_are_reported_once(built, roots, thr):
+    """At threshold 0 a quarter to all of 350,000 pairs match, more than the
+    first run's duplicate set holds."""
+    rng = np.random.Generator(np.random.PCG64(roots))
+    cl, cr = _util.random_tables(40 + roots, 499, 701, b"abc", 9, n_eq_values=2)
+    for t, n in ((cl, 499), (cr, 701)):
+        for k in (2, 3, 2):
+            t.append([b"k"] + [b"%d" % int(x) for x in rng.integers(0, k, size=n)])
+    docs = [_rule8(eq, [(col, thr)]) for eq, col in ROOTS[roots]]
+    want = api.run_block(api.CTable(cl), api.CTable(cr), rules.serialize(rules.sort_rules(
+        [rules.decode_rule(rules.parse_yaml(d)) for d in docs])), 1)
+    c = hb.Context(0)
+    plan = hb.Plan.from_yaml(docs, c)
+    left, right = hb.Table.from_columns(cl, c), hb.Table.from_columns(cr, c)
+    for mode in ("plain", "batched"):
+        got, st = hb.block(c, plan, left, right, 1, _util.INT_MAX, mode)
+        assert np.array_equal(_util.sorted_pairs(got), want.pairs), mode
+        assert st.pair_comparisons == want.pair_comparisons, mode
+    got, _ = hb.block_streamed(c, plan, left, right, 1, 1 << 18)
+    assert np.array_equal(_util.sorted_pairs(got), want.pairs)
+    with hb.Server(c, [plan], right) as srv:
+        srv.submit(1, 0, [col[1:] for col in cl])
+        got = srv.poll(20000)["pairs"]
+    served = want.pairs[want.pairs[:, 0] > 0] - np.array([1, 0], np.uint32)
+    assert np.array_equal(got, served)
+    c.close()
