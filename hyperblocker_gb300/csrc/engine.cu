@@ -51,8 +51,9 @@ struct RuleBufs {
 struct JoinLists {
   std::vector<uint32_t> count, scatter, block_task;
   std::vector<dev::ScanTask> scan;
-  DBuf<uint32_t> d_count, d_scatter, d_block_task;
-  DBuf<dev::ScanTask> d_scan;
+  // in hbx_session::lists
+  const uint32_t *d_count = nullptr, *d_scatter = nullptr, *d_block_task = nullptr;
+  const dev::ScanTask* d_scan = nullptr;
   uint64_t n_counts = 0;
 };
 
@@ -84,7 +85,8 @@ struct hbx_session {
   hbx::DBuf<uint32_t> counts;
   hbx::DBuf<unsigned long long> scan_sync;  // chunk totals and tickets (k_join_scan)
   hbx::JoinLists join_rules, join_groups;   // the joins of h_rules and of h_groups
-  hbx::DBuf<uint32_t> bound_idx;              // per rule, n_partitions + 1 key indices
+  hbx::DBuf<uint32_t> lists;                  // join tasks and bound_idx (upload_lists)
+  const uint32_t* bound_idx = nullptr;        // per rule, n_partitions + 1 key indices
   hbx::DBuf<unsigned long long> bound_val;    // item_off at those keys
   hbx::dev::Side side_l{}, side_r{};
   uint32_t warp_words = 4;
@@ -241,8 +243,8 @@ void launch_dependent(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, c
   HBX_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...));
 }
 
-// The join tasks of a rule array, uploaded on st.
-void list_join(const std::vector<dev::Rule>& rules, JoinLists* J, cudaStream_t st) {
+// The join tasks of a rule array.
+void list_join(const std::vector<dev::Rule>& rules, JoinLists* J) {
   for (uint32_t r = 0; r < (uint32_t)rules.size(); r++) {
     const dev::Rule& d = rules[r];
     if (!d.n_members) {
@@ -266,10 +268,39 @@ void list_join(const std::vector<dev::Rule>& rules, JoinLists* J, cudaStream_t s
       J->scan.push_back(t);
     }
   }
-  J->d_count.upload(J->count, st);
-  J->d_scatter.upload(J->scatter, st);
-  J->d_block_task.upload(J->block_task, st);
-  J->d_scan.upload(J->scan, st);
+}
+
+// Uploads both rule arrays' join tasks and the partition boundaries `bounds`
+// in one copy on st, from the returned words (to be kept until it is done).
+std::vector<uint32_t> upload_lists(hbx_session* S, const std::vector<uint32_t>& bounds,
+                                   cudaStream_t st) {
+  std::vector<uint32_t> all;
+  auto add = [&](const void* p, size_t words) {
+    const size_t at = all.size();
+    all.resize(at + (words + 3) / 4 * 4);  // 16-byte aligned pieces
+    if (words) std::memcpy(all.data() + at, p, words * 4);
+    return at;
+  };
+  size_t at[2][4];
+  JoinLists* lists[2] = {&S->join_rules, &S->join_groups};
+  for (int k = 0; k < 2; k++) {
+    const JoinLists& J = *lists[k];
+    at[k][0] = add(J.count.data(), J.count.size());
+    at[k][1] = add(J.scatter.data(), J.scatter.size());
+    at[k][2] = add(J.block_task.data(), J.block_task.size());
+    at[k][3] = add(J.scan.data(), J.scan.size() * sizeof(dev::ScanTask) / 4);
+  }
+  const size_t at_bounds = add(bounds.data(), bounds.size());
+  S->lists.upload(all, st);
+  for (int k = 0; k < 2; k++) {
+    JoinLists& J = *lists[k];
+    J.d_count = S->lists.p + at[k][0];
+    J.d_scatter = S->lists.p + at[k][1];
+    J.d_block_task = S->lists.p + at[k][2];
+    J.d_scan = reinterpret_cast<const dev::ScanTask*>(S->lists.p + at[k][3]);
+  }
+  S->bound_idx = S->lists.p + at_bounds;
+  return all;
 }
 
 // Do rules of the array share all their candidates (dev::Rule::dup_always)?
@@ -387,8 +418,8 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
       g.cur_r = d.cur_r;
     }
   }
-  list_join(S->h_rules, &S->join_rules, st);
-  list_join(S->h_groups, &S->join_groups, st);
+  list_join(S->h_rules, &S->join_rules);
+  list_join(S->h_groups, &S->join_groups);
   S->scan_sync.alloc(S->join_rules.block_task.size() + S->join_rules.scan.size());
   S->d_rules.alloc(E.rules.size());
   S->d_groups.alloc(E.rules.size());
@@ -430,7 +461,7 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
         const uint32_t cc = std::min<uint32_t>(c, S->h_rules[r].n_classes - 1);
         idx.push_back(cc * S->h_rules[r].domain + (uint32_t)E.rules[r].part_key_begin[p]);
       }
-  S->bound_idx.upload(idx, st);
+  const std::vector<uint32_t> lists = upload_lists(S, idx, st);
   S->bound_val.alloc(idx.size());
   // output slots for the caller's capacity, but never more than the
   // partitions can hold: a generous caller buffer does not size device buffers
@@ -452,7 +483,7 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
   HBX_CUDA(cudaEventCreate(&S->ev_eval0));
   HBX_CUDA(cudaEventCreate(&S->ev_eval1));
   uint64_t h2d = h2d_tables;
-  h2d += S->d_rules.n * sizeof(dev::Rule) + S->bound_idx.n * 4;
+  h2d += S->d_rules.n * sizeof(dev::Rule) + idx.size() * 4;
   S->stats.h2d_bytes = h2d;
   HBX_CUDA(cudaStreamSynchronize(st));
   S->stats.pairs_covered = E.pairs_covered;
@@ -628,12 +659,12 @@ uint32_t enqueue_join(hbx_session* S, cudaStream_t st, bool groups) {
   const size_t smem = std::min<uint32_t>(max_d, dev::kSharedHistKeys) * sizeof(uint32_t);
   const int row_blocks = row_grid(std::max(S->side_l.n_rows, S->side_r.n_rows), S->ctx->n_sm);
   launch_dependent(dev::k_join_count, dim3(row_blocks, (uint32_t)J.count.size()), dim3(256), smem,
-                   st, S->side_l, S->side_r, rules, J.d_count.p);
+                   st, S->side_l, S->side_r, rules, J.d_count);
   launch_dependent(dev::k_join_scan, dim3(n_blocks), dim3(1024), 0, st, rules, S->tile_right,
-                   J.d_scan.p, J.d_block_task.p, S->scan_sync.p, &S->d_ctr.p->comparisons, 0u,
+                   J.d_scan, J.d_block_task, S->scan_sync.p, &S->d_ctr.p->comparisons, 0u,
                    S->d_ctr.p);
   launch_dependent(dev::k_join_scatter, dim3(row_blocks, (uint32_t)J.scatter.size()), dim3(256), 0,
-                   st, S->side_l, S->side_r, rules, (uint32_t)S->rb.size(), J.d_scatter.p,
+                   st, S->side_l, S->side_r, rules, (uint32_t)S->rb.size(), J.d_scatter,
                    S->d_rule_base.p, S->d_ctr.p);
   launch_check("join kernels");
   return 4;
@@ -801,7 +832,7 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
   const uint32_t per_rule = per_class * n_classes(S);
   const uint32_t total = n_rules * per_rule;
   k_gather_bounds<<<(total + 255) / 256, 256, 0, st>>>(S->d_rules.p, n_rules, per_rule,
-                                                       S->bound_idx.p, S->bound_val.p);
+                                                       S->bound_idx, S->bound_val.p);
   n++;
   launch_check("k_gather_bounds");
   std::vector<unsigned long long> bounds(total), base(dev::item_base_words(n_rules));

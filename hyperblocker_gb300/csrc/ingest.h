@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <string>
+#include <vector>
 
 #include "device_buffers.h"
 #include "encode.h"
@@ -45,20 +46,47 @@ __device__ __forceinline__ uint32_t cell_len(const ColDev& c, uint32_t i, int64_
   return n;
 }
 
-__global__ void k_dict_insert(ColDev c, uint32_t n, uint32_t gid_base, unsigned long long* keys,
-                              uint32_t* rep, uint32_t mask, uint32_t* row_slot,
-                              unsigned long long* sum, unsigned long long seed);
-__global__ void k_occupied(const unsigned long long* keys, uint32_t cap, uint32_t* occ);
-__global__ void k_dict_assign(ColDev c, uint32_t n, uint32_t gid_base, const uint32_t* row_slot,
-                              const uint32_t* code, const uint32_t* rep, ColDev cl, ColDev cr,
-                              uint32_t n_left, int32_t* out, unsigned long long* sum);
+// Work of several columns in one launch (blockIdx.y over the entries): the
+// encoder's kernels are short, so small tables are bound by their number.
+//
+// A joint dictionary of two columns (n_left and n_right rows; the right one
+// alone with n_left = 0): its open-addressing table, codes and their number
+// (cleared by the caller, like keys to kEmpty).
+struct DictJob {
+  ColDev l, r;
+  int32_t *out_l, *out_r;
+  unsigned long long* keys;
+  uint32_t *code, *rep;
+  unsigned long long* card;
+};
+constexpr uint32_t kDictBatch = 8;
+struct DictBatch {
+  DictJob job[kDictBatch];
+  uint32_t n_left, n_right, mask;
+};
+__global__ void k_dict_insert(const __grid_constant__ DictBatch B, unsigned long long* sum,
+                              unsigned long long seed);
+__global__ void k_dict_assign(const __grid_constant__ DictBatch B, unsigned long long* sum);
+// One string column: its cells' arena units, then its symbols and metadata.
+struct StrJob {
+  ColDev c;
+  uint32_t n;
+  uint32_t* units;
+  const uint32_t* off16;
+  uint8_t* arena;
+  dev::StrMeta* meta;
+  unsigned long long* maxlen;
+};
+constexpr uint32_t kStrBatch = 8;
+struct StrBatch {
+  StrJob job[kStrBatch];
+};
 __global__ void k_scan_total(const uint32_t* scan, const uint32_t* in, uint32_t n,
                              unsigned long long extra, unsigned long long* dst);
-__global__ void k_byte_hist(ColDev c, uint32_t n, unsigned long long* hist);
+__global__ void k_byte_hist(const __grid_constant__ StrBatch B, unsigned long long* hist);
 __global__ void k_symbol_map(const unsigned long long* hist, uint8_t* sym, unsigned long long* sum);
-__global__ void k_units(ColDev c, uint32_t n, uint32_t* units);
-__global__ void k_pack(ColDev c, uint32_t n, const uint32_t* off16, const uint8_t* sym_g,
-                       uint8_t* arena, dev::StrMeta* meta, unsigned long long* maxlen);
+__global__ void k_units(const __grid_constant__ StrBatch B);
+__global__ void k_pack(const __grid_constant__ StrBatch B, const uint8_t* sym_g);
 
 }  // namespace ing
 
@@ -66,9 +94,22 @@ __global__ void k_pack(ColDev c, uint32_t n, const uint32_t* off16, const uint8_
 int grid_for(uint64_t n, int n_sm, int per_sm = 8);
 // Fails with HBX_ERR_CUDA if the last launch failed.
 void check_launch(const char* what);
-// Exclusive scan of n >= 1 u32 values into out (the join's scan kernels);
-// its scratch comes from the current pool (or arena).
+// Exclusive scan of n >= 1 u32 values into out; its scratch comes from the
+// current pool (or arena).
 void scan_u32(const uint32_t* in, uint32_t n, uint32_t* out, cudaStream_t st);
+
+// Launches over any number of string columns, kStrBatch at a time: the byte
+// histogram (work: the most 16-byte chunks or rows of a column), the arena
+// units, the arenas and metadata.
+void byte_hist(const std::vector<ing::StrJob>& jobs, uint64_t work, unsigned long long* hist,
+               int n_sm, cudaStream_t st);
+void str_units(const std::vector<ing::StrJob>& jobs, int n_sm, cudaStream_t st);
+void str_pack(const std::vector<ing::StrJob>& jobs, const uint8_t* sym, int n_sm, cudaStream_t st);
+// Joint dictionaries of a batch (its first n_jobs): clears the tables (keys:
+// one block of n_jobs tables) and builds them.
+void build_dictionaries(const ing::DictBatch& B, uint32_t n_jobs, unsigned long long* keys,
+                        unsigned long long* sum, unsigned long long seed, int n_sm,
+                        cudaStream_t st);
 
 // Seed of the dictionaries' first hash; a rebuild after a collision uses
 // kDictSeed + attempt.  With the environment variable

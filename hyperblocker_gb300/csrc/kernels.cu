@@ -98,6 +98,74 @@ __device__ __forceinline__ T block_excl_scan(T v, T* s_warp, T* total) {
   return r;
 }
 
+constexpr unsigned long long kScanFlag = 1ull << 63;
+constexpr uint32_t kScanWaitPolls = 1u << 20;
+
+// Adds the totals of the chunks before chunk c to *s_base (shared, cleared by
+// thread 0 before), a thread per chunk; every thread of the block calls it and
+// *s_base is complete when it returns.  false: a wait of this thread gave up.
+__device__ __forceinline__ bool scan_lookback(unsigned long long* totals, uint32_t c,
+                                              unsigned long long* s_base) {
+  bool ok = true;
+  if (c) {
+    __syncthreads();  // *s_base is 0
+    if ((threadIdx.x & ~31u) < c) {  // whole warps
+      unsigned long long t = 0;
+      for (uint32_t j = threadIdx.x; j < c; j += blockDim.x) {
+        unsigned long long f = 0;
+        uint32_t polls = 0;
+        while (!((f = atomicAdd(totals + j, 0ull)) & kScanFlag) && ++polls < kScanWaitPolls)
+          __nanosleep(64);
+        ok = ok && (f & kScanFlag);
+        t += f & ~kScanFlag;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+      if ((threadIdx.x & 31) == 0) atomicAdd(s_base, t);
+    }
+  }
+  __syncthreads();
+  return ok;
+}
+
+__global__ void k_scan_once_u32(const uint32_t* in, uint32_t n, uint32_t* out,
+                                unsigned long long* sync) {
+  __shared__ uint32_t s_warp[32];
+  __shared__ uint32_t s_total, s_chunk;
+  __shared__ unsigned long long s_base;
+  if (threadIdx.x == 0) s_chunk = (uint32_t)atomicAdd(sync + gridDim.x, 1ull);
+  __syncthreads();
+  const uint32_t c = s_chunk;
+  const uint64_t base = (uint64_t)c * kScanChunk + threadIdx.x * 4u;
+  uint32_t v[4], sum = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    v[k] = base + k < n ? in[base + k] : 0u;
+    sum += v[k];
+  }
+  uint32_t ex = block_excl_scan<uint32_t>(sum, s_warp, &s_total);
+  if (threadIdx.x == 0) {
+    s_base = 0;
+    __threadfence();
+    atomicExch(sync + c, s_total | kScanFlag);
+  }
+  const bool ok = scan_lookback(sync, c, &s_base);
+  if (__syncthreads_or(!ok)) {  // a wait gave up: the values themselves
+    if (threadIdx.x == 0) s_base = 0;
+    __syncthreads();
+    unsigned long long t = 0;
+    for (uint64_t k = threadIdx.x; k < (uint64_t)c * kScanChunk; k += blockDim.x) t += in[k];
+    atomicAdd(&s_base, t);
+    __syncthreads();
+  }
+  ex += (uint32_t)s_base;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    if (base + k < n) out[base + k] = ex;
+    ex += v[k];
+  }
+}
+
 __global__ void k_scan_partial_u32(const uint32_t* in, uint32_t n, uint32_t* partial) {
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_total;
@@ -273,9 +341,6 @@ __device__ __forceinline__ unsigned long long join_scan_value(const Rule& Q, uin
   return (what == 1 ? Q.cnt_r : Q.cnt_l)[k];
 }
 
-constexpr unsigned long long kScanFlag = 1ull << 63;
-constexpr uint32_t kScanWaitPolls = 1u << 20;
-
 // The scans of every rule with work items (ScanTask), one block of 1024
 // threads per chunk of kScanChunk keys, in one launch.  A block takes its
 // chunk from its task's ticket counter when it starts, publishes the chunk's
@@ -312,24 +377,7 @@ __global__ void k_join_scan(const Rule* rules, uint32_t tile_right, const ScanTa
     __threadfence();
     atomicExch(totals + c, chunk_total | kScanFlag);
   }
-  if (c) {  // the chunks before this one
-    __syncthreads();  // s_base is 0
-    if ((threadIdx.x & ~31u) < c) {  // whole warps
-      unsigned long long t = 0;
-      for (uint32_t j = threadIdx.x; j < c; j += blockDim.x) {
-        unsigned long long f = 0;
-        uint32_t polls = 0;
-        while (!((f = atomicAdd(totals + j, 0ull)) & kScanFlag) && ++polls < kScanWaitPolls)
-          __nanosleep(64);
-        if (!(f & kScanFlag)) atomicAdd(&ctr->watchdog_trips, 1ull);
-        t += f & ~kScanFlag;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
-      if ((threadIdx.x & 31) == 0) atomicAdd(&s_base, t);
-    }
-  }
-  __syncthreads();
+  if (!scan_lookback(totals, c, &s_base)) atomicAdd(&ctr->watchdog_trips, 1ull);
   const unsigned long long base = s_base;
   ex += base;
   if (T.what == 2) {

@@ -397,6 +397,13 @@ __global__ void k_scan_partial_u32(const uint32_t* in, uint32_t n, uint32_t* par
 __global__ void k_scan_top_u32(uint32_t* partial, uint32_t nb);
 __global__ void k_scan_final_u32(const uint32_t* in, uint32_t n, const uint32_t* partial,
                                  uint32_t* out);
+// The same in one launch for up to kScanOnceChunks chunks: a block per chunk
+// (taken from a ticket) adds the totals of the chunks before its own, as
+// k_join_scan does; sync: one word per chunk and the ticket, zero before the
+// launch.
+constexpr uint32_t kScanOnceChunks = 2048;
+__global__ void k_scan_once_u32(const uint32_t* in, uint32_t n, uint32_t* out,
+                                unsigned long long* sync);
 __global__ void k_items_partial(const Rule* rules, uint32_t rule, uint32_t tile_right,
                                 unsigned long long* partial, unsigned long long* comparisons);
 __global__ void k_scan_top_u64(unsigned long long* partial, uint32_t nb);

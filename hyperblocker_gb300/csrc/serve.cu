@@ -388,12 +388,13 @@ void pack_strings(const std::vector<ing::ColDev>& cols, const std::vector<uint64
   DBuf<uint32_t> units, off16;
   units.alloc(ns * n);
   off16.alloc(ns * n);
+  std::vector<ing::StrJob> jobs;
   for (size_t s = 0; s < ns; s++)
-    ing::k_units<<<grid_for(n, n_sm), 256, 0, st>>>(cols[s], n, units.p + s * n);
+    jobs.push_back(ing::StrJob{cols[s], n, units.p + s * n, off16.p + s * n, B->arena.p,
+                               B->meta.p + s * n, maxlen + s});
+  str_units(jobs, n_sm, st);
   scan_u32(units.p, (uint32_t)(ns * n), off16.p, st);
-  for (size_t s = 0; s < ns; s++)
-    ing::k_pack<<<grid_for((uint64_t)n * 32, n_sm), 256, 0, st>>>(
-        cols[s], n, off16.p + s * n, sym, B->arena.p, B->meta.p + s * n, maxlen + s);
+  str_pack(jobs, sym, n_sm, st);
   check_launch("serving string arenas");
 }
 
@@ -476,24 +477,16 @@ void open_server(hbx_server* S, const hbx_plan* const* plans, int32_t n_plans, c
     D.keys.alloc(D.cap);
     D.rep.alloc(D.cap);
     D.code.alloc(D.cap);
-    HBX_CUDA(cudaMemsetAsync(D.keys.p, 0xff, (size_t)D.cap * 8, st));
-    HBX_CUDA(cudaMemsetAsync(D.rep.p, 0xff, (size_t)D.cap * 4, st));
-    DBuf<uint32_t> row_slot, occ;
-    row_slot.alloc(std::max<uint32_t>(nR, 1));
-    occ.alloc(D.cap);
     codes_of_col.emplace_back();
     codes_of_col.back().alloc(std::max<uint32_t>(nR, 1));
     const ing::ColDev rc = S->rcols[pr.second].view();
-    if (nR)
-      ing::k_dict_insert<<<grid_for(nR, C->n_sm), 256, 0, st>>>(rc, nR, 0, D.keys.p, D.rep.p,
-                                                                 D.cap - 1, row_slot.p, sum.p,
-                                                                 kDictSeed);
-    ing::k_occupied<<<grid_for(D.cap, C->n_sm), 256, 0, st>>>(D.keys.p, D.cap, occ.p);
-    scan_u32(occ.p, D.cap, D.code.p, st);
-    if (nR)
-      ing::k_dict_assign<<<grid_for(nR, C->n_sm), 256, 0, st>>>(
-          rc, nR, 0, row_slot.p, D.code.p, D.rep.p, rc, rc, nR, codes_of_col.back().p, sum.p);
-    ing::k_scan_total<<<1, 32, 0, st>>>(D.code.p, occ.p, D.cap, 0, sum.p + ing::kSumFixed);
+    ing::DictBatch B{};
+    B.n_right = nR;
+    B.mask = D.cap - 1;
+    B.job[0] = ing::DictJob{rc, rc, nullptr, codes_of_col.back().p, D.keys.p, D.code.p, D.rep.p,
+                            sum.p + ing::kSumFixed};
+    HBX_CUDA(cudaMemsetAsync(sum.p + ing::kSumFixed, 0, 8, st));
+    build_dictionaries(B, 1, D.keys.p, sum.p, kDictSeed, C->n_sm, st);
     check_launch("serving dictionary");
     unsigned long long card = 0, flags = 0;
     HBX_CUDA(cudaMemcpyAsync(&card, sum.p + ing::kSumFixed, 8, cudaMemcpyDeviceToHost, st));
@@ -516,10 +509,15 @@ void open_server(hbx_server* S, const hbx_plan* const* plans, int32_t n_plans, c
   S->sym.alloc(256);
   S->lut.alloc(256);
   HBX_CUDA(cudaMemsetAsync(bhist.p, 0, 256 * 8, st));
-  for (int c : S->rstr) {
-    const Column& col = TR.cols[(size_t)c];
-    const uint64_t work = col.has_nul ? nR : (col.bytes.size() + 15) / 16;
-    if (nR) ing::k_byte_hist<<<grid_for(work, C->n_sm, 4), 256, 0, st>>>(S->rcols[c].view(), nR, bhist.p);
+  {
+    std::vector<ing::StrJob> jobs;
+    uint64_t work = 1;
+    for (int c : S->rstr) {
+      const Column& col = TR.cols[(size_t)c];
+      work = std::max<uint64_t>(work, col.has_nul ? nR : (col.bytes.size() + 15) / 16);
+      jobs.push_back(ing::StrJob{S->rcols[c].view(), nR, nullptr, nullptr, nullptr, nullptr, nullptr});
+    }
+    byte_hist(jobs, work, bhist.p, C->n_sm, st);
   }
   ing::k_symbol_map<<<1, 256, 0, st>>>(bhist.p, S->sym.p, sum.p);
   unsigned long long ns = 1;
