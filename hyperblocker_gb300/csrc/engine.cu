@@ -1050,6 +1050,74 @@ void autotune(hbx_session* S, cudaStream_t st) {
 
 }  // namespace
 
+// Counts of the sampled row pairs (x: left, y: right row of the encoded tables)
+// for every pair of columns, column-major.
+std::vector<PairCount> count_samples(const Encoded& E, const SideBufs& L, const SideBufs& R,
+                                     const std::vector<std::pair<int, int>>& columns,
+                                     const std::vector<uint2>& rows, cudaStream_t st) {
+  auto slot = [](const std::vector<int>& cols, int c) {
+    return (size_t)(std::find(cols.begin(), cols.end(), c) - cols.begin());
+  };
+  const uint32_t n = (uint32_t)rows.size();
+  DBuf<uint2> d_rows;
+  DBuf<uint4> d_out;
+  d_rows.upload(rows, st);
+  d_out.alloc((size_t)n * columns.size());
+  for (size_t c0 = 0; c0 < columns.size(); c0 += dev::kSampleBatch) {
+    dev::SampleCols cols{};
+    const size_t m = std::min<size_t>(columns.size() - c0, dev::kSampleBatch);
+    for (size_t k = 0; k < m; k++) {
+      cols.l[k] = L.meta.p + slot(E.L.str_col, columns[c0 + k].first) * (size_t)E.L.n_rows;
+      cols.r[k] = R.meta.p + slot(E.R.str_col, columns[c0 + k].second) * (size_t)E.R.n_rows;
+    }
+    dev::k_sample<<<dim3((n + 7) / 8, (uint32_t)m), 256, 0, st>>>(cols, L.arena.p, R.arena.p,
+                                                                  d_rows.p, n, d_out.p + c0 * n);
+  }
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) fail(HBX_ERR_CUDA, std::string("planner sample: ") + cudaGetErrorString(e));
+  std::vector<PairCount> counts((size_t)n * columns.size());
+  static_assert(sizeof(PairCount) == sizeof(uint4), "k_sample's records");
+  HBX_CUDA(cudaMemcpyAsync(counts.data(), d_out.p, counts.size() * sizeof(PairCount),
+                           cudaMemcpyDeviceToHost, st));
+  HBX_CUDA(cudaStreamSynchronize(st));
+  return counts;
+}
+
+void rank_by_counts(Plan* plan, const PlanSample& sample, const Table& left, const Table& right,
+                    const std::vector<PairCount>& counts) {
+  std::vector<ColumnSample> values;
+  for (size_t c = 0; c < sample.cols.size(); c++)
+    values.push_back(column_sample(sample, sample.cols[c], left, right,
+                                   counts.data() + c * sample.rows.size()));
+  rank_predicates(plan, sample, values);
+}
+
+namespace {
+
+// Orders the similarity predicates of *plan by the planner's sample, counted
+// on the encoded tables of the session, and the rules of S->E with them.
+void order_on_device(hbx_session* S, Plan* plan, const Table& left, const Table& right) {
+  Encoded& E = S->E;
+  const PlanSample sample = sample_plan(*plan, left, right);
+  if (sample.cols.empty()) return;
+  std::vector<uint2> rows;
+  for (auto& r : sample.rows) rows.push_back(make_uint2((uint32_t)r.first, (uint32_t)r.second));
+  rank_by_counts(plan, sample, left, right,
+                 count_samples(E, S->L, S->R, sample.cols, rows, S->ctx->stream));
+  auto slot = [](const std::vector<int>& cols, int c) {
+    return (int)(std::find(cols.begin(), cols.end(), c) - cols.begin());
+  };
+  for (size_t r = 0; r < E.rules.size(); r++)
+    for (size_t k = 0; k < plan->compiled[r].sims.size(); k++) {
+      const Pred& p = plan->compiled[r].sims[k];
+      E.rules[r].sim_slot_l[k] = slot(E.L.str_col, p.col_l);
+      E.rules[r].sim_slot_r[k] = slot(E.R.str_col, p.col_r);
+      E.rules[r].thr[k] = p.thr;
+    }
+}
+
+}  // namespace
+
 // Encodes the tables (on the device unless hbx_opts.ingest asks for the host
 // encoder, or only the host encoder is exact for the input) and builds the
 // session's device state.  The similarity predicates of each rule run in the
@@ -1062,28 +1130,18 @@ void create_session(hbx_session* S, const hbx_plan* plan, const hbx_table* left,
   PoolScope scope(C->pool, C->stream);
   Plan ordered;
   const Plan* use = &plan->p;
-  if (C->opts.pred_order == 0) {
-    hbx_plan* mp = const_cast<hbx_plan*>(plan);
-    const std::pair<uint64_t, uint64_t> key(left->uid, right->uid);
-    std::vector<CompiledRule> order;
-    bool have = false;
-    {
-      std::lock_guard<std::mutex> lock(mp->order_mu);
-      auto it = mp->order_cache.find(key);
-      if (it != mp->order_cache.end()) {
-        order = it->second;
-        have = true;
-      }
-    }
+  hbx_plan* mp = const_cast<hbx_plan*>(plan);
+  const std::pair<uint64_t, uint64_t> key(left->uid, right->uid);
+  bool to_order = C->opts.pred_order == 0;
+  if (to_order) {
     ordered = plan->p;
-    if (have) {
-      ordered.compiled = std::move(order);
-    } else {
-      order_predicates(&ordered, left->t, right->t);
-      std::lock_guard<std::mutex> lock(mp->order_mu);
-      mp->order_cache[key] = ordered.compiled;
+    std::lock_guard<std::mutex> lock(mp->order_mu);
+    auto it = mp->order_cache.find(key);
+    if (it != mp->order_cache.end()) {
+      ordered.compiled = it->second;
+      use = &ordered;
+      to_order = false;
     }
-    use = &ordered;
   }
   S->E = encode_schema(*use, left->t, right->t, n_partitions, prefix_idx);
   bool on_device = false;
@@ -1091,6 +1149,16 @@ void create_session(hbx_session* S, const hbx_plan* plan, const hbx_table* left,
   std::string why;
   if (C->opts.ingest == 0)
     on_device = device_encode(left, right, &S->E, &S->L, &S->R, C->n_sm, C->stream, &h2d, &why);
+  if (to_order) {
+    if (on_device) {
+      order_on_device(S, &ordered, left->t, right->t);
+    } else {
+      order_predicates(&ordered, left->t, right->t);
+      S->E = encode_schema(ordered, left->t, right->t, n_partitions, prefix_idx);
+    }
+    std::lock_guard<std::mutex> lock(mp->order_mu);
+    mp->order_cache[key] = ordered.compiled;
+  }
   if (!on_device) {
     encode_rows(left->t, right->t, &S->E);
     finish_rules(&S->E, true);

@@ -1,7 +1,10 @@
 // engine.h -- engine entry points used by other translation units.
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
+#include <utility>
 #include <vector>
 
 #include "../../include/hbx.h"
@@ -16,6 +19,18 @@ void run_to_host(hbx_session* s, hbx_mode mode, std::vector<uint32_t>* l, std::v
 // does not overflow and repeat.
 void reserve_output(hbx_session* s, uint64_t pairs);
 struct Table;
+struct Plan;
+struct PlanSample;
+struct PairCount;
+struct Encoded;
+struct SideBufs;
+// The planner's sample counted on encoded tables (rows: x left, y right), and
+// the order of *plan's predicates from those counts.
+std::vector<PairCount> count_samples(const Encoded& E, const SideBufs& L, const SideBufs& R,
+                                     const std::vector<std::pair<int, int>>& columns,
+                                     const std::vector<uint2>& rows, cudaStream_t st);
+void rank_by_counts(Plan* plan, const PlanSample& sample, const Table& left, const Table& right,
+                    const std::vector<PairCount>& counts);
 // sort.cu: sorts n device pairs by (left row, right row) in place; the first
 // form queues it on st.
 void queue_pair_sort(int n_sm, cudaStream_t st, uint32_t* l, uint32_t* r, uint64_t n,

@@ -92,7 +92,29 @@ constexpr size_t kDeviceCsvMin = 1u << 20;
 bool table_from_buffer_device(hbx_ctx* ctx, const char* data, size_t n, char sep, Table* out);
 Table table_from_columns(const hbx_columns* cols);
 
-// Measured-selectivity ordering of similarity predicates (planner.cpp).
+// Measured-selectivity ordering of similarity predicates (planner.cpp): the
+// sampled row pairs and the columns (left, right) to be compared on them (none:
+// nothing to order); their Jaro-Winkler values and mean cost per pair of
+// columns, and the order that follows from them.
+struct PlanSample {
+  std::vector<std::pair<int64_t, int64_t>> rows;
+  std::vector<std::pair<int, int>> cols;
+};
+PlanSample sample_plan(const Plan& plan, const Table& left, const Table& right);
+struct ColumnSample {
+  std::vector<double> jw;
+  double cost = 0;
+};
+// The samples of a pair of columns, from each pair's lengths, match count and
+// common prefix; a count of kNotCounted is made here from the tables.
+struct PairCount {
+  uint32_t la, lb, m, p;
+};
+constexpr uint32_t kNotCounted = 0xffffffffu;
+ColumnSample column_sample(const PlanSample& sample, std::pair<int, int> cols, const Table& left,
+                           const Table& right, const PairCount* counts);
+void rank_predicates(Plan* plan, const PlanSample& sample, const std::vector<ColumnSample>& values);
+// All of it on the host.
 void order_predicates(Plan* plan, const Table& left, const Table& right);
 
 }  // namespace hbx

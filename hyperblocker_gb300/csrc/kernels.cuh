@@ -469,6 +469,17 @@ __global__ void k_join_scatter(Side L, Side R, const Rule* rules, uint32_t n_rul
                                const uint32_t* tasks, unsigned long long* rule_base,
                                Counters* ctr);
 // ------------------------------------------------------------------ evaluation
+// The planner's sample: for row pair k (x: left row, y: right row) and each
+// pair of string columns (blockIdx.y; string metadata of the whole columns)
+// {left length, right length, match count, common prefix} into out[column *
+// n + k]; count 0xffffffff, not counted here, when both strings are longer
+// than kMaxTableLen symbols.  A warp per pair.
+constexpr uint32_t kSampleBatch = 8;
+struct SampleCols {
+  const StrMeta *l[kSampleBatch], *r[kSampleBatch];
+};
+__global__ void k_sample(const __grid_constant__ SampleCols cols, const uint8_t* arena_l,
+                         const uint8_t* arena_r, const uint2* rows, uint32_t n, uint4* out);
 // Peq tables of every left string of n_slots string slots (PeqShape).
 __global__ void k_peq_build(Side L, uint32_t n_slots, PeqShape shape, uint32_t* peq);
 // The evaluation kernel for masks of peq_w words (PeqShape::w): k_eval<W>

@@ -12,7 +12,6 @@
 // AND is commutative, so the order changes work, never the result.
 #include <algorithm>
 #include <cstring>
-#include <map>
 #include <numeric>
 
 #include "hbx_core.h"
@@ -35,18 +34,17 @@ inline size_t c_len(const Column& c, int64_t i) {
 // handling.
 class Sampler {
  public:
-  double jw(const char* a, size_t la, const char* b, size_t lb) {
-    if (la == 0 || lb == 0) return (la == 0 && lb == 0) ? 1.0 : 0.0;
+  PairCount count(const char* a, size_t la, const char* b, size_t lb) {
+    PairCount c{(uint32_t)la, (uint32_t)lb, 0, 0};
+    if (la == 0 || lb == 0) return c;
     if (la > lb) {
       std::swap(a, b);
       std::swap(la, lb);
     }
-    const size_t ls = la, ll = lb;
-    const size_t h = (ls + 1) / 2, words = (la + 63) / 64;
+    const size_t h = (la + 1) / 2, words = (la + 63) / 64;
     if (mask_.size() < 256 * words) mask_.assign(256 * words, 0);
     free_.assign(words, ~0ull);
     for (size_t j = 0; j < la; j++) mask_[(uint8_t)a[j] * words + j / 64] |= 1ull << (j % 64);
-    size_t m = 0;
     for (size_t i = 0; i < lb; i++) {
       const size_t lo = i > h ? i - h : 0, hi = std::min(la - 1, i + h);
       if (lo > hi) break;  // and for every later i
@@ -57,76 +55,93 @@ class Sampler {
         if (w == hi / 64) x &= ~0ull >> (63 - hi % 64);
         if (!x) continue;
         free_[w] &= ~(x & (0 - x));
-        m++;
+        c.m++;
         break;
       }
     }
     for (size_t j = 0; j < la; j++) mask_[(uint8_t)a[j] * words + j / 64] = 0;
-    if (!m) return 0.0;
-    double j = ((double)m / ls + (double)m / ll + 1.0) / 3.0;
-    size_t p = 0;
-    while (p < ls && a[p] == b[p]) p++;
-    j += (1.0 - j) * (double)p * 0.1;
-    return j > 1.0 ? 1.0 : j;
+    while (c.p < la && a[c.p] == b[c.p]) c.p++;
+    return c;
   }
 
  private:
   std::vector<uint64_t> mask_, free_;  // mask_: zero between calls
 };
 
-// The sampled pairs on one pair of columns: their Jaro-Winkler values and the
-// mean cost of one evaluation.
-struct ColumnSample {
-  std::vector<double> jw;
-  double cost = 0;
-};
+double jaro_winkler(const PairCount& c) {
+  if (c.la == 0 || c.lb == 0) return (c.la == 0 && c.lb == 0) ? 1.0 : 0.0;
+  if (!c.m) return 0.0;
+  const size_t ls = std::min(c.la, c.lb), ll = std::max(c.la, c.lb);
+  double j = ((double)c.m / ls + (double)c.m / ll + 1.0) / 3.0;
+  j += (1.0 - j) * (double)c.p * 0.1;
+  return j > 1.0 ? 1.0 : j;
+}
 
 }  // namespace
 
-void order_predicates(Plan* plan, const Table& left, const Table& right) {
-  if (left.n_rows == 0 || right.n_rows == 0) return;
+PlanSample sample_plan(const Plan& plan, const Table& left, const Table& right) {
+  PlanSample out;
+  if (left.n_rows == 0 || right.n_rows == 0) return out;
+  // rules test the same few columns at different thresholds: each pair of
+  // columns is sampled once
+  for (auto& cr : plan.compiled) {
+    if (cr.sims.size() < 2) continue;
+    for (auto& p : cr.sims) {
+      const std::pair<int, int> c(p.col_l, p.col_r);
+      if (p.col_l < left.n_cols() && p.col_r < right.n_cols() &&
+          std::find(out.cols.begin(), out.cols.end(), c) == out.cols.end())
+        out.cols.push_back(c);
+    }
+  }
+  if (out.cols.empty()) return out;
   const int kSamples = 2048;
   uint64_t state = 0x48594250ull;
   auto next = [&]() {
     state = state * 6364136223846793005ull + 1442695040888963407ull;
     return state >> 17;
   };
-  std::vector<std::pair<int64_t, int64_t>> pairs;
-  for (int i = 0; i < kSamples; i++)
-    pairs.emplace_back((int64_t)(next() % (uint64_t)left.n_rows),
-                       (int64_t)(next() % (uint64_t)right.n_rows));
-  // Rules test the same few columns at different thresholds: each pair of
-  // columns is sampled once (8 rules, 11 predicates, 25k x 40k rows, CSV files
-  // to pair file: 16.9 ms, with a byte-by-byte scan per predicate 77.8 ms).
-  std::map<std::pair<int, int>, ColumnSample> samples;
+  for (int i = 0; i < kSamples; i++) {
+    const int64_t l = (int64_t)(next() % (uint64_t)left.n_rows);
+    out.rows.emplace_back(l, (int64_t)(next() % (uint64_t)right.n_rows));
+  }
+  return out;
+}
+
+ColumnSample column_sample(const PlanSample& sample, std::pair<int, int> cols, const Table& left,
+                           const Table& right, const PairCount* counts) {
+  const Column& cl = left.cols[(size_t)cols.first];
+  const Column& cr = right.cols[(size_t)cols.second];
+  ColumnSample s;
   Sampler sampler;
-  auto sample = [&](int col_l, int col_r) -> const ColumnSample& {
-    ColumnSample& s = samples[{col_l, col_r}];
-    if (!s.jw.empty()) return s;
-    const Column& cl = left.cols[(size_t)col_l];
-    const Column& cr = right.cols[(size_t)col_r];
-    for (auto& pr : pairs) {
-      const size_t la = c_len(cl, pr.first), lb = c_len(cr, pr.second);
-      s.cost += (double)lb * (double)((std::min<size_t>(la, 256) + 31) / 32 + 2);
-      s.jw.push_back(sampler.jw(cl.ptr(pr.first), la, cr.ptr(pr.second), lb));
-    }
-    s.cost /= (double)pairs.size();
-    return s;
-  };
+  for (size_t k = 0; k < sample.rows.size(); k++) {
+    const auto& pr = sample.rows[k];
+    PairCount c = counts ? counts[k] : PairCount{0, 0, kNotCounted, 0};
+    if (c.m == kNotCounted)
+      c = sampler.count(cl.ptr(pr.first), c_len(cl, pr.first), cr.ptr(pr.second), c_len(cr, pr.second));
+    s.cost += (double)c.lb * (double)((std::min<size_t>(c.la, 256) + 31) / 32 + 2);
+    s.jw.push_back(jaro_winkler(c));
+  }
+  s.cost /= (double)sample.rows.size();
+  return s;
+}
+
+void rank_predicates(Plan* plan, const PlanSample& sample, const std::vector<ColumnSample>& values) {
+  if (sample.cols.empty()) return;
   for (auto& cr : plan->compiled) {
     if (cr.sims.size() < 2) continue;
     std::vector<double> rank(cr.sims.size());
     for (size_t s = 0; s < cr.sims.size(); s++) {
       const Pred& p = cr.sims[s];
-      if (p.col_l >= left.n_cols() || p.col_r >= right.n_cols()) {
+      const auto it = std::find(sample.cols.begin(), sample.cols.end(), std::make_pair(p.col_l, p.col_r));
+      if (it == sample.cols.end()) {
         rank[s] = 1e30;
         continue;
       }
-      const ColumnSample& c = sample(p.col_l, p.col_r);
+      const ColumnSample& c = values[(size_t)(it - sample.cols.begin())];
       double pass = 0;
       for (double v : c.jw)
         if (v >= (double)p.thr) pass += 1;
-      pass /= (double)pairs.size();
+      pass /= (double)c.jw.size();
       rank[s] = c.cost / std::max(1e-3, 1.0 - pass);
     }
     std::vector<size_t> ord(cr.sims.size());
@@ -136,6 +151,13 @@ void order_predicates(Plan* plan, const Table& left, const Table& right) {
     for (size_t k : ord) sorted.push_back(cr.sims[k]);
     cr.sims = std::move(sorted);
   }
+}
+
+void order_predicates(Plan* plan, const Table& left, const Table& right) {
+  const PlanSample sample = sample_plan(*plan, left, right);
+  std::vector<ColumnSample> values;
+  for (auto& c : sample.cols) values.push_back(column_sample(sample, c, left, right, nullptr));
+  rank_predicates(plan, sample, values);
 }
 
 }  // namespace hbx

@@ -66,6 +66,52 @@ void sub_table(const Table& t, const std::vector<int>& used, const uint32_t* idx
   }
 }
 
+// The planner's order for tables that are not on the device: the sampled rows
+// alone are encoded there.  (The host counts them when the context encodes on
+// the host, or the device encoder cannot.)
+void order_sampled(hbx_ctx* ctx, Plan* plan, const Table& left, const Table& right) {
+  const PlanSample sample = sample_plan(*plan, left, right);
+  if (sample.cols.empty()) return;
+  if (ctx->opts.ingest == 0) {
+    Plan few;  // the sampled columns as one rule without equalities
+    few.compiled.resize(1);
+    std::vector<int> used_l, used_r;
+    for (auto& c : sample.cols) {
+      few.compiled[0].sims.push_back(Pred{'s', c.first, c.second, 0.0f});
+      used_l.push_back(c.first);
+      used_r.push_back(c.second);
+    }
+    std::vector<uint32_t> il, ir;
+    std::vector<uint2> rows;
+    for (size_t k = 0; k < sample.rows.size(); k++) {
+      il.push_back((uint32_t)sample.rows[k].first);
+      ir.push_back((uint32_t)sample.rows[k].second);
+      rows.push_back(make_uint2((uint32_t)k, (uint32_t)k));
+    }
+    std::sort(used_l.begin(), used_l.end());
+    std::sort(used_r.begin(), used_r.end());
+    hbx_table sub_l, sub_r;
+    sub_l.pin_tried = sub_r.pin_tried = true;
+    sub_table(left, used_l, il.data(), il.size(), &sub_l.t);
+    sub_table(right, used_r, ir.data(), ir.size(), &sub_r.t);
+    PoolScope scope(ctx->pool, ctx->stream);
+    try {
+      Encoded E = encode_schema(few, sub_l.t, sub_r.t, 1, INT_MAX);
+      SideBufs L, R;
+      uint64_t h2d = 0;
+      std::string why;
+      if (device_encode(&sub_l, &sub_r, &E, &L, &R, ctx->n_sm, ctx->stream, &h2d, &why)) {
+        rank_by_counts(plan, sample, left, right,
+                       count_samples(E, L, R, sample.cols, rows, ctx->stream));
+        return;
+      }
+    } catch (const Error&) {
+      cudaGetLastError();
+    }
+  }
+  order_predicates(plan, left, right);
+}
+
 }  // namespace
 }  // namespace hbx
 
@@ -88,7 +134,7 @@ extern "C" hbx_status hbx_block_streamed(hbx_ctx* ctx, const hbx_plan* plan, con
     // the evaluation order is measured once on the whole tables
     hbx_plan ordered;
     ordered.p = plan->p;
-    if (ctx->opts.pred_order == 0) order_predicates(&ordered.p, TL, TR);
+    if (ctx->opts.pred_order == 0) order_sampled(ctx, &ordered.p, TL, TR);
     const Encoded schema = encode_schema(ordered.p, TL, TR, n_partitions, prefix_idx);
     std::vector<int> used_l, used_r;
     auto use = [](std::vector<int>& v, int c) {
