@@ -46,15 +46,17 @@ struct RuleBufs {
   DBuf<unsigned long long> item_off;
 };
 
-// The tasks of a rule array's join kernels (kernels.cuh), and the histogram
-// words that they use, all at the front of hbx_session::counts.
+// The tasks of a rule array's join kernels (kernels.cuh), and what a run clears
+// for them: key histograms and scatter cursors, chunk totals and tickets.
 struct JoinLists {
   std::vector<uint32_t> count, scatter, block_task;
   std::vector<dev::ScanTask> scan;
-  // in hbx_session::lists
+  std::vector<uint32_t> words;  // all of them, as uploaded
+  DBuf<uint32_t> lists;
   const uint32_t *d_count = nullptr, *d_scatter = nullptr, *d_block_task = nullptr;
   const dev::ScanTask* d_scan = nullptr;
-  uint64_t n_counts = 0;
+  DBuf<uint32_t> counts;
+  DBuf<unsigned long long> scan_sync;
 };
 
 template <class T>
@@ -81,12 +83,10 @@ struct hbx_session {
   hbx::dev::Counters* h_ctr = nullptr;  // page-locked copy of d_ctr (the context's), written by each run
   hbx::DBuf<uint32_t> out_l, out_r;
   hbx::DBuf<unsigned long long> seen;  // reported-pair set (plans with several rules)
-  // key histograms and scatter cursors of every rule, one block: one memset
-  hbx::DBuf<uint32_t> counts;
-  hbx::DBuf<unsigned long long> scan_sync;  // chunk totals and tickets (k_join_scan)
-  hbx::JoinLists join_rules, join_groups;   // the joins of h_rules and of h_groups
-  hbx::DBuf<uint32_t> lists;                  // join tasks and bound_idx (upload_lists)
-  const uint32_t* bound_idx = nullptr;        // per rule, n_partitions + 1 key indices
+  // the joins of h_groups (batched form) and of h_rules (plain form)
+  hbx::JoinLists join_groups, join_rules;
+  bool plain_ready = false;  // the plain form's buffers exist (ensure_plain)
+  hbx::DBuf<uint32_t> bound_idx;              // per rule, n_partitions + 1 key indices
   hbx::DBuf<unsigned long long> bound_val;    // item_off at those keys
   hbx::dev::Side side_l{}, side_r{};
   uint32_t warp_words = 4;
@@ -153,8 +153,8 @@ int row_grid(uint64_t n, int n_sm) {
 // Tile shape and kernel variant of a session: right rows per work item
 // (tile_right) and the evaluation kernel (0: 3 CTAs per SM, 1: 2 CTAs per SM
 // with more registers).  Lays out each warp's shared memory
-// (dev::warp_layout), uploads the rule descriptors, raises the kernel's
-// shared-memory limit if needed and drops the graph.
+// (dev::warp_layout), raises the kernel's shared-memory limit if needed and
+// drops the graph.
 void configure(hbx_session* S, uint32_t tile_right, int variant) {
   hbx_ctx* C = S->ctx;
   S->tile_right = std::min<uint32_t>(512, std::max<uint32_t>(32, (tile_right + 31) / 32 * 32));
@@ -168,11 +168,6 @@ void configure(hbx_session* S, uint32_t tile_right, int variant) {
   if (S->warp_words > cap_warp_words) fail(HBX_ERR_INVALID_ARG, "tile_right too large");
   // every warp region lies inside the dynamic allocation
   S->smem_bytes = (size_t)S->warp_words * 4 * dev::kWarpsPerCta;
-  HBX_CUDA(cudaMemcpyAsync(S->d_rules.p, S->h_rules.data(), S->h_rules.size() * sizeof(dev::Rule),
-                           cudaMemcpyHostToDevice, C->stream));
-  HBX_CUDA(cudaMemcpyAsync(S->d_groups.p, S->h_groups.data(), S->h_groups.size() * sizeof(dev::Rule),
-                           cudaMemcpyHostToDevice, C->stream));
-  HBX_CUDA(cudaStreamSynchronize(C->stream));
   for (bool g : {false, true}) raise_smem_limit(dev::eval_kernel(S->variant, g, S->peq_shape.w), S->smem_bytes);
   int bps = 0;
   HBX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -243,16 +238,60 @@ void launch_dependent(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, c
   HBX_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...));
 }
 
-// The join tasks of a rule array.
-void list_join(const std::vector<dev::Rule>& rules, JoinLists* J) {
-  for (uint32_t r = 0; r < (uint32_t)rules.size(); r++) {
-    const dev::Rule& d = rules[r];
+// A rule's join buffers, but for its counts.
+void alloc_join(RuleBufs& b, dev::Rule* d, uint32_t nL, uint32_t nR) {
+  b.key_l.alloc(nL);
+  b.key_r.alloc(nR);
+  b.off_l.alloc(d->domain_l);
+  b.off_r.alloc(d->domain);
+  b.sorted_l.alloc(nL);
+  b.sorted_r.alloc((size_t)nR + 4);
+  if (d->n_sim) b.sorted_meta_r.alloc(nR);
+  b.item_off.alloc((size_t)d->domain_l + 1);
+}
+
+void bind_join(const RuleBufs& b, dev::Rule* d) {
+  d->key_l = b.key_l.p;
+  d->key_r = b.key_r.p;
+  d->off_l = b.off_l.p;
+  d->off_r = b.off_r.p;
+  d->item_off = b.item_off.p;
+  d->sorted_l = b.sorted_l.p;
+  d->sorted_r = b.sorted_r.p;
+  d->sorted_meta_r = d->n_sim ? b.sorted_meta_r.p : nullptr;
+}
+
+// The join tasks of a rule array, uploaded on st (J->words stays for the copy),
+// and its counts: all of a rule with work items, the right histogram of a
+// member that only counts its comparisons.
+void list_join(std::vector<dev::Rule>* rules, JoinLists* J, cudaStream_t st) {
+  size_t n_counts = 0;
+  for (const dev::Rule& d : *rules) {
+    if (d.n_members)
+      n_counts += 2ull * d.domain_l + 2ull * d.domain;
+    else if (d.cmp_weight)
+      n_counts += d.domain;
+  }
+  J->counts.alloc(n_counts);
+  uint32_t* next = J->counts.p;
+  auto take = [&](size_t words) {
+    uint32_t* p = next;
+    next += words;
+    return p;
+  };
+  for (uint32_t r = 0; r < (uint32_t)rules->size(); r++) {
+    dev::Rule& d = (*rules)[r];
     if (!d.n_members) {
       if (!d.cmp_weight) continue;  // another rule's join counts its comparisons
+      d.cnt_r = take(d.domain);
       J->count.push_back(dev::join_task(r, 1));
       J->scatter.push_back(dev::join_task(r, 0));
       continue;
     }
+    d.cnt_l = take(d.domain_l);
+    d.cur_l = take(d.domain_l);
+    d.cnt_r = take(d.domain);
+    d.cur_r = take(d.domain);
     for (int side : {0, 1}) {
       J->count.push_back(dev::join_task(r, side));
       J->scatter.push_back(dev::join_task(r, side));
@@ -268,39 +307,22 @@ void list_join(const std::vector<dev::Rule>& rules, JoinLists* J) {
       J->scan.push_back(t);
     }
   }
-}
-
-// Uploads both rule arrays' join tasks and the partition boundaries `bounds`
-// in one copy on st, from the returned words (to be kept until it is done).
-std::vector<uint32_t> upload_lists(hbx_session* S, const std::vector<uint32_t>& bounds,
-                                   cudaStream_t st) {
-  std::vector<uint32_t> all;
+  J->scan_sync.alloc(J->block_task.size() + J->scan.size());
   auto add = [&](const void* p, size_t words) {
-    const size_t at = all.size();
-    all.resize(at + (words + 3) / 4 * 4);  // 16-byte aligned pieces
-    if (words) std::memcpy(all.data() + at, p, words * 4);
+    const size_t at = J->words.size();
+    J->words.resize(at + (words + 3) / 4 * 4);  // 16-byte aligned pieces
+    if (words) std::memcpy(J->words.data() + at, p, words * 4);
     return at;
   };
-  size_t at[2][4];
-  JoinLists* lists[2] = {&S->join_rules, &S->join_groups};
-  for (int k = 0; k < 2; k++) {
-    const JoinLists& J = *lists[k];
-    at[k][0] = add(J.count.data(), J.count.size());
-    at[k][1] = add(J.scatter.data(), J.scatter.size());
-    at[k][2] = add(J.block_task.data(), J.block_task.size());
-    at[k][3] = add(J.scan.data(), J.scan.size() * sizeof(dev::ScanTask) / 4);
-  }
-  const size_t at_bounds = add(bounds.data(), bounds.size());
-  S->lists.upload(all, st);
-  for (int k = 0; k < 2; k++) {
-    JoinLists& J = *lists[k];
-    J.d_count = S->lists.p + at[k][0];
-    J.d_scatter = S->lists.p + at[k][1];
-    J.d_block_task = S->lists.p + at[k][2];
-    J.d_scan = reinterpret_cast<const dev::ScanTask*>(S->lists.p + at[k][3]);
-  }
-  S->bound_idx = S->lists.p + at_bounds;
-  return all;
+  const size_t a0 = add(J->count.data(), J->count.size());
+  const size_t a1 = add(J->scatter.data(), J->scatter.size());
+  const size_t a2 = add(J->block_task.data(), J->block_task.size());
+  const size_t a3 = add(J->scan.data(), J->scan.size() * sizeof(dev::ScanTask) / 4);
+  J->lists.upload(J->words, st);
+  J->d_count = J->lists.p + a0;
+  J->d_scatter = J->lists.p + a1;
+  J->d_block_task = J->lists.p + a2;
+  J->d_scan = reinterpret_cast<const dev::ScanTask*>(J->lists.p + a3);
 }
 
 // Do rules of the array share all their candidates (dev::Rule::dup_always)?
@@ -357,72 +379,26 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
     d.domain = (uint32_t)re.domain;
     dev::set_classes(&d, S->long_left);
     dev::make_singleton(&d);
-    RuleBufs& b = S->rb[r];
-    b.key_l.alloc(nL);
-    b.key_r.alloc(nR);
-    b.off_l.alloc(d.domain_l);
-    b.off_r.alloc(re.domain);
-    b.sorted_l.alloc(nL);
-    b.sorted_r.alloc((size_t)nR + 4);
-    if (d.n_sim) b.sorted_meta_r.alloc(nR);
-    b.item_off.alloc((size_t)d.domain_l + 1);
-    d.key_l = b.key_l.p;
-    d.key_r = b.key_r.p;
-    d.off_l = b.off_l.p;
-    d.off_r = b.off_r.p;
-    d.item_off = b.item_off.p;
-    d.sorted_l = b.sorted_l.p;
-    d.sorted_r = b.sorted_r.p;
-    d.sorted_meta_r = d.n_sim ? b.sorted_meta_r.p : nullptr;
   }
   dev::set_overlaps(S->h_rules.data(), S->h_rules.size());
   S->h_groups = group_rules(S->h_rules);
   S->groups = false;
   for (const dev::Rule& g : S->h_groups)
     if (g.n_members > 1) S->groups = true;
-  // histograms and cursors of every rule, one block: first what the groups'
-  // join uses (a member that counts its comparisons: cnt_r), then the rest
-  {
-    size_t total = 0;
-    for (const dev::Rule& d : S->h_rules) total += 2ull * d.domain_l + 2ull * d.domain;
-    S->counts.alloc(std::max<size_t>(total, 1));
-    uint32_t* next = S->counts.p;
-    auto take = [&](size_t words) {
-      uint32_t* p = next;
-      next += words;
-      return p;
-    };
-    for (size_t r = 0; r < S->h_rules.size(); r++) {
-      dev::Rule& d = S->h_rules[r];
-      const dev::Rule& g = S->h_groups[r];
-      if (g.n_members || g.cmp_weight) d.cnt_r = take(d.domain);
-      if (!g.n_members) continue;
-      d.cnt_l = take(d.domain_l);
-      d.cur_l = take(d.domain_l);
-      d.cur_r = take(d.domain);
-    }
-    S->join_groups.n_counts = (uint64_t)(next - S->counts.p);
-    for (dev::Rule& d : S->h_rules) {
-      if (!d.cnt_r) d.cnt_r = take(d.domain);
-      if (!d.cnt_l) d.cnt_l = take(d.domain_l);
-      if (!d.cur_l) d.cur_l = take(d.domain_l);
-      if (!d.cur_r) d.cur_r = take(d.domain);
-    }
-    S->join_rules.n_counts = (uint64_t)(next - S->counts.p);
-    for (size_t r = 0; r < S->h_rules.size(); r++) {
-      const dev::Rule& d = S->h_rules[r];
-      dev::Rule& g = S->h_groups[r];
-      g.cnt_l = d.cnt_l;
-      g.cnt_r = d.cnt_r;
-      g.cur_l = d.cur_l;
-      g.cur_r = d.cur_r;
-    }
+  // the batched form's joins; rules evaluated in others' groups get their own
+  // when a plain run asks for them (ensure_plain): with key domains of several
+  // equalities that is nine tenths of the join state (8 rules, 64 partitions x
+  // 240 keys x 500 venues: 250 MB for one of them), whose mapping and release
+  // cost a one-shot call more than its run (CSV files to pair file, 25k x 40k
+  // rows: 7.05 against 8.7 ms)
+  for (size_t r = 0; r < E.rules.size(); r++) {
+    dev::Rule& g = S->h_groups[r];
+    if (!g.n_members) continue;
+    alloc_join(S->rb[r], &g, nL, nR);
+    bind_join(S->rb[r], &g);
   }
-  list_join(S->h_rules, &S->join_rules);
-  list_join(S->h_groups, &S->join_groups);
-  S->scan_sync.alloc(S->join_rules.block_task.size() + S->join_rules.scan.size());
-  S->d_rules.alloc(E.rules.size());
-  S->d_groups.alloc(E.rules.size());
+  list_join(&S->h_groups, &S->join_groups, st);
+  S->d_groups.upload(S->h_groups, st);
   S->d_rule_base.alloc(dev::item_base_words(E.rules.size()));
   S->d_ctr.alloc(1);
   // one page-locked counter block per context: its sessions run one at a time
@@ -452,17 +428,6 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
     }
   }
 
-  // partition boundaries of every rule's left key space, per class (plain
-  // form): entry (rule, class, p) = first left key of partition p
-  std::vector<uint32_t> idx;
-  for (size_t r = 0; r < E.rules.size(); r++)
-    for (uint32_t c = 0; c < n_classes(S); c++)
-      for (uint64_t p = 0; p <= E.n_partitions; p++) {
-        const uint32_t cc = std::min<uint32_t>(c, S->h_rules[r].n_classes - 1);
-        idx.push_back(cc * S->h_rules[r].domain + (uint32_t)E.rules[r].part_key_begin[p]);
-      }
-  const std::vector<uint32_t> lists = upload_lists(S, idx, st);
-  S->bound_val.alloc(idx.size());
   // output slots for the caller's capacity, but never more than the
   // partitions can hold: a generous caller buffer does not size device buffers
   // by itself.  The duplicate set: twice as many where rules may share every
@@ -483,11 +448,41 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
   HBX_CUDA(cudaEventCreate(&S->ev_eval0));
   HBX_CUDA(cudaEventCreate(&S->ev_eval1));
   uint64_t h2d = h2d_tables;
-  h2d += S->d_rules.n * sizeof(dev::Rule) + idx.size() * 4;
+  h2d += S->d_groups.n * sizeof(dev::Rule) + S->join_groups.words.size() * 4;
   S->stats.h2d_bytes = h2d;
   HBX_CUDA(cudaStreamSynchronize(st));
   S->stats.pairs_covered = E.pairs_covered;
   S->stats.n_partitions_used = E.n_partitions_used;
+}
+
+// The plain form's join state, made by its first run: every rule on its own.
+void ensure_plain(hbx_session* S) {
+  if (S->plain_ready) return;
+  hbx_ctx* C = S->ctx;
+  const Encoded& E = S->E;
+  cudaStream_t st = C->stream;
+  PoolScope scope(C->pool, st);
+  for (size_t r = 0; r < E.rules.size(); r++) {
+    dev::Rule& d = S->h_rules[r];
+    if (!S->h_groups[r].n_members) alloc_join(S->rb[r], &d, (uint32_t)E.L.n_rows, (uint32_t)E.R.n_rows);
+    bind_join(S->rb[r], &d);
+  }
+  S->join_rules = JoinLists{};
+  list_join(&S->h_rules, &S->join_rules, st);
+  S->d_rules.upload(S->h_rules, st);
+  // partition boundaries of every rule's left key space, per class: entry
+  // (rule, class, p) = first left key of partition p
+  std::vector<uint32_t> idx;
+  for (size_t r = 0; r < E.rules.size(); r++)
+    for (uint32_t c = 0; c < n_classes(S); c++)
+      for (uint64_t p = 0; p <= E.n_partitions; p++) {
+        const uint32_t cc = std::min<uint32_t>(c, S->h_rules[r].n_classes - 1);
+        idx.push_back(cc * S->h_rules[r].domain + (uint32_t)E.rules[r].part_key_begin[p]);
+      }
+  S->bound_idx.upload(idx, st);
+  S->bound_val.alloc(idx.size());
+  HBX_CUDA(cudaStreamSynchronize(st));
+  S->plain_ready = true;
 }
 
 // Groups of the batched form (dev::Rule, "Group evaluation"), from the
@@ -648,10 +643,10 @@ uint32_t enqueue_join(hbx_session* S, cudaStream_t st, bool groups) {
   const uint32_t n_blocks = (uint32_t)J.block_task.size();
   {  // counters, histograms, the duplicate set and the join scan's tickets, one launch
     const uint64_t n_seen = S->seen.p ? S->seen.n : 0;
-    const uint64_t n_sync = n_blocks + J.scan.size();
-    const uint64_t n = std::max<uint64_t>(std::max<uint64_t>(J.n_counts, n_seen), std::max<uint64_t>(n_sync, 32));
-    dev::k_reset<<<row_grid(n, S->ctx->n_sm), 256, 0, st>>>(S->d_ctr.p, S->counts.p, J.n_counts,
-                                                            S->seen.p, n_seen, S->scan_sync.p,
+    const uint64_t n_sync = J.scan_sync.n;
+    const uint64_t n = std::max<uint64_t>(std::max<uint64_t>(J.counts.n, n_seen), std::max<uint64_t>(n_sync, 32));
+    dev::k_reset<<<row_grid(n, S->ctx->n_sm), 256, 0, st>>>(S->d_ctr.p, J.counts.p, J.counts.n,
+                                                            S->seen.p, n_seen, J.scan_sync.p,
                                                             n_sync);
   }
   uint32_t max_d = 1;
@@ -661,7 +656,7 @@ uint32_t enqueue_join(hbx_session* S, cudaStream_t st, bool groups) {
   launch_dependent(dev::k_join_count, dim3(row_blocks, (uint32_t)J.count.size()), dim3(256), smem,
                    st, S->side_l, S->side_r, rules, J.d_count);
   launch_dependent(dev::k_join_scan, dim3(n_blocks), dim3(1024), 0, st, rules, S->tile_right,
-                   J.d_scan, J.d_block_task, S->scan_sync.p, &S->d_ctr.p->comparisons, 0u,
+                   J.d_scan, J.d_block_task, J.scan_sync.p, &S->d_ctr.p->comparisons, 0u,
                    S->d_ctr.p);
   launch_dependent(dev::k_join_scatter, dim3(row_blocks, (uint32_t)J.scatter.size()), dim3(256), 0,
                    st, S->side_l, S->side_r, rules, (uint32_t)S->rb.size(), J.d_scatter,
@@ -825,6 +820,7 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
     return *S->h_ctr;
   }
   // PLAIN: join, then one launch per (partition, rule)
+  ensure_plain(S);
   HBX_CUDA(cudaEventRecord(S->ev0, st));
   uint32_t n = enqueue_join(S, st, false);
   const uint32_t n_rules = (uint32_t)S->rb.size();
@@ -832,7 +828,7 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
   const uint32_t per_rule = per_class * n_classes(S);
   const uint32_t total = n_rules * per_rule;
   k_gather_bounds<<<(total + 255) / 256, 256, 0, st>>>(S->d_rules.p, n_rules, per_rule,
-                                                       S->bound_idx, S->bound_val.p);
+                                                       S->bound_idx.p, S->bound_val.p);
   n++;
   launch_check("k_gather_bounds");
   std::vector<unsigned long long> bounds(total), base(dev::item_base_words(n_rules));

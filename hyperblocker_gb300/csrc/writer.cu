@@ -94,8 +94,8 @@ void write_pairs_device(hbx_ctx* C, const Table& TL, const Table& TR, const uint
   const uint64_t max_line = (uint64_t)il.max_len + ir.max_len + 2;
   if (max_line >= (1ull << 31)) fail(HBX_ERR_INVALID_ARG, "id cells too long");
   // pairs per chunk: their text fits kTextChunkBytes (and u32 offsets)
-  const uint32_t per_chunk =
-      (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kTextChunkBytes / max_line, 1u << 24));
+  const uint32_t per_chunk = (uint32_t)std::max<uint64_t>(
+      1, std::min<uint64_t>({kTextChunkBytes / max_line, 1u << 24, n}));
   FILE* f = std::fopen(path, "ab");
   if (!f) fail(HBX_ERR_IO, std::string("cannot open ") + path);
   struct Closer {
@@ -128,6 +128,7 @@ void write_pairs_device(hbx_ctx* C, const Table& TL, const Table& TR, const uint
   total.alloc(1);
   HBX_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(unsigned int), st));
   for (Slot& s : slots) {
+    if (&s == &slots[1] && n <= per_chunk) break;  // one chunk
     s.len.alloc(per_chunk);
     s.off.alloc(per_chunk);
     s.text.alloc((uint64_t)per_chunk * max_line + 16);
