@@ -90,7 +90,8 @@ struct hbx_session {
   hbx::DBuf<unsigned long long> bound_val;    // item_off at those keys
   hbx::dev::Side side_l{}, side_r{};
   uint32_t warp_words = 4;
-  uint32_t tile_right = 128;
+  uint32_t tile_right = 128;  // right rows per work item
+  uint32_t stage_rows = 128;  // and per staging buffer
   hbx::dev::WarpLayout wl{};
   hbx::dev::PeqShape peq_shape{};
   hbx::DBuf<uint32_t> peq;  // Peq tables of the left strings [slot][row]
@@ -163,9 +164,16 @@ void configure(hbx_session* S, uint32_t tile_right, int variant) {
   // per block
   const size_t smem_cap = std::min<size_t>(C->smem_optin * 2, C->smem_per_sm - 2048);
   const uint32_t cap_warp_words = (uint32_t)(C->smem_optin / 4 / dev::kWarpsPerCta) / 4 * 4;
-  S->wl = dev::warp_layout_fit(S->tile_right, smem_cap);
+  // Items of more than 128 rows are staged 96 at a time: fewer claims, with the
+  // shared memory (and so the L1 left to the Peq rows) of 96-row items.  8
+  // rules, 150k x 150k rows, evaluation: 9.54 ms with 288 rows per item, 9.60
+  // with 192, 9.87 with 96; 2,601 x 64,264 rows are better off with 96 or 128
+  // (141 against 149 us: too few items to share out evenly), so the autotuner
+  // chooses.  What did not fit a warp's share in one piece is refused still.
+  if (768u + 17u * S->tile_right + 432u > cap_warp_words) fail(HBX_ERR_INVALID_ARG, "tile_right too large");
+  S->stage_rows = S->tile_right > 128 ? 96 : S->tile_right;
+  S->wl = dev::warp_layout_fit(S->stage_rows, smem_cap);
   S->warp_words = S->wl.warp_words;
-  if (S->warp_words > cap_warp_words) fail(HBX_ERR_INVALID_ARG, "tile_right too large");
   // every warp region lies inside the dynamic allocation
   S->smem_bytes = (size_t)S->warp_words * 4 * dev::kWarpsPerCta;
   for (bool g : {false, true}) raise_smem_limit(dev::eval_kernel(S->variant, g, S->peq_shape.w), S->smem_bytes);
@@ -695,6 +703,7 @@ dev::EvalParams eval_params(hbx_session* S, const dev::Rule* rules) {
   P.n_symbols = S->E.n_symbols;
   P.rule_item_base = S->d_rule_base.p;
   P.tile_right = S->tile_right;
+  P.stage_rows = S->stage_rows;
   dev::set_layout(&P, S->wl, S->peq_shape, S->peq.p);
   P.out_l = S->ext_l ? S->ext_l : S->out_l.p;
   P.out_r = S->ext_l ? S->ext_r : S->out_r.p;
@@ -996,7 +1005,7 @@ void autotune(hbx_session* S, cudaStream_t st) {
       return;
     }
   }
-  std::vector<uint32_t> tiles = {32, 64, 96, 128};
+  std::vector<uint32_t> tiles = {32, 64, 96, 128, 288};
   std::vector<int> variants = {0, 1};
   if (o.tile_right > 0) tiles = {(uint32_t)o.tile_right};
   if (o.eval_variant > 0) variants = {o.eval_variant - 1};

@@ -1219,6 +1219,7 @@ constexpr uint32_t kMaxClaimChunk = 16;
 // member of its group has extra equality slots; bits 8-11 hold the group's
 // member count.
 constexpr uint32_t kItemSim = 1u, kItemExtras = 2u, kItemMore = 4u;  // more: n_sim > 1
+constexpr uint32_t kItemLast = 8u;  // of a staged piece: the item's last one
 __device__ __forceinline__ uint32_t item_members(uint32_t kind) { return (kind >> 8) & 15u; }
 // A claimed work item: the sources of its bulk copies (right-row metadata
 // from the block's first row, right rows from the 16-byte boundary at or
@@ -1573,7 +1574,7 @@ __device__ __forceinline__ uint32_t claim_chunk(const EvalParams& P, WarpCtl* C,
 __device__ __forceinline__ void claim_item(const EvalParams& P, WarpCtl* C, uint32_t b,
                                            uint32_t* buf, uint64_t* bar, unsigned long long n_work,
                                            uint32_t chunk, long long t_start, bool* stop,
-                                           uint32_t* d_pos, uint32_t* d_n,
+                                           uint32_t* d_pos, uint32_t* d_n, uint32_t* d_off,
                                            unsigned long long* done) {
   const int lane = threadIdx.x & 31;
   while (!*stop) {
@@ -1590,7 +1591,7 @@ __device__ __forceinline__ void claim_item(const EvalParams& P, WarpCtl* C, uint
       *stop = true;
       break;
     }
-    const ItemDesc d = C->desc[(*d_pos)++];
+    ItemDesc d = C->desc[*d_pos];
     if (!(d.kind & kItemSim)) {  // equalities only: every candidate matches
       for (uint32_t e = 0; e < d.n; e += 32) {
         const uint32_t k = e + (uint32_t)lane;
@@ -1598,8 +1599,21 @@ __device__ __forceinline__ void claim_item(const EvalParams& P, WarpCtl* C, uint
         emit(P, &C->out, k < d.n, d.lrow, rrow, d.rule, lane);
       }
       (*done)++;
+      (*d_pos)++;
       continue;
     }
+    // the next piece of the item that a buffer holds
+    const uint32_t off = *d_off, left = d.n - off;
+    d.n = min(left, P.stage_rows);
+    if (left > P.stage_rows) {
+      *d_off = off + d.n;
+    } else {
+      *d_off = 0;
+      (*d_pos)++;
+      d.kind |= kItemLast;
+    }
+    d.meta_src += off;
+    d.rows_src += off;
     if (lane == 0) {
       const uint32_t mbytes = d.n * (uint32_t)sizeof(StrMeta);
       const uint32_t rbytes = ((d.n + (d.pos & 3u)) * 4u + 15u) & ~15u;
@@ -1653,10 +1667,12 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
   const uint32_t chunk =
       (uint32_t)max(1ull, min((unsigned long long)kMaxClaimChunk, n_work / (n_warps * 8ull)));
   bool stop = false;
-  uint32_t d_pos = 0, d_n = 0;  // the warp's claimed descriptors not yet taken
+  // the warp's claimed descriptors not yet taken, and the rows of the first one
+  // already staged
+  uint32_t d_pos = 0, d_n = 0, d_off = 0;
   for (uint32_t b = 0; b < P.n_bufs; b++)
     claim_item(P, C, b, region + P.buf_off + b * P.buf_words, bar0 + b, n_work, chunk, t_start,
-               &stop, &d_pos, &d_n, done);
+               &stop, &d_pos, &d_n, &d_off, done);
   uint32_t cb = 0;      // buffer of the current item (buffer cb + k holds the k-th next)
   uint32_t phs = 0;     // bit b: mbarrier phase of buffer b
   bool active = false;  // current item waited for and being filtered
@@ -1695,7 +1711,7 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
         // the item is filtered: its buffer takes the item after the next one
         active = false;
         __syncwarp();
-        claim_item(P, C, cb, buf, bar0 + cb, n_work, chunk, t_start, &stop, &d_pos, &d_n, done);
+        claim_item(P, C, cb, buf, bar0 + cb, n_work, chunk, t_start, &stop, &d_pos, &d_n, &d_off, done);
         cb = cb + 1u == P.n_bufs ? 0u : cb + 1u;
         buf = region + P.buf_off + cb * P.buf_words;
         cur_n = C->c_n[cb];
@@ -1715,8 +1731,8 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
       }
       active = true;
       in_pos = 0;
-      (*done)++;
       const uint32_t ir = C->c_rule[cb], il = C->c_lrow[cb], kind = C->c_kind[cb];
+      if (kind & kItemLast) (*done)++;
       const float thr = C->c_thr[cb];
       __syncwarp();  // the previous item's fields are read
       C->i_rule = ir;

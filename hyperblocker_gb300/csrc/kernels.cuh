@@ -357,7 +357,8 @@ struct EvalParams {
   uint32_t n_seg;
   unsigned long long seg_begin[kMaxSegments];
   unsigned long long seg_end[kMaxSegments];
-  uint32_t tile_right;  // TR
+  uint32_t tile_right;  // TR: right rows per work item
+  uint32_t stage_rows;  // right rows per staging buffer (a multiple of 32)
   // shared-memory words per warp and offsets inside a warp's region (warp_layout)
   uint32_t warp_words, n_bufs, buf_off, buf_words, buf_rows_off, buf_lmeta_off, mbar_off, ctl_off;
   // Peq tables of the left strings (PeqShape): [left string slot][left row]

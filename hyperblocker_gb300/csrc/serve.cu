@@ -885,6 +885,7 @@ void launch_eval(hbx_server* S, Slot& B) {
   P.rule_item_base = B.d_base;
   P.n_seg = 0;
   P.tile_right = S->tile_right;
+  P.stage_rows = P.tile_right;
   dev::set_layout(&P, S->wl, B.shape, B.peq.p);
   P.out_l = B.out_l.p;
   P.out_r = B.out_r.p;

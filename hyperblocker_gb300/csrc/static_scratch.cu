@@ -366,6 +366,7 @@ void run_static(int device, const hbx_plan* plan, const hbx_table* left, const h
   P.rule_item_base = Y.rule_base;
   P.n_seg = 0;
   P.tile_right = Y.tile_right;
+  P.stage_rows = P.tile_right;
   dev::set_layout(&P, Y.wl, Y.shape, Y.peq);
   P.out_l = out->l_row;
   P.out_r = out->r_row;
