@@ -98,6 +98,7 @@ struct hbx_session {
   int variant = 0;  // evaluation kernel: 0 = k_eval, 1 = k_eval_wide
   bool groups = false;  // some rule evaluates others in the batched form (h_groups)
   bool long_left = false;  // some left string has no Peq table (k_eval_long)
+  hbx::DBuf<uint4> defer;  // with long_left: pairs left to k_eval_long
   bool tuned = false;
   bool one_shot = false;  // runs once (hbx_block): no graph is captured
   // output slots to start with; a run needing more than cap_limit (the
@@ -364,6 +365,9 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
   for (const RuleEnc& re : E.rules)
     for (int sl : re.sim_slot_l)
       if (E.L.str_maxlen[(size_t)sl] > dev::kMaxTableLen) S->long_left = true;
+  // (a few for every row, so that a small window's list stays small)
+  if (S->long_left)
+    S->defer.alloc(std::min<size_t>(dev::kDeferPairs, 1024 + 4 * ((size_t)nL + nR)));
   // join state of every rule (independent of the tile shape)
   S->rb.clear();
   S->rb.resize(E.rules.size());
@@ -712,14 +716,18 @@ dev::EvalParams eval_params(hbx_session* S, const dev::Rule* rules) {
   P.watchdog_cycles = S->ctx->opts.watchdog_cycles;
   P.seen = S->seen.p;
   P.seen_mask = S->seen.p ? S->seen.n - 1 : 0;
+  P.defer = S->defer.p;
+  P.defer_cap = (uint32_t)S->defer.n;
   return P;
 }
 
 void queue_counters(hbx_session* S, cudaStream_t st);
 
-// The work items of long left strings (or the range of them in P's segment).
-void launch_long(hbx_session* S, dev::EvalParams P, cudaStream_t st) {
+// The work items of long left strings (or the range of them in P's segment)
+// and / or the deferred pairs.
+void launch_long(hbx_session* S, dev::EvalParams P, bool items, bool deferred, cudaStream_t st) {
   P.rule_item_base += P.n_rules + 1;
+  P.long_what = (items ? 1u : 0u) | (deferred ? 2u : 0u);
   dev::k_eval_long<<<dev::long_grid(S->ctx->n_sm), kThreads, 0, st>>>(P);
   launch_check("k_eval_long");
 }
@@ -743,7 +751,7 @@ uint32_t enqueue_batched(hbx_session* S, cudaStream_t st) {
   dev::eval_kernel(S->variant, S->groups, S->peq_shape.w)<<<grid, kThreads, S->smem_bytes, st>>>(P);
   launch_check("k_eval");
   if (S->long_left) {
-    launch_long(S, P, st);
+    launch_long(S, P, true, true, st);
     launches++;
   }
   HBX_CUDA(cudaEventRecordWithFlags(S->ev_eval1, st, rec_flags));
@@ -865,7 +873,7 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
         HBX_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned long long), st));
         n++;
         if (c) {
-          launch_long(S, P, st);
+          launch_long(S, P, true, false, st);
           continue;
         }
         const unsigned long long ctas =
@@ -875,6 +883,10 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
         launch_check("k_eval (plain)");
       }
     }
+  }
+  if (S->long_left) {  // pairs that any of the launches deferred
+    launch_long(S, P, false, true, st);
+    n++;
   }
   HBX_CUDA(cudaEventRecord(S->ev_eval1, st));
   *launches = n;

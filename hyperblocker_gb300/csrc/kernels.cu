@@ -912,6 +912,21 @@ __device__ __noinline__ bool sim_pass_slow(const StrMeta* am, const StrMeta* bm,
   return jw_exact(m, mn, max(la, lb), p, thr, &ctr->ambiguous);
 }
 
+// The same for a pair inside the evaluation loop: one lane's loops over two
+// long strings hold up its warp for half a millisecond, so a pair that can
+// reach the threshold is left to k_eval_long where the launch has room for it.
+// 0 = fails, 1 = passes, 2 + k = the caller puts it on the list at k (< cap).
+__device__ __noinline__ uint32_t sim_slow_or_defer(const StrMeta* am, const StrMeta* bm,
+                                                   const uint8_t* a, const uint8_t* b, float thr,
+                                                   Counters* ctr, uint32_t cap) {
+  const uint32_t la = am->loc.y, lb = bm->loc.y;
+  if (cap && la && lb && can_reach(am, bm->head, bm->sig[0], bm->sig[1], la, lb, thr)) {
+    const unsigned long long at = atomicAdd(&ctr->deferred, 1ull);
+    if (at < cap) return 2u + (uint32_t)at;
+  }
+  return sim_pass_slow(am, bm, a, b, thr, ctr) ? 1u : 0u;
+}
+
 // Per-lane work counts of the evaluation loop, summed into Counters at exit:
 // algorithmic JW word operations (every evaluation, scanned or not), pairs
 // that reached a bit-parallel scan, and scan steps (4 symbols each).
@@ -1075,14 +1090,21 @@ __device__ __forceinline__ int advance_rule(const EvalParams& P, uint32_t rule, 
     const uint32_t la = al.y, lb = bl.y;
     const uint8_t* a = P.L.arena + 16ull * al.x;
     const uint8_t* b = P.R.arena + 16ull * bl.x;
-    if (!has_table(P, la)) {  // the reference's own loops
-      if (la && lb) ops->ops += jw_eval_ops(min(la, lb), max(la, lb));
-      if (!sim_pass_slow(am, bm, a, b, thr, P.ctr)) return 0;
+    if (la == 0 || lb == 0) {
+      if (!jw_exact(0, la, lb, 0, thr, &P.ctr->ambiguous)) return 0;
       continue;
     }
-    if (lb == 0) {
-      if (!jw_exact(0, la, 0, 0, thr, &P.ctr->ambiguous)) return 0;
-      continue;
+    if constexpr (W == kMaxTableLen / 32) {  // narrower masks: every string has a table
+      if (!has_table(P, la)) {
+        const uint32_t st = sim_slow_or_defer(am, bm, a, b, thr, P.ctr, P.defer_cap);
+        if (st >= 2u) {
+          P.defer[st - 2u] = make_uint4(lrow, rrow, rule, 1u);
+          return 0;
+        }
+        ops->ops += jw_eval_ops(min(la, lb), max(la, lb));
+        if (!st) return 0;
+        continue;
+      }
     }
     const uint32_t ls = min(la, lb), ll = max(la, lb);
     ops->ops += jw_eval_ops(ls, ll);
@@ -1165,14 +1187,21 @@ __device__ __forceinline__ int advance_group(const EvalParams& P, uint32_t rule,
       const uint32_t la = al.y, lb = bl.y;
       const uint8_t* a = P.L.arena + 16ull * al.x;
       const uint8_t* b = P.R.arena + 16ull * bl.x;
-      if (!has_table(P, la)) {  // the reference's own loops
-        if (la && lb) ops->ops += jw_eval_ops(min(la, lb), max(la, lb));
-        if (!sim_pass_slow(am, bm, a, b, thr, P.ctr)) break;
+      if (la == 0 || lb == 0) {
+        if (!jw_exact(0, la, lb, 0, thr, &P.ctr->ambiguous)) break;
         continue;
       }
-      if (lb == 0) {
-        if (!jw_exact(0, la, 0, 0, thr, &P.ctr->ambiguous)) break;
-        continue;
+      if constexpr (W == kMaxTableLen / 32) {  // narrower masks: every string has a table
+        if (!has_table(P, la)) {
+          const uint32_t st = sim_slow_or_defer(am, bm, a, b, thr, P.ctr, P.defer_cap);
+          if (st >= 2u) {  // with the members still live
+            P.defer[st - 2u] = make_uint4(lrow, rrow, rule, *live);
+            return 0;
+          }
+          ops->ops += jw_eval_ops(min(la, lb), max(la, lb));
+          if (!st) break;
+          continue;
+        }
       }
       const uint32_t ls = min(la, lb), ll = max(la, lb);
       ops->ops += jw_eval_ops(ls, ll);
@@ -1958,7 +1987,10 @@ __device__ __noinline__ bool long_pair_rest(const EvalParams& P, const Rule* R, 
 // reference's loops -- they were most of the time: 40,014 x 60,000 rows of
 // 64-256 characters, 2 % of the authors over 256 symbols, evaluation 37.5 ms
 // against 2.51 ms; and the evaluation kernels without that path need fewer
-// registers (8 rules, 150k x 150k rows: 14.06 against 13.91 ms).
+// registers (8 rules, 150k x 150k rows: 14.06 against 13.91 ms).  Pairs that
+// meet such a string at a later predicate (EvalParams::defer) follow: left to
+// their lanes they kept a few warps busy for 1.2 ms after all others (2.29
+// against 1.03 ms).
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_eval_long(
     const __grid_constant__ EvalParams P) {
   __shared__ OutBuf s_out[kWarpsPerCta];
@@ -1966,8 +1998,9 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_eval_long(
   OutBuf* O = s_out + (threadIdx.x >> 5);
   if (lane == 0) O->n = 0;
   __syncwarp();
-  const unsigned long long n_work =
-      P.n_seg ? P.seg_end[0] - P.seg_begin[0] : P.rule_item_base[P.n_rules];
+  const unsigned long long n_work = !(P.long_what & 1u) ? 0ull
+                                    : P.n_seg ? P.seg_end[0] - P.seg_begin[0]
+                                              : P.rule_item_base[P.n_rules];
   const long long t_start = clock64();
   unsigned long long done = 0, word_ops = 0;
   for (;;) {
@@ -2042,6 +2075,22 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_eval_long(
       emit(P, O, match, lrow, rrow, r, lane);
     }
     done++;
+  }
+  // the deferred pairs, one at a time by a warp
+  const unsigned long long n_def =
+      P.long_what & 2u ? min(P.ctr->deferred, (unsigned long long)P.defer_cap) : 0ull;
+  for (;;) {
+    unsigned long long v = n_def;
+    if (lane == 0 && n_def) v = atomicAdd(&P.ctr->deferred_next, 1ull);
+    v = __shfl_sync(kFull, v, 0);
+    if (v >= n_def) break;
+    if (P.watchdog_cycles && (unsigned long long)(clock64() - t_start) > P.watchdog_cycles) {
+      if (lane == 0) atomicAdd(&P.ctr->watchdog_trips, 1ull);
+      break;
+    }
+    const uint4 e = P.defer[v];
+    const bool ok = long_pair_rest(P, P.rules + e.z, e.w, e.x, e.y);
+    emit(P, O, ok && lane == 0, e.x, e.y, e.z, lane);
   }
   emit_drain(P, O, lane);
 #pragma unroll

@@ -341,6 +341,8 @@ struct Counters {
   unsigned long long scan_warp_steps;  // warp-level scan steps (any lane scanning)
   unsigned long long rest_scans;       // scans of predicates after a rule's or group's first
   unsigned long long work_next_long;   // k_eval_long's work_next
+  unsigned long long deferred;       // pairs put on EvalParams::defer (and those it had no room for)
+  unsigned long long deferred_next;  // and taken from it
 };
 
 struct EvalParams {
@@ -369,6 +371,12 @@ struct EvalParams {
   unsigned long long capacity;
   Counters* ctr;
   unsigned long long watchdog_cycles;  // 0 = no budget
+  // Pairs that reached a predicate whose left string has no Peq table, for
+  // k_eval_long: {left row, right row, rule, live members}; null: decided in
+  // the lane, as are those it has no room for
+  uint4* defer;
+  uint32_t defer_cap;
+  uint32_t long_what;  // k_eval_long: bit 0 = work items, bit 1 = deferred pairs
   // set of the reported (left, right) keys that another rule may report too
   // (plans with several rules, else null)
   unsigned long long* seen;
@@ -489,10 +497,12 @@ __global__ void k_peq_build(Side L, uint32_t n_slots, PeqShape shape, uint32_t* 
 // k_eval_groups_wide<W>: launches where some rule evaluates others).
 using EvalKernel = void (*)(EvalParams);
 // The work items of left strings without a Peq table (class 1; rule_item_base
-// points at their bases), for groups and rules alike: grid
-// long_grid(number of SMs), kWarpsPerCta * 32 threads.
+// points at their bases) and the pairs that the evaluation kernels deferred
+// (EvalParams::long_what), for groups and rules alike: grid long_grid(number
+// of SMs), kWarpsPerCta * 32 threads.
 __global__ void k_eval_long(const __grid_constant__ EvalParams P);
 inline int long_grid(int n_sm) { return n_sm * 4; }
+constexpr uint32_t kDeferPairs = 1u << 20;  // most room for deferred pairs of a run
 EvalKernel eval_kernel(int wide, bool groups, uint32_t peq_w);
 constexpr uint32_t kPeqWidths[] = {1, 2, 3, 4, 8};  // every PeqShape::w
 

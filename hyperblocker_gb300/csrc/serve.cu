@@ -273,6 +273,7 @@ struct Slot {
   dev::PeqShape shape{};   // Peq tables of this batch's left strings
   bool long_left = false;  // some left string may have no Peq table (k_eval_long)
   DBuf<uint32_t> peq;
+  DBuf<uint4> defer;  // with long_left: pairs left to k_eval_long
   Pinned stage, h_out, h_ctr;  // h_ctr: total items + Counters + comparisons per instance
   ~Slot() {
     release();  // buffers return to the pool on this slot's stream first
@@ -291,6 +292,7 @@ struct Slot {
     out_l.reset();
     out_r.reset();
     peq.reset();
+    defer.reset();
     capacity = 0;
     state = 0;
   }
@@ -860,6 +862,7 @@ void launch_batch(hbx_server* S, Slot& B) {
   k_scatter_left<<<grid, 256, 0, st>>>(B.d_rules, ni, d_rows, B.d_base);
   check_launch("serving batch join");
 
+  if (B.long_left) B.defer.alloc(1 << 16);
   B.capacity = std::max<uint64_t>(1 << 16, 2ull * N);
   B.out_l.alloc(B.capacity);
   B.out_r.alloc(B.capacity);
@@ -887,6 +890,8 @@ void launch_eval(hbx_server* S, Slot& B) {
   P.tile_right = S->tile_right;
   P.stage_rows = P.tile_right;
   dev::set_layout(&P, S->wl, B.shape, B.peq.p);
+  P.defer = B.defer.p;
+  P.defer_cap = (uint32_t)B.defer.n;
   P.out_l = B.out_l.p;
   P.out_r = B.out_r.p;
   P.capacity = B.capacity;
@@ -898,6 +903,7 @@ void launch_eval(hbx_server* S, Slot& B) {
   dev::eval_kernel(S->variant, false, B.shape.w)<<<grid, kThreads, S->smem_bytes, st>>>(P);
   if (B.long_left) {
     P.rule_item_base += ni + 1;
+    P.long_what = 3u;
     dev::k_eval_long<<<dev::long_grid(S->ctx->n_sm), kThreads, 0, st>>>(P);
   }
   check_launch("serving k_eval");

@@ -389,6 +389,7 @@ void run_static(int device, const hbx_plan* plan, const hbx_table* left, const h
   kern<<<n_sm * std::max(1, bps), dev::kWarpsPerCta * 32, smem, st>>>(P);
   if (Y.long_left) {
     P.rule_item_base += P.n_rules + 1;
+    P.long_what = 1u;  // no room for deferred pairs in the scratch
     dev::k_eval_long<<<dev::long_grid(n_sm), dev::kWarpsPerCta * 32, 0, st>>>(P);
   }
   HBX_STATIC_CUDA(cudaGetLastError());

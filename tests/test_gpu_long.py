@@ -100,3 +100,27 @@ def test_serving_and_static(ctx, docs):
                                      None, ctypes.byref(st)) == hb.OK
     got = out[:, :p.n_written].cpu().numpy().view(np.uint32).T
     assert np.array_equal(_util.sorted_pairs(got), _oracle(docs, cl, cr, 1).pairs)
+
+
+@pytest.mark.parametrize("docs", [ONE, GROUP])
+def test_more_pairs_than_the_list_of_deferred_ones_holds(ctx, docs):
+    """Every pair passes a short first string and meets a long second one: 9,600 pairs for a list
+    of 1,024 + 4 x 200; the others are decided in their lanes."""
+    rng = np.random.Generator(np.random.PCG64(3))
+    base = bytes(rng.choice(list(b"abcdefgh"), size=300).tolist())
+
+    def table(n, prefix):
+        s2 = [base[:257 + i % 40] + bytes(rng.choice(list(b"ab"), size=3 * (i % 9)).tolist())
+              for i in range(n)]
+        return [[b"id"] + [f"{prefix}{i}".encode() for i in range(n)],
+                [b"s1"] + [b"abcd"] * n, [b"s2"] + s2,
+                [b"k1"] + [b"1"] * n, [b"k2"] + [b"%d" % (i % 2) for i in range(n)]]
+
+    cl, cr = table(80, "l"), table(120, "r")
+    want = _oracle(docs, cl, cr, 1)
+    assert len(want.pairs) > 1000
+    plan = hb.Plan.from_yaml(docs, ctx)
+    left, right = hb.Table.from_columns(cl, ctx), hb.Table.from_columns(cr, ctx)
+    for mode in ("plain", "batched"):
+        got, _ = hb.block(ctx, plan, left, right, 1, _util.INT_MAX, mode)
+        assert np.array_equal(_util.sorted_pairs(got), want.pairs), mode
