@@ -1,13 +1,12 @@
 // sort.cu -- (left row, right row) pairs sorted on the device, for output in
-// row order: a least-significant-digit radix sort of the 64-bit keys
-// left << 32 | right, 8 bits per pass, over the bytes the row counts use.
+// row order: a least-significant-digit radix sort of keys left << b | right
+// (b bits hold a right row), 8 bits per pass.
 //
-// A pass histograms the digit per tile of kTile keys, scans the histograms
-// digit-major (all tiles' counts of digit 0, then digit 1, ...) into the
-// first position of every (digit, tile), and scatters each tile's keys in
-// order: rounds of 256 keys, a warp ranks its 32 keys among equal digits with
-// __match_any_sync, per-warp counts give each warp's start per digit, and a
-// running count per digit carries across rounds, so the sort is stable.
+// One launch counts every pass's digits.  A pass is then one launch: a block
+// ranks a tile of kTile keys, publishes its counts per digit, adds the counts
+// of the tiles before it (looking back tile by tile, as far as the first that
+// has published its sum) and scatters.  The first pass reads the pairs and the
+// last one writes them back, so that no launch only converts.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -20,119 +19,213 @@
 namespace hbx {
 namespace srt {
 
-constexpr uint32_t kThreads = 256;
-constexpr uint32_t kRounds = 8;
-constexpr uint32_t kTile = kThreads * kRounds;  // keys per tile
+constexpr uint32_t kThreads = 256, kWarps = kThreads / 32;
+constexpr uint32_t kKeys = 8;                // keys per thread
+constexpr uint32_t kTile = kThreads * kKeys;  // keys per tile
+constexpr uint32_t kMaxPasses = 8;
+constexpr uint32_t kBack = 8;  // tiles read at once when looking back
+// A wait for another tile's counts ends after this many polls (each some
+// microsecond); the block then counts the keys before its tile itself.
+constexpr uint32_t kWaitPolls = 1u << 20;
 constexpr unsigned kFull = 0xffffffffu;
 
-__global__ void k_pack(const uint32_t* l, const uint32_t* r, uint64_t n, unsigned long long* key) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    key[i] = ((unsigned long long)l[i] << 32) | r[i];
-}
-
-__global__ void k_unpack(const unsigned long long* key, uint64_t n, uint32_t* l, uint32_t* r) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    l[i] = (uint32_t)(key[i] >> 32);
-    r[i] = (uint32_t)key[i];
+struct Pairs {
+  uint32_t *l, *r;
+  uint64_t n;
+  uint32_t bits_r;
+  __device__ unsigned long long key(uint64_t i) const {
+    return (unsigned long long)l[i] << bits_r | r[i];
   }
-}
+};
 
-// hist[digit * n_tiles + tile]: keys of the tile with that digit.
-__global__ void __launch_bounds__(kThreads) k_hist(const unsigned long long* key, uint64_t n,
-                                                   uint32_t shift, uint32_t n_tiles,
-                                                   uint32_t* hist) {
-  __shared__ uint32_t h[256];
-  const uint32_t tile = blockIdx.x;
-  h[threadIdx.x] = 0;
+// count[pass * 256 + digit] over all keys.
+__global__ void __launch_bounds__(kThreads) k_digits(Pairs p, uint32_t n_passes, uint32_t* count) {
+  __shared__ uint32_t h[kMaxPasses * 256];
+  for (uint32_t k = threadIdx.x; k < n_passes * 256; k += kThreads) h[k] = 0;
   __syncthreads();
-  const uint64_t base = (uint64_t)tile * kTile;
-  for (uint32_t k = 0; k < kRounds; k++) {
-    const uint64_t i = base + k * kThreads + threadIdx.x;
-    if (i < n) atomicAdd(&h[(uint32_t)(key[i] >> shift) & 0xffu], 1u);
+  for (uint64_t i = blockIdx.x * (uint64_t)kThreads + threadIdx.x; i < p.n;
+       i += (uint64_t)gridDim.x * kThreads) {
+    const unsigned long long v = p.key(i);
+    for (uint32_t q = 0; q < n_passes; q++)
+      atomicAdd(&h[q * 256 + ((uint32_t)(v >> (8 * q)) & 0xffu)], 1u);
   }
   __syncthreads();
-  hist[(uint64_t)threadIdx.x * n_tiles + tile] = h[threadIdx.x];
+  for (uint32_t k = threadIdx.x; k < n_passes * 256; k += kThreads)
+    if (h[k]) atomicAdd(&count[k], h[k]);
 }
 
-// Scatters one tile's keys, in order, to off[digit * n_tiles + tile] on.
-__global__ void __launch_bounds__(kThreads) k_scatter(const unsigned long long* key, uint64_t n,
-                                                      uint32_t shift, uint32_t n_tiles,
-                                                      const uint32_t* off,
-                                                      unsigned long long* out) {
-  __shared__ uint32_t wcnt[kThreads / 32][256];  // this round's keys per warp and digit
-  __shared__ uint32_t wpre[kThreads / 32][256];  // where each warp starts, per digit
-  __shared__ uint32_t run[256];                  // keys of earlier rounds per digit
-  const uint32_t tile = blockIdx.x;
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  run[threadIdx.x] = off[(uint64_t)threadIdx.x * n_tiles + tile];
-  const uint64_t base = (uint64_t)tile * kTile;
-  for (uint32_t k = 0; k < kRounds; k++) {
-    for (uint32_t w = 0; w < kThreads / 32; w++) wcnt[w][threadIdx.x] = 0;
-    __syncthreads();
-    const uint64_t i = base + k * kThreads + threadIdx.x;
-    const bool act = i < n;
-    const unsigned long long v = act ? key[i] : 0ull;
-    const uint32_t d = act ? (uint32_t)(v >> shift) & 0xffu : 256u + lane;  // inactive: unique
+// A tile's word per digit: the keys of the tile (kCount) or of it and all
+// tiles before it (kSum) with that digit, the state in the two highest bits.
+template <class T>
+struct State {
+  static constexpr int kShift = 8 * sizeof(T) - 2;
+  static constexpr T kCount = (T)1 << kShift, kSum = (T)2 << kShift, kValue = kCount - 1;
+};
+
+// One pass.  What bounds it at 10^5 pairs is latency: a launch, the ranks (a
+// warp ranks 8 rounds of its own 256 keys without a block barrier), the look
+// back (8 tiles at a time: their words arrive together).  In turn a
+// histogram, a scan and a scatter launch per pass took 24 us for 100,000
+// pairs, 126 us a sort with the packing launches.
+// Tiles are handed out by a ticket, so the tiles before a block's own are
+// running or done.  next: the other pass's words, cleared for it.
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_pass(Pairs p, const unsigned long long* src,
+                                                   unsigned long long* dst, uint32_t shift,
+                                                   const uint32_t* count, uint32_t* ticket, T* state,
+                                                   T* next) {
+  using S = State<T>;
+  __shared__ uint32_t s_cnt[kWarps][256];  // a warp's keys per digit, then where they start
+  __shared__ uint32_t s_base[256];         // the tile's first position per digit
+  __shared__ uint32_t s_warp[kWarps];
+  __shared__ uint32_t s_tile;
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  if (t == 0) s_tile = atomicAdd(ticket, 1u);
+  for (uint32_t k = lane; k < 256; k += 32) s_cnt[warp][k] = 0;
+  __syncthreads();
+  const uint32_t tile = s_tile;
+  const uint64_t base = (uint64_t)tile * kTile + warp * (32 * kKeys) + lane;
+  unsigned long long v[kKeys];
+  uint32_t rank[kKeys];
+#pragma unroll
+  for (uint32_t k = 0; k < kKeys; k++) {
+    const uint64_t i = base + 32 * k;
+    v[k] = i >= p.n ? 0ull : src ? src[i] : p.key(i);
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < kKeys; k++) {
+    const bool act = base + 32 * k < p.n;
+    const uint32_t d = act ? (uint32_t)(v[k] >> shift) & 0xffu : 256u + lane;  // inactive: unique
     const unsigned peers = __match_any_sync(kFull, d);
-    const uint32_t rank = (uint32_t)__popc(peers & ((1u << lane) - 1u));
-    if (act && rank == 0) wcnt[warp][d] = (uint32_t)__popc(peers);
-    __syncthreads();
-    {  // thread t: digit t over the warps, in order
-      uint32_t acc = run[threadIdx.x];
-      for (uint32_t w = 0; w < kThreads / 32; w++) {
-        wpre[w][threadIdx.x] = acc;
-        acc += wcnt[w][threadIdx.x];
-      }
-      run[threadIdx.x] = acc;
+    const uint32_t before = (uint32_t)__popc(peers & ((1u << lane) - 1u));
+    const uint32_t had = act ? s_cnt[warp][d] : 0u;
+    __syncwarp();
+    if (act && before == 0) s_cnt[warp][d] = had + (uint32_t)__popc(peers);
+    __syncwarp();
+    rank[k] = had + before;
+  }
+  __syncthreads();
+  // thread t: digit t
+  uint32_t mine = 0;
+#pragma unroll
+  for (uint32_t w = 0; w < kWarps; w++) {
+    const uint32_t c = s_cnt[w][t];
+    s_cnt[w][t] = mine;
+    mine += c;
+  }
+  volatile T* words = state;
+  const uint64_t at = (uint64_t)tile * 256 + t;
+  words[at] = (T)mine | (tile ? S::kCount : S::kSum);
+  next[at] = 0;
+  // where the digit starts: all keys with smaller digits
+  const uint32_t all = count[t];
+  uint32_t inc = all;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, inc, o);
+    if ((int)lane >= o) inc += y;
+  }
+  if (lane == 31) s_warp[warp] = inc;
+  __syncthreads();
+  uint32_t first = inc - all;
+  for (uint32_t w = 0; w < warp; w++) first += s_warp[w];
+  // the tiles before this one
+  T sum = 0;
+  int64_t j = (int64_t)tile - 1;
+  uint32_t polls = 0;
+  bool done = tile == 0;
+  while (!done && polls < kWaitPolls) {
+    T w[kBack];
+#pragma unroll
+    for (uint32_t u = 0; u < kBack; u++)
+      w[u] = j >= (int64_t)u ? (T)words[(uint64_t)(j - u) * 256 + t] : S::kSum;
+    uint32_t got = 0;
+#pragma unroll
+    for (uint32_t u = 0; u < kBack; u++) {
+      if (done || got != u || !(w[u] & ~S::kValue)) continue;
+      sum += w[u] & S::kValue;
+      got++;
+      done = (w[u] & S::kSum) != 0;
     }
+    j -= got;
+    if (got == 0) {
+      polls++;
+      __nanosleep(32);
+    }
+  }
+  if (__syncthreads_or(!done)) {  // a wait gave up: the keys themselves
+    s_base[t] = 0;
     __syncthreads();
-    if (act) out[wpre[warp][d] + rank] = v;
+    for (uint64_t i = t; i < (uint64_t)tile * kTile; i += kThreads)
+      atomicAdd(&s_base[(uint32_t)((src ? src[i] : p.key(i)) >> shift) & 0xffu], 1u);
+    __syncthreads();
+    sum = s_base[t];
     __syncthreads();
   }
+  if (tile) words[at] = (sum + (T)mine) | S::kSum;
+  s_base[t] = first + (uint32_t)sum;
+  __syncthreads();
+#pragma unroll
+  for (uint32_t k = 0; k < kKeys; k++) {
+    if (base + 32 * k >= p.n) continue;
+    const uint32_t d = (uint32_t)(v[k] >> shift) & 0xffu;
+    const uint32_t to = s_base[d] + s_cnt[warp][d] + rank[k];
+    if (dst) {
+      dst[to] = v[k];
+    } else {
+      p.l[to] = (uint32_t)(v[k] >> p.bits_r);
+      p.r[to] = (uint32_t)(v[k] & ((1ull << p.bits_r) - 1));
+    }
+  }
+}
+
+template <class T>
+void queue_passes(Pairs p, uint32_t n_passes, int n_sm, cudaStream_t st) {
+  const uint32_t n_tiles = (uint32_t)((p.n + kTile - 1) / kTile);
+  const uint64_t words = 256ull * n_tiles;
+  // two passes and more: the first reads the pairs that the last overwrites
+  DBuf<unsigned long long> a, b;
+  a.alloc(p.n);
+  if (n_passes > 2) b.alloc(p.n);
+  DBuf<uint32_t> count;  // digit counts, tickets
+  DBuf<T> state;
+  count.alloc((size_t)kMaxPasses * 256 + kMaxPasses);
+  state.alloc(2 * words);
+  HBX_CUDA(cudaMemsetAsync(count.p, 0, count.n * 4, st));
+  HBX_CUDA(cudaMemsetAsync(state.p, 0, words * sizeof(T), st));
+  k_digits<<<std::min<uint32_t>(n_tiles, (uint32_t)n_sm * 4), kThreads, 0, st>>>(p, n_passes, count.p);
+  for (uint32_t q = 0; q < n_passes; q++) {
+    const unsigned long long* src = q == 0 ? nullptr : q & 1 ? a.p : b.p;
+    unsigned long long* dst = q + 1 == n_passes ? nullptr : q & 1 ? b.p : a.p;
+    k_pass<T><<<n_tiles, kThreads, 0, st>>>(p, src, dst, 8 * q, count.p + 256 * q,
+                                            count.p + 256 * kMaxPasses + q, state.p + (q & 1) * words,
+                                            state.p + (~q & 1) * words);
+  }
+  check_launch("pair sort");
 }
 
 }  // namespace srt
 
 // Queues the sort of n pairs by (left row, right row) in place on st; rows
-// below n_left / n_right (the bytes of the keys beyond them are 0 and take no
-// pass).  Its buffers come from the calling thread's pool on st.
+// are below n_left / n_right, and bits of the keys beyond those take no pass.
+// Its buffers come from the calling thread's pool on st.
 void queue_pair_sort(int n_sm, cudaStream_t st, uint32_t* l, uint32_t* r, uint64_t n,
                      uint32_t n_left, uint32_t n_right) {
   if (n < 2) return;
   if (n >= (1ull << 32)) fail(HBX_ERR_UNSUPPORTED, "more than 2^32 pairs to sort");
-  auto bytes_of = [](uint32_t rows) {
+  auto bits_of = [](uint32_t rows) {
     uint32_t b = 0;
-    while (b < 4 && (uint64_t)rows > (1ull << (8 * b))) b++;
-    return b;  // digit bytes that hold row indices below rows
+    while ((uint64_t)rows > (1ull << b)) b++;
+    return b;  // bits that hold row indices below rows
   };
-  const uint32_t br = bytes_of(n_right), bl = bytes_of(n_left);
-  DBuf<unsigned long long> a, b;
-  a.alloc(n);
-  b.alloc(n);
-  const int g = grid_for(n, n_sm);
-  srt::k_pack<<<g, 256, 0, st>>>(l, r, n, a.p);
-  const uint32_t n_tiles = (uint32_t)((n + srt::kTile - 1) / srt::kTile);
-  const uint64_t nh = 256ull * n_tiles;
-  if (nh >= (1ull << 32)) fail(HBX_ERR_UNSUPPORTED, "too many pairs to sort");
-  DBuf<uint32_t> hist, off;
-  hist.alloc(nh);
-  off.alloc(nh);
-  unsigned long long* src = a.p;
-  unsigned long long* dst = b.p;
-  for (uint32_t byte = 0; byte < 8; byte++) {
-    const bool used = byte < 4 ? byte < br : byte - 4 < bl;
-    if (!used) continue;
-    const uint32_t shift = 8 * byte;
-    srt::k_hist<<<n_tiles, srt::kThreads, 0, st>>>(src, n, shift, n_tiles, hist.p);
-    scan_u32(hist.p, (uint32_t)nh, off.p, st);
-    srt::k_scatter<<<n_tiles, srt::kThreads, 0, st>>>(src, n, shift, n_tiles, off.p, dst);
-    check_launch("pair sort");
-    std::swap(src, dst);
-  }
-  srt::k_unpack<<<g, 256, 0, st>>>(src, n, l, r);
-  check_launch("pair sort");
+  const uint32_t br = bits_of(n_right), bl = bits_of(n_left);
+  const uint32_t n_passes = std::max(2u, (bl + br + 7) / 8);
+  const srt::Pairs p{l, r, n, br};
+  // the words' values go up to n
+  if (n < (1ull << 30))
+    srt::queue_passes<uint32_t>(p, n_passes, n_sm, st);
+  else
+    srt::queue_passes<unsigned long long>(p, n_passes, n_sm, st);
 }
 
 // The same on the context's stream; returns when the pairs are sorted.
