@@ -64,9 +64,9 @@ struct State {
 
 // One pass.  What bounds it at 10^5 pairs is latency: a launch, the ranks (a
 // warp ranks 8 rounds of its own 256 keys without a block barrier), the look
-// back (8 tiles at a time: their words arrive together).  In turn a
-// histogram, a scan and a scatter launch per pass took 24 us for 100,000
-// pairs, 126 us a sort with the packing launches.
+// back (8 tiles at a time: their words arrive together).  100,000 pairs take
+// 8.7 us a pass and 43 us a sort; a histogram, a scan and a scatter launch per
+// pass took 24 us, and 126 us a sort with the packing launches.
 // Tiles are handed out by a ticket, so the tiles before a block's own are
 // running or done.  next: the other pass's words, cleared for it.
 template <class T>
