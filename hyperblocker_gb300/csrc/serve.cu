@@ -270,6 +270,7 @@ struct Slot {
   DBuf<uint32_t> out_l, out_r;
   uint64_t capacity = 0;
   bool sorted = false;  // the pairs copied back were sorted on the device
+  bool copied = false;  // the pairs came with the evaluation's report
   dev::PeqShape shape{};   // Peq tables of this batch's left strings
   bool long_left = false;  // some left string may have no Peq table (k_eval_long)
   DBuf<uint32_t> peq;
@@ -880,7 +881,34 @@ void launch_batch(hbx_server* S, Slot& B) {
   B.h_ctr.ensure(sizeof(dev::Counters) + 8 + 8ull * ni);
 }
 
-// The evaluation launch of a batch and the copy of its counters.
+// A batch's pairs are sorted by (batch row, right row), so that each entry's
+// are one run: on the device from this many on, else on the host.  A device
+// sort is about 8 operations, whatever it sorts, the host's takes longer with
+// every pair: a burst of 24 requests, 14,011 records, 279,498 pairs, takes
+// 2.3 ms with device sorts and 14.5 ms with host sorts.
+constexpr uint64_t kDeviceSortPairs = 2048;
+
+// What the host reads after a batch's evaluation, written to page-locked host
+// memory by one launch: the items' total, the counters and the comparisons
+// (words, side by side), and the pairs when there are fewer than a device
+// sort takes (left rows, then right rows).  A batch's few pairs need no copy
+// of their own then, nor the host a second wait: a request of 16 records
+// takes 174 us, with copies of the counters and then of the pairs 257 us.
+static_assert(sizeof(dev::Counters) % 8 == 0, "reported in 8-byte words");
+__global__ void k_report(const unsigned long long* words, uint32_t n_words, const dev::Counters* ctr,
+                         const uint32_t* l, const uint32_t* r, unsigned long long capacity,
+                         unsigned long long* h_words, uint32_t* h_out) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  for (uint32_t i = t; i < n_words; i += step) h_words[i] = words[i];
+  const unsigned long long n = ctr->out_count;
+  if (n >= kDeviceSortPairs || n > capacity) return;
+  for (uint32_t i = t; i < (uint32_t)n; i += step) {
+    h_out[i] = l[i];
+    h_out[n + i] = r[i];
+  }
+}
+
+// The evaluation launch of a batch and the report to the host.
 void launch_eval(hbx_server* S, Slot& B) {
   cudaStream_t st = B.st;
   const uint32_t ni = (uint32_t)B.inst_entry.size();
@@ -913,9 +941,12 @@ void launch_eval(hbx_server* S, Slot& B) {
     dev::k_eval_long<<<dev::long_grid(S->ctx->n_sm), kThreads, 0, st>>>(P);
   }
   check_launch("serving k_eval");
-  // the items' total, the counters and the comparisons lie side by side
-  HBX_CUDA(cudaMemcpyAsync(B.h_ctr.p, B.d_base + dev::item_base_words(ni) - 1,
-                           8 + sizeof(dev::Counters) + 8ull * ni, cudaMemcpyDeviceToHost, st));
+  B.h_out.ensure(8 * kDeviceSortPairs);
+  k_report<<<4, 512, 0, st>>>(B.d_base + dev::item_base_words(ni) - 1,
+                              1 + (uint32_t)(sizeof(dev::Counters) / 8) + ni, B.d_ctr, B.out_l.p,
+                              B.out_r.p, B.capacity, static_cast<unsigned long long*>(B.h_ctr.p),
+                              static_cast<uint32_t*>(B.h_out.p));
+  check_launch("serving report");
   HBX_CUDA(cudaEventRecord(B.ev_eval, st));
   B.state = 1;
 }
@@ -974,12 +1005,6 @@ void fail_batch(hbx_server* S, Slot& B, hbx_status status, const std::string& wh
   S->in_use -= B.est;
 }
 
-// A batch's pairs are sorted by (batch row, right row), so that each entry's
-// are one run: on the device from this many on, else on the host.  A device
-// sort is about 8 operations, whatever it sorts, the host's takes longer with
-// every pair: a burst of 24 requests, 14,011 records, 279,498 pairs, takes
-// 2.3 ms with device sorts and 14.5 ms with host sorts.
-constexpr uint64_t kDeviceSortPairs = 2048;
 
 // Advances one batch; returns true when something happened.
 bool progress(hbx_server* S, Slot& B) {
@@ -1015,10 +1040,14 @@ bool progress(hbx_server* S, Slot& B) {
       return true;
     }
     const uint64_t n = c.out_count;
-    B.h_out.ensure(std::max<uint64_t>(8 * n, 16));
-    uint32_t* ho = (uint32_t*)B.h_out.p;
     B.sorted = false;
-    if (n >= kDeviceSortPairs && n < (1ull << 31)) {
+    B.capacity = n;  // from here on: the number of pairs copied back
+    B.state = 2;
+    B.copied = n < kDeviceSortPairs;
+    if (B.copied) return true;  // by the report
+    B.h_out.ensure(8 * n);
+    uint32_t* ho = (uint32_t*)B.h_out.p;
+    if (n < (1ull << 31)) {
       PoolScope scope(S->ctx->pool, B.st);
       try {
         queue_pair_sort(S->ctx->n_sm, B.st, B.out_l.p, B.out_r.p, n, B.n_rows, S->n_right);
@@ -1028,17 +1057,13 @@ bool progress(hbx_server* S, Slot& B) {
         cudaGetLastError();
       }
     }
-    if (n) {
-      HBX_CUDA(cudaMemcpyAsync(ho, B.out_l.p, 4 * n, cudaMemcpyDeviceToHost, B.st));
-      HBX_CUDA(cudaMemcpyAsync(ho + n, B.out_r.p, 4 * n, cudaMemcpyDeviceToHost, B.st));
-    }
+    HBX_CUDA(cudaMemcpyAsync(ho, B.out_l.p, 4 * n, cudaMemcpyDeviceToHost, B.st));
+    HBX_CUDA(cudaMemcpyAsync(ho + n, B.out_r.p, 4 * n, cudaMemcpyDeviceToHost, B.st));
     HBX_CUDA(cudaEventRecord(B.ev_out, B.st));
-    B.capacity = n;  // from here on: the number of pairs copied back
-    B.state = 2;
     return true;
   }
   if (B.state == 2) {
-    const cudaError_t q = cudaEventQuery(B.ev_out);
+    const cudaError_t q = B.copied ? cudaSuccess : cudaEventQuery(B.ev_out);
     if (q == cudaErrorNotReady) return false;
     HBX_CUDA(q);
     float ms = 0;
