@@ -18,8 +18,10 @@ struct hbx_ctx {
   std::string err;
   std::string device_name;  // keys the autotuner's cache
   void* h_ctr = nullptr;    // page-locked counters of the context's session runs
-  // page-locked staging of one-shot results: two chunks of kOutChunkBytes,
-  // each with the event of its device-to-host copy (allocated on first use)
+  void* h_few = nullptr;    // page-locked pairs of small one-shot results (on first use)
+  // page-locked staging of larger ones: two chunks of h_out_chunk bytes, each
+  // with the event of its device-to-host copy (as large as a result needed)
   void* h_out = nullptr;
+  size_t h_out_chunk = 0;
   cudaEvent_t h_out_ev[2] = {nullptr, nullptr};
 };

@@ -101,6 +101,7 @@ struct hbx_session {
   hbx::DBuf<uint4> defer;  // with long_left: pairs left to k_eval_long
   bool tuned = false;
   bool one_shot = false;  // runs once (hbx_block): no graph is captured
+  uint32_t* h_few = nullptr;  // page-locked room for kFewPairs pairs, reported with the counters
   // output slots to start with; a run needing more than cap_limit (the
   // caller's buffer, 0 = none) returns its count without growing and rerunning
   uint64_t out_hint = 1 << 16, cap_limit = 0;
@@ -788,9 +789,22 @@ void grow_output(hbx_session* S, const dev::Counters& c) {
   }
 }
 
+// A one-shot result of at most this many pairs comes with the counters.  Up
+// to there the report's launch stays short (512 KB over the link, some 10 us);
+// a larger result's copies run at the link's rate through large chunks.
+constexpr uint32_t kFewPairs = 1u << 16;
+
 // Queues the copy of the counters (with the run's work-item total) into the
 // context's page-locked block (a graph node when captured).
 void queue_counters(hbx_session* S, cudaStream_t st) {
+  if (S->h_few) {
+    dev::k_report<<<32, 256, 0, st>>>(reinterpret_cast<const unsigned long long*>(S->d_ctr.p),
+                                      (uint32_t)(sizeof(dev::Counters) / 8), S->d_ctr.p, S->out_l.p,
+                                      S->out_r.p, S->out_l.n, kFewPairs,
+                                      reinterpret_cast<unsigned long long*>(S->h_ctr), S->h_few);
+    launch_check("k_report");
+    return;
+  }
   HBX_CUDA(cudaMemcpyAsync(S->h_ctr, S->d_ctr.p, sizeof(dev::Counters), cudaMemcpyDeviceToHost, st));
 }
 
@@ -1313,14 +1327,25 @@ void parallel_copy(void* dst, const void* src, size_t bytes) {
 // into place.  (Straight into a caller's pageable arrays the copy ran at
 // 5.5 GB/s on GB300; through one staging buffer of the whole output it
 // slowed from 190 to about 30 GB/s once the host had read that buffer.)
+// The chunks are as large as the largest array of a result so far, from 1 to
+// 256 MiB (page-locking twice 256 MiB takes 17 ms).
 constexpr size_t kOutChunkBytes = 256ull << 20;
 void copy_out(hbx_ctx* ctx, cudaStream_t st, void* const* dst, const void* const* src,
               const size_t* bytes, int n_arrays) {
-  if (!ctx->h_out) {
-    HBX_CUDA(cudaHostAlloc(&ctx->h_out, 2 * kOutChunkBytes, cudaHostAllocPortable));
-    for (cudaEvent_t& e : ctx->h_out_ev)
-      HBX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  size_t chunk = 1ull << 20;
+  for (int a = 0; a < n_arrays; a++)
+    while (chunk < bytes[a] && chunk < kOutChunkBytes) chunk *= 2;
+  if (chunk > ctx->h_out_chunk) {
+    void* old = ctx->h_out;
+    ctx->h_out = nullptr;
+    ctx->h_out_chunk = 0;
+    if (old) HBX_CUDA(cudaFreeHost(old));
+    HBX_CUDA(cudaHostAlloc(&ctx->h_out, 2 * chunk, cudaHostAllocPortable));
+    ctx->h_out_chunk = chunk;
   }
+  chunk = ctx->h_out_chunk;
+  for (cudaEvent_t& e : ctx->h_out_ev)
+    if (!e) HBX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   struct Piece {
     char* dst;
     const char* src;
@@ -1328,10 +1353,10 @@ void copy_out(hbx_ctx* ctx, cudaStream_t st, void* const* dst, const void* const
   };
   std::vector<Piece> pieces;
   for (int a = 0; a < n_arrays; a++)
-    for (size_t off = 0; off < bytes[a]; off += kOutChunkBytes)
+    for (size_t off = 0; off < bytes[a]; off += chunk)
       pieces.push_back({static_cast<char*>(dst[a]) + off, static_cast<const char*>(src[a]) + off,
-                        std::min(kOutChunkBytes, bytes[a] - off)});
-  char* slot[2] = {static_cast<char*>(ctx->h_out), static_cast<char*>(ctx->h_out) + kOutChunkBytes};
+                        std::min(chunk, bytes[a] - off)});
+  char* slot[2] = {static_cast<char*>(ctx->h_out), static_cast<char*>(ctx->h_out) + chunk};
   auto issue = [&](size_t i) {
     HBX_CUDA(cudaMemcpyAsync(slot[i & 1], pieces[i].src, pieces[i].n, cudaMemcpyDeviceToHost, st));
     HBX_CUDA(cudaEventRecord(ctx->h_out_ev[i & 1], st));
@@ -1417,6 +1442,7 @@ hbx_status hbx_ctx_destroy(hbx_ctx* ctx) {
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->h_ctr) cudaFreeHost(ctx->h_ctr);
+  if (ctx->h_few) cudaFreeHost(ctx->h_few);
   if (ctx->h_out) cudaFreeHost(ctx->h_out);
   for (cudaEvent_t e : ctx->h_out_ev)
     if (e) cudaEventDestroy(e);
@@ -1506,6 +1532,9 @@ hbx_status hbx_block(hbx_ctx* ctx, const hbx_plan* plan, const hbx_table* left,
     // the session is encoded on the context's stream (its creation ends with
     // that stream idle); the run and the copies go to the caller's stream
     hbx::create_session(s, plan, left, right, n_partitions, prefix_idx);
+    if (!ctx->h_few)
+      HBX_CUDA(cudaHostAlloc(&ctx->h_few, 8ull * hbx::kFewPairs, cudaHostAllocPortable));
+    s->h_few = static_cast<uint32_t*>(ctx->h_few);
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     hbx::session_run(s, mode, st);
     const uint64_t n = s->stats.n_matches;
@@ -1515,6 +1544,11 @@ hbx_status hbx_block(hbx_ctx* ctx, const hbx_plan* plan, const hbx_table* left,
     if (n > out->capacity) hbx::fail(HBX_ERR_CAPACITY, "output capacity below the match count");
     if (n) {
       if (!out->l_row || !out->r_row) hbx::fail(HBX_ERR_INVALID_ARG, "null output pointer");
+    }
+    if (n && n <= hbx::kFewPairs) {  // reported with the counters
+      std::memcpy(out->l_row, s->h_few, n * 4);
+      std::memcpy(out->r_row, s->h_few + n, n * 4);
+    } else if (n) {
       void* dst[2] = {out->l_row, out->r_row};
       const void* src[2] = {s->out_l.p, s->out_r.p};
       const size_t bytes[2] = {n * 4, n * 4};

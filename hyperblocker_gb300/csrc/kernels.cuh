@@ -345,6 +345,8 @@ struct Counters {
   unsigned long long deferred_next;  // and taken from it
 };
 
+static_assert(sizeof(Counters) % 8 == 0, "reported in 8-byte words");
+
 struct EvalParams {
   Side L, R;
   const Rule* rules;
@@ -504,6 +506,11 @@ __global__ void k_eval_long(const __grid_constant__ EvalParams P);
 inline int long_grid(int n_sm) { return n_sm * 4; }
 constexpr uint32_t kDeferPairs = 1u << 20;  // most room for deferred pairs of a run
 EvalKernel eval_kernel(int wide, bool groups, uint32_t peq_w);
+// words and, if there are at most limit of them (and capacity), the pairs to
+// page-locked host memory: h_out holds the left rows, then the right rows.
+__global__ void k_report(const unsigned long long* words, uint32_t n_words, const Counters* ctr,
+                         const uint32_t* l, const uint32_t* r, unsigned long long capacity,
+                         unsigned long long limit, unsigned long long* h_words, uint32_t* h_out);
 constexpr uint32_t kPeqWidths[] = {1, 2, 3, 4, 8};  // every PeqShape::w
 
 constexpr uint32_t kScanChunk = 4096;  // elements per CTA in the scans (1024 threads x 4)

@@ -888,26 +888,6 @@ void launch_batch(hbx_server* S, Slot& B) {
 // 2.3 ms with device sorts and 14.5 ms with host sorts.
 constexpr uint64_t kDeviceSortPairs = 2048;
 
-// What the host reads after a batch's evaluation, written to page-locked host
-// memory by one launch: the items' total, the counters and the comparisons
-// (words, side by side), and the pairs when there are fewer than a device
-// sort takes (left rows, then right rows).  A batch's few pairs need no copy
-// of their own then, nor the host a second wait: a request of 16 records
-// takes 174 us, with copies of the counters and then of the pairs 257 us.
-static_assert(sizeof(dev::Counters) % 8 == 0, "reported in 8-byte words");
-__global__ void k_report(const unsigned long long* words, uint32_t n_words, const dev::Counters* ctr,
-                         const uint32_t* l, const uint32_t* r, unsigned long long capacity,
-                         unsigned long long* h_words, uint32_t* h_out) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
-  for (uint32_t i = t; i < n_words; i += step) h_words[i] = words[i];
-  const unsigned long long n = ctr->out_count;
-  if (n >= kDeviceSortPairs || n > capacity) return;
-  for (uint32_t i = t; i < (uint32_t)n; i += step) {
-    h_out[i] = l[i];
-    h_out[n + i] = r[i];
-  }
-}
-
 // The evaluation launch of a batch and the report to the host.
 void launch_eval(hbx_server* S, Slot& B) {
   cudaStream_t st = B.st;
@@ -942,10 +922,12 @@ void launch_eval(hbx_server* S, Slot& B) {
   }
   check_launch("serving k_eval");
   B.h_out.ensure(8 * kDeviceSortPairs);
-  k_report<<<4, 512, 0, st>>>(B.d_base + dev::item_base_words(ni) - 1,
-                              1 + (uint32_t)(sizeof(dev::Counters) / 8) + ni, B.d_ctr, B.out_l.p,
-                              B.out_r.p, B.capacity, static_cast<unsigned long long*>(B.h_ctr.p),
-                              static_cast<uint32_t*>(B.h_out.p));
+  // the items' total, the counters and the comparisons lie side by side
+  dev::k_report<<<4, 512, 0, st>>>(B.d_base + dev::item_base_words(ni) - 1,
+                                   1 + (uint32_t)(sizeof(dev::Counters) / 8) + ni, B.d_ctr,
+                                   B.out_l.p, B.out_r.p, B.capacity, kDeviceSortPairs - 1,
+                                   static_cast<unsigned long long*>(B.h_ctr.p),
+                                   static_cast<uint32_t*>(B.h_out.p));
   check_launch("serving report");
   HBX_CUDA(cudaEventRecord(B.ev_eval, st));
   B.state = 1;
