@@ -797,15 +797,12 @@ constexpr uint32_t kFewPairs = 1u << 16;
 // Queues the copy of the counters (with the run's work-item total) into the
 // context's page-locked block (a graph node when captured).
 void queue_counters(hbx_session* S, cudaStream_t st) {
-  if (S->h_few) {
-    dev::k_report<<<32, 256, 0, st>>>(reinterpret_cast<const unsigned long long*>(S->d_ctr.p),
-                                      (uint32_t)(sizeof(dev::Counters) / 8), S->d_ctr.p, S->out_l.p,
-                                      S->out_r.p, S->out_l.n, kFewPairs,
-                                      reinterpret_cast<unsigned long long*>(S->h_ctr), S->h_few);
-    launch_check("k_report");
-    return;
-  }
-  HBX_CUDA(cudaMemcpyAsync(S->h_ctr, S->d_ctr.p, sizeof(dev::Counters), cudaMemcpyDeviceToHost, st));
+  dev::k_report<<<S->h_few ? 32 : 1, 256, 0, st>>>(
+      reinterpret_cast<const unsigned long long*>(S->d_ctr.p),
+      (uint32_t)(sizeof(dev::Counters) / 8), S->d_ctr.p, S->out_l.p, S->out_r.p,
+      S->h_few ? S->out_l.n : 0, S->h_few ? kFewPairs : 0,
+      reinterpret_cast<unsigned long long*>(S->h_ctr), S->h_few);
+  launch_check("k_report");
 }
 
 unsigned long long items_total(const hbx_session* S) { return S->h_ctr->items_total; }
