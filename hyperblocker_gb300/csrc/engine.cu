@@ -50,6 +50,7 @@ struct RuleBufs {
 // for them: key histograms and scatter cursors, chunk totals and tickets.
 struct JoinLists {
   std::vector<uint32_t> count, scatter, block_task;
+  uint32_t chunk = 0;  // scan_chunks
   std::vector<dev::ScanTask> scan;
   std::vector<uint32_t> words;  // all of them, as uploaded
   DBuf<uint32_t> lists;
@@ -274,7 +275,7 @@ void bind_join(const RuleBufs& b, dev::Rule* d) {
 // The join tasks of a rule array, uploaded on st (J->words stays for the copy),
 // and its counts: all of a rule with work items, the right histogram of a
 // member that only counts its comparisons.
-void list_join(std::vector<dev::Rule>* rules, JoinLists* J, cudaStream_t st) {
+void list_join(std::vector<dev::Rule>* rules, JoinLists* J, int n_sm, cudaStream_t st) {
   size_t n_counts = 0;
   for (const dev::Rule& d : *rules) {
     if (d.n_members)
@@ -308,15 +309,10 @@ void list_join(std::vector<dev::Rule>* rules, JoinLists* J, cudaStream_t st) {
     }
     for (uint32_t what = 0; what < 3; what++) {
       const uint32_t D = what == 1 ? d.domain : d.domain_l;
-      dev::ScanTask t;
-      t.rule = r;
-      t.what = what;
-      t.first_block = (uint32_t)J->block_task.size();
-      t.n_chunks = (D + dev::kScanChunk - 1) / dev::kScanChunk;
-      J->block_task.insert(J->block_task.end(), t.n_chunks, (uint32_t)J->scan.size());
-      J->scan.push_back(t);
+      J->scan.push_back(dev::ScanTask{r, what, 0, D});
     }
   }
+  J->chunk = dev::scan_chunks(n_sm, &J->scan, &J->block_task);
   J->scan_sync.alloc(J->block_task.size() + J->scan.size());
   auto add = [&](const void* p, size_t words) {
     const size_t at = J->words.size();
@@ -410,7 +406,7 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
     alloc_join(S->rb[r], &g, nL, nR);
     bind_join(S->rb[r], &g);
   }
-  list_join(&S->h_groups, &S->join_groups, st);
+  list_join(&S->h_groups, &S->join_groups, S->ctx->n_sm, st);
   S->d_groups.upload(S->h_groups, st);
   S->d_rule_base.alloc(dev::item_base_words(E.rules.size()));
   S->d_ctr.alloc(1);
@@ -481,7 +477,7 @@ void ensure_plain(hbx_session* S) {
     bind_join(S->rb[r], &d);
   }
   S->join_rules = JoinLists{};
-  list_join(&S->h_rules, &S->join_rules, st);
+  list_join(&S->h_rules, &S->join_rules, S->ctx->n_sm, st);
   S->d_rules.upload(S->h_rules, st);
   // partition boundaries of every rule's left key space, per class: entry
   // (rule, class, p) = first left key of partition p
@@ -668,7 +664,8 @@ uint32_t enqueue_join(hbx_session* S, cudaStream_t st, bool groups) {
   const int row_blocks = row_grid(std::max(S->side_l.n_rows, S->side_r.n_rows), S->ctx->n_sm);
   launch_dependent(dev::k_join_count, dim3(row_blocks, (uint32_t)J.count.size()), dim3(256), smem,
                    st, S->side_l, S->side_r, rules, J.d_count);
-  launch_dependent(dev::k_join_scan, dim3(n_blocks), dim3(1024), 0, st, rules, S->tile_right,
+  const dev::JoinScan scan = dev::join_scan(J.chunk);
+  launch_dependent(scan.kernel, dim3(n_blocks), dim3(scan.threads), 0, st, rules, S->tile_right,
                    J.d_scan, J.d_block_task, J.scan_sync.p, &S->d_ctr.p->comparisons, 0u,
                    S->d_ctr.p);
   launch_dependent(dev::k_join_scatter, dim3(row_blocks, (uint32_t)J.scatter.size()), dim3(256), 0,

@@ -430,8 +430,8 @@ void check_launch(const char* what) {
 void scan_u32(const uint32_t* in, uint32_t n, uint32_t* out, cudaStream_t st) {
   const uint32_t nb = (n + dev::kScanChunk - 1) / dev::kScanChunk;
   if (nb <= dev::kScanOnceChunks) {
-    // one launch and a clear instead of three launches; above, the chunks'
-    // look-backs (a word per chunk before) would cost more than the passes
+    // one launch and a clear instead of three launches, where launches are
+    // what a scan costs; above, the passes take longer than their launches
     DBuf<unsigned long long> sync;
     sync.alloc(nb + 1);
     HBX_CUDA(cudaMemsetAsync(sync.p, 0, (nb + 1) * 8ull, st));

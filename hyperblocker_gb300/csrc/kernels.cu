@@ -69,7 +69,7 @@ __global__ void k_scatter(Side S, const Rule* rules, uint32_t rule, int side) {
   }
 }
 
-// Block-wide exclusive scan of 4 values per thread (1024 threads).
+// Block-wide exclusive scan of a value per thread.
 template <typename T>
 __device__ __forceinline__ T block_excl_scan(T v, T* s_warp, T* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -98,34 +98,71 @@ __device__ __forceinline__ T block_excl_scan(T v, T* s_warp, T* total) {
   return r;
 }
 
-constexpr unsigned long long kScanFlag = 1ull << 63;
+// A chunk's word in a single-launch scan: the chunk's total, or the sum of it
+// and of all chunks before (kScanSum has the bit of kScanCount too).
+constexpr unsigned long long kScanCount = 1ull << 63, kScanSum = 3ull << 62;
+constexpr unsigned long long kScanValue = ~kScanSum;
 constexpr uint32_t kScanWaitPolls = 1u << 20;
 
-// Adds the totals of the chunks before chunk c to *s_base (shared, cleared by
-// thread 0 before), a thread per chunk; every thread of the block calls it and
-// *s_base is complete when it returns.  false: a wait of this thread gave up.
-__device__ __forceinline__ bool scan_lookback(unsigned long long* totals, uint32_t c,
+// Publishes chunk c's total and sums the chunks before it into *s_base
+// (shared; complete when this returns): a window of blockDim.x chunks at a
+// time, a thread each, back to the nearest that has published its sum, which
+// is one window as long as fewer blocks run at once.  (Adding up every chunk
+// before, by atomic reads, was most of the join's scans at large domains:
+// 5,860 chunks of three rules' scans took 227 us, with this and vector
+// accesses 203.)  Every thread of the block calls it; false: a wait of this
+// thread gave up.  The caller publishes the sum.
+__device__ __forceinline__ bool scan_lookback(unsigned long long* words, uint32_t c,
+                                              unsigned long long total,
                                               unsigned long long* s_base) {
+  __shared__ uint32_t s_near;
+  volatile unsigned long long* w = words;
   bool ok = true;
-  if (c) {
-    __syncthreads();  // *s_base is 0
-    if ((threadIdx.x & ~31u) < c) {  // whole warps
-      unsigned long long t = 0;
-      for (uint32_t j = threadIdx.x; j < c; j += blockDim.x) {
-        unsigned long long f = 0;
-        uint32_t polls = 0;
-        while (!((f = atomicAdd(totals + j, 0ull)) & kScanFlag) && ++polls < kScanWaitPolls)
-          __nanosleep(64);
-        ok = ok && (f & kScanFlag);
-        t += f & ~kScanFlag;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
-      if ((threadIdx.x & 31) == 0) atomicAdd(s_base, t);
+  if (threadIdx.x == 0) {
+    *s_base = 0;
+    w[c] = total | (c ? kScanCount : kScanSum);
+  }
+  for (uint32_t end = c; end != 0; end = end > blockDim.x ? end - blockDim.x : 0u) {
+    if (threadIdx.x == 0) s_near = ~0u;
+    __syncthreads();
+    unsigned long long f = 0;
+    if (threadIdx.x < end) {
+      uint32_t polls = 0;
+      while (!((f = w[end - 1 - threadIdx.x]) & kScanCount) && ++polls < kScanWaitPolls)
+        __nanosleep(64);
+      ok = ok && (f & kScanCount);
     }
+    const unsigned sums = __ballot_sync(kFull, (f & kScanSum) == kScanSum);
+    if (sums && (int)(threadIdx.x & 31) == __ffs(sums) - 1) atomicMin(&s_near, threadIdx.x);
+    __syncthreads();
+    const uint32_t near = s_near;
+    unsigned long long t = threadIdx.x <= near ? f & kScanValue : 0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+    if ((threadIdx.x & 31) == 0 && t) atomicAdd(s_base, t);
+    __syncthreads();
+    if (near != ~0u) break;
   }
   __syncthreads();
   return ok;
+}
+
+// Four consecutive values from index b on, those at n and above 0; in one
+// access where they lie on a 16-byte boundary.
+__device__ __forceinline__ uint4 load4(const uint32_t* p, uint32_t b, uint32_t n) {
+  if (b + 3 < n && ((uintptr_t)(p + b) & 15) == 0) return *reinterpret_cast<const uint4*>(p + b);
+  return make_uint4(b < n ? p[b] : 0u, b + 1 < n ? p[b + 1] : 0u, b + 2 < n ? p[b + 2] : 0u,
+                    b + 3 < n ? p[b + 3] : 0u);
+}
+__device__ __forceinline__ void store4(uint32_t* p, uint32_t b, uint32_t n, uint4 v) {
+  if (b + 3 < n && ((uintptr_t)(p + b) & 15) == 0) {
+    *reinterpret_cast<uint4*>(p + b) = v;
+    return;
+  }
+  if (b < n) p[b] = v.x;
+  if (b + 1 < n) p[b + 1] = v.y;
+  if (b + 2 < n) p[b + 2] = v.z;
+  if (b + 3 < n) p[b + 3] = v.w;
 }
 
 __global__ void k_scan_once_u32(const uint32_t* in, uint32_t n, uint32_t* out,
@@ -136,20 +173,10 @@ __global__ void k_scan_once_u32(const uint32_t* in, uint32_t n, uint32_t* out,
   if (threadIdx.x == 0) s_chunk = (uint32_t)atomicAdd(sync + gridDim.x, 1ull);
   __syncthreads();
   const uint32_t c = s_chunk;
-  const uint64_t base = (uint64_t)c * kScanChunk + threadIdx.x * 4u;
-  uint32_t v[4], sum = 0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    v[k] = base + k < n ? in[base + k] : 0u;
-    sum += v[k];
-  }
-  uint32_t ex = block_excl_scan<uint32_t>(sum, s_warp, &s_total);
-  if (threadIdx.x == 0) {
-    s_base = 0;
-    __threadfence();
-    atomicExch(sync + c, s_total | kScanFlag);
-  }
-  const bool ok = scan_lookback(sync, c, &s_base);
+  const uint32_t b = c * kScanChunk + threadIdx.x * 4u;
+  const uint4 v = load4(in, b, n);
+  uint32_t ex = block_excl_scan<uint32_t>(v.x + v.y + v.z + v.w, s_warp, &s_total);
+  const bool ok = scan_lookback(sync, c, s_total, &s_base);
   if (__syncthreads_or(!ok)) {  // a wait gave up: the values themselves
     if (threadIdx.x == 0) s_base = 0;
     __syncthreads();
@@ -158,12 +185,10 @@ __global__ void k_scan_once_u32(const uint32_t* in, uint32_t n, uint32_t* out,
     atomicAdd(&s_base, t);
     __syncthreads();
   }
+  if (threadIdx.x == 0)
+    *static_cast<volatile unsigned long long*>(sync + c) = (s_base + s_total) | kScanSum;
   ex += (uint32_t)s_base;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    if (base + k < n) out[base + k] = ex;
-    ex += v[k];
-  }
+  store4(out, b, n, make_uint4(ex, ex + v.x, ex + v.x + v.y, ex + v.x + v.y + v.z));
 }
 
 __global__ void k_scan_partial_u32(const uint32_t* in, uint32_t n, uint32_t* partial) {
@@ -215,14 +240,19 @@ __global__ void k_scan_final_u32(const uint32_t* in, uint32_t n, const uint32_t*
   }
 }
 
+// Work items of a key with nl left and nr right rows, and its pairs.
+__device__ __forceinline__ unsigned long long n_items(uint32_t nl, uint32_t nr, uint32_t tile_right,
+                                                      unsigned long long* pairs) {
+  *pairs = (unsigned long long)nl * nr;
+  if (!nl || !nr) return 0;
+  return (unsigned long long)nl * ((nr + tile_right - 1) / tile_right);
+}
+
 // Work items of left key j (class j / D, join key j % D).
 __device__ __forceinline__ unsigned long long key_items(const Rule& R, uint32_t j,
                                                         uint32_t tile_right,
                                                         unsigned long long* pairs) {
-  const uint32_t nl = R.cnt_l[j], nr = R.cnt_r[j % R.domain];
-  *pairs = (unsigned long long)nl * nr;
-  if (!nl || !nr) return 0;
-  return (unsigned long long)nl * ((nr + tile_right - 1) / tile_right);
+  return n_items(R.cnt_l[j], R.cnt_r[j % R.domain], tile_right, pairs);
 }
 
 __global__ void k_items_partial(const Rule* rules, uint32_t rule, uint32_t tile_right,
@@ -327,78 +357,121 @@ __global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* 
   }
 }
 
-// The value of key k (< D): its row count, or its work items (what = 2, with
-// the key's pair comparisons added to *pairs).
-__device__ __forceinline__ unsigned long long join_scan_value(const Rule& Q, uint32_t what,
-                                                              uint32_t tile_right, uint32_t k,
-                                                              unsigned long long* pairs) {
-  if (what == 2) {
-    unsigned long long p = 0;
-    const unsigned long long v = key_items(Q, k, tile_right, &p);
-    *pairs += p;
-    return v;
-  }
-  return (what == 1 ? Q.cnt_r : Q.cnt_l)[k];
-}
-
-// The scans of every rule with work items (ScanTask), one block of 1024
-// threads per chunk of kScanChunk keys, in one launch.  A block takes its
+// The scans of every rule with work items (ScanTask), one block per
+// chunk of keys, in one launch.  A block takes its
 // chunk from its task's ticket counter when it starts, publishes the chunk's
-// total (flag bit kScanFlag set) before it reads anything of the other
-// chunks, then adds the totals of the chunks before its own, a thread per
-// chunk: those blocks took their tickets earlier, so they are running or
-// done, and every wait ends (bounded all the same: a wait that gives up
-// counts a watchdog trip, which fails the run).
-__global__ void k_join_scan(const Rule* rules, uint32_t tile_right, const ScanTask* tasks,
-                            const uint32_t* block_task, unsigned long long* sync,
-                            unsigned long long* comparisons, uint32_t cmp_stride, Counters* ctr) {
+// total before it reads anything of the other chunks, and looks back over
+// those before its own: their blocks took their tickets earlier, so they are
+// running or done, and every wait ends (bounded all the same: a wait that
+// gives up counts a watchdog trip, which fails the run).
+// A block takes some 10 us whatever it holds (its task, its ticket, the look
+// back), so where there are more chunks than blocks run at once a block holds
+// 8,192 keys, 16 a thread, instead of 4,096, four a thread (scan_chunks):
+// 24 million keys of three rules' scans take 108 us against 203, but 1 to 2 us
+// more where all chunks run at once (2,601 x 2,295 rows: 17.6 against 15.6 us
+// of join).
+template <int kThreads, int kKeys>
+__global__ void __launch_bounds__(kThreads, 2) k_join_scan(
+    const Rule* rules, uint32_t tile_right, const ScanTask* tasks, const uint32_t* block_task,
+    unsigned long long* sync, unsigned long long* comparisons, uint32_t cmp_stride, Counters* ctr) {
   __shared__ unsigned long long s_w64[32];
   __shared__ unsigned long long s_t64, s_base;
   __shared__ uint32_t s_chunk;
+  constexpr int kVec = kKeys / 4;
   pdl_trigger();
   pdl_wait();  // the histograms are complete (k_join_count)
   const uint32_t ti = block_task[blockIdx.x];
+  if (threadIdx.x == 0) s_chunk = (uint32_t)atomicAdd(sync + gridDim.x + ti, 1ull);
   const ScanTask T = tasks[ti];
   unsigned long long* totals = sync + T.first_block;
-  if (threadIdx.x == 0) s_chunk = (uint32_t)atomicAdd(sync + gridDim.x + ti, 1ull);
-  __syncthreads();
-  const uint32_t c = s_chunk;
   const Rule& Q = rules[T.rule];
   const uint32_t D = T.what == 1 ? Q.domain : Q.domain_l;
-  const uint32_t b = c * kScanChunk + threadIdx.x * 4u;
-  unsigned long long v[4], pairs = 0;
+  __syncthreads();
+  const uint32_t c = s_chunk;
+  const uint32_t b = (c * kThreads + threadIdx.x) * kKeys;
+  if (T.what != 2) {  // row counts
+    const uint32_t* cnt = T.what == 1 ? Q.cnt_r : Q.cnt_l;
+    uint4 v[kVec];
+    unsigned long long sum = 0;
 #pragma unroll
-  for (int k = 0; k < 4; k++)
-    v[k] = b + k < D ? join_scan_value(Q, T.what, tile_right, b + k, &pairs) : 0ull;
-  unsigned long long ex = block_excl_scan<unsigned long long>(v[0] + v[1] + v[2] + v[3], s_w64, &s_t64);
-  const unsigned long long chunk_total = s_t64;
-  if (threadIdx.x == 0) {
-    s_base = 0;
-    __threadfence();
-    atomicExch(totals + c, chunk_total | kScanFlag);
-  }
-  if (!scan_lookback(totals, c, &s_base)) atomicAdd(&ctr->watchdog_trips, 1ull);
-  const unsigned long long base = s_base;
-  ex += base;
-  if (T.what == 2) {
+    for (int k = 0; k < kVec; k++) v[k] = load4(cnt, b + 4 * k, D);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (b + k < D) Q.item_off[b + k] = ex;
-      ex += v[k];
-    }
-    if (c + 1 == T.n_chunks && threadIdx.x == 0) Q.item_off[D] = base + chunk_total;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(kFull, pairs, o);
-    if ((threadIdx.x & 31) == 0 && pairs)
-      atomicAdd(comparisons + (size_t)T.rule * cmp_stride, pairs * Q.cmp_weight);
-  } else {
+    for (int k = 0; k < kVec; k++) sum += v[k].x + v[k].y + v[k].z + v[k].w;
+    uint32_t ex = (uint32_t)block_excl_scan<unsigned long long>(sum, s_w64, &s_t64);
+    if (!scan_lookback(totals, c, s_t64, &s_base)) atomicAdd(&ctr->watchdog_trips, 1ull);
+    if (threadIdx.x == 0)
+      *static_cast<volatile unsigned long long*>(totals + c) = (s_base + s_t64) | kScanSum;
+    ex += (uint32_t)s_base;
     uint32_t* off = T.what == 1 ? Q.off_r : Q.off_l;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (b + k < D) off[b + k] = (uint32_t)ex;
-      ex += v[k];
+    for (int k = 0; k < kVec; k++) {
+      const uint4 o = make_uint4(ex, ex + v[k].x, ex + v[k].x + v[k].y, ex + v[k].x + v[k].y + v[k].z);
+      store4(off, b + 4 * k, D, o);
+      ex = o.w + v[k].w;
     }
+    return;
   }
+  // work items; a class's keys repeat the right side's
+  uint4 nl[kVec], nr[kVec];
+  const uint32_t m = Q.domain;
+#pragma unroll
+  for (int k = 0; k < kVec; k++) {
+    const uint32_t j = b + 4 * k;
+    nl[k] = load4(Q.cnt_l, j, D);
+    nr[k] = make_uint4(0, 0, 0, 0);
+    if (j + 3 < m)
+      nr[k] = load4(Q.cnt_r, j, m);
+    else if (j < D)
+      nr[k] = make_uint4(Q.cnt_r[j % m], Q.cnt_r[(j + 1) % m], Q.cnt_r[(j + 2) % m],
+                         Q.cnt_r[(j + 3) % m]);
+  }
+  unsigned long long items = 0, pairs = 0, p;
+#pragma unroll
+  for (int k = 0; k < kVec; k++) {
+    items += n_items(nl[k].x, nr[k].x, tile_right, &p);
+    pairs += p;
+    items += n_items(nl[k].y, nr[k].y, tile_right, &p);
+    pairs += p;
+    items += n_items(nl[k].z, nr[k].z, tile_right, &p);
+    pairs += p;
+    items += n_items(nl[k].w, nr[k].w, tile_right, &p);
+    pairs += p;
+  }
+  unsigned long long ex = block_excl_scan<unsigned long long>(items, s_w64, &s_t64);
+  if (!scan_lookback(totals, c, s_t64, &s_base)) atomicAdd(&ctr->watchdog_trips, 1ull);
+  if (threadIdx.x == 0) {
+    const unsigned long long sum = s_base + s_t64;
+    *static_cast<volatile unsigned long long*>(totals + c) = sum | kScanSum;
+    if (c + 1 == T.n_chunks) Q.item_off[D] = sum;
+  }
+  ex += s_base;
+#pragma unroll
+  for (int k = 0; k < kVec; k++) {
+    const uint32_t j = b + 4 * k;
+    const unsigned long long e1 = ex + n_items(nl[k].x, nr[k].x, tile_right, &p);
+    const unsigned long long e2 = e1 + n_items(nl[k].y, nr[k].y, tile_right, &p);
+    const unsigned long long e3 = e2 + n_items(nl[k].z, nr[k].z, tile_right, &p);
+    if (j + 3 < D && ((uintptr_t)(Q.item_off + j) & 15) == 0) {
+      ulonglong2* to = reinterpret_cast<ulonglong2*>(Q.item_off + j);
+      to[0] = make_ulonglong2(ex, e1);
+      to[1] = make_ulonglong2(e2, e3);
+    } else {
+      if (j < D) Q.item_off[j] = ex;
+      if (j + 1 < D) Q.item_off[j + 1] = e1;
+      if (j + 2 < D) Q.item_off[j + 2] = e2;
+      if (j + 3 < D) Q.item_off[j + 3] = e3;
+    }
+    ex = e3 + n_items(nl[k].w, nr[k].w, tile_right, &p);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(kFull, pairs, o);
+  if ((threadIdx.x & 31) == 0 && pairs)
+    atomicAdd(comparisons + (size_t)T.rule * cmp_stride, pairs * Q.cmp_weight);
+}
+
+JoinScan join_scan(uint32_t chunk) {
+  if (chunk == kJoinChunk) return {k_join_scan<1024, 4>, 1024};
+  return {k_join_scan<512, 16>, 512};
 }
 
 // Rows of every rule with work items grouped by key (counting-sort scatter,

@@ -38,6 +38,7 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <vector>
 
 namespace hbx {
 namespace dev {
@@ -456,10 +457,9 @@ __global__ void k_reset(Counters* ctr, uint32_t* counts, uint64_t n_counts,
 // items, the right one of the members that only count their comparisons;
 // kSharedHistKeys * 4 bytes of dynamic shared memory, or 4 bytes per key of
 // the largest domain when that is less.  Scatter: both tables of the rules
-// with work items, the left one of the members.  k_join_scan runs 1024
-// threads per chunk of kScanChunk keys of each ScanTask; sync holds one total
-// per block of its grid, then one ticket per task, zero before the launch
-// (k_reset).
+// with work items, the left one of the members.  k_join_scan runs
+// a block per chunk of keys of each ScanTask; sync holds one word per block of
+// its grid, then one ticket per task, zero before the launch (k_reset).
 constexpr uint32_t kSharedHistKeys = 8192;
 constexpr uint32_t kTaskRight = 1u << 31;
 __host__ __device__ inline uint32_t join_task(uint32_t rule, int side) {
@@ -470,12 +470,34 @@ __host__ __device__ inline uint32_t join_task(uint32_t rule, int side) {
 struct ScanTask {
   uint32_t rule, what, first_block, n_chunks;
 };
+// Keys of k_join_scan's chunks: kJoinChunk as long as all of them run at once
+// (two blocks per SM), kWideJoinChunk above.
+constexpr uint32_t kJoinChunk = 4096, kWideJoinChunk = 8192;
+// Lays out the tasks' chunks (n_chunks holds their keys on entry); block_task
+// gets the task of every block.  Returns the chunk.
+inline uint32_t scan_chunks(int n_sm, std::vector<ScanTask>* tasks,
+                            std::vector<uint32_t>* block_task) {
+  uint64_t n = 0;
+  for (const ScanTask& t : *tasks) n += ((uint64_t)t.n_chunks + kJoinChunk - 1) / kJoinChunk;
+  const uint32_t chunk = n <= 2ull * (uint64_t)n_sm ? kJoinChunk : kWideJoinChunk;
+  for (size_t i = 0; i < tasks->size(); i++) {
+    ScanTask& t = (*tasks)[i];
+    t.first_block = (uint32_t)block_task->size();
+    t.n_chunks = (uint32_t)(((uint64_t)t.n_chunks + chunk - 1) / chunk);
+    block_task->insert(block_task->end(), t.n_chunks, (uint32_t)i);
+  }
+  return chunk;
+}
 __global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* tasks);
 // comparisons: rule r's pair-comparisons are added to comparisons[r *
 // cmp_stride].
-__global__ void k_join_scan(const Rule* rules, uint32_t tile_right, const ScanTask* tasks,
-                            const uint32_t* block_task, unsigned long long* sync,
-                            unsigned long long* comparisons, uint32_t cmp_stride, Counters* ctr);
+struct JoinScan {
+  void (*kernel)(const Rule* rules, uint32_t tile_right, const ScanTask* tasks,
+                 const uint32_t* block_task, unsigned long long* sync,
+                 unsigned long long* comparisons, uint32_t cmp_stride, Counters* ctr);
+  int threads;
+};
+JoinScan join_scan(uint32_t chunk);  // k_join_scan for a chunk of scan_chunks
 __global__ void k_join_scatter(Side L, Side R, const Rule* rules, uint32_t n_rules,
                                const uint32_t* tasks, unsigned long long* rule_base,
                                Counters* ctr);

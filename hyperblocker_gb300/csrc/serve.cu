@@ -665,7 +665,8 @@ uint64_t estimate(const hbx_server* S, const Table& t, int32_t plan, uint32_t r0
   b += sizeof(dev::StrMeta) * n * S->lstr.size() + 4 * n * S->pairs.size();
   for (int r : S->plan_rules[(size_t)plan]) {
     const dev::Rule& d = S->rules[(size_t)r]->d;
-    // an upper bound on the classes of left keys
+    // room for five classes of left keys, more than are in use: what the
+    // budget refuses does not depend on them
     const uint64_t keys_l = (uint64_t)d.domain * (d.n_sim && d.domain * 5ull <= (1ull << 22) ? 5 : 1);
     b += 12ull * n + 20ull * keys_l + 64 + 8 * ((keys_l + dev::kScanChunk - 1) / dev::kScanChunk + 1);
   }
@@ -707,19 +708,14 @@ void launch_batch(hbx_server* S, Slot& B) {
       dev::Rule d = S->rules[(size_t)r]->d;
       dev::set_classes(&d, B.long_left);
       for (uint32_t what : {0u, 2u}) {
-        dev::ScanTask t;
-        t.rule = (uint32_t)rules.size();
-        t.what = what;
-        t.first_block = (uint32_t)block_task.size();
-        t.n_chunks = (d.domain_l + dev::kScanChunk - 1) / dev::kScanChunk;
-        block_task.insert(block_task.end(), t.n_chunks, (uint32_t)tasks.size());
-        tasks.push_back(t);
+        tasks.push_back(dev::ScanTask{(uint32_t)rules.size(), what, 0, d.domain_l});
       }
       rules.push_back(d);
       rows.push_back({B.base[q], B.ents[q].n()});
       max_n = std::max(max_n, B.ents[q].n());
       B.inst_entry.push_back((uint32_t)q);
     }
+  const dev::JoinScan scan = dev::join_scan(dev::scan_chunks(C->n_sm, &tasks, &block_task));
   const uint32_t ni = (uint32_t)rules.size();
   const size_t n_base = dev::item_base_words(ni);
   {
@@ -857,7 +853,7 @@ void launch_batch(hbx_server* S, Slot& B) {
   const InstRows* d_rows = reinterpret_cast<const InstRows*>(B.d_stage.p + at_rows);
   const dim3 grid(grid_for(max_n, C->n_sm), std::min<uint32_t>(ni, 65535u));
   k_keys<<<grid, 256, 0, st>>>(B.d_rules, ni, d_rows, B.side_l);
-  dev::k_join_scan<<<(uint32_t)block_task.size(), 1024, 0, st>>>(
+  scan.kernel<<<(uint32_t)block_task.size(), scan.threads, 0, st>>>(
       B.d_rules, S->tile_right, reinterpret_cast<const dev::ScanTask*>(B.d_stage.p + at_tasks),
       reinterpret_cast<const uint32_t*>(B.d_stage.p + at_blocks), B.d_sync, B.d_cmp, 1u, B.d_ctr);
   k_scatter_left<<<grid, 256, 0, st>>>(B.d_rules, ni, d_rows, B.d_base);
@@ -885,7 +881,7 @@ void launch_batch(hbx_server* S, Slot& B) {
 // are one run: on the device from this many on, else on the host.  A device
 // sort is about 8 operations, whatever it sorts, the host's takes longer with
 // every pair: a burst of 24 requests, 14,011 records, 279,498 pairs, takes
-// 2.3 ms with device sorts and 14.5 ms with host sorts.
+// 2.1 ms with device sorts and 14.5 ms with host sorts.
 constexpr uint64_t kDeviceSortPairs = 2048;
 
 // The evaluation launch of a batch and the report to the host.

@@ -80,3 +80,25 @@ def test_pairs_of_several_rules_are_reported_once(built, roots, thr):
     served = want.pairs[want.pairs[:, 0] > 0] - np.array([1, 0], np.uint32)
     assert np.array_equal(got, served)
     c.close()
+
+
+@pytest.mark.parametrize("n_keys", [413696, 417793, 421888, 425985])
+def test_domains_around_the_wide_chunks(ctx, n_keys):
+    """Three scans of 101 to 105 chunks of 4,096 keys: one wave of blocks takes
+    304, so the larger sizes take chunks of 8,192."""
+    cl, cr = _util.random_tables(n_keys, 300, 2000, b"abc", 10)
+    n = n_keys // 4
+    cr[3][1:] = [b"%d" % (i * 37 % n) for i in range(2000)]
+    cl[3][1:] = [b"%d" % (n - 1 - 7 * i) for i in range(300)]
+    # 4 partitions and a filler column value per key: the right table lists them all
+    for c in range(len(cr)):
+        cr[c] += [b"%d" % i for i in range(n - 1)] if c == 3 else [b"zz"] * (n - 1)
+    docs = RULES[:1]
+    want = api.run_block(api.CTable(cl), api.CTable(cr), rules.serialize(rules.sort_rules(
+        [rules.decode_rule(rules.parse_yaml(d)) for d in docs])), 4)
+    plan = hb.Plan.from_yaml(docs, ctx)
+    left, right = hb.Table.from_columns(cl, ctx), hb.Table.from_columns(cr, ctx)
+    for mode in ("plain", "batched"):
+        got, st = hb.block(ctx, plan, left, right, 4, _util.INT_MAX, mode)
+        assert np.array_equal(_util.sorted_pairs(got), want.pairs), mode
+        assert st.pair_comparisons == want.pair_comparisons, mode
