@@ -3,7 +3,7 @@
 // (b bits hold a right row), 8 bits per pass.
 //
 // One launch counts every pass's digits.  A pass is then one launch: a block
-// ranks a tile of kTile keys, publishes its counts per digit, adds the counts
+// ranks a tile of keys, publishes its counts per digit, adds the counts
 // of the tiles before it (looking back tile by tile, as far as the first that
 // has published its sum) and scatters.  The first pass reads the pairs and the
 // last one writes them back, so that no launch only converts.
@@ -20,8 +20,6 @@ namespace hbx {
 namespace srt {
 
 constexpr uint32_t kThreads = 256, kWarps = kThreads / 32;
-constexpr uint32_t kKeys = 8;                // keys per thread
-constexpr uint32_t kTile = kThreads * kKeys;  // keys per tile
 constexpr uint32_t kMaxPasses = 8;
 constexpr uint32_t kBack = 8;  // tiles read at once when looking back
 // A wait for another tile's counts ends after this many polls (each some
@@ -66,15 +64,20 @@ struct State {
 // warp ranks 8 rounds of its own 256 keys without a block barrier), the look
 // back (8 tiles at a time: their words arrive together).  100,000 pairs take
 // 8.7 us a pass and 43 us a sort; a histogram, a scan and a scatter launch per
-// pass took 24 us, and 126 us a sort with the packing launches.
+// pass took 24 us, and 126 us a sort with the packing launches.  Above what
+// four blocks per SM hold, a thread takes 16 keys instead of 8: half as many
+// tiles look back over half as many (24.5 million pairs: 255 us a pass and
+// 1.12 ms a sort, 300 us and 1.30 ms with 8 keys, 282 us and 1.27 ms with
+// three launches a pass).
 // Tiles are handed out by a ticket, so the tiles before a block's own are
 // running or done.  next: the other pass's words, cleared for it.
-template <class T>
+template <class T, uint32_t kKeys>
 __global__ void __launch_bounds__(kThreads) k_pass(Pairs p, const unsigned long long* src,
                                                    unsigned long long* dst, uint32_t shift,
                                                    const uint32_t* count, uint32_t* ticket, T* state,
                                                    T* next) {
   using S = State<T>;
+  constexpr uint32_t kTile = kThreads * kKeys;
   __shared__ uint32_t s_cnt[kWarps][256];  // a warp's keys per digit, then where they start
   __shared__ uint32_t s_base[256];         // the tile's first position per digit
   __shared__ uint32_t s_warp[kWarps];
@@ -179,8 +182,9 @@ __global__ void __launch_bounds__(kThreads) k_pass(Pairs p, const unsigned long 
   }
 }
 
-template <class T>
+template <class T, uint32_t kKeys>
 void queue_passes(Pairs p, uint32_t n_passes, int n_sm, cudaStream_t st) {
+  constexpr uint32_t kTile = kThreads * kKeys;
   const uint32_t n_tiles = (uint32_t)((p.n + kTile - 1) / kTile);
   const uint64_t words = 256ull * n_tiles;
   // two passes and more: the first reads the pairs that the last overwrites
@@ -197,7 +201,7 @@ void queue_passes(Pairs p, uint32_t n_passes, int n_sm, cudaStream_t st) {
   for (uint32_t q = 0; q < n_passes; q++) {
     const unsigned long long* src = q == 0 ? nullptr : q & 1 ? a.p : b.p;
     unsigned long long* dst = q + 1 == n_passes ? nullptr : q & 1 ? b.p : a.p;
-    k_pass<T><<<n_tiles, kThreads, 0, st>>>(p, src, dst, 8 * q, count.p + 256 * q,
+    k_pass<T, kKeys><<<n_tiles, kThreads, 0, st>>>(p, src, dst, 8 * q, count.p + 256 * q,
                                             count.p + 256 * kMaxPasses + q, state.p + (q & 1) * words,
                                             state.p + (~q & 1) * words);
   }
@@ -222,10 +226,12 @@ void queue_pair_sort(int n_sm, cudaStream_t st, uint32_t* l, uint32_t* r, uint64
   const uint32_t n_passes = std::max(2u, (bl + br + 7) / 8);
   const srt::Pairs p{l, r, n, br};
   // the words' values go up to n
-  if (n < (1ull << 30))
-    srt::queue_passes<uint32_t>(p, n_passes, n_sm, st);
+  if (n <= 4ull * n_sm * 8 * srt::kThreads)
+    srt::queue_passes<uint32_t, 8>(p, n_passes, n_sm, st);
+  else if (n < (1ull << 30))
+    srt::queue_passes<uint32_t, 16>(p, n_passes, n_sm, st);
   else
-    srt::queue_passes<unsigned long long>(p, n_passes, n_sm, st);
+    srt::queue_passes<unsigned long long, 16>(p, n_passes, n_sm, st);
 }
 
 // The same on the context's stream; returns when the pairs are sorted.
