@@ -186,9 +186,10 @@ hbx_status hbx_session_destroy(hbx_session* s);
  * out holds HOST pointers.  The tables are encoded on the context's stream;
  * the run and the copy of the pairs go to `stream` (a cudaStream_t, NULL =
  * the context's stream), the stream the reference's AsyncSubmit takes
- * (host_producer.h:109-112).  The pairs come back through 512 MiB of
- * page-locked host memory the context allocates on its first call (two
- * chunks, each copied into out while the next one transfers).  Returns when
+ * (host_producer.h:109-112).  The pairs come back through page-locked host
+ * memory that the context keeps: up to 65,536 pairs with the run's counters,
+ * more through two chunks of up to 256 MiB, as large as results needed so far
+ * (each copied into out while the next one transfers).  Returns when
  * the pairs are in out. */
 hbx_status hbx_block(hbx_ctx* ctx, const hbx_plan* plan, const hbx_table* left,
                      const hbx_table* right, uint64_t n_partitions, int64_t prefix_idx,
