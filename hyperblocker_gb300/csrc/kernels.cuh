@@ -21,6 +21,10 @@
 //                     from the left string's table, exact early-fail bound),
 //                     and go on with the rule's next predicate in the same
 //                     lane; matches leave by warp-aggregated atomics.
+//   6. k_eval_long    where some left string has over 256 symbols (no table):
+//                     the items of those strings, and the pairs that met one
+//                     at a later predicate, by whole warps.
+//   7. k_report       counters, and a small result's pairs, to the host.
 //
 // Semantics reproduced (reference = HyperBlocker):
 //   * pairs are compared only inside a partition (data_mngr.h:150-216, the
