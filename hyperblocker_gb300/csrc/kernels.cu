@@ -723,13 +723,15 @@ __device__ __noinline__ bool jw_exact(uint32_t m, uint32_t ls, uint32_t ll, uint
 
 // Decision from the match count m and the common prefix p: a float estimate
 // settles every pair whose JW lies farther than kDecisionMargin from the
-// threshold (the estimate's error is below 2e-6); the rest take the exact path.
+// threshold (the estimate's error is below 2e-6 up to p = 10); the rest take
+// the exact path.  The prefix has no cap, so from p = 10 on the sum reaches 1
+// and more: cut at 1 like the value it stands for, it is 1 but for the rounding.
 __device__ __forceinline__ bool jw_decide(uint32_t m, uint32_t ls, uint32_t ll, uint32_t p,
                                           float thr, unsigned long long* ambiguous) {
   const float fm = (float)m;
   const float ja = m ? (__fdividef(fm, (float)ls) + __fdividef(fm, (float)ll) + 1.0f) * (1.0f / 3.0f)
                      : 0.0f;
-  const float jwa = ja + (1.0f - ja) * (0.1f * (float)p);
+  const float jwa = fminf(ja + (1.0f - ja) * (0.1f * (float)p), 1.0f);
   if (jwa >= thr + kDecisionMargin) return true;
   if (jwa < thr - kDecisionMargin) return false;
   return jw_exact(m, ls, ll, p, thr, ambiguous);
