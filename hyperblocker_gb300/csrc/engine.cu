@@ -615,22 +615,22 @@ std::vector<dev::Rule> group_rules(const std::vector<dev::Rule>& singles) {
     if (G.n_members) dev::fill_extras_table(&G);
   // rules with the same equalities have the same pair-comparisons: one of
   // them counts for all, a rule with work items where there is one
+  std::vector<char> counted(n, 0);
   for (size_t r = 0; r < n; r++) {
-    if (!g[r].cmp_weight) continue;
+    if (counted[r]) continue;
     size_t keep = r;
     std::vector<size_t> same;
     for (size_t q = r; q < n; q++)
-      if (g[q].cmp_weight && eqset(q) == eqset(r)) {
+      if (!counted[q] && eqset(q) == eqset(r)) {
+        counted[q] = 1;
         same.push_back(q);
         if (g[q].n_members && !g[keep].n_members) keep = q;
       }
-    uint32_t rest = 0;
     for (size_t q : same)
       if (q != keep && !g[q].n_members) {
-        rest++;
+        g[keep].cmp_weight++;
         g[q].cmp_weight = 0;
       }
-    g[keep].cmp_weight = 1 + rest;
   }
   dev::set_overlaps(g.data(), n);
   return g;
