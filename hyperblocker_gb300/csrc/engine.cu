@@ -116,6 +116,7 @@ struct hbx_session {
   uint64_t ext_cap = 0;
   const uint32_t* graph_out = nullptr;  // output the captured graph writes
   uint64_t graph_cap = 0;
+  uint32_t graph_launches = 0;  // kernels in it
   uint64_t seen_pairs = 1 << 16;  // distinct pairs the duplicate set is sized for
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;      // whole run
   cudaEvent_t ev_eval0 = nullptr, ev_eval1 = nullptr;  // join ends / evaluation ends
@@ -756,7 +757,7 @@ uint32_t enqueue_batched(hbx_session* S, cudaStream_t st) {
   // the counters travel back inside the run (graph nodes when captured)
   queue_counters(S, st);
   HBX_CUDA(cudaEventRecordWithFlags(S->ev1, st, rec_flags));
-  return launches + 1;
+  return launches + 2;  // with the evaluation and the report
 }
 
 void grow_output(hbx_session* S, uint64_t need) {
@@ -834,10 +835,10 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
         cudaError_t e = cudaGraphInstantiate(&S->graph, g, 0);
         cudaGraphDestroy(g);
         HBX_CUDA(e);
-        S->stats.n_launches = n;
+        S->graph_launches = n;
       }
       HBX_CUDA(cudaGraphLaunch(S->graph, st));
-      *launches = S->stats.n_launches;
+      *launches = S->graph_launches;
     } else {
       *launches = enqueue_batched(S, st);
     }
@@ -897,9 +898,9 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
     n++;
   }
   HBX_CUDA(cudaEventRecord(S->ev_eval1, st));
-  *launches = n;
-  S->stats.n_launches = n;
   queue_counters(S, st);
+  n++;
+  *launches = n;
   HBX_CUDA(cudaEventRecord(S->ev1, st));
   HBX_CUDA(cudaStreamSynchronize(st));
   return *S->h_ctr;
