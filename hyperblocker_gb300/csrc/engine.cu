@@ -668,7 +668,7 @@ uint32_t enqueue_join(hbx_session* S, cudaStream_t st, bool groups) {
   const dev::JoinScan scan = dev::join_scan(J.chunk);
   launch_dependent(scan.kernel, dim3(n_blocks), dim3(scan.threads), 0, st, rules, S->tile_right,
                    J.d_scan, J.d_block_task, J.scan_sync.p, &S->d_ctr.p->comparisons, 0u,
-                   S->d_ctr.p);
+                   dev::scan_polls());
   launch_dependent(dev::k_join_scatter, dim3(row_blocks, (uint32_t)J.scatter.size()), dim3(256), 0,
                    st, S->side_l, S->side_r, rules, (uint32_t)S->rb.size(), J.d_scatter,
                    S->d_rule_base.p, S->d_ctr.p);

@@ -435,7 +435,7 @@ void scan_u32(const uint32_t* in, uint32_t n, uint32_t* out, cudaStream_t st) {
     DBuf<unsigned long long> sync;
     sync.alloc(nb + 1);
     HBX_CUDA(cudaMemsetAsync(sync.p, 0, (nb + 1) * 8ull, st));
-    dev::k_scan_once_u32<<<nb, 1024, 0, st>>>(in, n, out, sync.p);
+    dev::k_scan_once_u32<<<nb, 1024, 0, st>>>(in, n, out, sync.p, dev::scan_polls());
     check_launch("ingest scan");
     return;
   }

@@ -1,4 +1,7 @@
 // kernels.cu -- sm_103a kernels of the blocking engine (see kernels.cuh).
+#include <cstdlib>
+#include <cstring>
+
 #include "kernels.cuh"
 #include "bitscan.cuh"
 
@@ -102,7 +105,11 @@ __device__ __forceinline__ T block_excl_scan(T v, T* s_warp, T* total) {
 // and of all chunks before (kScanSum has the bit of kScanCount too).
 constexpr unsigned long long kScanCount = 1ull << 63, kScanSum = 3ull << 62;
 constexpr unsigned long long kScanValue = ~kScanSum;
-constexpr uint32_t kScanWaitPolls = 1u << 20;
+
+uint32_t scan_polls() {
+  const char* e = std::getenv("HBX_TEST_SCAN_GIVE_UP");
+  return e && std::strcmp(e, "1") == 0 ? 0u : 1u << 20;
+}
 
 // Publishes chunk c's total and sums the chunks before it into *s_base
 // (shared; complete when this returns): a window of blockDim.x chunks at a
@@ -110,10 +117,11 @@ constexpr uint32_t kScanWaitPolls = 1u << 20;
 // is one window as long as fewer blocks run at once.  (Adding up every chunk
 // before, by atomic reads, was most of the join's scans at large domains:
 // 5,860 chunks of three rules' scans took 227 us, with this and vector
-// accesses 203.)  Every thread of the block calls it; false: a wait of this
-// thread gave up.  The caller publishes the sum.
+// accesses 203.)  Every thread of the block calls it; false in all of them: a
+// wait gave up after `polls` polls (scan_polls), and the caller adds up what
+// lies before the chunk itself (scan_recount).  The caller publishes the sum.
 __device__ __forceinline__ bool scan_lookback(unsigned long long* words, uint32_t c,
-                                              unsigned long long total,
+                                              unsigned long long total, uint32_t polls,
                                               unsigned long long* s_base) {
   __shared__ uint32_t s_near;
   volatile unsigned long long* w = words;
@@ -127,9 +135,11 @@ __device__ __forceinline__ bool scan_lookback(unsigned long long* words, uint32_
     __syncthreads();
     unsigned long long f = 0;
     if (threadIdx.x < end) {
-      uint32_t polls = 0;
-      while (!((f = w[end - 1 - threadIdx.x]) & kScanCount) && ++polls < kScanWaitPolls)
+      uint32_t left = polls;
+      while (left && !((f = w[end - 1 - threadIdx.x]) & kScanCount)) {
+        left--;
         __nanosleep(64);
+      }
       ok = ok && (f & kScanCount);
     }
     const unsigned sums = __ballot_sync(kFull, (f & kScanSum) == kScanSum);
@@ -143,8 +153,19 @@ __device__ __forceinline__ bool scan_lookback(unsigned long long* words, uint32_
     __syncthreads();
     if (near != ~0u) break;
   }
+  return !__syncthreads_or(!ok);
+}
+
+// The block's sum of value(k) for k below n, into *s_base (complete when this
+// returns).
+template <class F>
+__device__ __forceinline__ void scan_recount(uint64_t n, unsigned long long* s_base, F&& value) {
+  if (threadIdx.x == 0) *s_base = 0;
   __syncthreads();
-  return ok;
+  unsigned long long t = 0;
+  for (uint64_t k = threadIdx.x; k < n; k += blockDim.x) t += value(k);
+  atomicAdd(s_base, t);
+  __syncthreads();
 }
 
 // Four consecutive values from index b on, those at n and above 0; in one
@@ -166,7 +187,7 @@ __device__ __forceinline__ void store4(uint32_t* p, uint32_t b, uint32_t n, uint
 }
 
 __global__ void k_scan_once_u32(const uint32_t* in, uint32_t n, uint32_t* out,
-                                unsigned long long* sync) {
+                                unsigned long long* sync, uint32_t polls) {
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_total, s_chunk;
   __shared__ unsigned long long s_base;
@@ -176,15 +197,8 @@ __global__ void k_scan_once_u32(const uint32_t* in, uint32_t n, uint32_t* out,
   const uint32_t b = c * kScanChunk + threadIdx.x * 4u;
   const uint4 v = load4(in, b, n);
   uint32_t ex = block_excl_scan<uint32_t>(v.x + v.y + v.z + v.w, s_warp, &s_total);
-  const bool ok = scan_lookback(sync, c, s_total, &s_base);
-  if (__syncthreads_or(!ok)) {  // a wait gave up: the values themselves
-    if (threadIdx.x == 0) s_base = 0;
-    __syncthreads();
-    unsigned long long t = 0;
-    for (uint64_t k = threadIdx.x; k < (uint64_t)c * kScanChunk; k += blockDim.x) t += in[k];
-    atomicAdd(&s_base, t);
-    __syncthreads();
-  }
+  if (!scan_lookback(sync, c, s_total, polls, &s_base))
+    scan_recount((uint64_t)c * kScanChunk, &s_base, [&](uint64_t k) { return in[k]; });
   if (threadIdx.x == 0)
     *static_cast<volatile unsigned long long*>(sync + c) = (s_base + s_total) | kScanSum;
   ex += (uint32_t)s_base;
@@ -357,23 +371,37 @@ __global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* 
   }
 }
 
+// The rows of keys below n, and the work items of left keys below n, for a
+// block whose wait gave up (out of line: the scans' registers are for their keys).
+__device__ __noinline__ void recount_rows(const uint32_t* cnt, uint32_t n, unsigned long long* s_base) {
+  scan_recount(n, s_base, [&](uint64_t k) { return cnt[k]; });
+}
+__device__ __noinline__ void recount_items(const Rule& R, uint32_t tile_right, uint32_t n,
+                                           unsigned long long* s_base) {
+  scan_recount(n, s_base, [&](uint64_t k) {
+    unsigned long long pairs;
+    return key_items(R, (uint32_t)k, tile_right, &pairs);
+  });
+}
+
 // The scans of every rule with work items (ScanTask), one block per
 // chunk of keys, in one launch.  A block takes its
 // chunk from its task's ticket counter when it starts, publishes the chunk's
 // total before it reads anything of the other chunks, and looks back over
 // those before its own: their blocks took their tickets earlier, so they are
-// running or done, and every wait ends (bounded all the same: a wait that
-// gives up counts a watchdog trip, which fails the run).
+// running or done, and every wait ends (bounded all the same: a block whose
+// wait gave up adds up the counts before its chunk itself).
 // A block takes some 10 us whatever it holds (its task, its ticket, the look
 // back), so where there are more chunks than blocks run at once a block holds
-// 8,192 keys, 16 a thread, instead of 4,096, four a thread (scan_chunks):
+// 8,192 keys, 16 a thread, instead of 4,096, eight a thread (scan_chunks):
 // 24 million keys of three rules' scans take 108 us against 203, but 1 to 2 us
-// more where all chunks run at once (2,601 x 2,295 rows: 17.6 against 15.6 us
-// of join).
+// more where all chunks run at once (2,617 x 2,295 rows: 17.6 against 15.6 us
+// of join, measured with 1,024 threads of four keys; 512 of eight take the same
+// and have the registers for the recount without spills).
 template <int kThreads, int kKeys>
 __global__ void __launch_bounds__(kThreads, 2) k_join_scan(
     const Rule* rules, uint32_t tile_right, const ScanTask* tasks, const uint32_t* block_task,
-    unsigned long long* sync, unsigned long long* comparisons, uint32_t cmp_stride, Counters* ctr) {
+    unsigned long long* sync, unsigned long long* comparisons, uint32_t cmp_stride, uint32_t polls) {
   __shared__ unsigned long long s_w64[32];
   __shared__ unsigned long long s_t64, s_base;
   __shared__ uint32_t s_chunk;
@@ -388,17 +416,22 @@ __global__ void __launch_bounds__(kThreads, 2) k_join_scan(
   const uint32_t D = T.what == 1 ? Q.domain : Q.domain_l;
   __syncthreads();
   const uint32_t c = s_chunk;
-  const uint32_t b = (c * kThreads + threadIdx.x) * kKeys;
+  const uint32_t chunk0 = c * (kThreads * kKeys), b = chunk0 + threadIdx.x * kKeys;
   if (T.what != 2) {  // row counts
     const uint32_t* cnt = T.what == 1 ? Q.cnt_r : Q.cnt_l;
     uint4 v[kVec];
-    unsigned long long sum = 0;
+    uint32_t ex;
+    for (bool again = false;; again = true) {
+      unsigned long long sum = 0;
 #pragma unroll
-    for (int k = 0; k < kVec; k++) v[k] = load4(cnt, b + 4 * k, D);
+      for (int k = 0; k < kVec; k++) v[k] = load4(cnt, b + 4 * k, D);
 #pragma unroll
-    for (int k = 0; k < kVec; k++) sum += v[k].x + v[k].y + v[k].z + v[k].w;
-    uint32_t ex = (uint32_t)block_excl_scan<unsigned long long>(sum, s_w64, &s_t64);
-    if (!scan_lookback(totals, c, s_t64, &s_base)) atomicAdd(&ctr->watchdog_trips, 1ull);
+      for (int k = 0; k < kVec; k++) sum += v[k].x + v[k].y + v[k].z + v[k].w;
+      ex = (uint32_t)block_excl_scan<unsigned long long>(sum, s_w64, &s_t64);
+      // (after a recount the keys are loaded again: nothing is kept across it)
+      if (again || scan_lookback(totals, c, s_t64, polls, &s_base)) break;
+      recount_rows(cnt, chunk0, &s_base);
+    }
     if (threadIdx.x == 0)
       *static_cast<volatile unsigned long long*>(totals + c) = (s_base + s_t64) | kScanSum;
     ex += (uint32_t)s_base;
@@ -414,31 +447,36 @@ __global__ void __launch_bounds__(kThreads, 2) k_join_scan(
   // work items; a class's keys repeat the right side's
   uint4 nl[kVec], nr[kVec];
   const uint32_t m = Q.domain;
+  unsigned long long pairs, ex, p;
+  for (bool again = false;; again = true) {
 #pragma unroll
-  for (int k = 0; k < kVec; k++) {
-    const uint32_t j = b + 4 * k;
-    nl[k] = load4(Q.cnt_l, j, D);
-    nr[k] = make_uint4(0, 0, 0, 0);
-    if (j + 3 < m)
-      nr[k] = load4(Q.cnt_r, j, m);
-    else if (j < D)
-      nr[k] = make_uint4(Q.cnt_r[j % m], Q.cnt_r[(j + 1) % m], Q.cnt_r[(j + 2) % m],
-                         Q.cnt_r[(j + 3) % m]);
-  }
-  unsigned long long items = 0, pairs = 0, p;
+    for (int k = 0; k < kVec; k++) {
+      const uint32_t j = b + 4 * k;
+      nl[k] = load4(Q.cnt_l, j, D);
+      nr[k] = make_uint4(0, 0, 0, 0);
+      if (j + 3 < m)
+        nr[k] = load4(Q.cnt_r, j, m);
+      else if (j < D)
+        nr[k] = make_uint4(Q.cnt_r[j % m], Q.cnt_r[(j + 1) % m], Q.cnt_r[(j + 2) % m],
+                           Q.cnt_r[(j + 3) % m]);
+    }
+    unsigned long long items = 0;
+    pairs = 0;
 #pragma unroll
-  for (int k = 0; k < kVec; k++) {
-    items += n_items(nl[k].x, nr[k].x, tile_right, &p);
-    pairs += p;
-    items += n_items(nl[k].y, nr[k].y, tile_right, &p);
-    pairs += p;
-    items += n_items(nl[k].z, nr[k].z, tile_right, &p);
-    pairs += p;
-    items += n_items(nl[k].w, nr[k].w, tile_right, &p);
-    pairs += p;
+    for (int k = 0; k < kVec; k++) {
+      items += n_items(nl[k].x, nr[k].x, tile_right, &p);
+      pairs += p;
+      items += n_items(nl[k].y, nr[k].y, tile_right, &p);
+      pairs += p;
+      items += n_items(nl[k].z, nr[k].z, tile_right, &p);
+      pairs += p;
+      items += n_items(nl[k].w, nr[k].w, tile_right, &p);
+      pairs += p;
+    }
+    ex = block_excl_scan<unsigned long long>(items, s_w64, &s_t64);
+    if (again || scan_lookback(totals, c, s_t64, polls, &s_base)) break;
+    recount_items(Q, tile_right, chunk0, &s_base);
   }
-  unsigned long long ex = block_excl_scan<unsigned long long>(items, s_w64, &s_t64);
-  if (!scan_lookback(totals, c, s_t64, &s_base)) atomicAdd(&ctr->watchdog_trips, 1ull);
   if (threadIdx.x == 0) {
     const unsigned long long sum = s_base + s_t64;
     *static_cast<volatile unsigned long long*>(totals + c) = sum | kScanSum;
@@ -470,7 +508,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_join_scan(
 }
 
 JoinScan join_scan(uint32_t chunk) {
-  if (chunk == kJoinChunk) return {k_join_scan<1024, 4>, 1024};
+  if (chunk == kJoinChunk) return {k_join_scan<512, 8>, 512};
   return {k_join_scan<512, 16>, 512};
 }
 

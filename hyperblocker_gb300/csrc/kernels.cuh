@@ -418,8 +418,12 @@ __global__ void k_scan_final_u32(const uint32_t* in, uint32_t n, const uint32_t*
 // k_join_scan does; sync: one word per chunk and the ticket, zero before the
 // launch.
 constexpr uint32_t kScanOnceChunks = 2048;
+// Polls (some 100 ns each) after which a single-launch scan or the sort gives
+// up waiting for a chunk before its own and counts what lies before it itself;
+// 0 with HBX_TEST_SCAN_GIVE_UP=1 in the environment: they count at once.
+uint32_t scan_polls();
 __global__ void k_scan_once_u32(const uint32_t* in, uint32_t n, uint32_t* out,
-                                unsigned long long* sync);
+                                unsigned long long* sync, uint32_t polls);
 __global__ void k_items_partial(const Rule* rules, uint32_t rule, uint32_t tile_right,
                                 unsigned long long* partial, unsigned long long* comparisons);
 __global__ void k_scan_top_u64(unsigned long long* partial, uint32_t nb);
@@ -498,7 +502,7 @@ __global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* 
 struct JoinScan {
   void (*kernel)(const Rule* rules, uint32_t tile_right, const ScanTask* tasks,
                  const uint32_t* block_task, unsigned long long* sync,
-                 unsigned long long* comparisons, uint32_t cmp_stride, Counters* ctr);
+                 unsigned long long* comparisons, uint32_t cmp_stride, uint32_t polls);
   int threads;
 };
 JoinScan join_scan(uint32_t chunk);  // k_join_scan for a chunk of scan_chunks

@@ -855,7 +855,8 @@ void launch_batch(hbx_server* S, Slot& B) {
   k_keys<<<grid, 256, 0, st>>>(B.d_rules, ni, d_rows, B.side_l);
   scan.kernel<<<(uint32_t)block_task.size(), scan.threads, 0, st>>>(
       B.d_rules, S->tile_right, reinterpret_cast<const dev::ScanTask*>(B.d_stage.p + at_tasks),
-      reinterpret_cast<const uint32_t*>(B.d_stage.p + at_blocks), B.d_sync, B.d_cmp, 1u, B.d_ctr);
+      reinterpret_cast<const uint32_t*>(B.d_stage.p + at_blocks), B.d_sync, B.d_cmp, 1u,
+      dev::scan_polls());
   k_scatter_left<<<grid, 256, 0, st>>>(B.d_rules, ni, d_rows, B.d_base);
   check_launch("serving batch join");
 

@@ -5,11 +5,15 @@
 // One launch counts every pass's digits.  A pass is then one launch: a block
 // ranks a tile of keys, publishes its counts per digit, adds the counts
 // of the tiles before it (looking back tile by tile, as far as the first that
-// has published its sum) and scatters.  The first pass reads the pairs and the
-// last one writes them back, so that no launch only converts.
+// has published its sum) and scatters: the published one-sweep radix sort
+// (Adinets and Merrill) with decoupled look-back (Merrill and Garland).  The
+// first pass reads the pairs and the last one writes them back, so that no
+// launch only converts.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdlib>
+#include <cstring>
 
 #include "context.h"
 #include "device_buffers.h"
@@ -22,9 +26,6 @@ namespace srt {
 constexpr uint32_t kThreads = 256, kWarps = kThreads / 32;
 constexpr uint32_t kMaxPasses = 8;
 constexpr uint32_t kBack = 8;  // tiles read at once when looking back
-// A wait for another tile's counts ends after this many polls (each some
-// microsecond); the block then counts the keys before its tile itself.
-constexpr uint32_t kWaitPolls = 1u << 20;
 constexpr unsigned kFull = 0xffffffffu;
 
 struct Pairs {
@@ -70,12 +71,14 @@ struct State {
 // 1.12 ms a sort, 300 us and 1.30 ms with 8 keys, 282 us and 1.27 ms with
 // three launches a pass).
 // Tiles are handed out by a ticket, so the tiles before a block's own are
-// running or done.  next: the other pass's words, cleared for it.
+// running or done; a wait for their counts ends after max_polls polls
+// (dev::scan_polls), and the block counts the keys before its tile itself.
+// next: the other pass's words, cleared for it.
 template <class T, uint32_t kKeys>
 __global__ void __launch_bounds__(kThreads) k_pass(Pairs p, const unsigned long long* src,
                                                    unsigned long long* dst, uint32_t shift,
                                                    const uint32_t* count, uint32_t* ticket, T* state,
-                                                   T* next) {
+                                                   T* next, uint32_t max_polls) {
   using S = State<T>;
   constexpr uint32_t kTile = kThreads * kKeys;
   __shared__ uint32_t s_cnt[kWarps][256];  // a warp's keys per digit, then where they start
@@ -137,7 +140,7 @@ __global__ void __launch_bounds__(kThreads) k_pass(Pairs p, const unsigned long 
   int64_t j = (int64_t)tile - 1;
   uint32_t polls = 0;
   bool done = tile == 0;
-  while (!done && polls < kWaitPolls) {
+  while (!done && polls < max_polls) {
     T w[kBack];
 #pragma unroll
     for (uint32_t u = 0; u < kBack; u++)
@@ -203,7 +206,7 @@ void queue_passes(Pairs p, uint32_t n_passes, int n_sm, cudaStream_t st) {
     unsigned long long* dst = q + 1 == n_passes ? nullptr : q & 1 ? b.p : a.p;
     k_pass<T, kKeys><<<n_tiles, kThreads, 0, st>>>(p, src, dst, 8 * q, count.p + 256 * q,
                                             count.p + 256 * kMaxPasses + q, state.p + (q & 1) * words,
-                                            state.p + (~q & 1) * words);
+                                            state.p + (~q & 1) * words, dev::scan_polls());
   }
   check_launch("pair sort");
 }
@@ -225,8 +228,11 @@ void queue_pair_sort(int n_sm, cudaStream_t st, uint32_t* l, uint32_t* r, uint64
   const uint32_t br = bits_of(n_right), bl = bits_of(n_left);
   const uint32_t n_passes = std::max(2u, (bl + br + 7) / 8);
   const srt::Pairs p{l, r, n, br};
-  // the words' values go up to n
-  if (n <= 4ull * n_sm * 8 * srt::kThreads)
+  // the words' values go up to n; 64-bit words at any n for a test
+  const char* wide = std::getenv("HBX_TEST_SORT_WIDE");
+  if (wide && std::strcmp(wide, "1") == 0)
+    srt::queue_passes<unsigned long long, 16>(p, n_passes, n_sm, st);
+  else if (n <= 4ull * n_sm * 8 * srt::kThreads)
     srt::queue_passes<uint32_t, 8>(p, n_passes, n_sm, st);
   else if (n < (1ull << 30))
     srt::queue_passes<uint32_t, 16>(p, n_passes, n_sm, st);
