@@ -41,7 +41,7 @@
 namespace hbx {
 
 struct RuleBufs {
-  DBuf<uint32_t> key_l, key_r, off_l, off_r, sorted_l, sorted_r;
+  DBuf<uint32_t> key_l, key_r, off_l, off_r, sorted_l, sorted_r, long_key;
   DBuf<dev::StrMeta> sorted_meta_r;
   DBuf<unsigned long long> item_off;
 };
@@ -260,6 +260,7 @@ void alloc_join(RuleBufs& b, dev::Rule* d, uint32_t nL, uint32_t nR) {
   b.sorted_r.alloc((size_t)nR + 4);
   if (d->n_sim) b.sorted_meta_r.alloc(nR);
   b.item_off.alloc((size_t)d->domain_l + 1);
+  if (d->ranked) b.long_key.alloc(nL);
 }
 
 void bind_join(const RuleBufs& b, dev::Rule* d) {
@@ -271,6 +272,7 @@ void bind_join(const RuleBufs& b, dev::Rule* d) {
   d->sorted_l = b.sorted_l.p;
   d->sorted_r = b.sorted_r.p;
   d->sorted_meta_r = d->n_sim ? b.sorted_meta_r.p : nullptr;
+  d->long_key = b.long_key.p;
 }
 
 // The join tasks of a rule array, uploaded on st (J->words stays for the copy),
@@ -280,7 +282,7 @@ void list_join(std::vector<dev::Rule>* rules, JoinLists* J, int n_sm, cudaStream
   size_t n_counts = 0;
   for (const dev::Rule& d : *rules) {
     if (d.n_members)
-      n_counts += 2ull * d.domain_l + 2ull * d.domain;
+      n_counts += 2ull * d.domain_l + 2ull * d.domain + (d.ranked ? 4 : 0);
     else if (d.cmp_weight)
       n_counts += d.domain;
   }
@@ -304,6 +306,7 @@ void list_join(std::vector<dev::Rule>* rules, JoinLists* J, int n_sm, cudaStream
     d.cur_l = take(d.domain_l);
     d.cnt_r = take(d.domain);
     d.cur_r = take(d.domain);
+    d.n_long = d.ranked ? take(4) : nullptr;  // one of a 16-byte piece
     for (int side : {0, 1}) {
       J->count.push_back(dev::join_task(r, side));
       J->scatter.push_back(dev::join_task(r, side));
@@ -338,9 +341,6 @@ bool overlap(const std::vector<dev::Rule>& rules) {
     if (d.n_members && d.dup_always) return true;
   return false;
 }
-
-// Classes of left rows of the session's rules (dev::Rule).
-uint32_t n_classes(const hbx_session* S) { return S->long_left ? 2u : 1u; }
 
 // Device state of a session whose side buffers hold the encoded tables.
 void setup_session(hbx_session* S, uint64_t h2d_tables) {
@@ -387,7 +387,7 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
       d.thr[s] = re.thr[s];
     }
     d.domain = (uint32_t)re.domain;
-    dev::set_classes(&d, S->long_left);
+    dev::set_classes(&d, S->long_left, nL);
     dev::make_singleton(&d);
   }
   dev::set_overlaps(S->h_rules.data(), S->h_rules.size());
@@ -480,15 +480,12 @@ void ensure_plain(hbx_session* S) {
   S->join_rules = JoinLists{};
   list_join(&S->h_rules, &S->join_rules, S->ctx->n_sm, st);
   S->d_rules.upload(S->h_rules, st);
-  // partition boundaries of every rule's left key space, per class: entry
-  // (rule, class, p) = first left key of partition p
+  // partition boundaries of every rule's join keys: entry (rule, p) = first
+  // key of partition p
   std::vector<uint32_t> idx;
   for (size_t r = 0; r < E.rules.size(); r++)
-    for (uint32_t c = 0; c < n_classes(S); c++)
-      for (uint64_t p = 0; p <= E.n_partitions; p++) {
-        const uint32_t cc = std::min<uint32_t>(c, S->h_rules[r].n_classes - 1);
-        idx.push_back(cc * S->h_rules[r].domain + (uint32_t)E.rules[r].part_key_begin[p]);
-      }
+    for (uint64_t p = 0; p <= E.n_partitions; p++)
+      idx.push_back((uint32_t)E.rules[r].part_key_begin[p]);
   S->bound_idx.upload(idx, st);
   S->bound_val.alloc(idx.size());
   HBX_CUDA(cudaStreamSynchronize(st));
@@ -850,8 +847,7 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
   HBX_CUDA(cudaEventRecord(S->ev0, st));
   uint32_t n = enqueue_join(S, st, false);
   const uint32_t n_rules = (uint32_t)S->rb.size();
-  const uint32_t per_class = (uint32_t)S->E.n_partitions + 1;
-  const uint32_t per_rule = per_class * n_classes(S);
+  const uint32_t per_rule = (uint32_t)S->E.n_partitions + 1;
   const uint32_t total = n_rules * per_rule;
   k_gather_bounds<<<(total + 255) / 256, 256, 0, st>>>(S->d_rules.p, n_rules, per_rule,
                                                        S->bound_idx.p, S->bound_val.p);
@@ -866,33 +862,31 @@ dev::Counters run_once(hbx_session* S, hbx_mode mode, cudaStream_t st, uint32_t*
   dev::EvalParams P = eval_params(S, S->d_rules.p);
   const int max_grid = S->ctx->n_sm * S->blocks_per_sm;
   HBX_CUDA(cudaEventRecord(S->ev_eval0, st));
-  for (uint64_t p = 0; p < S->E.n_partitions; p++) {
-    for (uint32_t r = 0; r < n_rules; r++) {
-      // the partition's items, those of long left strings in a launch of
-      // their own
-      for (uint32_t c = 0; c < S->h_rules[r].n_classes; c++) {
-        const size_t k = (size_t)r * per_rule + (size_t)c * per_class;
-        // the class's first item of the rule, in its item space and in item_off
-        const unsigned long long base_c = base[c * (n_rules + 1) + r], off_c = bounds[k];
-        P.n_seg = 1;
-        P.seg_begin[0] = base_c + bounds[k + p] - off_c;
-        P.seg_end[0] = base_c + bounds[k + p + 1] - off_c;
-        if (P.seg_end[0] <= P.seg_begin[0]) continue;
-        unsigned long long* next = c ? &S->d_ctr.p->work_next_long : &S->d_ctr.p->work_next;
-        HBX_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned long long), st));
-        n++;
-        if (c) {
-          launch_long(S, P, true, false, st);
-          continue;
-        }
-        const unsigned long long ctas =
-            (P.seg_end[0] - P.seg_begin[0] + dev::kWarpsPerCta - 1) / dev::kWarpsPerCta;
-        const int grid = (int)std::min<unsigned long long>(ctas, (unsigned long long)max_grid);
-        dev::eval_kernel(S->variant, false, S->peq_shape.w)<<<grid, kThreads, S->smem_bytes, st>>>(P);
-        launch_check("k_eval (plain)");
-      }
+  // launches the items [b0, b1) of a class's item space
+  auto launch_range = [&](unsigned long long b0, unsigned long long b1, bool of_long) {
+    if (b1 <= b0) return;
+    P.n_seg = 1;
+    P.seg_begin[0] = b0;
+    P.seg_end[0] = b1;
+    unsigned long long* next = of_long ? &S->d_ctr.p->work_next_long : &S->d_ctr.p->work_next;
+    HBX_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned long long), st));
+    n++;
+    if (of_long) {
+      launch_long(S, P, true, false, st);
+      return;
     }
-  }
+    const unsigned long long ctas = (b1 - b0 + dev::kWarpsPerCta - 1) / dev::kWarpsPerCta;
+    const int grid = (int)std::min<unsigned long long>(ctas, (unsigned long long)max_grid);
+    dev::eval_kernel(S->variant, false, S->peq_shape.w)<<<grid, kThreads, S->smem_bytes, st>>>(P);
+    launch_check("k_eval (plain)");
+  };
+  for (uint64_t p = 0; p < S->E.n_partitions; p++)
+    for (uint32_t r = 0; r < n_rules; r++)
+      launch_range(base[r] + bounds[(size_t)r * per_rule + p],
+                   base[r] + bounds[(size_t)r * per_rule + p + 1], false);
+  // the items of long left strings, whose keys need not follow the partitions
+  const unsigned long long* base_long = base.data() + n_rules + 1;
+  for (uint32_t r = 0; r < n_rules; r++) launch_range(base_long[r], base_long[r + 1], true);
   if (S->long_left) {  // pairs that any of the launches deferred
     launch_long(S, P, false, true, st);
     n++;
@@ -1453,6 +1447,18 @@ const char* hbx_last_error(const hbx_ctx* ctx) {
 
 void hbx_internal_set_error(hbx_ctx* ctx, const char* msg) {
   if (ctx) ctx->err = msg ? msg : "";
+}
+
+// The most device memory in use from the context's pool since the last call
+// with reset; then what is in use now starts the next span.
+uint64_t hbx_internal_pool_peak(hbx_ctx* ctx, int reset) {
+  uint64_t v = 0;
+  cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemHigh, &v);
+  if (reset) {
+    uint64_t zero = 0;
+    cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrUsedMemHigh, &zero);
+  }
+  return v;
 }
 
 hbx_status hbx_session_create(hbx_ctx* ctx, const hbx_plan* plan, const hbx_table* left,

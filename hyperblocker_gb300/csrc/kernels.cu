@@ -26,11 +26,10 @@ __global__ void k_keys_hist(Side S, const Rule* rules, uint32_t rule, int side) 
   const Rule& R = rules[rule];
   uint32_t* keys = side ? R.key_r : R.key_l;
   uint32_t* cnt = side ? R.cnt_r : R.cnt_l;
-  const bool split = !side && R.n_classes > 1;
   for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < S.n_rows;
        row += gridDim.x * blockDim.x) {
     uint32_t k = row_key(S, R, row);
-    if (split) k += R.domain * left_class(S.str_meta[(size_t)R.class_slot * S.n_rows + row].loc.y);
+    if (!side) k = left_key(R, S, row, k);
     keys[row] = k;
     atomicAdd(cnt + k, 1u);
   }
@@ -262,11 +261,12 @@ __device__ __forceinline__ unsigned long long n_items(uint32_t nl, uint32_t nr, 
   return (unsigned long long)nl * ((nr + tile_right - 1) / tile_right);
 }
 
-// Work items of left key j (class j / D, join key j % D).
+// Work items of left key j.
 __device__ __forceinline__ unsigned long long key_items(const Rule& R, uint32_t j,
                                                         uint32_t tile_right,
                                                         unsigned long long* pairs) {
-  return n_items(R.cnt_l[j], R.cnt_r[j % R.domain], tile_right, pairs);
+  const uint32_t nl = R.cnt_l[j];
+  return n_items(nl, nl ? R.cnt_r[join_key(R, j)] : 0u, tile_right, pairs);
 }
 
 __global__ void k_items_partial(const Rule* rules, uint32_t rule, uint32_t tile_right,
@@ -352,7 +352,6 @@ __global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* 
   const uint32_t D = side ? Q.domain : Q.domain_l;
   uint32_t* keys = !Q.n_members ? nullptr : side ? Q.key_r : Q.key_l;
   uint32_t* cnt = side ? Q.cnt_r : Q.cnt_l;
-  const bool split = !side && Q.n_classes > 1;
   const bool sh = D <= kSharedHistKeys;
   if (sh) {
     for (uint32_t k = threadIdx.x; k < D; k += blockDim.x) s_cnt[k] = 0;
@@ -360,7 +359,7 @@ __global__ void k_join_count(Side L, Side R, const Rule* rules, const uint32_t* 
   }
   for (uint32_t row = t0; row < S.n_rows; row += stride) {
     uint32_t k = row_key(S, Q, row);
-    if (split) k += Q.domain * left_class(S.str_meta[(size_t)Q.class_slot * S.n_rows + row].loc.y);
+    if (!side) k = left_key(Q, S, row, k);
     if (keys) keys[row] = k;
     atomicAdd(sh ? s_cnt + k : cnt + k, 1u);
   }
@@ -444,7 +443,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_join_scan(
     }
     return;
   }
-  // work items; a class's keys repeat the right side's
+  // work items
   uint4 nl[kVec], nr[kVec];
   const uint32_t m = Q.domain;
   unsigned long long pairs, ex, p;
@@ -453,12 +452,14 @@ __global__ void __launch_bounds__(kThreads, 2) k_join_scan(
     for (int k = 0; k < kVec; k++) {
       const uint32_t j = b + 4 * k;
       nl[k] = load4(Q.cnt_l, j, D);
-      nr[k] = make_uint4(0, 0, 0, 0);
-      if (j + 3 < m)
+      if (j + 3 < m) {
         nr[k] = load4(Q.cnt_r, j, m);
-      else if (j < D)
-        nr[k] = make_uint4(Q.cnt_r[j % m], Q.cnt_r[(j + 1) % m], Q.cnt_r[(j + 2) % m],
-                           Q.cnt_r[(j + 3) % m]);
+      } else {  // class 1, or beyond the keys (0 left rows)
+        nr[k].x = nl[k].x ? Q.cnt_r[join_key(Q, j)] : 0u;
+        nr[k].y = nl[k].y ? Q.cnt_r[join_key(Q, j + 1)] : 0u;
+        nr[k].z = nl[k].z ? Q.cnt_r[join_key(Q, j + 2)] : 0u;
+        nr[k].w = nl[k].w ? Q.cnt_r[join_key(Q, j + 3)] : 0u;
+      }
     }
     unsigned long long items = 0;
     pairs = 0;
@@ -1636,11 +1637,10 @@ __device__ __forceinline__ uint32_t find_key_in(const unsigned long long* item_o
 }
 
 // The left row and the rows [rb0, rb1) of sorted_r of item `local` of a rule's
-// item space, under left key jl.
+// item space, under left key jl with join key `key`.
 __device__ __forceinline__ void item_rows(const EvalParams& P, const Rule& R, uint32_t jl,
-                                          unsigned long long local, uint32_t* lrow, uint32_t* rb0,
-                                          uint32_t* rb1) {
-  const uint32_t key = jl < R.domain ? jl : jl - R.domain;  // join key
+                                          uint32_t key, unsigned long long local, uint32_t* lrow,
+                                          uint32_t* rb0, uint32_t* rb1) {
   const unsigned long long in_key = local - R.item_off[jl];
   const uint32_t nl = R.cnt_l[jl];
   const uint32_t ri = (uint32_t)(in_key / nl);
@@ -1682,7 +1682,7 @@ __device__ __forceinline__ uint32_t claim_chunk(const EvalParams& P, WarpCtl* C,
     jl = find_key(R.item_off, R.domain, local);
   }
   uint32_t lrow, rb0, rb1;
-  item_rows(P, R, jl, local, &lrow, &rb0, &rb1);
+  item_rows(P, R, jl, jl, local, &lrow, &rb0, &rb1);
   const uint32_t a0 = rb0 & ~3u;
   ItemDesc d;
   const bool sim = R.n_sim != 0;
@@ -2133,7 +2133,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_eval_long(
     const uint32_t jl =
         R->domain + find_key(R->item_off + R->domain, R->domain_l - R->domain, local);
     uint32_t lrow, rb0, rb1;
-    item_rows(P, *R, jl, local, &lrow, &rb0, &rb1);
+    item_rows(P, *R, jl, join_key(*R, jl), local, &lrow, &rb0, &rb1);
     const StrMeta* lm = P.L.str_meta + (size_t)R->sim_l[0] * P.L.n_rows + lrow;
     const uint32_t la = lm->loc.y;
     const uint8_t* a = P.L.arena + 16ull * lm->loc.x;

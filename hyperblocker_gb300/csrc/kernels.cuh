@@ -129,10 +129,18 @@ struct Rule {
   // Where some left string has no Peq table (more than kMaxTableLen symbols),
   // left rows are grouped by (class, key): class 1 holds the rows whose
   // string of the first similarity predicate is that long.  Their work items
-  // follow all items of class 0 and are evaluated by k_eval_long.
+  // follow all items of class 0 and are evaluated by k_eval_long.  The left
+  // keys of class 1 follow the D of class 0: one per join key, or, where there
+  // are at least twice as many join keys as left rows, one per row of the
+  // class (ranked: in the order of arrival, *n_long so far, with their join
+  // keys in long_key), so that few long strings do not double the state of a
+  // large key domain (20 bytes a key).
   uint32_t n_classes;   // 1, or 2 with long left strings
   uint32_t class_slot;  // left string slot that decides the class
-  uint32_t domain_l;    // n_classes * D: left keys
+  uint32_t ranked;
+  uint32_t domain_l;    // left keys of all classes
+  uint32_t* long_key;   // [left rows], ranked only
+  uint32_t* n_long;
   uint32_t* key_l;
   uint32_t* key_r;
   uint32_t* cnt_l;  // [domain_l]
@@ -252,13 +260,31 @@ inline void set_overlaps(Rule* rules, size_t n) {
 constexpr uint32_t kMaxTableLen = 256;
 __host__ __device__ inline uint32_t left_class(uint32_t len) { return len > kMaxTableLen ? 1u : 0u; }
 
-// Host: a rule's left keys, in two classes when some left string is longer
-// than kMaxTableLen.  After domain, n_sim and sim_l are set.
-inline void set_classes(Rule* d, bool long_left) {
+// Host: the left keys of a rule over n_left rows, in two classes when some left
+// string is longer than kMaxTableLen.  After domain, n_sim and sim_l are set.
+inline void set_classes(Rule* d, bool long_left, uint32_t n_left) {
   d->n_classes = long_left && d->n_sim ? 2u : 1u;
   d->class_slot = d->n_sim ? d->sim_l[0] : 0u;
-  d->domain_l = d->n_classes * d->domain;
+  d->ranked = d->n_classes > 1 && d->domain / 2 >= n_left ? 1u : 0u;
+  d->domain_l = d->domain + (d->n_classes == 1 ? 0u : d->ranked ? n_left : d->domain);
 }
+#ifdef __CUDACC__
+// Left key of a row with join key `key`; class 1 ranks are handed out here.
+__device__ __forceinline__ uint32_t left_key(const Rule& R, const Side& L, uint32_t row,
+                                             uint32_t key) {
+  if (R.n_classes == 1 || !left_class(L.str_meta[(size_t)R.class_slot * L.n_rows + row].loc.y))
+    return key;
+  if (!R.ranked) return R.domain + key;
+  const uint32_t k = atomicAdd(R.n_long, 1u);
+  R.long_key[k] = key;
+  return R.domain + k;
+}
+// Join key of left key j, which holds rows.
+__device__ __forceinline__ uint32_t join_key(const Rule& R, uint32_t j) {
+  if (j < R.domain) return j;
+  return R.ranked ? R.long_key[j - R.domain] : j - R.domain;
+}
+#endif
 constexpr uint32_t kMaxSegments = 1;
 constexpr uint32_t kRingEntries = 64;
 constexpr uint32_t kRingWords = 12;  // words per ring entry (three 16-byte records)

@@ -123,8 +123,7 @@ __global__ void k_keys(const dev::Rule* rules, uint32_t n_inst, const InstRows* 
         R.key_l[i] = 0xffffffffu;
         continue;
       }
-      if (R.n_classes > 1)
-        key += R.domain * dev::left_class(L.str_meta[(size_t)R.class_slot * L.n_rows + row].loc.y);
+      key = dev::left_key(R, L, row, key);
       R.key_l[i] = key;
       atomicAdd(R.cnt_l + key, 1u);
     }
@@ -575,7 +574,7 @@ void open_server(hbx_server* S, const hbx_plan* const* plans, int32_t n_plans, c
         d.thr[s] = pr.thr[s];
       }
       d.domain = (uint32_t)D;
-      dev::set_classes(&d, false);  // a batch with long left strings sets two
+      dev::set_classes(&d, false, 0);  // a batch with long left strings sets two
       dev::make_singleton(&d);
       // right half of the join: rows grouped by key, metadata in that order
       T->key_r.alloc(std::max<uint32_t>(nR, 1));
@@ -706,7 +705,7 @@ void launch_batch(hbx_server* S, Slot& B) {
   for (size_t q = 0; q < nq; q++)
     for (int r : S->plan_rules[(size_t)B.ents[q].r->plan]) {
       dev::Rule d = S->rules[(size_t)r]->d;
-      dev::set_classes(&d, B.long_left);
+      dev::set_classes(&d, B.long_left, B.ents[q].n());
       for (uint32_t what : {0u, 2u}) {
         tasks.push_back(dev::ScanTask{(uint32_t)rules.size(), what, 0, d.domain_l});
       }
@@ -730,9 +729,11 @@ void launch_batch(hbx_server* S, Slot& B) {
     const size_t o_base = take(8 * n_base), o_ctr = take(sizeof(dev::Counters));
     const size_t o_cmp = take(8ull * ni), o_sync = take(8 * (block_task.size() + tasks.size()));
     std::vector<size_t> o_cnt(ni), o_cur(ni), o_off(ni), o_item(ni), o_key(ni), o_row(ni);
+    std::vector<size_t> o_long(ni), o_nlong(ni);
     for (uint32_t i = 0; i < ni; i++) {
       o_cnt[i] = take(4ull * rules[i].domain_l);
       o_cur[i] = take(4ull * rules[i].domain_l);
+      if (rules[i].ranked) o_nlong[i] = take(4);
     }
     const size_t n_zero = words;
     for (uint32_t i = 0; i < ni; i++) {
@@ -740,6 +741,7 @@ void launch_batch(hbx_server* S, Slot& B) {
       o_item[i] = take(8ull * (rules[i].domain_l + 1));
       o_key[i] = take(4ull * rows[i].n);
       o_row[i] = take(4ull * rows[i].n);
+      if (rules[i].ranked) o_long[i] = take(4ull * rows[i].n);
     }
     B.join.alloc(words);
     unsigned long long* p = B.join.p;
@@ -755,6 +757,8 @@ void launch_batch(hbx_server* S, Slot& B) {
       d.item_off = p + o_item[i];
       d.key_l = u32(o_key[i]);
       d.sorted_l = u32(o_row[i]);
+      d.long_key = d.ranked ? u32(o_long[i]) : nullptr;
+      d.n_long = d.ranked ? u32(o_nlong[i]) : nullptr;
     }
     B.d_cmp = p + o_cmp;
     B.d_sync = p + o_sync;

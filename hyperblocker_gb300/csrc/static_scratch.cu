@@ -183,24 +183,20 @@ void place(Carve& c, const hbx::Encoded& E, size_t smem_cap, Layout* Y) {
       d.thr[s] = re.thr[s];
     }
     d.domain = (uint32_t)re.domain;
-    dev::set_classes(&d, long_left);
-    // room for five classes of left keys where they stay below four times
-    // kMaxKeyDomain, else for one (which long left strings may double): the
-    // sizes that are refused do not depend on the classes in use
-    const uint64_t room_l =
-        d.n_sim && re.domain * 5 <= (uint64_t)hbx::kMaxKeyDomain * 4
-            ? re.domain * 5 : std::max<uint64_t>(re.domain, d.domain_l);
+    dev::set_classes(&d, long_left, nL);
     dev::make_singleton(&d);
     d.dup_always = E.rules.size() > 1 ? 1u : 0u;  // the set is sized for every report
     d.key_l = c.take<uint32_t>(nL);
     d.key_r = c.take<uint32_t>(nR);
-    d.cnt_l = c.take<uint32_t>(room_l);
+    d.cnt_l = c.take<uint32_t>(d.domain_l);
     d.cnt_r = c.take<uint32_t>(d.domain);
-    d.off_l = c.take<uint32_t>(room_l);
+    d.off_l = c.take<uint32_t>(d.domain_l);
     d.off_r = c.take<uint32_t>(d.domain);
-    d.cur_l = c.take<uint32_t>(room_l);
+    d.cur_l = c.take<uint32_t>(d.domain_l);
     d.cur_r = c.take<uint32_t>(d.domain);
-    d.item_off = c.take<unsigned long long>((size_t)room_l + 1);
+    d.item_off = c.take<unsigned long long>((size_t)d.domain_l + 1);
+    d.long_key = d.ranked ? c.take<uint32_t>(nL) : nullptr;
+    d.n_long = d.ranked ? c.take<uint32_t>(1) : nullptr;
     d.sorted_l = c.take<uint32_t>(nL);
     d.sorted_r = c.take<uint32_t>((size_t)nR + 4);
     d.sorted_meta_r = d.n_sim ? c.take<dev::StrMeta>(nR) : nullptr;
@@ -334,6 +330,7 @@ void run_static(int device, const hbx_plan* plan, const hbx_table* left, const h
     HBX_STATIC_CUDA(cudaMemsetAsync(d.cnt_r, 0, d.domain * 4, st));
     HBX_STATIC_CUDA(cudaMemsetAsync(d.cur_l, 0, d.domain_l * 4, st));
     HBX_STATIC_CUDA(cudaMemsetAsync(d.cur_r, 0, d.domain * 4, st));
+    if (d.n_long) HBX_STATIC_CUDA(cudaMemsetAsync(d.n_long, 0, 4, st));
     const uint32_t ru = (uint32_t)r;
     if (nL) dev::k_keys_hist<<<grid_for(nL), 256, 0, st>>>(Y.L, Y.d_rules, ru, 0);
     if (nR) dev::k_keys_hist<<<grid_for(nR), 256, 0, st>>>(Y.R, Y.d_rules, ru, 1);
