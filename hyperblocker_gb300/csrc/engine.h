@@ -35,6 +35,8 @@ void rank_by_counts(Plan* plan, const PlanSample& sample, const Table& left, con
 // form queues it on st.
 void queue_pair_sort(int n_sm, cudaStream_t st, uint32_t* l, uint32_t* r, uint64_t n,
                      uint32_t n_left, uint32_t n_right);
+// Device memory that takes besides the pairs, while it runs.
+uint64_t pair_sort_bytes(int n_sm, uint64_t n, uint32_t n_left, uint32_t n_right);
 void sort_pairs_device(hbx_ctx* ctx, uint32_t* l, uint32_t* r, uint64_t n, uint32_t n_left,
                        uint32_t n_right);
 // writer.cu: appends the id lines of n device pairs to path.

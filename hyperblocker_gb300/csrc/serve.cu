@@ -202,6 +202,7 @@ struct Request {
 struct Entry {
   Request* r = nullptr;
   uint32_t r0 = 0, r1 = 0;
+  int64_t longest = 1;  // longest_left
   uint32_t n() const { return r1 - r0; }
 };
 
@@ -648,9 +649,31 @@ void open_server(hbx_server* S, const hbx_plan* const* plans, int32_t n_plans, c
   S->st.resident_bytes = S->resident_bytes;
 }
 
+// The longest left string a similarity predicate reads in rows [r0, r1) of a
+// request, in bytes (which bound its symbols).
+int64_t longest_left(const hbx_server* S, const Table& t, uint32_t r0, uint32_t r1) {
+  int64_t mx = 1;
+  for (int c : S->lstr) {
+    const Column& col = t.cols[(size_t)c];
+    for (uint32_t i = r0; i < r1; i++) mx = std::max<int64_t>(mx, col.off[i + 1] - col.off[i]);
+  }
+  return mx;
+}
+
+bool is_long(int64_t longest) { return longest > (int64_t)dev::kMaxTableLen; }
+
+// A rule's instance over n request rows, its left half unplaced.
+dev::Rule instance(const hbx_server* S, int rule, uint32_t n, int64_t longest) {
+  dev::Rule d = S->rules[(size_t)rule]->d;
+  dev::set_classes(&d, is_long(longest), n);
+  return d;
+}
+
 // Device memory rows [r0, r1) of a request need while their batch is in
-// flight (upper bound).
-uint64_t estimate(const hbx_server* S, const Table& t, int32_t plan, uint32_t r0, uint32_t r1) {
+// flight (upper bound), but for entry_share and batch_share; longest: of those
+// rows' left strings.
+uint64_t estimate(const hbx_server* S, const Table& t, int32_t plan, uint32_t r0, uint32_t r1,
+                  int64_t longest) {
   const uint64_t n = r1 - r0;
   uint64_t b = 0;
   auto bytes = [&](int c) {
@@ -658,19 +681,49 @@ uint64_t estimate(const hbx_server* S, const Table& t, int32_t plan, uint32_t r0
     return (uint64_t)(col.off[r1] - col.off[r0]);
   };
   for (int c : S->left_cols) b += bytes(c) + 8 * (n + 1) + 16;
-  for (int c : S->lstr) b += bytes(c) + 15 * n + 16 + 40 * n;  // arena, metadata, scan
+  // arena; its units, offsets and their scan
+  for (int c : S->lstr) b += bytes(c) + 15 * n + 16 + 8 * n + 8 * (n / dev::kScanChunk + 2);
   // Peq tables, at most 8 words per symbol row
   b += 4ull * ((8ull * S->n_symbols + 3) / 4 * 4) * n * S->lstr.size() + 16;
   b += sizeof(dev::StrMeta) * n * S->lstr.size() + 4 * n * S->pairs.size();
   for (int r : S->plan_rules[(size_t)plan]) {
-    const dev::Rule& d = S->rules[(size_t)r]->d;
-    // room for five classes of left keys, more than are in use: what the
-    // budget refuses does not depend on them
-    const uint64_t keys_l = (uint64_t)d.domain * (d.n_sim && d.domain * 5ull <= (1ull << 22) ? 5 : 1);
-    b += 12ull * n + 20ull * keys_l + 64 + 8 * ((keys_l + dev::kScanChunk - 1) / dev::kScanChunk + 1);
+    const dev::Rule d = instance(S, r, r1 - r0, longest);
+    b += 8ull * n + 20ull * d.domain_l + (d.ranked ? 4 * n : 0) + 64;
   }
-  b += 16 * n + (S->any_multi_rule ? 64 * n : 0) + 4096;  // output share (grows if needed)
+  b += 16 * n + (S->any_multi_rule ? 64 * n : 0);  // output share (more is added if it grows)
+  return b + 4096;
+}
+
+// Pairs that a batch with long left strings may leave to k_eval_long.
+constexpr size_t kServeDefer = 1 << 16;
+
+// What an entry's rule instances take besides: the rules, the words of their
+// join scans.
+uint64_t entry_share(const hbx_server* S, int32_t plan, uint32_t n, int64_t longest) {
+  uint64_t b = 0;
+  for (int r : S->plan_rules[(size_t)plan]) {
+    const uint64_t chunks = instance(S, r, n, longest).domain_l / dev::kJoinChunk + 1;
+    b += sizeof(dev::Rule) + sizeof(InstRows) + 2 * sizeof(dev::ScanTask) + 24 * chunks + 64;
+  }
   return b;
+}
+
+// What a batch takes whatever it holds: the smallest output and duplicate set,
+// the list of deferred pairs, the counters and the pool's rounding of some
+// twenty buffers.
+uint64_t batch_share(const hbx_server* S, bool any_long) {
+  return (8ull << 16) + (S->any_multi_rule ? 8ull << 17 : 0) +
+         (any_long ? sizeof(uint4) * kServeDefer : 0) + sizeof(dev::Counters) + 20 * 1024;
+}
+
+// A batch takes more device memory than it was admitted with (a negative
+// number: gives some back).
+void hold(hbx_server* S, Slot& B, int64_t bytes) {
+  std::lock_guard<std::mutex> lock(S->mu);
+  B.est += (uint64_t)bytes;
+  S->in_use += (uint64_t)bytes;
+  S->peak = std::max(S->peak, S->in_use);
+  S->st.peak_bytes = S->peak;
 }
 
 void launch_batch(hbx_server* S, Slot& B) {
@@ -684,16 +737,11 @@ void launch_batch(hbx_server* S, Slot& B) {
   B.n_rows = N;
   HBX_CUDA(cudaEventRecord(B.ev_start, st));
 
-  // Peq tables shaped for the batch's longest left string (bytes bound symbols)
+  // Peq tables shaped for the batch's longest left string
   int64_t max_len = 1;
-  for (size_t sl = 0; sl < S->lstr.size(); sl++)
-    for (auto& e : B.ents) {
-      const Column& col = e.r->rows.cols[(size_t)S->lstr[sl]];
-      for (uint32_t i = e.r0; i < e.r1; i++)
-        max_len = std::max<int64_t>(max_len, col.off[i + 1] - col.off[i]);
-    }
+  for (auto& e : B.ents) max_len = std::max(max_len, e.longest);
   B.shape = dev::peq_shape((uint32_t)std::min<int64_t>(max_len, 1 << 20), S->n_symbols);
-  B.long_left = max_len > (int64_t)dev::kMaxTableLen;
+  B.long_left = is_long(max_len);
 
   // ---- rule instances: (request, rule of its plan), and their join tasks
   B.inst_entry.clear();
@@ -704,8 +752,7 @@ void launch_batch(hbx_server* S, Slot& B) {
   uint32_t max_n = 1;
   for (size_t q = 0; q < nq; q++)
     for (int r : S->plan_rules[(size_t)B.ents[q].r->plan]) {
-      dev::Rule d = S->rules[(size_t)r]->d;
-      dev::set_classes(&d, B.long_left, B.ents[q].n());
+      const dev::Rule d = instance(S, r, B.ents[q].n(), B.ents[q].longest);
       for (uint32_t what : {0u, 2u}) {
         tasks.push_back(dev::ScanTask{(uint32_t)rules.size(), what, 0, d.domain_l});
       }
@@ -864,7 +911,7 @@ void launch_batch(hbx_server* S, Slot& B) {
   k_scatter_left<<<grid, 256, 0, st>>>(B.d_rules, ni, d_rows, B.d_base);
   check_launch("serving batch join");
 
-  if (B.long_left) B.defer.alloc(1 << 16);
+  if (B.long_left) B.defer.alloc(kServeDefer);
   // Output slots: more than there are room for repeat the evaluation (150 to
   // 210 us of a batch of 4,096 records with 20 pairs each, two batches of five
   // in a burst).  So up to 64 a record, as far as the masks that the Peq
@@ -1010,14 +1057,13 @@ bool progress(hbx_server* S, Slot& B) {
       uint64_t cap = B.capacity;
       const uint64_t need = c.out_count + (c.seen_overflow ? c.passes : 0);
       while (cap < need || cap == B.capacity) cap *= 2;
+      uint64_t slots = B.seen.n;
+      while (B.seen.p && slots < 2 * cap) slots *= 2;
+      hold(S, B, (int64_t)(8 * (cap - B.capacity) + (B.seen.p ? 8 * (slots - B.seen.n) : 0)));
       B.capacity = cap;
       B.out_l.alloc(cap);
       B.out_r.alloc(cap);
-      if (B.seen.p) {
-        uint64_t slots = B.seen.n;
-        while (slots < 2 * cap) slots *= 2;
-        B.seen.alloc(slots);
-      }
+      if (B.seen.p) B.seen.alloc(slots);
       HBX_CUDA(cudaMemsetAsync(B.d_ctr, 0, sizeof(dev::Counters), B.st));
       launch_eval(S, B);
       return true;
@@ -1030,14 +1076,22 @@ bool progress(hbx_server* S, Slot& B) {
     if (B.copied) return true;  // by the report
     B.h_out.ensure(8 * n);
     uint32_t* ho = (uint32_t*)B.h_out.p;
-    if (n < (1ull << 31)) {
+    const uint64_t sort_bytes = pair_sort_bytes(S->ctx->n_sm, n, B.n_rows, S->n_right);
+    bool room;
+    {
+      std::lock_guard<std::mutex> lock(S->mu);
+      room = S->in_use + sort_bytes <= S->budget;
+    }
+    if (n < (1ull << 31) && room) {
       PoolScope scope(S->ctx->pool, B.st);
       try {
+        hold(S, B, (int64_t)sort_bytes);
         queue_pair_sort(S->ctx->n_sm, B.st, B.out_l.p, B.out_r.p, n, B.n_rows, S->n_right);
         B.sorted = true;
       } catch (const Error& e) {  // no room for its buffers: the pairs are as they were
         if (e.status != HBX_ERR_OOM) throw;
         cudaGetLastError();
+        hold(S, B, -(int64_t)sort_bytes);
       }
     }
     HBX_CUDA(cudaMemcpyAsync(ho, B.out_l.p, 4 * n, cudaMemcpyDeviceToHost, B.st));
@@ -1161,12 +1215,19 @@ void worker_loop(hbx_server* S) {
           return x->t_submit < y->t_submit;
         });
         uint64_t rows = 0;
+        bool any_long = false;
         for (Request* r : cand) {
           const uint32_t take = (uint32_t)std::min<uint64_t>(r->n - r->next, max_rows - rows);
           if (take == 0) break;
-          const uint64_t e = estimate(S, r->rows, r->plan, r->next, r->next + take);
-          if (S->in_use + est + e > S->budget && !(S->in_use == 0 && ents.empty())) break;
-          ents.push_back(Entry{r, r->next, r->next + take});
+          const int64_t longest = longest_left(S, r->rows, r->next, r->next + take);
+          const uint64_t e = estimate(S, r->rows, r->plan, r->next, r->next + take, longest) +
+                             entry_share(S, r->plan, take, longest);
+          const bool with_long = any_long || is_long(longest);
+          if (S->in_use + est + e + batch_share(S, with_long) > S->budget &&
+              !(S->in_use == 0 && ents.empty()))
+            break;
+          any_long = with_long;
+          ents.push_back(Entry{r, r->next, r->next + take, longest});
           r->next += take;
           r->outstanding++;
           if (!r->admitted) {
@@ -1176,6 +1237,7 @@ void worker_loop(hbx_server* S) {
           rows += take;
           est += e;
         }
+        if (!ents.empty()) est += batch_share(S, any_long);
         S->in_use += est;
         S->peak = std::max(S->peak, S->in_use);
         S->st.peak_bytes = S->peak;
@@ -1260,7 +1322,8 @@ hbx_status hbx_serve_submit(hbx_server* s, uint64_t req_id, int32_t plan, const 
     r->n = (uint32_t)r->rows.n_rows;
     // the largest chunk the request can be dispatched in must fit the budget
     const uint64_t max_rows = s->opts.max_batch_rows > 0 ? (uint64_t)s->opts.max_batch_rows : 4096u;
-    need = estimate(s, r->rows, plan, 0, (uint32_t)std::min<uint64_t>(r->n, max_rows));
+    const uint32_t n = (uint32_t)std::min<uint64_t>(r->n, max_rows);
+    need = estimate(s, r->rows, plan, 0, n, longest_left(s, r->rows, 0, n));
   } catch (const Error& e) {
     std::lock_guard<std::mutex> lock(s->mu);
     s->err = e.what();

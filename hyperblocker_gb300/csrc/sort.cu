@@ -213,6 +213,39 @@ void queue_passes(Pairs p, uint32_t n_passes, int n_sm, cudaStream_t st) {
 
 }  // namespace srt
 
+namespace {
+
+struct SortShape {
+  uint32_t bits_r, n_passes, keys;  // keys a thread
+  bool wide;                        // 64-bit words
+};
+
+SortShape sort_shape(int n_sm, uint64_t n, uint32_t n_left, uint32_t n_right) {
+  auto bits_of = [](uint32_t rows) {
+    uint32_t b = 0;
+    while ((uint64_t)rows > (1ull << b)) b++;
+    return b;  // bits that hold row indices below rows
+  };
+  SortShape s;
+  s.bits_r = bits_of(n_right);
+  s.n_passes = std::max(2u, (bits_of(n_left) + s.bits_r + 7) / 8);
+  // the words' values go up to n; 64-bit words at any n for a test
+  const char* wide = std::getenv("HBX_TEST_SORT_WIDE");
+  s.wide = n >= (1ull << 30) || (wide && std::strcmp(wide, "1") == 0);
+  s.keys = !s.wide && n <= 4ull * n_sm * 8 * srt::kThreads ? 8 : 16;
+  return s;
+}
+
+}  // namespace
+
+uint64_t pair_sort_bytes(int n_sm, uint64_t n, uint32_t n_left, uint32_t n_right) {
+  if (n < 2) return 0;
+  const SortShape s = sort_shape(n_sm, n, n_left, n_right);
+  const uint64_t tile = (uint64_t)srt::kThreads * s.keys, words = 512 * ((n + tile - 1) / tile);
+  return 8 * n * (s.n_passes > 2 ? 2 : 1) + words * (s.wide ? 8 : 4) +
+         4 * (srt::kMaxPasses * 257) + 4 * 1024;
+}
+
 // Queues the sort of n pairs by (left row, right row) in place on st; rows
 // are below n_left / n_right, and bits of the keys beyond those take no pass.
 // Its buffers come from the calling thread's pool on st.
@@ -220,24 +253,14 @@ void queue_pair_sort(int n_sm, cudaStream_t st, uint32_t* l, uint32_t* r, uint64
                      uint32_t n_left, uint32_t n_right) {
   if (n < 2) return;
   if (n >= (1ull << 32)) fail(HBX_ERR_UNSUPPORTED, "more than 2^32 pairs to sort");
-  auto bits_of = [](uint32_t rows) {
-    uint32_t b = 0;
-    while ((uint64_t)rows > (1ull << b)) b++;
-    return b;  // bits that hold row indices below rows
-  };
-  const uint32_t br = bits_of(n_right), bl = bits_of(n_left);
-  const uint32_t n_passes = std::max(2u, (bl + br + 7) / 8);
-  const srt::Pairs p{l, r, n, br};
-  // the words' values go up to n; 64-bit words at any n for a test
-  const char* wide = std::getenv("HBX_TEST_SORT_WIDE");
-  if (wide && std::strcmp(wide, "1") == 0)
-    srt::queue_passes<unsigned long long, 16>(p, n_passes, n_sm, st);
-  else if (n <= 4ull * n_sm * 8 * srt::kThreads)
-    srt::queue_passes<uint32_t, 8>(p, n_passes, n_sm, st);
-  else if (n < (1ull << 30))
-    srt::queue_passes<uint32_t, 16>(p, n_passes, n_sm, st);
+  const SortShape s = sort_shape(n_sm, n, n_left, n_right);
+  const srt::Pairs p{l, r, n, s.bits_r};
+  if (s.wide)
+    srt::queue_passes<unsigned long long, 16>(p, s.n_passes, n_sm, st);
+  else if (s.keys == 8)
+    srt::queue_passes<uint32_t, 8>(p, s.n_passes, n_sm, st);
   else
-    srt::queue_passes<unsigned long long, 16>(p, n_passes, n_sm, st);
+    srt::queue_passes<uint32_t, 16>(p, s.n_passes, n_sm, st);
 }
 
 // The same on the context's stream; returns when the pairs are sorted.

@@ -257,7 +257,11 @@ typedef struct hbx_serve_opts {
   uint32_t struct_size;     /* sizeof(hbx_serve_opts) */
   int32_t max_inflight;     /* batches on the device at once, 0 = 2 */
   int64_t max_batch_rows;   /* left records per batch, 0 = 4096 */
-  uint64_t budget_bytes;    /* device memory for batches in flight, 0 = half of the free memory */
+  uint64_t budget_bytes;    /* device memory for batches in flight, 0 = half of the free memory.
+                               A batch that runs alone may take 3 MiB more (its smallest output
+                               and duplicate set, the list of pairs left to a later launch), and
+                               what its output grows by; pairs are sorted on the host when the
+                               device's sort would not fit */
   int32_t tile_right;       /* right rows per work item, 0 = 128 */
   int32_t eval_variant;     /* evaluation kernel as hbx_opts, 0 = 2 CTAs/SM */
 } hbx_serve_opts;
@@ -284,7 +288,7 @@ typedef struct hbx_serve_stats {
   uint64_t n_pairs;
   double ms_device;           /* summed device time of the batches (CUDA events) */
   uint64_t budget_bytes;
-  uint64_t peak_bytes;        /* largest device memory held by batches in flight */
+  uint64_t peak_bytes;        /* largest device memory held by batches in flight (upper bound) */
   uint64_t resident_bytes;    /* device memory of the resident table and its joins */
 } hbx_serve_stats;
 
