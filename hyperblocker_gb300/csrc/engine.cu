@@ -768,15 +768,13 @@ void grow_output(hbx_session* S, uint64_t need) {
   }
 }
 
-// Distinct pairs of a run; with a full duplicate set an upper bound (its
-// reports, and all that it might have reported besides).
-uint64_t pair_count(const dev::Counters& c) {
-  return c.out_count + (c.seen_overflow ? c.passes : 0);
+void count_firsts(hbx_session* S, dev::Counters* c, cudaStream_t st) {
+  if (c->seen_overflow) read_firsts(S->seen.p, S->seen.n, S->d_ctr.p, c, S->ctx->n_sm, st);
 }
 
 // A run's output or duplicate set was too small: room for its pairs.
 void grow_output(hbx_session* S, const dev::Counters& c) {
-  const uint64_t need = pair_count(c);
+  const uint64_t need = dev::pair_count(c);
   if (need > S->out_l.n) grow_output(S, need);
   if (c.seen_overflow) {
     S->seen_pairs = std::max<uint64_t>(S->seen_pairs, c.passes);
@@ -1041,7 +1039,8 @@ void autotune(hbx_session* S, cudaStream_t st) {
     for (size_t k = 0; k < cand.size(); k++) {
       configure(S, cand[k].first, cand[k].second);
       float ms = timed_batched_run(S, st, &flush);
-      const dev::Counters c = read_counters(S, st);
+      dev::Counters c = read_counters(S, st);
+      count_firsts(S, &c, st);
       if (S->ext_l ? (bool)c.seen_overflow : (c.out_count > S->out_l.n || c.seen_overflow)) {
         if (S->ext_l) {
           S->seen_pairs = std::max<uint64_t>(2 * S->seen_pairs, c.passes);
@@ -1069,6 +1068,14 @@ void autotune(hbx_session* S, cudaStream_t st) {
 }
 
 }  // namespace
+
+void read_firsts(const unsigned long long* seen, uint64_t n_seen, dev::Counters* d_ctr,
+                 dev::Counters* c, int n_sm, cudaStream_t st) {
+  dev::k_count_firsts<<<grid_for(n_seen, n_sm), 256, 0, st>>>(seen, n_seen, d_ctr);
+  HBX_CUDA(cudaGetLastError());
+  HBX_CUDA(cudaMemcpyAsync(&c->firsts, &d_ctr->firsts, sizeof c->firsts, cudaMemcpyDeviceToHost, st));
+  HBX_CUDA(cudaStreamSynchronize(st));
+}
 
 // Counts of the sampled row pairs (x: left, y: right row of the encoded tables)
 // for every pair of columns, column-major.
@@ -1200,6 +1207,7 @@ void session_run(hbx_session* S, hbx_mode mode, cudaStream_t st) {
   fit_seen(S, S->seen_pairs);
   for (int attempt = 0; attempt < 8; attempt++) {
     dev::Counters c = run_once(S, mode, st, &launches);  // returns with the stream idle
+    count_firsts(S, &c, st);
     float ms = 0, ms_join = 0, ms_eval = 0;
     HBX_CUDA(cudaEventElapsedTime(&ms, S->ev0, S->ev1));
     HBX_CUDA(cudaEventElapsedTime(&ms_join, S->ev0, S->ev_eval0));
@@ -1239,7 +1247,7 @@ void session_run(hbx_session* S, hbx_mode mode, cudaStream_t st) {
       // the caller's buffer: a result larger than it is only counted; a
       // full duplicate set is grown and the run repeated
       if (c.out_count > S->ext_cap) {
-        S->stats.n_matches = pair_count(c);
+        S->stats.n_matches = dev::pair_count(c);
         return;
       }
       fit_seen(S, S->seen_pairs);
@@ -1248,7 +1256,7 @@ void session_run(hbx_session* S, hbx_mode mode, cudaStream_t st) {
     if (S->cap_limit && c.out_count > S->cap_limit) {
       // the caller's buffer is too small anyway: report the count (an upper
       // bound when the duplicate set overflowed) instead of running again
-      S->stats.n_matches = pair_count(c);
+      S->stats.n_matches = dev::pair_count(c);
       return;
     }
     grow_output(S, c);

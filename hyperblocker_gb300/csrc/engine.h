@@ -31,6 +31,10 @@ std::vector<PairCount> count_samples(const Encoded& E, const SideBufs& L, const 
                                      const std::vector<uint2>& rows, cudaStream_t st);
 void rank_by_counts(Plan* plan, const PlanSample& sample, const Table& left, const Table& right,
                     const std::vector<PairCount>& counts);
+// After a run whose duplicate set (n_seen slots) overflowed: c->firsts, counted
+// on st and waited for.
+void read_firsts(const unsigned long long* seen, uint64_t n_seen, dev::Counters* d_ctr,
+                 dev::Counters* c, int n_sm, cudaStream_t st);
 // sort.cu: sorts n device pairs by (left row, right row) in place; the first
 // form queues it on st.
 void queue_pair_sort(int n_sm, cudaStream_t st, uint32_t* l, uint32_t* r, uint64_t n,

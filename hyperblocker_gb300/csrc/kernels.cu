@@ -2212,6 +2212,16 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_eval_long(
   if (lane == 0 && word_ops) atomicAdd(&P.ctr->jw_word_ops, word_ops);
 }
 
+__global__ void k_count_firsts(const unsigned long long* seen, uint64_t n_seen, Counters* ctr) {
+  uint32_t k = 0;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_seen;
+       i += (uint64_t)gridDim.x * blockDim.x)
+    k += seen[i] != ~0ull;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(kFull, k, o);
+  if ((threadIdx.x & 31) == 0 && k) atomicAdd(&ctr->firsts, (unsigned long long)k);
+}
+
 // What the host reads after an evaluation, written to its page-locked memory
 // by one launch; few pairs need no copy of their own then, nor the host a
 // second wait.  Bound by the latency of one pass of stores over the link: a

@@ -366,6 +366,7 @@ struct Counters {
   unsigned long long jw_word_ops;  // algorithmic work of the JW evaluations
   unsigned long long seen_overflow;  // nonzero: the duplicate set had no room (run repeats)
   unsigned long long passes;  // matches taken through the duplicate set (first_report)
+  unsigned long long firsts;  // those of them that were reported (k_count_firsts, after an overflow)
   unsigned long long scans;       // pairs that reached a bit-parallel scan
   unsigned long long scan_steps;  // scan steps of 4 symbols
   unsigned long long items_total; // work items of the run (written by the join)
@@ -377,6 +378,12 @@ struct Counters {
 };
 
 static_assert(sizeof(Counters) % 8 == 0, "reported in 8-byte words");
+
+// Distinct pairs of a run; with a full duplicate set an upper bound: the pairs
+// that did not go through it, and every match that did (after read_firsts).
+inline unsigned long long pair_count(const Counters& c) {
+  return c.seen_overflow ? c.out_count - c.firsts + c.passes : c.out_count;
+}
 
 struct EvalParams {
   Side L, R;
@@ -562,6 +569,10 @@ __global__ void k_eval_long(const __grid_constant__ EvalParams P);
 inline int long_grid(int n_sm) { return n_sm * 4; }
 constexpr uint32_t kDeferPairs = 1u << 20;  // most room for deferred pairs of a run
 EvalKernel eval_kernel(int wide, bool groups, uint32_t peq_w);
+// Counts the reports that went through a duplicate set, its taken slots (a run
+// whose set overflowed only: the evaluation itself does not count them, which
+// would cost it 0.6 %).
+__global__ void k_count_firsts(const unsigned long long* seen, uint64_t n_seen, Counters* ctr);
 // words and, if there are at most limit of them (and capacity), the pairs to
 // page-locked host memory: h_out holds the left rows, then the right rows.
 __global__ void k_report(const unsigned long long* words, uint32_t n_words, const Counters* ctr,

@@ -1054,8 +1054,9 @@ bool progress(hbx_server* S, Slot& B) {
     if (c.out_count > B.capacity || c.seen_overflow) {
       // grow and evaluate again (the join is unchanged)
       PoolScope scope(S->ctx->pool, B.st);
+      if (c.seen_overflow) read_firsts(B.seen.p, B.seen.n, B.d_ctr, &c, S->ctx->n_sm, B.st);
       uint64_t cap = B.capacity;
-      const uint64_t need = c.out_count + (c.seen_overflow ? c.passes : 0);
+      const uint64_t need = dev::pair_count(c);
       while (cap < need || cap == B.capacity) cap *= 2;
       uint64_t slots = B.seen.n;
       while (B.seen.p && slots < 2 * cap) slots *= 2;

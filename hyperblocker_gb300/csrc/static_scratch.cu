@@ -45,6 +45,7 @@
 
 #include "device_buffers.h"
 #include "encode.h"
+#include "engine.h"
 #include "hbx_core.h"
 #include "ingest.h"
 #include "kernels.cuh"
@@ -398,9 +399,10 @@ void run_static(int device, const hbx_plan* plan, const hbx_table* left, const h
                                   Y.rule_base + dev::item_base_words(Y.rules.size()) - 1, 8,
                                   cudaMemcpyDeviceToHost, st));
   HBX_STATIC_CUDA(cudaStreamSynchronize(st));
+  if (c.seen_overflow) hbx::read_firsts(Y.seen, Y.seen_slots, Y.ctr, &c, n_sm, st);
   drain.armed = false;  // the stream is idle
   if (c.items_done != total_items) hbx::fail(HBX_ERR_CUDA, "evaluation did not finish its work");
-  out->n_required = c.seen_overflow ? std::max<uint64_t>(c.out_count, c.passes) : c.out_count;
+  out->n_required = dev::pair_count(c);
   out->n_written = 0;
   if (stats) {
     *stats = hbx_stats{};
