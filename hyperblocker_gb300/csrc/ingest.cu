@@ -709,13 +709,10 @@ bool device_encode(const hbx_table* left, const hbx_table* right, Encoded* Ep, S
   const size_t n_tab = current_arena() ? 1 : std::max<size_t>(1, std::min<size_t>(
       {n_eq, (size_t)ing::kDictBatch, (size_t)((1ull << 30) / (16ull * cap))}));
   DBuf<unsigned long long> keys;
-  DBuf<uint32_t> rep, code, spare;
+  DBuf<uint32_t> rep, code;
   keys.alloc(n_tab * cap);
   rep.alloc(n_tab * cap);
   code.alloc(n_tab * cap);
-  // the scratch of the entry point without allocation refuses an input at the
-  // same size whatever the tables need
-  if (current_arena()) spare.alloc((size_t)cap + nL + nR);
   const char* collide_env = std::getenv("HBX_TEST_DICT_COLLIDE");
   const bool collide_test = collide_env && std::strcmp(collide_env, "1") == 0;
   // attempt k hashes with seed kDictSeed + k; the test build of attempt 0
@@ -745,14 +742,34 @@ bool device_encode(const hbx_table* left, const hbx_table* right, Encoded* Ep, S
   };
   eq_dictionaries(seed_of(0));
 
-  // ---- symbol alphabet, arenas and string metadata
+  // ---- symbol alphabet
   {
     std::vector<ing::StrJob> jobs;
-    DBuf<uint32_t> units_l, units_r, off_l, off_r;
-    uint64_t hist_work = 1;
+    uint64_t work = 1;
     auto side = [&](std::map<int, DevCol>& m, const std::vector<int>& str_col, uint32_t n,
-                    const Table& t, SideBufs* B, DBuf<uint32_t>& units, DBuf<uint32_t>& off16,
-                    size_t i_mx) {
+                    const Table& t) {
+      for (int col : str_col) {
+        if (!n) continue;
+        const Column& c = t.cols[(size_t)col];
+        work = std::max<uint64_t>(work, c.has_nul ? n : (c.bytes.size() + 15) / 16);
+        jobs.push_back(ing::StrJob{view(m, col), n, nullptr, nullptr, nullptr, nullptr, nullptr});
+      }
+    };
+    side(cols_l, E.L.str_col, nL, TL);
+    side(cols_r, E.R.str_col, nR, TR);
+    byte_hist(jobs, work, sum.p + i_bhist, n_sm, st);
+    ing::k_symbol_map<<<1, 256, 0, st>>>(sum.p + i_bhist, sym, sum.p);
+    check_launch("ingest symbols");
+  }
+
+  // ---- arenas and string metadata: both tables in each launch, or one after the
+  // other in the scratch of the entry point without allocation, where the
+  // units and offsets of a table are given back before the next is placed
+  auto strings = [&](bool of_left, bool of_right) {
+    std::vector<ing::StrJob> jobs;
+    DBuf<uint32_t> tmp_l, tmp_r;  // arena units, then their offsets
+    auto side = [&](std::map<int, DevCol>& m, const std::vector<int>& str_col, uint32_t n,
+                    const Table& t, SideBufs* B, DBuf<uint32_t>& tmp, size_t i_mx) {
       const size_t ns = str_col.size();
       uint64_t bound = 16;  // the zero block at the end
       for (int col : str_col) bound += t.cols[(size_t)col].bytes.size() + 15ull * n;
@@ -763,24 +780,25 @@ bool device_encode(const hbx_table* left, const hbx_table* right, Encoded* Ep, S
       B->meta.alloc(std::max<size_t>(ns * n, 1));
       if (!ns || !n) return;
       if ((uint64_t)ns * n > UINT32_MAX) fail(HBX_ERR_UNSUPPORTED, "more than 2^32 strings");
-      units.alloc(ns * n);
-      off16.alloc(ns * n);
-      for (size_t k = 0; k < ns; k++) {
-        const Column& c = t.cols[(size_t)str_col[k]];
-        hist_work = std::max<uint64_t>(hist_work, c.has_nul ? n : (c.bytes.size() + 15) / 16);
-        jobs.push_back(ing::StrJob{view(m, str_col[k]), n, units.p + k * n, off16.p + k * n,
+      const size_t half = (ns * n + 63) / 64 * 64;  // 256-byte aligned pieces
+      tmp.alloc(2 * half);
+      for (size_t k = 0; k < ns; k++)
+        jobs.push_back(ing::StrJob{view(m, str_col[k]), n, tmp.p + k * n, tmp.p + half + k * n,
                                    B->arena.p, B->meta.p + k * n, sum.p + i_mx + k});
-      }
     };
-    side(cols_l, E.L.str_col, nL, TL, LB, units_l, off_l, i_mxl);
-    side(cols_r, E.R.str_col, nR, TR, RB, units_r, off_r, i_mxr);
-    byte_hist(jobs, hist_work, sum.p + i_bhist, n_sm, st);
-    ing::k_symbol_map<<<1, 256, 0, st>>>(sum.p + i_bhist, sym, sum.p);
+    if (of_left) side(cols_l, E.L.str_col, nL, TL, LB, tmp_l, i_mxl);
+    if (of_right) side(cols_r, E.R.str_col, nR, TR, RB, tmp_r, i_mxr);
     str_units(jobs, n_sm, st);
-    if (units_l.p) scan_u32(units_l.p, (uint32_t)units_l.n, off_l.p, st);
-    if (units_r.p) scan_u32(units_r.p, (uint32_t)units_r.n, off_r.p, st);
+    if (tmp_l.p) scan_u32(tmp_l.p, (uint32_t)(n_sl * nL), tmp_l.p + tmp_l.n / 2, st);
+    if (tmp_r.p) scan_u32(tmp_r.p, (uint32_t)(n_sr * nR), tmp_r.p + tmp_r.n / 2, st);
     str_pack(jobs, sym, n_sm, st);
     check_launch("ingest arenas");
+  };
+  if (current_arena()) {
+    strings(true, false);
+    strings(false, true);
+  } else {
+    strings(true, true);
   }
 
   // ---- summary
