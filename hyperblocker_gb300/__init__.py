@@ -502,8 +502,9 @@ def block(ctx: Context, plan: Plan, left: Table, right: Table, n_partitions: int
 def block_streamed(ctx: Context, plan: Plan, left: Table, right: Table, n_partitions: int,
                    window_bytes: int, prefix_idx: int = INT_MAX, mode="batched",
                    capacity: Optional[int] = None):
-    """``hbx_block_streamed``: partition windows of at most ``window_bytes``
-    of device memory, two in flight; returns (pairs (n, 2) uint32, stats)."""
+    """``hbx_block_streamed``: partition windows whose rows take at most
+    ``window_bytes`` of device memory (include/hbx.h says what comes on top),
+    two in flight; returns (pairs (n, 2) uint32, stats)."""
     if capacity is None:
         capacity = getattr(ctx, "_capacity_hint", 1 << 16)
     while True:

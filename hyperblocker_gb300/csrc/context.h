@@ -17,6 +17,9 @@ struct hbx_ctx {
   hbx_opts opts{};
   std::string err;
   std::string device_name;  // keys the autotuner's cache
+  // its sessions are windows under a memory budget: one dictionary at a time
+  bool windows = false;
+  uint64_t window_peak = 0;  // most device memory a window of the last streamed call took
   void* h_ctr = nullptr;    // page-locked counters of the context's session runs
   void* h_few = nullptr;    // page-locked pairs of small one-shot results (on first use)
   // page-locked staging of larger ones: two chunks of h_out_chunk bytes, each

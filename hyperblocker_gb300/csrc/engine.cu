@@ -1175,7 +1175,8 @@ void create_session(hbx_session* S, const hbx_plan* plan, const hbx_table* left,
   uint64_t h2d = 0;
   std::string why;
   if (C->opts.ingest == 0)
-    on_device = device_encode(left, right, &S->E, &S->L, &S->R, C->n_sm, C->stream, &h2d, &why);
+    on_device = device_encode(left, right, &S->E, &S->L, &S->R, C->n_sm, C->stream, &h2d, &why,
+                              true, C->windows ? 0 : 1ull << 30);
   if (to_order) {
     if (on_device) {
       order_on_device(S, &ordered, left->t, right->t);
@@ -1468,6 +1469,9 @@ uint64_t hbx_internal_pool_peak(hbx_ctx* ctx, int reset) {
   }
   return v;
 }
+
+// The most device memory a window of the context's last streamed call took.
+uint64_t hbx_internal_window_peak(const hbx_ctx* ctx) { return ctx->window_peak; }
 
 hbx_status hbx_session_create(hbx_ctx* ctx, const hbx_plan* plan, const hbx_table* left,
                               const hbx_table* right, uint64_t n_partitions, int64_t prefix_idx,

@@ -568,7 +568,7 @@ void unpin_table(hbx_table* t) {
 
 bool device_encode(const hbx_table* left, const hbx_table* right, Encoded* Ep, SideBufs* LB,
                    SideBufs* RB, int n_sm, cudaStream_t st, uint64_t* h2d, std::string* why,
-                   bool pin) {
+                   bool pin, size_t dict_bytes) {
   Encoded& E = *Ep;
   const Table& TL = left->t;
   const Table& TR = right->t;
@@ -701,13 +701,13 @@ bool device_encode(const hbx_table* left, const hbx_table* right, Encoded* Ep, S
   check_launch("ingest buckets");
 
   // ---- joint dictionaries (rebuilt with a fresh seed after a collision,
-  // below), several slots to a launch where their tables stay below 1 GiB
+  // below), as many slots to a launch as keep their tables within dict_bytes
   LB->eq.alloc(std::max<size_t>(n_eq * nL, 1));
   RB->eq.alloc(std::max<size_t>(n_eq * nR, 1));
   uint32_t cap = 1024;
   while (cap < 2ull * ((uint64_t)nL + nR)) cap <<= 1;
   const size_t n_tab = current_arena() ? 1 : std::max<size_t>(1, std::min<size_t>(
-      {n_eq, (size_t)ing::kDictBatch, (size_t)((1ull << 30) / (16ull * cap))}));
+      {n_eq, (size_t)ing::kDictBatch, (size_t)(dict_bytes / (16ull * cap))}));
   DBuf<unsigned long long> keys;
   DBuf<uint32_t> rep, code;
   keys.alloc(n_tab * cap);

@@ -138,9 +138,11 @@ constexpr unsigned long long kDictSeed = 0xc70f6907ull;
 // or more, or collisions under four seeds); the side buffers are then left
 // empty.  pin = false leaves the host tables pageable (no cudaHostRegister:
 // the entry point without device allocation copies from pageable memory).
+// The dictionaries of several equality slots are built at once while their
+// tables (16 bytes a slot, two to four slots a row) take at most dict_bytes.
 bool device_encode(const hbx_table* left, const hbx_table* right, Encoded* E, SideBufs* L,
                    SideBufs* R, int n_sm, cudaStream_t st, uint64_t* h2d, std::string* why,
-                   bool pin = true);
+                   bool pin = true, size_t dict_bytes = 1ull << 30);
 
 // Partition bucket of every row of a table (data_mngr.h:150-202) computed on
 // the device from the partition and prefix columns only, in chunks of rows.

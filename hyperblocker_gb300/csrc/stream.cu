@@ -33,6 +33,8 @@
 #include "hbx_core.h"
 #include "ingest.h"
 
+extern "C" uint64_t hbx_internal_pool_peak(hbx_ctx* ctx, int reset);
+
 namespace hbx {
 namespace {
 
@@ -180,11 +182,17 @@ extern "C" hbx_status hbx_block_streamed(hbx_ctx* ctx, const hbx_plan* plan, con
     group(bl, &sl, &rl);
     group(br, &sr, &rr);
 
-    // ---- device bytes of a row in a window (encoded strings, metadata, codes,
-    // join state), an upper bound
+    // ---- device bytes of a row in a window: the columns, encoded strings,
+    // metadata, codes and join rows; with long left strings the list of
+    // deferred pairs, and left keys of their own
+    bool long_left = false;
+    for (int col : schema.L.str_col)
+      for (int64_t i = 0; i < TL.n_rows && !long_left; i++)
+        long_left = TL.cols[(size_t)col].len(i) > (int64_t)dev::kMaxTableLen;
     auto row_cost = [&](const Table& t, const std::vector<int>& used, const std::vector<int>& str,
                         size_t n_eq, uint32_t row) {
       uint64_t c = 64 + 4 * n_eq + 16 * schema.rules.size();
+      if (long_left) c += 64 + (&t == &TL ? 24 * schema.rules.size() : 0);
       for (int col : used) c += (uint64_t)t.cols[(size_t)col].len(row) + 8;
       for (int col : str) c += (uint64_t)t.cols[(size_t)col].len(row) + 16 + sizeof(dev::StrMeta);
       return c;
@@ -274,6 +282,7 @@ extern "C" hbx_status hbx_block_streamed(hbx_ctx* ctx, const hbx_plan* plan, con
         return;
       }
       (void)id;
+      wc->windows = true;
       std::vector<uint32_t> il, ir, l, r;
       for (;;) {
         {
@@ -370,8 +379,14 @@ extern "C" hbx_status hbx_block_streamed(hbx_ctx* ctx, const hbx_plan* plan, con
         agg.rest_scans += ws.rest_scans;
         agg.scan_words = std::max(agg.scan_words, ws.scan_words);
       }
+      uint64_t peak = hbx_internal_pool_peak(wc, 0);
+      {
+        std::lock_guard<std::mutex> lock(mu);
+        ctx->window_peak = std::max(ctx->window_peak, peak);
+      }
       hbx_ctx_destroy(wc);
     };
+    ctx->window_peak = 0;
     const int n_workers = windows.size() > 1 ? 2 : 1;
     std::vector<std::thread> th;
     for (int i = 0; i < n_workers; i++) th.emplace_back(worker, i);

@@ -213,12 +213,18 @@ hbx_status hbx_write_pairs_device(hbx_ctx* ctx, const hbx_table* left, const hbx
 
 /* hbx_block for tables whose encoding need not fit the device at once (the
  * reference's per-partition pipeline, host_producer.h:75-104, with a memory
- * bound): partitions are grouped into windows of at most window_bytes of
- * device memory (a partition larger than that is split by its left rows), and
+ * bound): partitions are grouped into windows whose rows -- their columns,
+ * encoded strings, codes and join rows -- take at most window_bytes of device
+ * memory (a partition larger than that is split by its left rows), and
  * two workers with their own streams process windows in turn, so one
- * window's copies and encoding overlap another's evaluation.  A window's
- * pair output (up to window_bytes / 8 pairs, more if it needs them) comes on
- * top of the budget.  Same pairs as
+ * window's copies and encoding overlap another's evaluation.  On top of the
+ * budget come, per window: the pair output (up to window_bytes / 8 pairs, more
+ * if it needs them); the left strings' masks (up to 32 bytes for each symbol
+ * of the alphabet and string); the join keys' state (32 bytes a key of a
+ * rule's domain, partitions x distinct values, however few rows the window
+ * has); one equality's dictionary while it is built (64 bytes a row at most);
+ * and the right rows' string records in each rule's join order (64 bytes).
+ * Same pairs as
  * hbx_block (in another order); stats->n_windows counts the windows and
  * ms_last_run is the wall time of the call.  out holds HOST pointers. */
 hbx_status hbx_block_streamed(hbx_ctx* ctx, const hbx_plan* plan, const hbx_table* left,
