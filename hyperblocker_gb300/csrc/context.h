@@ -19,6 +19,7 @@ struct hbx_ctx {
   std::string device_name;  // keys the autotuner's cache
   // its sessions are windows under a memory budget: one dictionary at a time
   bool windows = false;
+  bool sampled_on_device = false;  // the last streamed call's planner sample
   uint64_t window_peak = 0;  // most device memory a window of the last streamed call took
   void* h_ctr = nullptr;    // page-locked counters of the context's session runs
   void* h_few = nullptr;    // page-locked pairs of small one-shot results (on first use)

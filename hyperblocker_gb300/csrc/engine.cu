@@ -1472,6 +1472,8 @@ uint64_t hbx_internal_pool_peak(hbx_ctx* ctx, int reset) {
 
 // The most device memory a window of the context's last streamed call took.
 uint64_t hbx_internal_window_peak(const hbx_ctx* ctx) { return ctx->window_peak; }
+// Was that call's planner sample counted on the device?
+int hbx_internal_sampled_on_device(const hbx_ctx* ctx) { return ctx->sampled_on_device ? 1 : 0; }
 
 hbx_status hbx_session_create(hbx_ctx* ctx, const hbx_plan* plan, const hbx_table* left,
                               const hbx_table* right, uint64_t n_partitions, int64_t prefix_idx,

@@ -105,9 +105,11 @@ void order_sampled(hbx_ctx* ctx, Plan* plan, const Table& left, const Table& rig
       if (device_encode(&sub_l, &sub_r, &E, &L, &R, ctx->n_sm, ctx->stream, &h2d, &why)) {
         rank_by_counts(plan, sample, left, right,
                        count_samples(E, L, R, sample.cols, rows, ctx->stream));
+        ctx->sampled_on_device = true;
         return;
       }
-    } catch (const Error&) {
+    } catch (const Error& e) {  // no room or no way there; other errors are the call's
+      if (e.status != HBX_ERR_OOM && e.status != HBX_ERR_UNSUPPORTED) throw;
       cudaGetLastError();
     }
   }
@@ -136,6 +138,7 @@ extern "C" hbx_status hbx_block_streamed(hbx_ctx* ctx, const hbx_plan* plan, con
     // the evaluation order is measured once on the whole tables
     hbx_plan ordered;
     ordered.p = plan->p;
+    ctx->sampled_on_device = false;
     if (ctx->opts.pred_order == 0) order_sampled(ctx, &ordered.p, TL, TR);
     const Encoded schema = encode_schema(ordered.p, TL, TR, n_partitions, prefix_idx);
     std::vector<int> used_l, used_r;
