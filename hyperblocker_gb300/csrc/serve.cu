@@ -1169,6 +1169,9 @@ bool progress(hbx_server* S, Slot& B) {
   return false;
 }
 
+// Rule instances of a batch: the evaluation holds an instance in 16 bits.
+constexpr size_t kMaxInstances = 65535;
+
 // Requests waiting longer than this go ahead of shorter ones.
 constexpr double kAgingMs = 200.0;
 
@@ -1216,10 +1219,13 @@ void worker_loop(hbx_server* S) {
           return x->t_submit < y->t_submit;
         });
         uint64_t rows = 0;
+        size_t instances = 0;
         bool any_long = false;
         for (Request* r : cand) {
           const uint32_t take = (uint32_t)std::min<uint64_t>(r->n - r->next, max_rows - rows);
           if (take == 0) break;
+          instances += S->plan_rules[(size_t)r->plan].size();
+          if (instances > kMaxInstances) break;
           const int64_t longest = longest_left(S, r->rows, r->next, r->next + take);
           const uint64_t e = estimate(S, r->rows, r->plan, r->next, r->next + take, longest) +
                              entry_share(S, r->plan, take, longest);
