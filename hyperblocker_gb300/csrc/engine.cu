@@ -155,6 +155,10 @@ int row_grid(uint64_t n, int n_sm) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(g, (uint64_t)n_sm * 8));
 }
 
+// The largest work item that hbx_opts.tile_right may ask for: more rows than a
+// warp's share of shared memory held in one piece.
+constexpr uint32_t kMaxTileRight = 352;
+
 // Tile shape and kernel variant of a session: right rows per work item
 // (tile_right) and the evaluation kernel (0: 3 CTAs per SM, 1: 2 CTAs per SM
 // with more registers).  Lays out each warp's shared memory
@@ -167,14 +171,13 @@ void configure(hbx_session* S, uint32_t tile_right, int variant) {
   // two blocks per SM: the SM's shared memory less 1 KB the hardware keeps
   // per block
   const size_t smem_cap = std::min<size_t>(C->smem_optin * 2, C->smem_per_sm - 2048);
-  const uint32_t cap_warp_words = (uint32_t)(C->smem_optin / 4 / dev::kWarpsPerCta) / 4 * 4;
   // Items of more than 128 rows are staged 96 at a time: fewer claims, with the
   // shared memory (and so the L1 left to the Peq rows) of 96-row items.  8
   // rules, 150k x 150k rows, evaluation: 9.54 ms with 288 rows per item, 9.60
   // with 192, 9.87 with 96; 2,601 x 64,264 rows are better off with 96 or 128
   // (141 against 149 us: too few items to share out evenly), so the autotuner
-  // chooses.  What did not fit a warp's share in one piece is refused still.
-  if (768u + 17u * S->tile_right + 432u > cap_warp_words) fail(HBX_ERR_INVALID_ARG, "tile_right too large");
+  // chooses.
+  if (S->tile_right > kMaxTileRight) fail(HBX_ERR_INVALID_ARG, "tile_right too large");
   S->stage_rows = S->tile_right > 128 ? 96 : S->tile_right;
   S->wl = dev::warp_layout_fit(S->stage_rows, smem_cap);
   S->warp_words = S->wl.warp_words;

@@ -331,9 +331,9 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // counts in the scatter launch, so no pass runs over its key domain (8 rules,
 // 30,012 x 29,990 rows: the key + venue rules have 64 partitions x 250 keys x
 // 500 venues = 8M keys).  Bound by launches and memory latency: reset, count,
-// scan and scatter take 46 us there and 158 us at 150k x 150k rows, against
+// scan and scatter take 36 us there and 115 us at 150k x 150k rows, against
 // 1.57 and 1.83 ms with a scan of every rule's domain, times 5 length
-// classes, in launches per rule; 38 us against 44 us for 2 rules, 2,601 x
+// classes, in launches per rule; 35 us against 44 us for 2 rules, 2,601 x
 // 64,264 rows.
 
 // Keys and key histograms of every task's rule and table; histograms of
@@ -393,7 +393,7 @@ __device__ __noinline__ void recount_items(const Rule& R, uint32_t tile_right, u
 // A block takes some 10 us whatever it holds (its task, its ticket, the look
 // back), so where there are more chunks than blocks run at once a block holds
 // 8,192 keys, 16 a thread, instead of 4,096, eight a thread (scan_chunks):
-// 24 million keys of three rules' scans take 108 us against 203, but 1 to 2 us
+// three scans of 8 million keys each take 108 us against 203, but 1 to 2 us
 // more where all chunks run at once (2,617 x 2,295 rows: 17.6 against 15.6 us
 // of join, measured with 1,024 threads of four keys; 512 of eight take the same
 // and have the registers for the recount without spills).
@@ -2016,7 +2016,7 @@ __device__ __forceinline__ void eval_loop(const EvalParams& P, uint32_t* region,
 template <int W, bool G>
 __device__ __forceinline__ void eval_body(const EvalParams& P) {
   extern __shared__ __align__(16) uint32_t smem[];
-  pdl_wait();  // the join is complete (launched after it with launch_dependent)
+  pdl_wait();  // nothing to wait for: launched in stream order, after the join
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   uint32_t* region = smem + (size_t)warp * P.warp_words;
