@@ -155,6 +155,9 @@ int row_grid(uint64_t n, int n_sm) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(g, (uint64_t)n_sm * 8));
 }
 
+// Least slots of the duplicate set and of the output.
+constexpr uint64_t kMinSeen = 1 << 17, kMinOut = 1 << 16;
+
 // The largest work item that hbx_opts.tile_right may ask for: more rows than a
 // warp's share of shared memory held in one piece.
 constexpr uint32_t kMaxTileRight = 352;
@@ -447,11 +450,11 @@ void setup_session(hbx_session* S, uint64_t h2d_tables) {
   // pair (load factor at most one half), else a quarter (dev::set_overlaps;
   // a run that needs more repeats with a set of the size it asked for)
   const uint64_t cap0 =
-      std::max<uint64_t>(1 << 16, std::min<uint64_t>(S->out_hint, E.pairs_covered + 1));
+      std::max<uint64_t>(kMinOut, std::min<uint64_t>(S->out_hint, E.pairs_covered + 1));
   S->out_l.alloc(cap0);
   S->out_r.alloc(cap0);
   if (E.rules.size() > 1) {
-    uint64_t slots = 1 << 17;
+    uint64_t slots = kMinSeen;
     const uint64_t want = overlap(S->h_groups) ? 2 * cap0 : cap0 / 4;
     while (slots < want) slots *= 2;
     S->seen.alloc(slots);
@@ -686,14 +689,23 @@ void drop_graph(hbx_session* S) {
   }
 }
 
-// The duplicate set holds at least 2 x `pairs` slots (load at most one half).
+// A session's buffers are allocated on its context's stream, whatever stream a
+// run takes: they may outlive that one.  Any stream may use them once the
+// allocation is done.
+void settle(hbx_session* S) { HBX_CUDA(cudaStreamSynchronize(S->ctx->stream)); }
+
+// The duplicate set (plans with several rules) holds at least 2 x `pairs`
+// slots (load at most one half).
 void fit_seen(hbx_session* S, uint64_t pairs) {
-  if (!S->seen.p) return;
-  uint64_t slots = S->seen.n;
+  if (S->E.rules.size() < 2) return;
+  // (no set is left after an allocation that failed)
+  uint64_t slots = std::max<uint64_t>(S->seen.p ? S->seen.n : 0, kMinSeen);
   while (slots < 2 * pairs) slots *= 2;
-  if (slots != S->seen.n) {
-    S->seen.alloc(slots);
+  if (!S->seen.p || slots != S->seen.n) {
+    PoolScope scope(S->ctx->pool, S->ctx->stream);
     drop_graph(S);
+    S->seen.alloc(slots);
+    settle(S);
   }
 }
 
@@ -761,14 +773,13 @@ uint32_t enqueue_batched(hbx_session* S, cudaStream_t st) {
 }
 
 void grow_output(hbx_session* S, uint64_t need) {
-  uint64_t cap = S->out_l.n;
+  uint64_t cap = std::max<uint64_t>(S->out_l.n, kMinOut);
   while (cap < need) cap *= 2;
+  PoolScope scope(S->ctx->pool, S->ctx->stream);
+  drop_graph(S);
   S->out_l.alloc(cap);
   S->out_r.alloc(cap);
-  if (S->graph) {
-    cudaGraphExecDestroy(S->graph);
-    S->graph = nullptr;
-  }
+  settle(S);
 }
 
 void count_firsts(hbx_session* S, dev::Counters* c, cudaStream_t st) {
@@ -1209,6 +1220,7 @@ void session_run(hbx_session* S, hbx_mode mode, cudaStream_t st) {
   if (mode == HBX_MODE_PLAIN && overlap(S->h_rules))
     S->seen_pairs = std::max<uint64_t>(S->seen_pairs, std::min(out_cap(S), S->E.pairs_covered));
   fit_seen(S, S->seen_pairs);
+  if (!S->out_l.p || !S->out_r.p) grow_output(S, kMinOut);  // an earlier allocation failed
   for (int attempt = 0; attempt < 8; attempt++) {
     dev::Counters c = run_once(S, mode, st, &launches);  // returns with the stream idle
     count_firsts(S, &c, st);
@@ -1269,7 +1281,6 @@ void session_run(hbx_session* S, hbx_mode mode, cudaStream_t st) {
 }
 
 void reserve_output(hbx_session* S, uint64_t pairs) {
-  PoolScope scope(S->ctx->pool, S->ctx->stream);
   if (pairs > S->out_l.n) grow_output(S, pairs);
   if (overlap(S->h_groups)) S->seen_pairs = std::max<uint64_t>(S->seen_pairs, pairs);
 }
