@@ -16,7 +16,6 @@
 
 #include <cuda_runtime.h>
 
-#include <cstdlib>
 #include <string>
 #include <vector>
 
@@ -81,13 +80,6 @@ struct ArenaScope {
   ArenaScope& operator=(const ArenaScope&) = delete;
 };
 
-// Bytes above which an allocation fails: HBX_TEST_ALLOC_LIMIT in the environment
-// (a test's lack of device memory), else none.
-inline size_t alloc_limit() {
-  const char* e = std::getenv("HBX_TEST_ALLOC_LIMIT");
-  return e ? (size_t)std::strtoull(e, nullptr, 10) : ~(size_t)0;
-}
-
 template <class T>
 struct DBuf {
   T* p = nullptr;
@@ -147,7 +139,6 @@ struct DBuf {
       a->peak = a->used > a->peak ? a->used : a->peak;
       return;
     }
-    if (count * sizeof(T) > alloc_limit()) fail(HBX_ERR_OOM, "above HBX_TEST_ALLOC_LIMIT");
     const DevPool* dp = current_pool();
     if (dp) {
       HBX_CUDA(cudaMallocFromPoolAsync((void**)&p, count * sizeof(T), dp->pool, dp->stream));

@@ -689,10 +689,20 @@ void drop_graph(hbx_session* S) {
   }
 }
 
-// A session's buffers are allocated on its context's stream, whatever stream a
-// run takes: they may outlive that one.  Any stream may use them once the
-// allocation is done.
-void settle(hbx_session* S) { HBX_CUDA(cudaStreamSynchronize(S->ctx->stream)); }
+// A new size for a session's buffer, whose contents go.  It is allocated on the
+// context's stream, whatever stream a run takes: it may outlive that one; any
+// stream may use it once this returns.  More bytes than HBX_TEST_ALLOC_LIMIT in
+// the environment are a test's lack of device memory.
+template <class T>
+void resize(hbx_session* S, DBuf<T>* b, uint64_t n) {
+  PoolScope scope(S->ctx->pool, S->ctx->stream);
+  b->reset();
+  const char* limit = std::getenv("HBX_TEST_ALLOC_LIMIT");
+  if (limit && n * sizeof(T) > std::strtoull(limit, nullptr, 10))
+    fail(HBX_ERR_OOM, "above HBX_TEST_ALLOC_LIMIT");
+  b->alloc(n);
+  HBX_CUDA(cudaStreamSynchronize(S->ctx->stream));
+}
 
 // The duplicate set (plans with several rules) holds at least 2 x `pairs`
 // slots (load at most one half).
@@ -702,10 +712,8 @@ void fit_seen(hbx_session* S, uint64_t pairs) {
   uint64_t slots = std::max<uint64_t>(S->seen.p ? S->seen.n : 0, kMinSeen);
   while (slots < 2 * pairs) slots *= 2;
   if (!S->seen.p || slots != S->seen.n) {
-    PoolScope scope(S->ctx->pool, S->ctx->stream);
     drop_graph(S);
-    S->seen.alloc(slots);
-    settle(S);
+    resize(S, &S->seen, slots);
   }
 }
 
@@ -775,11 +783,9 @@ uint32_t enqueue_batched(hbx_session* S, cudaStream_t st) {
 void grow_output(hbx_session* S, uint64_t need) {
   uint64_t cap = std::max<uint64_t>(S->out_l.n, kMinOut);
   while (cap < need) cap *= 2;
-  PoolScope scope(S->ctx->pool, S->ctx->stream);
   drop_graph(S);
-  S->out_l.alloc(cap);
-  S->out_r.alloc(cap);
-  settle(S);
+  resize(S, &S->out_l, cap);
+  resize(S, &S->out_r, cap);
 }
 
 void count_firsts(hbx_session* S, dev::Counters* c, cudaStream_t st) {

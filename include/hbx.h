@@ -99,7 +99,8 @@ typedef struct hbx_pairs {
   uint32_t* r_row;
   uint64_t capacity;
   uint64_t n_written;   /* out */
-  uint64_t n_required;  /* out: total matches (also when HBX_ERR_CAPACITY) */
+  uint64_t n_required;  /* out: total matches; when HBX_ERR_CAPACITY, with several rules, an
+                           upper bound of them if the set of reported pairs filled up */
 } hbx_pairs;
 
 typedef struct hbx_stats {
@@ -219,7 +220,8 @@ hbx_status hbx_write_pairs_device(hbx_ctx* ctx, const hbx_table* left, const hbx
  * two workers with their own streams process windows in turn, so one
  * window's copies and encoding overlap another's evaluation.  On top of the
  * budget come, per window: the pair output (up to window_bytes / 8 pairs, more
- * if it needs them); the left strings' masks (up to 32 bytes for each symbol
+ * if it needs them) and, with several rules, the set of reported pairs (up to 32
+ * bytes a pair of the output); the left strings' masks (up to 32 bytes for each symbol
  * of the alphabet and string); the join keys' state (32 bytes a key of a
  * rule's domain, partitions x distinct values, however few rows the window
  * has); one equality's dictionary while it is built (64 bytes a row at most);
